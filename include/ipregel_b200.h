@@ -227,6 +227,19 @@ typedef struct ipg_bins {
 int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1,
                    ipg_bins* bins);
 
+/* The rows of more than hub_min edges, cut into chunks of `chunk` edges
+ * (cached per direction, owned by the graph): hub[h] = {vertex, first chunk,
+ * chunks, 0} in no particular order, owner[c] = h of chunk c; a hub's chunks
+ * are numbered in a row. */
+typedef struct ipg_hubs {
+    const uint32_t* d_hub;   /* 4 words each */
+    uint64_t hubs;
+    const uint32_t* d_owner;
+    uint64_t chunks;
+} ipg_hubs;
+int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64_t chunk,
+                   ipg_hubs* hubs);
+
 /* The same degree classes without allocating anything -- no counterpart in
  * the reference.  Meant for callers that must not call cudaMalloc: code
  * running while a stream is being captured, serving loops that cannot afford

@@ -637,11 +637,21 @@ struct ipx_consts {
      * active count, edges traversed, direction, unused */
     uint32_t* lcnt;
     unsigned long long* hist;
-    /* single_broadcast hub chunks: per chunk the partial fold ({message,
-     * has} in a slot, has in the stamp word), per hub the chunks arrived */
+    /* single_broadcast: the vertices by degree class (short, middle and
+     * long rows, the hubs among the long ones; their numbers in class_n),
+     * and the hubs (rows above hub_min, ipg_graph_hubs) {vertex, first
+     * chunk, chunks} with, per chunk, the index of its hub and the partial
+     * fold ({message, has} in a slot, has in the stamp word), per hub the
+     * chunks arrived */
+    const uint32_t* class_list[3];
+    uint32_t class_n[3];
+    const uint4* hub;
     ipx_bslot* hub_part;
     uint32_t* hub_arrived;
-    /* chunk -> index of its hub in the static hub class (built at attach) */
+    uint64_t hub_min;
+    uint32_t chunks, hub_chunk;
+    /* chunk -> index of its hub: of those hubs, or of the static hub class
+     * of a pulling push version */
     const uint32_t* hub_owner;
     /* the in-lists with the flag of the most gathered vertices (null: none) */
     const uint32_t* in_adj_hot;
@@ -804,9 +814,9 @@ __device__ __forceinline__ void ipx_deliver(int p, uint64_t w, ipx_msg m)
 #ifndef IPX_HUB_WARP
 #define IPX_HUB_WARP 1
 #endif
-/* In-edges per chunk of the single_broadcast gather's hub class (a warp's
- * with IPX_HUB_WARP; 2,048 for a CTA's: the staging buffers of larger
- * chunks do not fit the 48 KB of static shared memory). */
+/* Most in-edges per chunk of the single_broadcast gather's hubs (a warp's
+ * with IPX_HUB_WARP, fewer on small graphs; 2,048 for a CTA's: the staging
+ * buffers of larger chunks do not fit the 48 KB of static shared memory). */
 #ifndef IPX_GATHER_CHUNK
 #if IPX_HUB_WARP
 #define IPX_GATHER_CHUNK 8192
@@ -1370,20 +1380,6 @@ __device__ __forceinline__ void ipx_warp_fold(bool& has, ipx_msg& acc)
     }
 }
 
-/* The same over the G lanes of one group (G a power of two <= 32); `mask`
- * holds the group's lanes. */
-template <int G>
-__device__ __forceinline__ void ipx_group_fold(bool& has, ipx_msg& acc, unsigned mask)
-{
-    typedef typename ipx_word<ipx_msg>::type W;
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-        const bool oh = __shfl_down_sync(mask, has, o, G);
-        const ipx_msg om = ipx_from_word<ipx_msg>(__shfl_down_sync(mask, ipx_to_word(acc), o, G));
-        ipx_fold(has, acc, oh, om);
-    }
-}
-
 /* Folds the broadcasts of the in-neighbours at edges e0 + lane, e0 + lane +
  * lanes, ... below e1, in that order.  IPX_UNROLL edges a step: their ids,
  * then their broadcast slots are each loaded for all IPX_UNROLL edges before
@@ -1797,11 +1793,11 @@ __global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_sb0()
 /* After vertex v's gather of superstep s: whether v is active (it was after
  * compute(s), or a message reactivates it, :65-71), and if so its compute
  * phase of superstep s+1 (:185-201) with the gathered message; a broadcast
- * goes to `out` stamped s+1.  Returns the activity that superstep s counts. */
-__device__ __forceinline__ bool ipx_sb_compute_next(uint64_t v, bool has, const ipx_msg& acc, ipx_sbslot* out,
-                                                    uint32_t next_stamp)
+ * goes to `out` stamped s+1.  a0 and v0: the vertex's activity and value.
+ * Returns the activity that superstep s counts. */
+__device__ __forceinline__ bool ipx_sb_compute_next(uint64_t v, bool has, const ipx_msg& acc, bool a0,
+                                                    const ipx_val& v0, ipx_sbslot* out, uint32_t next_stamp)
 {
-    const bool a0 = ipx_c.active_b[v] != 0;
     if (!a0 && !has) {
         ipx_sb_put(&out[v], false, acc, next_stamp);
         return false;
@@ -1811,7 +1807,6 @@ __device__ __forceinline__ bool ipx_sb_compute_next(uint64_t v, bool has, const 
     x.active = true;
     x.has_message = has;
     if (has) x.message = acc;
-    const ipx_val v0 = ipx_c.value[v];
     x.value = v0;
     x.ipx_has_out = false;
     ipx_fill_topology(x, v);
@@ -1877,18 +1872,18 @@ struct ipx_hub_chunk {
     uint32_t c, c0, nch, pad;
 };
 
-__device__ __forceinline__ void ipx_locate_chunk(const uint32_t* __restrict__ list, uint64_t n,
-                                                 const uint32_t* __restrict__ prefix, const uint64_t* __restrict__ row,
-                                                 uint32_t c, ipx_hub_chunk& h)
+__device__ __forceinline__ void ipx_locate_chunk(const uint64_t* __restrict__ row, uint32_t c, ipx_hub_chunk& h)
 {
     h.c = c;
-    h.i = ipx_c.hub_owner ? ipx_c.hub_owner[c] : ipx_hub_of_chunk(prefix, n, c);
-    h.v = list[h.i];
-    h.c0 = prefix[h.i];
-    h.nch = prefix[h.i + 1] - h.c0;
-    h.e0 = row[h.v] + (uint64_t)(c - h.c0) * IPX_GATHER_CHUNK;
+    h.i = ipx_c.hub_owner[c];
+    const uint4 hub = ipx_c.hub[h.i];
+    h.v = hub.x;
+    h.c0 = hub.y;
+    h.nch = hub.z;
+    const uint64_t chunk = ipx_c.hub_chunk;
+    h.e0 = row[h.v] + (uint64_t)(c - h.c0) * chunk;
     const uint64_t end = row[h.v + 1];
-    h.e1 = (h.e0 + IPX_GATHER_CHUNK < end) ? h.e0 + IPX_GATHER_CHUNK : end;
+    h.e1 = (h.e0 + chunk < end) ? h.e0 + chunk : end;
     h.a0 = h.e0 & ~3ULL;
     h.b = h.e1 & ~3ULL;
 }
@@ -1940,112 +1935,10 @@ __device__ __forceinline__ unsigned long long ipx_hub_chunk_done(const ipx_hub_c
             ipx_c.hub_arrived[h.i] = 0; /* every chunk of the hub has arrived */
         }
     }
-    if (threadIdx.x == 0 && last != 0) return (unsigned long long)ipx_sb_compute_next(h.v, has, acc, out, next_stamp);
+    if (threadIdx.x == 0 && last != 0)
+        return (unsigned long long)ipx_sb_compute_next(h.v, has, acc, ipx_c.active_b[h.v] != 0, ipx_c.value[h.v], out,
+                                                       next_stamp);
     return 0ULL;
-}
-
-/* 1: the warp class of the fused pull kernel takes 32 vertices per warp and
- * spreads their concatenated in-edges over its lanes (ipx_gather_expand);
- * 0: a warp per vertex.  Measured on directed R-MAT scale 25 (FP64
- * PageRank, 30 rounds): 191 ms with the expansion against 135 ms without
- * (its shuffles and segmented folds cost more than the idle lanes of the
- * warp per vertex), so it is off. */
-#ifndef IPX_GATHER_EXPAND
-#define IPX_GATHER_EXPAND 0
-#endif
-#ifndef IPX_EXPAND_STEPS
-#define IPX_EXPAND_STEPS 4
-#endif
-
-/* The warp class of ipx_k_gather_compute, edge-balanced.  Most vertices of
- * the class have a few dozen in-edges, so a warp per vertex leaves most
- * lanes idle and pays the list -> row -> ids -> slots chain once per vertex.
- * Here a warp takes 32 vertices of the list (lane j owns vertex j), scans
- * their in-degrees, and walks the concatenated edges 32 per step, lane by
- * lane: each lane finds its vertex by a 5-step search of the exclusive
- * degree prefix, loads the id and the slot (IPX_EXPAND_STEPS steps' loads
- * in flight), the lanes of each vertex fold their messages by a segmented
- * reduction (a lane folds in its right neighbour's partial while it belongs
- * to the same vertex), and the vertex's owner lane folds the segment's
- * result into its own.  A vertex's messages are folded in edge order within
- * a step, as a tree, and step after step: only the order of the ip_combine
- * calls differs from the reference's sequential fold.  Then every lane runs
- * the compute phase of its own vertex.  Degrees are below 2^32 / 32 (the
- * class bound t1). */
-__device__ __forceinline__ unsigned long long ipx_gather_expand(const uint32_t* __restrict__ list, uint64_t n,
-                                                                const ipx_vid* __restrict__ adj,
-                                                                const uint64_t* __restrict__ row,
-                                                                const ipx_sbslot* __restrict__ bs, uint32_t stamp,
-                                                                ipx_sbslot* __restrict__ out)
-{
-    const int lane = threadIdx.x & 31;
-    const uint64_t nwarps = ipx_gstride() >> 5;
-    unsigned long long cnt = 0;
-    for (uint64_t base = (ipx_gtid() >> 5) * 32; base < n; base += nwarps * 32) {
-        const bool valid = base + lane < n;
-        uint64_t v = 0, r0 = 0;
-        uint32_t deg = 0;
-        if (valid) {
-            v = list[base + lane];
-            r0 = row[v];
-            deg = (uint32_t)(row[v + 1] - r0);
-        }
-        uint32_t inc = deg;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(IPX_FULL, inc, o);
-            if (lane >= o) inc += t;
-        }
-        const uint32_t excl = inc - deg;
-        const uint32_t total = __shfl_sync(IPX_FULL, inc, 31);
-        bool has = false;
-        ipx_msg acc;
-        for (uint32_t t0 = 0; t0 < total; t0 += 32 * IPX_EXPAND_STEPS) {
-            int jk[IPX_EXPAND_STEPS];
-            ipx_sbslot w[IPX_EXPAND_STEPS];
-#pragma unroll
-            for (int k = 0; k < IPX_EXPAND_STEPS; k++) {
-                const uint32_t pos = t0 + (uint32_t)(32 * k + lane);
-                int j = 0;
-#pragma unroll
-                for (int st = 16; st > 0; st >>= 1) {
-                    const uint32_t ex = __shfl_sync(IPX_FULL, excl, j + st);
-                    if (ex <= pos) j += st;
-                }
-                const uint64_t rj = __shfl_sync(IPX_FULL, r0, j);
-                const uint32_t xj = __shfl_sync(IPX_FULL, excl, j);
-                jk[k] = pos < total ? j : 32 + lane; /* past the end: a segment of its own */
-                w[k] = ipx_no_slot<ipx_sbslot>();
-                if (pos < total) {
-                    const uint64_t u = (uint64_t)ipx_ld_stream(&adj[rj + (pos - xj)]);
-                    w[k] = __ldg(&bs[u]);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < IPX_EXPAND_STEPS; k++) {
-                ipx_msg m;
-                bool h = ipx_slot_take(w[k], stamp, m);
-                const int j = jk[k];
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const bool h2 = __shfl_down_sync(IPX_FULL, h, o);
-                    const ipx_msg m2 = ipx_shfl_down(m, o);
-                    const int j2 = __shfl_down_sync(IPX_FULL, j, o);
-                    if (lane + o < 32 && j2 == j) ipx_fold(h, m, h2, m2);
-                }
-                /* lane j's segment in this step starts at its first edge
-                 * here (or at lane 0 when it began in an earlier step) */
-                const uint32_t ts = t0 + 32u * k;
-                const bool meets = deg && excl < ts + 32 && excl + deg > ts;
-                const int src = meets ? (int)(excl > ts ? excl - ts : 0u) : lane;
-                const bool hs = __shfl_sync(IPX_FULL, h, src);
-                const ipx_msg ms = ipx_shfl_idx(m, src);
-                if (meets) ipx_fold(has, acc, hs, ms);
-            }
-        }
-        if (valid) cnt += ipx_sb_compute_next(v, has, acc, out, stamp + 1);
-    }
-    return cnt;
 }
 
 #ifndef IPX_HUB_SMEM
@@ -2055,14 +1948,6 @@ __device__ __forceinline__ unsigned long long ipx_gather_expand(const uint32_t* 
 #ifndef IPX_HUB_UNROLL
 #define IPX_HUB_UNROLL 4
 #endif
-/* Lanes per vertex in the middle class of the fused pull kernel.  On
- * directed R-MAT scale 25 (FP64 PageRank, 30 rounds) 16 lanes took 118 ms,
- * 8 lanes 119 ms and a whole warp 135 ms: most vertices of the class have a
- * few dozen in-edges. */
-#ifndef IPX_GATHER_GROUP
-#define IPX_GATHER_GROUP 16
-#endif
-
 /* The hub class of ipx_k_gather_compute with ids staged in shared memory:
  * two id buffers, each filled by one bulk copy per chunk and completed on
  * its own mbarrier.  Thread 0 locates chunk k+1 and starts its copy before
@@ -2074,57 +1959,13 @@ __device__ __forceinline__ unsigned long long ipx_gather_expand(const uint32_t* 
  * IPX_ERR_COPY_TIMEOUT, and the CTA reads ids from global memory for the
  * rest of the launch; results stay exact. */
 
-/* The hub class with a warp per chunk: the warp folds its chunk, lane 0
- * stores the fold, and the warp whose chunk arrives last folds the hub's
- * partials -- each lane a contiguous run of them, then the runs in order by
- * shuffles -- and lane 0 runs the vertex's compute phase. */
-template <bool HOT>
-__device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
-    const ipx_vid* __restrict__ adj, const uint64_t* __restrict__ row, const uint32_t* __restrict__ list, uint64_t n,
-    const uint32_t* __restrict__ prefix, uint32_t chunks, const ipx_sbslot* __restrict__ bs, uint32_t stamp,
-    ipx_sbslot* __restrict__ out)
-{
-    const int lane = threadIdx.x & 31;
-    const uint64_t nwarps = ipx_gstride() >> 5;
-    unsigned long long cnt = 0;
-    for (uint64_t c = ipx_gtid() >> 5; c < chunks; c += nwarps) {
-        ipx_hub_chunk h;
-        ipx_locate_chunk(list, n, prefix, row, (uint32_t)c, h);
-        bool has = false;
-        ipx_msg acc;
-        ipx_gather_fold_edges<HOT>(adj, bs, stamp, h.e0, h.e1, lane, 32, has, acc);
-        ipx_warp_fold(has, acc);
-        int last = 2; /* a hub of one chunk: its fold is the hub's */
-        if (lane == 0 && h.nch != 1) {
-            ipx_bslot_put(&ipx_c.hub_part[h.c], acc, has ? 1u : 0u);
-            __threadfence();
-            last = atomicAdd(&ipx_c.hub_arrived[h.i], 1u) == h.nch - 1 ? 1 : 0;
-        }
-        last = __shfl_sync(IPX_FULL, last, 0);
-        if (last == 1) {
-            __threadfence();
-            const uint32_t per = (h.nch + 31) / 32;
-            const uint32_t k0 = (uint32_t)lane * per, k1 = min(k0 + per, h.nch);
-            has = false;
-            for (uint32_t k = k0; k < k1; k++) {
-                const ipx_bslot p = __ldcg(&ipx_c.hub_part[h.c0 + k]);
-                ipx_msg m;
-                if (ipx_bslot_take(p, 1u, m)) ipx_fold(has, acc, true, m);
-            }
-            ipx_warp_fold(has, acc);
-            if (lane == 0) ipx_c.hub_arrived[h.i] = 0; /* every chunk of the hub has arrived */
-        }
-        if (lane == 0 && last != 0) cnt += ipx_sb_compute_next(h.v, has, acc, out, stamp + 1);
-    }
-    return cnt;
-}
-
+#if !IPX_HUB_WARP
 template <bool HOT>
 __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
-    const uint32_t* __restrict__ adj, const uint64_t* __restrict__ row, const uint32_t* __restrict__ list, uint64_t n,
-    const uint32_t* __restrict__ prefix, uint32_t chunks, const ipx_sbslot* __restrict__ bs, uint32_t stamp,
-    ipx_sbslot* __restrict__ out)
+    const uint32_t* __restrict__ adj, const uint64_t* __restrict__ row, const ipx_sbslot* __restrict__ bs,
+    uint32_t stamp, ipx_sbslot* __restrict__ out)
 {
+    const uint32_t chunks = ipx_c.chunks;
     __shared__ __align__(16) uint32_t s_ids[2][IPX_GATHER_CHUNK + 4];
     __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ ipx_hub_chunk s_h[2];
@@ -2144,7 +1985,7 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
     __syncthreads();
     auto issue = [&](uint32_t c, int buf) {
         ipx_hub_chunk& h = s_h[buf];
-        ipx_locate_chunk(list, n, prefix, row, c, h);
+        ipx_locate_chunk(row, c, h);
         if (h.b > h.a0 && !s_fail) {
             const uint32_t bytes = (uint32_t)((h.b - h.a0) * 4);
             ipx_mbar_arrive_tx(&s_bar[buf], bytes);
@@ -2218,37 +2059,228 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
     __syncthreads();
     return cnt;
 }
+#endif /* !IPX_HUB_WARP */
+
+/* ---- the rows of the fused pull kernel ----
+ *
+ * G lanes fold one row at a time, each lane four consecutive in-edges per
+ * step: one 128-bit load of their ids (aligned down; edges of the rows before
+ * and after are masked out), then four slot loads in flight, folded in edge
+ * order, and the lanes' folds meet in a tree.  What bounds a row is the chain
+ * list entry -> row bounds -> ids -> slots, four dependent loads for a few
+ * dozen edges, so the chain is pipelined over the group's next rows: while
+ * the slots of one row are in flight, the ids of the next row, the bounds of
+ * the one after it and the list entry of the one after that are loaded.
+ * Measured (FP64 PageRank, directed R-MAT scale 25, 31 supersteps; ms with
+ * one launch per class and no pipeline -> with it): 88 -> 74; FP64
+ * personalised PageRank, undirected, 4 M vertices: 11.7 -> 9.8.  The rows of
+ * 17 and more edges go from 203 to 263 G edges/s; the same ids gathered flat,
+ * without rows, reach 314 G/s, which the L2 bounds. */
+
+/* Edges p .. p+3 as loaded (p a multiple of 4): which of them belong to the
+ * row is decided when they are used, so that nothing waits for the load
+ * before. */
+__device__ __forceinline__ uint4 ipx_ld_quad(const uint32_t* __restrict__ adj, uint64_t p, uint64_t e1, uint64_t E)
+{
+    return __ldcs(reinterpret_cast<const uint4*>(adj + ((p < e1 && p + 4 <= E) ? p : 0)));
+}
+
+/* Folds the broadcasts of edges p .. p+3 that lie in [e0, e1), in order; q:
+ * ipx_ld_quad of p.  The array's last, incomplete quad is read here. */
+template <bool HOT>
+__device__ __forceinline__ void ipx_fold_quad(const uint32_t* __restrict__ adj, const ipx_sbslot* __restrict__ bs,
+                                              uint32_t stamp, uint4 q, uint64_t p, uint64_t e0, uint64_t e1, uint64_t E,
+                                              bool& has, ipx_msg& acc)
+{
+    const int lo = p < e0 ? (int)(e0 - p) : 0;
+    const int hi = p < e1 ? (e1 - p < 4 ? (int)(e1 - p) : 4) : 0;
+    if (p + 4 > E && hi > 0) {
+        q.x = adj[p];
+        if (hi > 1) q.y = adj[p + 1];
+        if (hi > 2) q.z = adj[p + 2];
+    }
+    const uint32_t id[4] = {q.x, q.y, q.z, q.w};
+    ipx_sbslot w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        w[k] = (k >= lo && k < hi) ? ipx_slot_ld<HOT>(bs, (uint64_t)id[k]) : ipx_no_slot<ipx_sbslot>();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        ipx_msg m;
+        if (ipx_slot_take(w[k], stamp, m)) ipx_fold(has, acc, true, m);
+    }
+}
+
+/* The tree over the G lanes of one group (G a power of two <= 32); `mask`
+ * holds the group's lanes. */
+template <int G>
+__device__ __forceinline__ void ipx_group_fold(bool& has, ipx_msg& acc, unsigned mask)
+{
+    typedef typename ipx_word<ipx_msg>::type W;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        const bool oh = __shfl_down_sync(mask, has, o, G);
+        const ipx_msg om = ipx_from_word<ipx_msg>(__shfl_down_sync(mask, ipx_to_word(acc), o, G));
+        ipx_fold(has, acc, oh, om);
+    }
+}
+
+/* Gather + next compute phase of the list's vertices, G lanes each; SKIP:
+ * hubs are passed over. */
+template <int G, bool SKIP, bool HOT>
+__device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* __restrict__ list, uint32_t n,
+                                                              const ipx_vid* __restrict__ ids, bool quads,
+                                                              const uint64_t* __restrict__ row,
+                                                              const ipx_sbslot* __restrict__ bs, uint32_t stamp,
+                                                              ipx_sbslot* __restrict__ out)
+{
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const unsigned mask = (G == 32) ? IPX_FULL : (((1u << (G & 31)) - 1u) << (lane & ~(G - 1)));
+    const uint64_t step = ipx_gstride() / G;
+    uint64_t i = ipx_gtid() / G;
+    unsigned long long cnt = 0;
+    if (!quads) {
+        for (; i < n; i += step) {
+            const uint64_t v = list[i];
+            if (SKIP && row[v + 1] - row[v] > ipx_c.hub_min) continue;
+            bool has = false;
+            ipx_msg acc;
+            ipx_gather_fold_edges<HOT>(ids, bs, stamp, row[v], row[v + 1], gl, G, has, acc);
+            if (G > 1) ipx_group_fold<G>(has, acc, mask);
+            if (gl == 0) cnt += ipx_sb_compute_next(v, has, acc, ipx_c.active_b[v] != 0, ipx_c.value[v], out, stamp + 1);
+        }
+        return cnt;
+    }
+    const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ids);
+    const uint64_t E = ipx_c.E;
+    if (i >= n) return cnt;
+    /* a: the row being folded, b: the next, c: the one after it.  Past the
+     * list's end vertex 0 stands in: loaded, never folded. */
+    uint32_t va = list[i], vb = i + step < n ? list[i + step] : 0u, vc = i + 2 * step < n ? list[i + 2 * step] : 0u;
+    uint64_t a0 = row[va], a1 = row[va + 1], b0 = row[vb], b1 = row[vb + 1];
+    uint4 qa = ipx_ld_quad(adj, (a0 & ~3ULL) + 4 * gl, a1, E);
+    for (; i < n; i += step) {
+        const bool act = gl == 0 ? ipx_c.active_b[va] != 0 : false;
+        const ipx_val v0 = gl == 0 ? ipx_c.value[va] : ipx_val();
+        const uint32_t vd = i + 3 * step < n ? list[i + 3 * step] : 0u;
+        const uint64_t c0 = row[vc], c1 = row[vc + 1];
+        const uint4 qb = ipx_ld_quad(adj, (b0 & ~3ULL) + 4 * gl, b1, E);
+        bool has = false;
+        ipx_msg acc;
+        const bool skip = SKIP && a1 - a0 > ipx_c.hub_min;
+        if (skip) a1 = a0;
+        uint64_t p = (a0 & ~3ULL) + 4 * gl;
+        ipx_fold_quad<HOT>(adj, bs, stamp, qa, p, a0, a1, E, has, acc);
+        for (p += 4 * G; p < a1; p += 4 * G)
+            ipx_fold_quad<HOT>(adj, bs, stamp, ipx_ld_quad(adj, p, a1, E), p, a0, a1, E, has, acc);
+        if (G > 1) ipx_group_fold<G>(has, acc, mask);
+        if (gl == 0 && !skip) cnt += ipx_sb_compute_next(va, has, acc, act, v0, out, stamp + 1);
+        va = vb;
+        vb = vc;
+        vc = vd;
+        a0 = b0;
+        a1 = b1;
+        b0 = c0;
+        b1 = c1;
+        qa = qb;
+    }
+    return cnt;
+}
+
+/* The hub class with a warp per chunk: the warp folds its chunk, lane 0
+ * stores the fold, and the warp whose chunk arrives last folds the hub's
+ * partials -- each lane a contiguous run of them, then the runs in order by
+ * shuffles -- and lane 0 runs the vertex's compute phase. */
+template <bool HOT>
+__device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
+    const ipx_vid* __restrict__ ids, bool quads, const uint64_t* __restrict__ row, const ipx_sbslot* __restrict__ bs,
+    uint32_t stamp, ipx_sbslot* __restrict__ out)
+{
+    const int lane = threadIdx.x & 31;
+    const uint64_t E = ipx_c.E;
+    const uint64_t nwarps = ipx_gstride() >> 5;
+    unsigned long long cnt = 0;
+    for (uint64_t c = ipx_gtid() >> 5; c < ipx_c.chunks; c += nwarps) {
+        ipx_hub_chunk h;
+        ipx_locate_chunk(row, (uint32_t)c, h);
+        bool has = false;
+        ipx_msg acc;
+        if (quads) {
+            const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ids);
+            uint64_t p = (h.e0 & ~3ULL) + 4 * lane;
+            uint4 q = ipx_ld_quad(adj, p, h.e1, E);
+            for (; p < h.e1; p += 128) {
+                const uint4 next = ipx_ld_quad(adj, p + 128, h.e1, E);
+                ipx_fold_quad<HOT>(adj, bs, stamp, q, p, h.e0, h.e1, E, has, acc);
+                q = next;
+            }
+        } else {
+            ipx_gather_fold_edges<HOT>(ids, bs, stamp, h.e0, h.e1, lane, 32, has, acc);
+        }
+        ipx_warp_fold(has, acc);
+        int last = 2; /* a hub of one chunk: its fold is the hub's */
+        if (lane == 0 && h.nch != 1) {
+            ipx_bslot_put(&ipx_c.hub_part[h.c], acc, has ? 1u : 0u);
+            __threadfence();
+            last = atomicAdd(&ipx_c.hub_arrived[h.i], 1u) == h.nch - 1 ? 1 : 0;
+        }
+        last = __shfl_sync(IPX_FULL, last, 0);
+        if (last == 1) {
+            __threadfence();
+            const uint32_t per = (h.nch + 31) / 32;
+            const uint32_t k0 = (uint32_t)lane * per, k1 = min(k0 + per, h.nch);
+            has = false;
+            for (uint32_t k = k0; k < k1; k++) {
+                const ipx_bslot p = __ldcg(&ipx_c.hub_part[h.c0 + k]);
+                ipx_msg m;
+                if (ipx_bslot_take(p, 1u, m)) ipx_fold(has, acc, true, m);
+            }
+            ipx_warp_fold(has, acc);
+            if (lane == 0) ipx_c.hub_arrived[h.i] = 0; /* every chunk of the hub has arrived */
+        }
+        if (lane == 0 && last != 0)
+            cnt += ipx_sb_compute_next(h.v, has, acc, ipx_c.active_b[h.v] != 0, ipx_c.value[h.v], out, stamp + 1);
+    }
+    return cnt;
+}
+
+/* Lanes per row of the middle and the long class, and the longest middle
+ * row (rows up to t0 take a thread each): about as many lanes as a row has
+ * quads.  PageRank at scale 25 / personalised PageRank at 4 M vertices took
+ * 74.1 / 9.8 ms with 8 lanes up to 64 edges and 16 beyond, 77.6 / 10.3 with 16
+ * for both, 73.5 / 10.9 with 8 for both, 75.9 / 10.2 with 32 beyond 64. */
+#ifndef IPX_GATHER_GROUP
+#define IPX_GATHER_GROUP 8
+#endif
+#ifndef IPX_GATHER_LONG
+#define IPX_GATHER_LONG 16
+#endif
+#ifndef IPX_GATHER_MID
+#define IPX_GATHER_MID 64
+#endif
+
+/* Resident CTAs per SM the fused pull kernel is compiled for: it carries
+ * ip_compute and the pipeline's registers besides the gather (64 a thread;
+ * with 48 or 40 it spills: PageRank at scale 25 78.0 ms with 4 CTAs, 83.4
+ * with 5, 95.0 with 6, 80 with 3). */
+#ifndef IPX_GATHER_CTAS
+#define IPX_GATHER_CTAS 4
+#endif
 
 /* Single broadcast (pull), one superstep s >= 0 after its compute phase:
  * ip_fetch_broadcast_messages (combiner_single_broadcast_postamble.h:57-89)
- * for the vertices of one in-degree class, then, vertex by vertex, the
- * compute phase of superstep s+1.  The gather reads buffer s & 1 (slots
- * stamped s) and the compute writes buffer (s+1) & 1, which no gather of
- * superstep s reads, so the two phases need no grid-wide barrier between
- * them and the message goes from the fold to ip_compute in registers.
- * Count of superstep s: the vertices active after the gather.  When it is
- * 0 no vertex was active or received a message, so no compute phase of
- * superstep s+1 ran, and the loop ends (:164).  MODE 0: a thread per vertex,
- * folding in adjacency order as the reference does; 1: a warp; 2: a block
- * (lane-strided runs folded in order, then a tree, per chunk of a hub's
- * row; chunks folded in order: only the order of the ip_combine calls
- * differs). */
-/* Resident CTAs per SM the fused pull kernel is compiled for: it carries
- * ip_compute besides the gather, which needs more registers than the other
- * edge kernels. */
-#ifndef IPX_GATHER_CTAS
-#define IPX_GATHER_CTAS 5
-#endif
-
-#ifndef IPX_EXPAND_CTAS
-#define IPX_EXPAND_CTAS 4
-#endif
-
-template <int MODE, bool HOT>
-__global__ void __launch_bounds__(IPX_THREADS, (MODE == 1 && IPX_GATHER_EXPAND) ? IPX_EXPAND_CTAS : IPX_GATHER_CTAS)
-    ipx_k_gather_compute(const uint32_t* __restrict__ list,
-                                                                                  uint64_t n,
-                                                                                  const uint32_t* __restrict__ prefix)
+ * and then, vertex by vertex, the compute phase of superstep s+1.  The
+ * gather reads buffer s & 1 (slots stamped s) and the compute writes buffer
+ * (s+1) & 1, which no gather of superstep s reads, so the two phases need no
+ * grid-wide barrier between them and the message goes from the fold to
+ * ip_compute in registers.  Count of superstep s: the vertices active after
+ * the gather.  When it is 0 no vertex was active or received a message, so
+ * no compute phase of superstep s+1 ran, and the loop ends (:164).  All
+ * degree classes in one launch, the longest rows first: three launches of
+ * 16 k to 500 k threads each end in a tail of their own, which on a graph of
+ * 65,536 vertices was half of the superstep. */
+template <bool HOT>
+__global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_compute()
 {
     const uint64_t s = ipx_step();
     const uint32_t stamp = (uint32_t)s;
@@ -2257,117 +2289,73 @@ __global__ void __launch_bounds__(IPX_THREADS, (MODE == 1 && IPX_GATHER_EXPAND) 
     const uint64_t* __restrict__ row = ipx_c.in_row;
     const ipx_sbslot* __restrict__ bs = ipx_c.sbslot[s & 1];
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[(s + 1) & 1];
+    /* 128-bit id loads need 32-bit ids and a 16-byte aligned array (a
+     * caller's may not be) of one load at least */
+    const bool quads = sizeof(ipx_vid) == 4 && (reinterpret_cast<uintptr_t>(adj) & 15) == 0 && ipx_c.E >= 4;
     unsigned long long cnt = 0;
-    if constexpr (MODE == 0) {
-        /* the next vertex's list entry is loaded while this vertex's
-         * in-edges are folded */
-        const uint64_t stride = ipx_gstride();
-        uint64_t i = ipx_gtid(), v = (i < n) ? list[i] : 0;
-        for (; i < n; i += stride) {
-            const uint64_t vn = (i + stride < n) ? list[i + stride] : 0;
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges<HOT>(adj, bs, stamp, row[v], row[v + 1], 0, 1, has, acc);
-            cnt += ipx_sb_compute_next(v, has, acc, out, stamp + 1);
-            v = vn;
-        }
-    } else if constexpr (MODE == 1 && IPX_GATHER_EXPAND && !HOT) {
-        cnt += ipx_gather_expand(list, n, adj, row, bs, stamp, out);
-    } else if constexpr (MODE == 1 && IPX_GATHER_GROUP < 32) {
-        /* IPX_GATHER_GROUP lanes per vertex: most vertices of the class have
-         * a few dozen in-edges, which 8 lanes reading four ids each cover
-         * in one or two steps, so a warp works on 32 / G vertices at once */
-        constexpr int G = IPX_GATHER_GROUP;
-        const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-        const unsigned mask = (G == 32) ? IPX_FULL : (((1u << G) - 1u) << (lane & ~(G - 1)));
-        const uint64_t groups = ipx_gstride() / G;
-        for (uint64_t i = ipx_gtid() / G; i < n; i += groups) {
-            const uint64_t v = list[i];
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges<HOT>(adj, bs, stamp, row[v], row[v + 1], gl, G, has, acc);
-            ipx_group_fold<G>(has, acc, mask);
-            if (gl == 0) cnt += ipx_sb_compute_next(v, has, acc, out, stamp + 1);
-        }
-    } else if constexpr (MODE == 1) {
-        /* the next vertex's list entry and row bounds are loaded while this
-         * vertex's in-edges are folded */
-        const int lane = threadIdx.x & 31;
-        const uint64_t stride = ipx_gstride() >> 5;
-        uint64_t i = ipx_gtid() >> 5, v = 0, r0 = 0, r1 = 0;
-        if (i < n) {
-            v = list[i];
-            r0 = row[v];
-            r1 = row[v + 1];
-        }
-        for (; i < n; i += stride) {
-            uint64_t vn = 0, r0n = 0, r1n = 0;
-            if (i + stride < n) {
-                vn = list[i + stride];
-                r0n = row[vn];
-                r1n = row[vn + 1];
-            }
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges<HOT>(adj, bs, stamp, r0, r1, lane, 32, has, acc);
-            ipx_warp_fold(has, acc);
-            if (lane == 0) cnt += ipx_sb_compute_next(v, has, acc, out, stamp + 1);
-            v = vn;
-            r0 = r0n;
-            r1 = r1n;
-        }
-    } else {
-        /* hubs in chunks of IPX_GATHER_CHUNK in-edges, spread over all CTAs
-         * (one hub's row would otherwise keep one CTA busy long after the
-         * others finished): each chunk's fold is stored, and the CTA whose
-         * chunk arrives last folds the partials in chunk order, then runs
-         * the compute phase (ipx_hub_chunk_done).  No CTA waits for another.
-         * With 32-bit ids the chunk's ids are staged through shared memory:
-         * while the CTA gathers one chunk, a bulk copy brings the ids of its
-         * next chunk, so the slot loads are issued from shared memory
-         * instead of behind a global id load each. */
-        if (n == 0) return;
-        const uint32_t chunks = prefix[n];
-        if constexpr (IPX_HUB_WARP) {
-            cnt += ipx_gather_hubs_warp<HOT>(adj, row, list, n, prefix, chunks, bs, stamp, out);
+    /* the longest work items first */
+    if constexpr (IPX_HUB_WARP) cnt += ipx_gather_hubs_warp<HOT>(adj, quads, row, bs, stamp, out);
+    cnt += ipx_gather_rows<IPX_GATHER_LONG, true, HOT>(ipx_c.class_list[2], ipx_c.class_n[2], adj, quads, row, bs,
+                                                       stamp, out);
+    cnt += ipx_gather_rows<IPX_GATHER_GROUP, false, HOT>(ipx_c.class_list[1], ipx_c.class_n[1], adj, quads, row, bs,
+                                                         stamp, out);
+    cnt += ipx_gather_rows<1, false, HOT>(ipx_c.class_list[0], ipx_c.class_n[0], adj, quads, row, bs, stamp, out);
+    ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
+}
+
+#if !IPX_HUB_WARP
+/* The hub chunks of the fused pull kernel in a launch of their own, a CTA
+ * per chunk (IPX_HUB_WARP = 0): each chunk's fold is stored, and the CTA
+ * whose chunk arrives last folds the partials in chunk order, then runs the
+ * compute phase (ipx_hub_chunk_done).  No CTA waits for another.  With
+ * 32-bit ids the chunk's ids are staged through shared memory: while the CTA
+ * gathers one chunk, a bulk copy brings the ids of its next chunk, so the
+ * slot loads are issued from shared memory instead of behind a global id
+ * load each. */
+template <bool HOT>
+__global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hubs()
+{
+    const uint64_t s = ipx_step();
+    const uint32_t stamp = (uint32_t)s;
+    const ipx_vid* __restrict__ adj = HOT ? reinterpret_cast<const ipx_vid*>(ipx_c.in_adj_hot) : ipx_c.in_adj;
+    const uint64_t* __restrict__ row = ipx_c.in_row;
+    const ipx_sbslot* __restrict__ bs = ipx_c.sbslot[s & 1];
+    ipx_sbslot* __restrict__ out = ipx_c.sbslot[(s + 1) & 1];
+    unsigned long long cnt = 0;
+    if constexpr (sizeof(ipx_vid) == 4 && IPX_HUB_SMEM) {
+        if ((reinterpret_cast<uintptr_t>(adj) & 15) == 0) {
+            cnt += ipx_gather_hubs_staged<HOT>(reinterpret_cast<const uint32_t*>(adj), row, bs, stamp, out);
             ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
             return;
         }
-        if constexpr (sizeof(ipx_vid) == 4 && IPX_HUB_SMEM) {
-            if ((reinterpret_cast<uintptr_t>(adj) & 15) == 0) {
-                cnt += ipx_gather_hubs_staged<HOT>(reinterpret_cast<const uint32_t*>(adj), row, list, n, prefix, chunks,
-                                              bs, stamp, out);
-                ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
-                return;
-            }
+    }
+    __shared__ bool s_has[IPX_THREADS / 32];
+    __shared__ ipx_msg s_acc[IPX_THREADS / 32];
+    __shared__ ipx_hub_chunk s_h;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint32_t c = blockIdx.x; c < ipx_c.chunks; c += gridDim.x) {
+        if (threadIdx.x == 0) ipx_locate_chunk(row, c, s_h);
+        __syncthreads();
+        const ipx_hub_chunk h = s_h;
+        bool has = false;
+        ipx_msg acc;
+        ipx_gather_fold_edges<HOT>(adj, bs, stamp, h.e0, h.e1, threadIdx.x, blockDim.x, has, acc);
+        ipx_warp_fold(has, acc);
+        if (lane == 0) {
+            s_has[warp] = has;
+            s_acc[warp] = acc;
         }
-        __shared__ bool s_has[IPX_THREADS / 32];
-        __shared__ ipx_msg s_acc[IPX_THREADS / 32];
-        __shared__ ipx_hub_chunk s_h;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-            if (threadIdx.x == 0) ipx_locate_chunk(list, n, prefix, row, c, s_h);
-            __syncthreads();
-            const ipx_hub_chunk h = s_h;
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges<HOT>(adj, bs, stamp, h.e0, h.e1, threadIdx.x, blockDim.x, has, acc);
-            ipx_warp_fold(has, acc);
-            if (lane == 0) {
-                s_has[warp] = has;
-                s_acc[warp] = acc;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                has = false;
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) ipx_fold(has, acc, s_has[w], s_acc[w]);
-            }
-            cnt += ipx_hub_chunk_done(h, has, acc, out, stamp + 1, s_has, s_acc);
-            __syncthreads();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            has = false;
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) ipx_fold(has, acc, s_has[w], s_acc[w]);
         }
+        cnt += ipx_hub_chunk_done(h, has, acc, out, stamp + 1, s_has, s_acc);
+        __syncthreads();
     }
     ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
 }
+#endif /* !IPX_HUB_WARP */
 
 /* Spread + single broadcast compute phase: combiner_spread_single_broadcast_
  * postamble.h:228-237, over the targets (all vertices at superstep 0). */

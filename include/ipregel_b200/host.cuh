@@ -84,7 +84,8 @@ struct ipx_host_state {
     uint32_t* h_lcnt = nullptr;                        /* pinned mirror of lcnt */
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    ipg_bins gbins;                                    /* static in-degree classes (pull) */
+    ipg_bins gbins;                                    /* static in-degree classes (pulling push versions) */
+    ipg_hubs ghubs;                                    /* hub chunks of the single_broadcast gather */
     std::vector<uint64_t> counts;
     double total_seconds = 0.0;
     uint64_t edges = 0;
@@ -104,7 +105,7 @@ struct ipx_host_state {
     int tb = IPX_THREADS;      /* CTA size in use */
     uint32_t grid_compute = 0; /* resident CTAs of the compute kernel */
     uint32_t grid_edge = 0;    /* resident CTAs of the edge kernels */
-    uint32_t grid_gather[3] = {0, 0, 0}; /* single_broadcast: of each class's fused kernel */
+    uint32_t grid_hubs = 0;    /* single_broadcast, a CTA per hub chunk: of the hub kernel */
     std::vector<struct ip_vertex_t> host_vertices;
     bool host_valid = false;
     char err[512] = {0};
@@ -268,7 +269,7 @@ static int ipx_reset_vertex_state()
     /* every stamp IPX_NO_STAMP: no slot counts in any superstep */
     IPX_CU(cudaMemsetAsync(c.sbslot[0], 0xff, (V ? V : 1) * sizeof(ipx_sbslot), st));
     IPX_CU(cudaMemsetAsync(c.sbslot[1], 0xff, (V ? V : 1) * sizeof(ipx_sbslot), st));
-    IPX_CU(cudaMemsetAsync(c.hub_arrived, 0, (ipx_h.gbins.count[2] + 1) * sizeof(uint32_t), st));
+    IPX_CU(cudaMemsetAsync(c.hub_arrived, 0, (ipx_h.ghubs.hubs + 1) * sizeof(uint32_t), st));
 #else
     IPX_CU(cudaMemsetAsync(c.hasmsg_b, 0, V + 1, st));
     IPX_CU(cudaMemsetAsync(c.bslot[0], 0xff, (V ? V : 1) * sizeof(ipx_bslot), st));
@@ -336,6 +337,20 @@ static int ipx_build_hot_ids(ipx_consts& c)
 }
 #else
 static int ipx_build_hot_ids(ipx_consts&) { return IPG_OK; }
+#endif
+
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+/* In-edges per hub chunk: a quarter of a resident warp's share of the edges,
+ * so that every warp gets several and they even out, within [256,
+ * IPX_GATHER_CHUNK]. */
+static uint64_t ipx_hub_chunk_edges(uint64_t E)
+{
+    if (!IPX_HUB_WARP) return IPX_GATHER_CHUNK;
+    const uint64_t share = E / ((uint64_t)ipg_sm_count() * IPX_GATHER_CTAS * (IPX_THREADS / 32) * 4);
+    uint64_t chunk = 256;
+    while (chunk < IPX_GATHER_CHUNK && chunk * 2 <= share) chunk *= 2;
+    return chunk;
+}
 #endif
 
 /* Allocates the version's device state for the attached graph. */
@@ -454,26 +469,28 @@ static int ipx_setup_state()
     IPX_OK(ipx_alloc(&c.sbslot[0], V));
     IPX_OK(ipx_alloc(&c.sbslot[1], V));
     IPX_OK(ipx_alloc(&c.active_b, V + 1));
-    IPX_OK(ipg_graph_bins(ipx_h.gw, 1, ipx_h.tune.t0, ipx_h.tune.t1, &ipx_h.gbins));
     {
-        /* chunks of the hub class: prefix, partial folds, arrival counters */
-        const ipg_bins& b = ipx_h.gbins;
-        const uint64_t n2 = b.count[2];
-        const uint64_t max_chunks = b.edges[2] / IPX_GATHER_CHUNK + n2 + 1;
-        IPX_OK(ipx_alloc(&ipx_h.pull_prefix, n2 + 2));
-        IPX_OK(ipx_alloc(&c.hub_part, max_chunks));
-        IPX_OK(ipx_alloc(&c.hub_arrived, n2 + 1));
-        IPX_CU(cudaMemset(c.hub_arrived, 0, (n2 + 1) * sizeof(uint32_t)));
-        uint32_t* dcount = nullptr;
-        IPX_OK(ipx_alloc(&dcount, 1));
-        const uint32_t n2u = (uint32_t)n2;
-        IPX_CU(cudaMemcpy(dcount, &n2u, 4, cudaMemcpyHostToDevice));
-        uint32_t* owner = nullptr;
-        IPX_OK(ipx_alloc(&owner, max_chunks));
-        ipx_k_hub_prefix<IPX_GATHER_CHUNK><<<1, 1024>>>(b.d_list[2], dcount, c.in_row, ipx_h.pull_prefix, owner);
-        IPX_CU(cudaGetLastError());
-        IPX_CU(cudaDeviceSynchronize());
-        c.hub_owner = owner;
+        /* rows above a chunk are hubs: on a large graph rows up to t1 stay
+         * in the middle class, which needs no partial folds */
+        const uint64_t chunk = ipx_hub_chunk_edges(gv.E);
+        const uint64_t hub_min = ipx_h.tune.t1 < chunk ? ipx_h.tune.t1 : chunk;
+        const uint64_t t0 = ipx_h.tune.t0 < hub_min ? ipx_h.tune.t0 : hub_min;
+        const uint64_t mid = IPX_GATHER_MID < hub_min ? IPX_GATHER_MID : hub_min;
+        IPX_OK(ipg_graph_bins(ipx_h.gw, 1, t0, mid > t0 ? mid : t0, &ipx_h.gbins));
+        IPX_OK(ipg_graph_hubs(ipx_h.gw, 1, hub_min, chunk, &ipx_h.ghubs));
+        c.hub_min = hub_min;
+        for (int k = 0; k < 3; k++) {
+            c.class_list[k] = ipx_h.gbins.d_list[k];
+            c.class_n[k] = (uint32_t)ipx_h.gbins.count[k];
+        }
+        const ipg_hubs& n = ipx_h.ghubs;
+        c.hub = (const uint4*)n.d_hub;
+        c.hub_owner = n.d_owner;
+        c.chunks = (uint32_t)n.chunks;
+        c.hub_chunk = (uint32_t)chunk;
+        IPX_OK(ipx_alloc(&c.hub_part, n.chunks));
+        IPX_OK(ipx_alloc(&c.hub_arrived, n.hubs + 1));
+        IPX_CU(cudaMemset(c.hub_arrived, 0, (n.hubs + 1) * sizeof(uint32_t)));
     }
     IPX_OK(ipx_build_hot_ids(c));
 #endif
@@ -507,16 +524,12 @@ static int ipx_setup_state()
         ipx_h.grid_edge = ipx_resident_grid(ipx_k_push<1>, tb, per_sm);
 #elif IPX_VERSION == IPX_SINGLE_BROADCAST
         ipx_h.grid_compute = ipx_resident_grid(ipx_k_compute_sb0, tb, per_sm);
-        if (c.in_adj_hot) {
-            ipx_h.grid_edge = ipx_resident_grid(ipx_k_gather_compute<1, true>, tb, per_sm);
-            ipx_h.grid_gather[0] = ipx_resident_grid(ipx_k_gather_compute<0, true>, tb, per_sm);
-            ipx_h.grid_gather[2] = ipx_resident_grid(ipx_k_gather_compute<2, true>, tb, per_sm);
-        } else {
-            ipx_h.grid_edge = ipx_resident_grid(ipx_k_gather_compute<1, false>, tb, per_sm);
-            ipx_h.grid_gather[0] = ipx_resident_grid(ipx_k_gather_compute<0, false>, tb, per_sm);
-            ipx_h.grid_gather[2] = ipx_resident_grid(ipx_k_gather_compute<2, false>, tb, per_sm);
-        }
-        ipx_h.grid_gather[1] = ipx_h.grid_edge;
+        ipx_h.grid_edge = c.in_adj_hot ? ipx_resident_grid(ipx_k_gather_compute<true>, tb, per_sm)
+                                       : ipx_resident_grid(ipx_k_gather_compute<false>, tb, per_sm);
+#if !IPX_HUB_WARP
+        ipx_h.grid_hubs = c.in_adj_hot ? ipx_resident_grid(ipx_k_gather_hubs<true>, tb, per_sm)
+                                       : ipx_resident_grid(ipx_k_gather_hubs<false>, tb, per_sm);
+#endif
 #else
         ipx_h.grid_compute = ipx_resident_grid(ipx_k_compute_ssb, tb, per_sm);
         ipx_h.grid_edge = ipx_resident_grid(ipx_k_gather<1, false>, tb, per_sm);
@@ -703,16 +716,13 @@ static void ipx_account_bytes(uint64_t s, uint64_t frontier)
 #endif
 #elif IPX_VERSION == IPX_SINGLE_BROADCAST
     /* superstep 0's compute: activity, value read and write, broadcast;
-     * the fused kernels: per vertex its list entry, in-row bounds, activity
-     * and value read + write, out-row bounds and a broadcast (the compute
-     * phase of the next superstep); per in-edge its id and the gathered
-     * message */
-    const ipg_bins& b = ipx_h.gbins;
+     * the fused kernel: per vertex its in-row bounds, activity, value read
+     * and write and a broadcast (the compute phase of the next superstep);
+     * per in-edge its id and the gathered message */
     (void)frontier;
     if (s == 0) B[IPX_K_COMPUTE] += V * (1.0 + 2 * vb + 16.0 + mb);
-    for (int k = 0; k < 3; k++)
-        B[IPX_K_GATHER0 + k] += b.count[k] * (4.0 + 16.0 + 1.0 + 2 * vb + mb) + b.edges[k] * (ib + mb);
-    for (int k = 0; k < 3; k++) N[IPX_K_GATHER0 + k] += b.edges[k];
+    B[IPX_K_GATHER1] += V * (16.0 + 1.0 + 2 * vb + mb) + (double)ipx_h.c.E * (ib + mb);
+    N[IPX_K_GATHER1] += (double)ipx_h.c.E;
 #else
     const double nb = (double)l[0] + l[1] + l[2];
     B[IPX_K_COMPUTE] += frontier * (4.0 + 2 * vb + 1 + mb) + nb * mb;
@@ -821,23 +831,14 @@ static int ipx_enqueue_superstep()
 #elif IPX_VERSION == IPX_SINGLE_BROADCAST
     {
         /* gather of this superstep fused with the next one's compute phase */
-        const ipg_bins& b = ipx_h.gbins;
-        const bool hot = ipx_h.c.in_adj_hot != nullptr;
-        if (b.count[0])
-            IPX_LAUNCH(IPX_K_GATHER0, hot ? ipx_k_gather_compute<0, true><<<ipx_h.grid_gather[0], ipx_h.tb, 0, st>>>(
-                                                b.d_list[0], b.count[0], nullptr)
-                                          : ipx_k_gather_compute<0, false><<<ipx_h.grid_gather[0], ipx_h.tb, 0, st>>>(
-                                                b.d_list[0], b.count[0], nullptr));
-        if (b.count[1])
-            IPX_LAUNCH(IPX_K_GATHER1, hot ? ipx_k_gather_compute<1, true><<<ipx_h.grid_gather[1], ipx_h.tb, 0, st>>>(
-                                                b.d_list[1], b.count[1], nullptr)
-                                          : ipx_k_gather_compute<1, false><<<ipx_h.grid_gather[1], ipx_h.tb, 0, st>>>(
-                                                b.d_list[1], b.count[1], nullptr));
-        if (b.count[2])
-            IPX_LAUNCH(IPX_K_GATHER2, hot ? ipx_k_gather_compute<2, true><<<ipx_h.grid_gather[2], ipx_h.tb, 0, st>>>(
-                                                b.d_list[2], b.count[2], ipx_h.pull_prefix)
-                                          : ipx_k_gather_compute<2, false><<<ipx_h.grid_gather[2], ipx_h.tb, 0, st>>>(
-                                                b.d_list[2], b.count[2], ipx_h.pull_prefix));
+        const bool hot = c.in_adj_hot != nullptr;
+#if !IPX_HUB_WARP
+        if (c.chunks)
+            IPX_LAUNCH(IPX_K_GATHER2, hot ? ipx_k_gather_hubs<true><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>()
+                                          : ipx_k_gather_hubs<false><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>());
+#endif
+        IPX_LAUNCH(IPX_K_GATHER1, hot ? ipx_k_gather_compute<true><<<ge, ipx_h.tb, 0, st>>>()
+                                      : ipx_k_gather_compute<false><<<ge, ipx_h.tb, 0, st>>>());
     }
 #else
     uint64_t* edges_b = (uint64_t*)(c.ctr + 8);

@@ -219,6 +219,24 @@ struct ipg_graph {
         uint64_t bytes = 0;
         ipg_bins bins;
     } bins[2];
+    struct HubCache {
+        bool valid = false;
+        uint64_t hub_min = 0, chunk = 0;
+        void* mem = nullptr;
+        uint64_t bytes = 0;
+        ipg_hubs hubs = {};
+    } hubs[2];
+    // what was derived from the rows (which = 0), the in-lists (1) or both (-1)
+    void drop_derived(int which = -1)
+    {
+        for (int k = 0; k < 2; k++) {
+            if (which >= 0 && which != k) continue;
+            ipg_dev_free(bins[k].lists, bins[k].bytes);
+            bins[k] = BinCache();
+            ipg_dev_free(hubs[k].mem, hubs[k].bytes);
+            hubs[k] = HubCache();
+        }
+    }
     // ipg_graph_refill_host's own stream, device words (check bits, degree
     // maxima), pinned words and offset staging, made at its first call
     cudaStream_t refill_st = nullptr;
@@ -267,7 +285,7 @@ struct ipg_graph {
         ipg_dev_free(in_row, in_row_bytes);
         ipg_dev_free(in_adj, in_adj_bytes);
         ipg_dev_free(in_wgt, in_wgt_bytes);
-        for (auto& b : bins) ipg_dev_free(b.lists, b.bytes);
+        drop_derived();
     }
 };
 
@@ -866,10 +884,7 @@ extern "C" int ipg_graph_degree_order(ipg_graph* g, int need_in, ipg_order* out)
     if (!fresh) {
         g->ord_valid = false;
         o->v.has_in = 0;  // rebuilt below with the rows
-        for (auto& b : o->bins) {  // derived from the old contents
-            ipg_dev_free(b.lists, b.bytes);
-            b = ipg_graph::BinCache();
-        }
+        o->drop_derived();  // from the old contents
         if (V) {
             uint32_t* occ = (uint32_t*)deg;
             const uint64_t s = ord_sample_stride();
@@ -973,11 +988,7 @@ extern "C" int ipg_graph_refill_host(ipg_graph* g, const void* idx, int idx_byte
     // contents are not validated (bad).
     g->generation++;
     g->bad = true;
-    // derived data of the old contents
-    for (auto& b : g->bins) {
-        ipg_dev_free(b.lists, b.bytes);
-        b = ipg_graph::BinCache();
-    }
+    g->drop_derived();  // from the old contents
     g->v.symmetric = 0;
     const bool own_in = g->in_row != nullptr;
     if (own_in) {
@@ -1627,8 +1638,7 @@ extern "C" int ipg_graph_set_directed(ipg_graph* g, int directed)
     ipg_dev_free(g->in_wgt, g->in_wgt_bytes);
     g->in_row = g->in_adj = g->in_wgt = nullptr;
     g->in_row_bytes = g->in_adj_bytes = g->in_wgt_bytes = 0;
-    ipg_dev_free(g->bins[1].lists, g->bins[1].bytes);
-    g->bins[1] = ipg_graph::BinCache();
+    g->drop_derived(1);
     g->v.has_in = 0;
     g->v.d_in_row = nullptr;
     g->v.d_in_adj = nullptr;
@@ -1898,5 +1908,63 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
     c.t1 = t1;
     c.valid = true;
     *bins = c.bins;
+    return IPG_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Hub rows cut into chunks (cached per direction).
+// ---------------------------------------------------------------------------
+__global__ void k_hub_chunks(const uint64_t* __restrict__ row, uint64_t V, uint64_t hub_min, uint64_t chunk,
+                             uint4* __restrict__ hub, uint32_t* __restrict__ owner, uint32_t* __restrict__ cnt)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t d = row[i + 1] - row[i];
+        if (d > hub_min) {
+            const uint32_t n = (uint32_t)((d + chunk - 1) / chunk);
+            const uint32_t h = atomicAdd(&cnt[0], 1u), c0 = atomicAdd(&cnt[1], n);
+            hub[h] = make_uint4((uint32_t)i, c0, n, 0u);
+            for (uint32_t k = 0; k < n; k++) owner[c0 + k] = h;
+        }
+    }
+}
+
+extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64_t chunk, ipg_hubs* hubs)
+{
+    if (!g || !hubs) return fail(IPG_EINVAL, "ipg_graph_hubs: null argument");
+    if (chunk < 1) return fail(IPG_EINVAL, "ipg_graph_hubs: chunks hold at least one edge");
+    if (use_in && !g->v.has_in) IPG_TRY(ipg_graph_build_in(g));
+    auto& c = g->hubs[use_in ? 1 : 0];
+    if (c.valid && c.hub_min == hub_min && c.chunk == chunk) {
+        *hubs = c.hubs;
+        return IPG_OK;
+    }
+    const uint64_t V = g->v.V, E = g->v.E;
+    uint64_t hubs_max = E / (hub_min + 1) + 1;
+    if (hubs_max > V) hubs_max = V;
+    const uint64_t chunks_max = E / chunk + hubs_max + 1;
+    if (chunks_max >= (1ULL << 32)) return fail(IPG_EINVAL, "ipg_graph_hubs: too many chunks for 32-bit indices");
+    ipg_dev_free(c.mem, c.bytes);
+    c = ipg_graph::HubCache();
+    const uint64_t hub_b = align256((hubs_max + 1) * 16), own_b = align256(chunks_max * 4);
+    IPG_TRY(ipg_dev_alloc(&c.mem, hub_b + own_b + 256));
+    c.bytes = hub_b + own_b + 256;
+    uint4* hub = (uint4*)c.mem;
+    uint32_t* owner = (uint32_t*)((char*)c.mem + hub_b);
+    uint32_t* cnt = (uint32_t*)((char*)c.mem + hub_b + own_b);
+    uint32_t h[2] = {0, 0};
+    if (V) {
+        IPG_CUDA(cudaMemsetAsync(cnt, 0, 8, 0));
+        k_hub_chunks<<<grid_for(V, 256), 256>>>(use_in ? g->v.d_in_row : g->v.d_row, V, hub_min, chunk, hub, owner, cnt);
+        IPG_CUDA(cudaGetLastError());
+        IPG_CUDA(cudaMemcpy(h, cnt, 8, cudaMemcpyDeviceToHost));
+    }
+    c.hubs.d_hub = (const uint32_t*)hub;
+    c.hubs.hubs = h[0];
+    c.hubs.d_owner = owner;
+    c.hubs.chunks = h[1];
+    c.hub_min = hub_min;
+    c.chunk = chunk;
+    c.valid = true;
+    *hubs = c.hubs;
     return IPG_OK;
 }

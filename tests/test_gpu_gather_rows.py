@@ -1,0 +1,60 @@
+"""The single_broadcast gather at the sizes where its rows change hands: row
+lengths around the 128-bit id loads, the lanes per row, the degree classes and
+the hub chunks, with the edge array ending at every position of a load."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# around quads (4), 8 and 16 lanes of quads (32, 64), the classes (16, 64), hub chunks (256 on a small graph)
+LENGTHS = (0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 32, 33, 35, 36, 63, 64, 65, 67, 68, 127, 128, 129, 255, 256, 257,
+           511, 512, 513, 1500, 4096, 4097)
+PR_TOL = 1e-12  # the oracle folds a row in order, the warp classes in a tree
+
+
+def _graph(tail):
+    """Rows of LENGTHS in a shuffled order, then `tail` edges in the last row (the edge count modulo 4 varies)."""
+    rng = np.random.default_rng(7 + tail)
+    V = 5000
+    deg = np.zeros(V, dtype=np.int64)
+    deg[rng.permutation(V - 1)[:len(LENGTHS)]] = LENGTHS
+    deg[V - 1] = tail
+    idx = np.concatenate(([0], np.cumsum(deg)[:-1])).astype(np.uint64)
+    adj = np.concatenate([rng.choice(V, int(d), replace=False) for d in deg]).astype(np.uint32)
+    return O.CSR(V, int(deg.sum()), idx, adj, None)
+
+
+@pytest.mark.parametrize("tail", [0, 1, 2, 3])
+@pytest.mark.parametrize("app,version,id_bits,variant", [
+    ("pagerank", "single_broadcast", 32, ""), ("pagerank", "single_broadcast", 32, "staged"),
+    ("cc", "single_broadcast", 32, ""), ("cc", "single_broadcast", 64, "")])
+def test_rows_of_every_length(app, version, id_bits, variant, tail):
+    import ipregel_b200 as ip
+    g = _graph(tail)
+    want, counts, _ = O.run(g, app, version, id_bytes=id_bits // 8)
+    adj = g.adj if id_bits == 32 else g.adj.astype(np.uint64)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, adj, id_bytes=id_bits // 8)
+    eng = ip.Engine(app, version, id_bits, variant=variant)
+    eng.set_quiet(True)
+    try:
+        if app == "pagerank":
+            eng.set_param("rounds", 10)
+        # the default classes; classes of one lane a row up to a quad; every row above 3 edges a hub; small CTAs
+        for tune in (dict(), dict(t0=4, t1=4096), dict(t0=2, t1=3), dict(block=64, t0=64, t1=200)):
+            for order in (True, False):
+                eng.set_order(order)
+                eng.set_tuning(**tune)
+                eng.attach(graph)
+                res = eng.run()
+                assert res.counts == [int(c) for c in counts], (tune, order)
+                if app == "pagerank":
+                    assert float(np.max(np.abs(res.values - want))) <= PR_TOL, (tune, order)
+                else:
+                    np.testing.assert_array_equal(res.values.astype(np.uint64), want.astype(np.uint64))
+    finally:
+        eng.set_tuning()
+        eng.set_order(True)
+        eng.release()
+        graph.free()
