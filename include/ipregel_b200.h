@@ -236,6 +236,9 @@ typedef struct ipg_hubs {
     uint64_t hubs;
     const uint32_t* d_owner;
     uint64_t chunks;
+    uint64_t edges;          /* of all hubs */
+    uint64_t ids_readable;   /* ids of the list array that may be read: E, or E
+                              * rounded up to a multiple of 4 */
 } ipg_hubs;
 int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64_t chunk,
                    ipg_hubs* hubs);
@@ -297,11 +300,12 @@ int ipg_sm_count(void);
 typedef struct ipg_pr_plan ipg_pr_plan;
 
 /* Degree classes and scratch for runs on graph g (32-bit ids); holds
- * 12 bytes per vertex plus 8 bytes per 4096 hub edges of HBM until freed
+ * 12 bytes per vertex plus 8 bytes per hub chunk of HBM until freed
  * (and builds the graph's in-lists if it is directed). */
 int ipg_pr_plan_create(ipg_graph* g, ipg_pr_plan** plan);
 void ipg_pr_plan_free(ipg_pr_plan* plan);
-/* Vertices and edge sums of the thread / warp / hub classes, hub chunks. */
+/* Vertices and edge sums of the rows of a thread each, of several lanes each,
+ * and of the hubs; hub chunks. */
 int ipg_pr_plan_info(const ipg_pr_plan* plan, uint64_t* class_counts, uint64_t* class_edges,
                      uint64_t* hub_chunks);
 

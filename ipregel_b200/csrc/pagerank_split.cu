@@ -22,15 +22,15 @@
 // of x over vertices without out-edges) and the L1 residual sum |x - x_prev| --
 // are reduced in FP64.
 //
-// Kernels per superstep: one gather+update kernel per degree class (thread
-// per vertex up to t0 edges, warp per vertex up to t1 edges), and for the
-// hubs a chunk kernel (one CTA per PR_CHUNK edges, partial pairs to scratch)
-// followed by a finalising kernel that merges each hub's chunk partials in
-// chunk order.  Everything is enqueued on one stream without host
+// One kernel per superstep gathers, updates and sums the diagnostics: the
+// hubs' rows in chunks, a warp each (partial pairs to scratch, merged in chunk
+// order by the warp whose chunk arrives last), then rows by length with 16, 8
+// and 1 lanes each.  Everything is enqueued on one stream without host
 // synchronisation or allocation, so a run can be captured into a CUDA graph.
 #include "ipregel_b200.h"
 
 #include <cuda_runtime.h>
+#include <cub/cub.cuh>
 
 #include <cstdlib>
 #include <new>
@@ -40,12 +40,21 @@
 extern "C" int ipg_internal_fail(int code, const char* msg);
 
 #define PR_THREADS 256
-#define PR_UNROLL 4
-#define PR_CHUNK 4096
+#define PR_CHUNK 4096 /* most edges of a hub chunk, and so of a row that is no hub */
+#define PR_MID 64     /* rows up to here take PR_GROUP lanes, longer ones PR_LONG */
 #ifndef PR_GROUP
-#define PR_GROUP 16 /* lanes per vertex of the middle degree class */
+#define PR_GROUP 8
 #endif
-#define PR_CTAS_PER_SM 8 /* upper bound; the resident count decides */
+#ifndef PR_SHORT
+#define PR_SHORT 1
+#endif
+#ifndef PR_LONG
+#define PR_LONG 16
+#endif
+#ifndef PR_CTAS
+#define PR_CTAS 4 /* resident CTAs per SM the gather is compiled for */
+#endif
+#define PR_CTAS_PER_SM 8 /* upper bound of the other kernels; the resident count decides */
 
 #define PR_CUDA(call)                                                      \
     do {                                                                   \
@@ -70,12 +79,15 @@ struct ipg_pr_plan {
     // writes the values in the caller's (null: the graph's own numbering)
     const uint32_t* new_of_old = nullptr;
     float* xs2 = nullptr;
-    uint32_t* hub_prefix = nullptr;    // first chunk of each hub, then the total
-    uint32_t* hub_owner = nullptr;     // chunk -> index of its hub
+    ipg_hubs hubs{};                   // rows above hub_min in chunks
+    uint64_t hub_min = 0, chunk = 0;
     float2* partial = nullptr;         // (sum, compensation) of every hub chunk
-    uint64_t chunks = 0;
+    uint32_t* arrived = nullptr;       // per hub the chunks arrived (0 between supersteps)
+    uint32_t* shorts = nullptr;        // the short class: first the vertices with in-edges
+    uint64_t empty = 0, empty_dangling = 0;  // the rest of it
+    uint64_t class_count[3] = {0, 0, 0}, class_edges[3] = {0, 0, 0};
     int sms = 148;
-    uint32_t grid = 0;  // resident CTAs of the gather kernels, all SMs
+    uint32_t grid = 0, grid_flat = 0;  // resident CTAs of the gather / of the others, all SMs
     std::vector<std::pair<void*, uint64_t>> allocs;
 };
 
@@ -121,10 +133,23 @@ struct PrStep {
     const uint64_t* __restrict__ row;     // out-rows: the degrees
     const uint64_t* __restrict__ in_row;  // gather lists (the rows themselves
     const uint32_t* __restrict__ in_adj;  // unless the graph is directed)
-    const float* __restrict__ b_cur;  // read by the gathers
-    float* __restrict__ b_next;       // written for the next superstep
-    float* __restrict__ x_out;        // this superstep's values
+    const float* __restrict__ b_cur;   // read by the gathers
+    float* __restrict__ b_next;        // written for the next superstep
+    float* __restrict__ x_out;         // this superstep's values
+    const float* __restrict__ x_prev;  // the last superstep's
+    double* __restrict__ diag;         // this superstep's mass, dangling mass, residual
     float ratio, damping;
+    const uint32_t* __restrict__ list[3];  // short, middle, long rows (hubs among the long)
+    uint64_t n[3];
+    const uint4* __restrict__ hub;         // {vertex, first chunk, chunks}
+    const uint32_t* __restrict__ owner;    // chunk -> hub
+    float2* __restrict__ partial;
+    uint32_t* __restrict__ arrived;
+    uint64_t chunks, chunk, hub_min;
+    uint64_t empty, empty_dangling;  // vertices without in-edges; of those, without out-edges
+    float x0;                        // superstep 0's value
+    bool first;                      // superstep 1
+    bool quads;  // 128-bit id loads: an aligned array of whole loads
 };
 
 // Sum of the vertex diagnostics over the CTA, added to diag[0..2].
@@ -156,107 +181,76 @@ __device__ __forceinline__ void pr_block_diag(double m, double d, double r, doub
     }
 }
 
-// Vertex update of pagerank.c:51-52 and the broadcast of :57-63.  The
-// values are double-buffered: the gathers only write, and the diagnostics
-// come from a separate streaming pass over both buffers (reading the old
-// value here, one more dependent load per vertex, cost more than doubling
-// the superstep on R-MAT scale 24).
+// Diagnostics of the vertices a thread updated.
+struct PrDiag {
+    double m = 0, d = 0, r = 0;
+};
+
+// Vertex update of pagerank.c:51-52 and the broadcast of :57-63; the values
+// are double-buffered.  deg and x_prev were loaded before the gather, so the
+// update waits for nothing (read after it, the old value more than doubled
+// the superstep on R-MAT scale 24, and a pass of its own took 4 % of the run).
 template <bool LAST>
-__device__ __forceinline__ void pr_finish(const PrStep& a, uint64_t v, uint64_t deg, float sum)
+__device__ __forceinline__ void pr_finish(const PrStep& a, uint64_t v, uint64_t deg, float x_prev, float sum, PrDiag& g)
 {
     const float xn = __fadd_rn(a.ratio, __fmul_rn(a.damping, sum));
     a.x_out[v] = xn;
     if constexpr (!LAST) a.b_next[v] = deg ? __fdiv_rn(xn, (float)deg) : 0.0f;
+    g.m += (double)xn;
+    if (!deg) g.d += (double)xn;
+    g.r += fabs((double)xn - (double)x_prev);
 }
 
-// Lane-strided compensated sum of b_cur over adj[e0, e1), PR_UNROLL loads in
-// flight per lane (warps and blocks: pr_gather_v4).  Ids are loaded evict-first where a warp reads consecutive
-// ids in one instruction (lanes >= 32); a thread walking a row alone comes
-// back to the same line in its next loads, so it keeps the line cached.
-template <bool COMP>
-__device__ __forceinline__ void pr_gather_v4(const PrStep& a, uint64_t e0, uint64_t e1, uint64_t lane,
-                                             uint64_t lanes, float& s, float& c)
+// The aligned four ids at position rel (a multiple of 4) from row start r0
+// rounded down to one; which of them belong to the row of deg edges is
+// decided when they are used, so that nothing waits for the load before.
+__device__ __forceinline__ uint4 pr_ld_quad(const PrStep& a, uint64_t r0, uint32_t deg, uint32_t rel)
 {
-    // a warp or block reads four consecutive ids per lane with one 128-bit
-    // load; the up to 3 ids before the first 16-byte boundary and after the
-    // last take a lane each
-    uint64_t al = (e0 + 3) & ~3ULL;
-    if (al > e1) al = e1;
-    const uint64_t b = al + ((e1 - al) & ~3ULL);
-    {
-        const uint64_t nh = al - e0, nt = e1 - b;
-        uint64_t e = e1;
-        if (lane < nh) e = e0 + lane;
-        else if (lane < nh + nt) e = b + (lane - nh);
-        if (e < e1) pr_add<COMP>(s, c, __ldg(&a.b_cur[a.in_adj[e]]));
-    }
-    const uint4* __restrict__ q4 = reinterpret_cast<const uint4*>(a.in_adj + al);
-    const uint64_t groups = (b - al) >> 2;
-    for (uint64_t g = lane; g < groups; g += lanes) {
-        const uint4 id = __ldcs(q4 + g);
-        const float q0 = __ldg(&a.b_cur[id.x]), q1 = __ldg(&a.b_cur[id.y]);
-        const float q2 = __ldg(&a.b_cur[id.z]), q3 = __ldg(&a.b_cur[id.w]);
-        pr_add<COMP>(s, c, q0);
-        pr_add<COMP>(s, c, q1);
-        pr_add<COMP>(s, c, q2);
-        pr_add<COMP>(s, c, q3);
-    }
+    const uint32_t off = (uint32_t)r0 & 3u;
+    return __ldcs(reinterpret_cast<const uint4*>(a.in_adj + (rel < off + deg ? r0 - off + rel : 0)));
 }
 
+// Adds the quotients of the row's edges among them, in order.
+template <bool COMP>
+__device__ __forceinline__ void pr_add_quad(const PrStep& a, const uint4& q, uint64_t r0, uint32_t deg, uint32_t rel,
+                                            float& s, float& c)
+{
+    const uint32_t t = rel - ((uint32_t)r0 & 3u);  // edge of the row; before its first: wraps
+    const uint32_t id[4] = {q.x, q.y, q.z, q.w};
+    float w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = t + k < deg ? __ldg(&a.b_cur[id[k]]) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) pr_add<COMP>(s, c, w[k]);  // 0 leaves the pair as it is
+}
+
+// Lane-strided sum over in_adj[e0, e1) for arrays without 128-bit loads.
 template <bool COMP>
 __device__ __forceinline__ void pr_gather(const PrStep& a, uint64_t e0, uint64_t e1, uint64_t lane, uint64_t lanes,
                                           float& s, float& c)
 {
-    if (lanes >= 8 && (reinterpret_cast<uintptr_t>(a.in_adj) & 15) == 0) {
-        pr_gather_v4<COMP>(a, e0, e1, lane, lanes, s, c);
-        return;
-    }
-    for (uint64_t e = e0 + lane; e < e1; e += PR_UNROLL * lanes) {
-        uint32_t u[PR_UNROLL];
-        float q[PR_UNROLL];
-#pragma unroll
-        for (int k = 0; k < PR_UNROLL; k++) {
-            const uint64_t ek = e + k * lanes;
-            u[k] = ek < e1 ? (lanes >= 32 ? __ldcs(&a.in_adj[ek]) : a.in_adj[ek]) : 0u;
-        }
-#pragma unroll
-        for (int k = 0; k < PR_UNROLL; k++) q[k] = (e + k * lanes < e1) ? __ldg(&a.b_cur[u[k]]) : 0.0f;
-#pragma unroll
-        for (int k = 0; k < PR_UNROLL; k++)
-            if (e + k * lanes < e1) pr_add<COMP>(s, c, q[k]);
-    }
+    for (uint64_t e = e0 + lane; e < e1; e += lanes) pr_add<COMP>(s, c, __ldg(&a.b_cur[a.in_adj[e]]));
 }
 
-// Out-degree of v whose gather list is in_adj[e0, e1).
-__device__ __forceinline__ uint64_t pr_deg(const PrStep& a, uint64_t v, uint64_t e0, uint64_t e1)
+// Out-degree of v whose gather list holds n ids.
+__device__ __forceinline__ uint64_t pr_deg(const PrStep& a, uint64_t v, uint64_t n)
 {
-    return a.row == a.in_row ? e1 - e0 : a.row[v + 1] - a.row[v];
+    return a.row == a.in_row ? n : a.row[v + 1] - a.row[v];
 }
 
-// Superstep 0: x = 1/V, broadcast x/deg.
-__global__ void __launch_bounds__(PR_THREADS) k_pr_init(PrStep a, uint64_t V, float x0)
+// Superstep 0: x = 1/V, broadcast x/deg, and its diagnostics {sum x, sum of x
+// over vertices without out-edges, 0}.
+__global__ void __launch_bounds__(PR_THREADS) k_pr_init(const PrStep a, uint64_t V, float x0)
 {
+    double m = 0, d = 0;
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t deg = a.row[v + 1] - a.row[v];
         a.x_out[v] = x0;
         a.b_next[v] = deg ? __fdiv_rn(x0, (float)deg) : 0.0f;
+        m += (double)x0;
+        if (!deg) d += (double)x0;
     }
-}
-
-// FP64 diagnostics of a superstep: diag = {sum x, sum of x over vertices
-// without out-edges, sum |x - x_prev|} (x_prev null at superstep 0).
-__global__ void __launch_bounds__(PR_THREADS) k_pr_diag(const float* __restrict__ x, const float* __restrict__ x_prev,
-                                                        const uint64_t* __restrict__ row, uint64_t V,
-                                                        double* __restrict__ diag)
-{
-    double m = 0, d = 0, r = 0;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
-        const double xv = (double)x[v];
-        m += xv;
-        if (row[v + 1] == row[v]) d += xv;
-        if (x_prev) r += fabs(xv - (double)x_prev[v]);
-    }
-    pr_block_diag(m, d, r, diag);
+    pr_block_diag(m, d, 0.0, a.diag);
 }
 
 // out[i] = x[new_of_old[i]]: the values in the caller's numbering.
@@ -267,130 +261,167 @@ __global__ void k_pr_by_id(const float* __restrict__ x, const uint32_t* __restri
         out[i] = x[new_of_old[i]];
 }
 
-// Class 0: a thread per vertex.
-template <bool COMP, bool LAST>
-__global__ void __launch_bounds__(PR_THREADS) k_pr_thread(PrStep a, const uint32_t* __restrict__ list, uint64_t n)
+// Edges of a row; no row but a hub's comes near the limit.
+__device__ __forceinline__ uint32_t pr_edges(uint64_t r0, uint64_t r1)
 {
-    // the next vertex's list entry and row bounds are loaded while this
-    // vertex's in-edges are gathered
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, v = 0, e0 = 0, e1 = 0;
-    if (i < n) {
-        v = list[i];
-        e0 = a.in_row[v];
-        e1 = a.in_row[v + 1];
-    }
-    for (; i < n; i += stride) {
-        uint64_t vn = 0, e0n = 0, e1n = 0;
-        if (i + stride < n) {
-            vn = list[i + stride];
-            e0n = a.in_row[vn];
-            e1n = a.in_row[vn + 1];
-        }
-        float s = 0.0f, c = 0.0f;
-        pr_gather<COMP>(a, e0, e1, 0, 1, s, c);
-        pr_finish<LAST>(a, v, pr_deg(a, v, e0, e1), __fadd_rn(s, c));
-        v = vn;
-        e0 = e0n;
-        e1 = e1n;
-    }
+    return r1 - r0 < 0x7fffffffull ? (uint32_t)(r1 - r0) : 0x7fffffffu;
 }
 
-// Class 1: PR_GROUP lanes per vertex (most vertices of the class have a few
-// dozen in-edges, which 16 lanes reading four ids each cover in a step or
-// two; a whole warp per vertex left most lanes idle).
-template <bool COMP, bool LAST>
-__global__ void __launch_bounds__(PR_THREADS) k_pr_warp(PrStep a, const uint32_t* __restrict__ list, uint64_t n)
+// The list's vertices, G lanes each; SKIP: hubs are passed over.  What bounds
+// a row is the chain list entry -> row bounds -> ids -> quotients, so it is
+// pipelined over the group's next rows as in the FP64 engine's gather: while
+// a row's quotients are in flight, the next row's ids, the bounds of the one
+// after it and the list entry of the one after that are loaded.  Directed
+// R-MAT scale 25, 30 rounds: 63.0 ms with a launch per class, unpipelined, and
+// a diagnostics pass; 60.6 ms now, of which rows of 17 to 4,096 edges 32.5
+// (345 G edges/s, where the same ids gathered flat reach 354), hubs 16 (245
+// G/s: their ids hit the L1 least), short rows 10.  16 lanes for all longer
+// rows 63.1, 2 or 4 lanes for the short ones 62.3 / 67.6, 5 CTAs per SM (it
+// spills) 65.5, 3 CTAs 62.5 ms.
+template <int G, bool SKIP, bool COMP, bool LAST>
+__device__ __forceinline__ void pr_rows(const PrStep& a, const uint32_t* __restrict__ list, uint64_t n, PrDiag& g)
 {
-    constexpr int G = PR_GROUP;
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-    const unsigned mask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / G;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / G; i < n; i += groups) {
-        const uint64_t v = list[i];
-        const uint64_t e0 = a.in_row[v], e1 = a.in_row[v + 1];
+    const unsigned mask = (((1u << G) - 1u) << (lane & ~(G - 1)));
+    const uint64_t step = ((uint64_t)gridDim.x * blockDim.x) / G;
+    uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / G;
+    if (i >= n) return;
+    const bool quads = a.quads;
+    // v: the row being summed, u: the next, t: the one after it.  Past the
+    // list's end vertex 0 stands in: loaded, never summed.
+    uint32_t v = list[i], u = i + step < n ? list[i + step] : 0u, t = i + 2 * step < n ? list[i + 2 * step] : 0u;
+    uint64_t v0 = a.in_row[v], u0 = a.in_row[u];
+    uint32_t vd = pr_edges(v0, a.in_row[v + 1]), ud = pr_edges(u0, a.in_row[u + 1]);
+    uint4 qv = make_uint4(0, 0, 0, 0);
+    if (quads) qv = pr_ld_quad(a, v0, vd, 4 * gl);
+    for (; i < n; i += step) {
+        const float xp = gl == 0 ? a.x_prev[v] : 0.0f;
+        const uint64_t deg = gl == 0 ? pr_deg(a, v, vd) : 0;
+        const uint32_t w = i + 3 * step < n ? list[i + 3 * step] : 0u;
+        const uint64_t t0 = a.in_row[t], t1 = a.in_row[t + 1];
+        uint4 qu = make_uint4(0, 0, 0, 0);
+        if (quads) qu = pr_ld_quad(a, u0, ud, 4 * gl);
         float s = 0.0f, c = 0.0f;
-        pr_gather<COMP>(a, e0, e1, gl, G, s, c);
+        const bool skip = SKIP && vd > a.hub_min;
+        if (skip) vd = 0;
+        if (quads) {
+            pr_add_quad<COMP>(a, qv, v0, vd, 4 * gl, s, c);
+            const uint32_t len = ((uint32_t)v0 & 3u) + vd;
+            for (uint32_t rel = 4 * gl + 4 * G; rel < len; rel += 4 * G)
+                pr_add_quad<COMP>(a, pr_ld_quad(a, v0, vd, rel), v0, vd, rel, s, c);
+        } else {
+            pr_gather<COMP>(a, v0, v0 + vd, gl, G, s, c);
+        }
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) {
             const float s2 = __shfl_down_sync(mask, s, o, G);
             const float c2 = __shfl_down_sync(mask, c, o, G);
             pr_merge<COMP>(s, c, s2, c2);
         }
-        if (gl == 0) pr_finish<LAST>(a, v, pr_deg(a, v, e0, e1), __fadd_rn(s, c));
+        if (gl == 0 && !skip) pr_finish<LAST>(a, v, deg, xp, __fadd_rn(s, c), g);
+        v = u;
+        u = t;
+        t = w;
+        v0 = u0;
+        vd = ud;
+        u0 = t0;
+        ud = pr_edges(t0, t1);
+        qv = qu;
     }
 }
 
-// Class 2, pass 1: a warp per chunk of PR_CHUNK edges of a hub (no CTA-wide
-// barriers per chunk: 15 - 20 % shorter in the FP64 engine's gather).
-template <bool COMP>
-__global__ void __launch_bounds__(PR_THREADS) k_pr_hub_chunks(PrStep a, const uint32_t* __restrict__ list, uint64_t n,
-                                                              const uint32_t* __restrict__ prefix,
-                                                              const uint32_t* __restrict__ owner,
-                                                              float2* __restrict__ partial)
-{
-    if (n == 0) return;
-    const uint32_t chunks = prefix[n];
-    const int lane = threadIdx.x & 31;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t ch = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; ch < chunks; ch += warps) {
-        const uint64_t i = owner[ch];  // one load, not a binary search over the prefix
-        const uint64_t v = list[i];
-        const uint64_t end = a.in_row[v + 1];
-        const uint64_t e0 = a.in_row[v] + (ch - prefix[i]) * (uint64_t)PR_CHUNK;
-        const uint64_t e1 = e0 + PR_CHUNK < end ? e0 + PR_CHUNK : end;
-        float s = 0.0f, c = 0.0f;
-        pr_gather<COMP>(a, e0, e1, lane, 32, s, c);
-        pr_warp_merge<COMP>(s, c);
-        if (lane == 0) partial[ch] = make_float2(s, c);
-    }
-}
-
-// Class 2, pass 2: a warp per hub merges its chunk partials in chunk order.
+// Hubs, a warp per chunk: the chunk's pair is stored, and the warp whose chunk
+// arrives last merges the hub's pairs in chunk order and updates the vertex;
+// no warp waits for another.
 template <bool COMP, bool LAST>
-__global__ void __launch_bounds__(PR_THREADS) k_pr_hub_finish(PrStep a, const uint32_t* __restrict__ list, uint64_t n,
-                                                              const uint32_t* __restrict__ prefix,
-                                                              const float2* __restrict__ partial)
+__device__ __forceinline__ void pr_hubs(const PrStep& a, PrDiag& g)
 {
     const int lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const uint64_t v = list[i];
+    for (uint64_t ch = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; ch < a.chunks; ch += warps) {
+        const uint32_t i = a.owner[ch];
+        const uint4 hub = a.hub[i];
+        const uint64_t v = hub.x, row0 = a.in_row[v], end = a.in_row[v + 1];
+        const uint64_t e0 = row0 + (ch - hub.y) * a.chunk, e1 = e0 + a.chunk < end ? e0 + a.chunk : end;
         float s = 0.0f, c = 0.0f;
-        for (uint32_t ch = prefix[i] + lane; ch < prefix[i + 1]; ch += 32) {
-            const float2 p = partial[ch];
-            pr_merge<COMP>(s, c, p.x, p.y);
+        if (a.quads) {
+            const uint32_t deg = (uint32_t)(e1 - e0), len = ((uint32_t)e0 & 3u) + deg;
+            uint4 q = pr_ld_quad(a, e0, deg, 4 * lane);
+            for (uint32_t rel = 4 * lane; rel < len; rel += 128) {
+                const uint4 next = pr_ld_quad(a, e0, deg, rel + 128);
+                pr_add_quad<COMP>(a, q, e0, deg, rel, s, c);
+                q = next;
+            }
+        } else {
+            pr_gather<COMP>(a, e0, e1, lane, 32, s, c);
         }
         pr_warp_merge<COMP>(s, c);
-        if (lane == 0) pr_finish<LAST>(a, v, a.row[v + 1] - a.row[v], __fadd_rn(s, c));
+        int last = hub.z == 1 ? 1 : 0;
+        if (lane == 0 && hub.z != 1) {
+            a.partial[ch] = make_float2(s, c);
+            __threadfence();
+            last = atomicAdd(&a.arrived[i], 1u) == hub.z - 1 ? 1 : 0;
+        }
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last && hub.z != 1) {
+            __threadfence();
+            s = c = 0.0f;
+            for (uint32_t k = lane; k < hub.z; k += 32) {
+                const float2 p = __ldcg(&a.partial[hub.y + k]);
+                pr_merge<COMP>(s, c, p.x, p.y);
+            }
+            pr_warp_merge<COMP>(s, c);
+            if (lane == 0) a.arrived[i] = 0;  // every chunk of the hub has arrived
+        }
+        if (lane == 0 && last) pr_finish<LAST>(a, v, pr_deg(a, v, end - row0), a.x_prev[v], __fadd_rn(s, c), g);
     }
 }
 
-__global__ void k_pr_hub_chunk_counts(const uint32_t* __restrict__ list, uint64_t n, const uint64_t* __restrict__ row,
-                                      uint32_t* __restrict__ out)
+// A vertex without in-edges has the value ratio from superstep 1 on.  Its
+// value and quotient are written in supersteps 1 and 2, once into each buffer,
+// and stand there for the rest of the run; k_pr_step adds its diagnostics.
+// About half of an R-MAT graph's vertices are such.
+__global__ void __launch_bounds__(PR_THREADS) k_pr_empty(const PrStep a, const uint32_t* __restrict__ list)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t v = list[i];
-        out[i] = (uint32_t)((row[v + 1] - row[v] + PR_CHUNK - 1) / PR_CHUNK);
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < a.empty; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = list[i], deg = a.row[v + 1] - a.row[v];
+        a.x_out[v] = a.ratio;
+        a.b_next[v] = deg ? __fdiv_rn(a.ratio, (float)deg) : 0.0f;
     }
+}
+
+struct PrHasEdges {
+    const uint64_t* row;
+    __device__ bool operator()(uint32_t v) const { return row[v + 1] > row[v]; }
+};
+
+// cnt += vertices of the list without out-edges
+__global__ void k_pr_count_dangling(const uint32_t* __restrict__ list, uint64_t n, const uint64_t* __restrict__ row,
+                                    unsigned long long* __restrict__ cnt)
+{
+    unsigned long long c = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        c += row[list[i] + 1] == row[list[i]];
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(cnt, c);
 }
 
 template <bool COMP, bool LAST>
-int pr_superstep(ipg_pr_plan* p, const PrStep& a, cudaStream_t st)
+__global__ void __launch_bounds__(PR_THREADS, PR_CTAS) k_pr_step(const PrStep a)
 {
-    const ipg_bins& b = p->bins;
-    const uint32_t grid = p->grid;
-    if (b.count[0]) k_pr_thread<COMP, LAST><<<grid, PR_THREADS, 0, st>>>(a, b.d_list[0], b.count[0]);
-    if (b.count[1]) k_pr_warp<COMP, LAST><<<grid, PR_THREADS, 0, st>>>(a, b.d_list[1], b.count[1]);
-    if (b.count[2]) {
-        k_pr_hub_chunks<COMP><<<grid, PR_THREADS, 0, st>>>(a, b.d_list[2], b.count[2], p->hub_prefix, p->hub_owner,
-                                                             p->partial);
-        const uint32_t g2 = (uint32_t)((b.count[2] * 32 + PR_THREADS - 1) / PR_THREADS);
-        k_pr_hub_finish<COMP, LAST><<<g2 < grid ? g2 : grid, PR_THREADS, 0, st>>>(a, b.d_list[2], b.count[2],
-                                                                                  p->hub_prefix, p->partial);
+    PrDiag g;
+    pr_hubs<COMP, LAST>(a, g);  // the longest work items first
+    pr_rows<PR_LONG, true, COMP, LAST>(a, a.list[2], a.n[2], g);
+    pr_rows<PR_GROUP, false, COMP, LAST>(a, a.list[1], a.n[1], g);
+    pr_rows<PR_SHORT, false, COMP, LAST>(a, a.list[0], a.n[0], g);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // the vertices without in-edges: a.ratio each
+        const double x = (double)a.ratio;
+        g.m += (double)a.empty * x;
+        g.d += (double)a.empty_dangling * x;
+        if (a.first) g.r += (double)a.empty * fabs(x - (double)a.x0);
     }
-    PR_CUDA(cudaGetLastError());
-    return IPG_OK;
+    pr_block_diag(g.m, g.d, g.r, a.diag);
 }
 
 // Grid-stride kernels get exactly the CTAs that are resident at once: more
@@ -407,18 +438,10 @@ int pr_min_occupancy()
 {
     int n = PR_CTAS_PER_SM;
     auto low = [&](int k) { n = k < n ? k : n; };
-    low(pr_occupancy(k_pr_init));
-    low(pr_occupancy(k_pr_diag));
-    low(pr_occupancy(k_pr_thread<true, false>));
-    low(pr_occupancy(k_pr_thread<true, true>));
-    low(pr_occupancy(k_pr_thread<false, false>));
-    low(pr_occupancy(k_pr_thread<false, true>));
-    low(pr_occupancy(k_pr_warp<true, false>));
-    low(pr_occupancy(k_pr_warp<true, true>));
-    low(pr_occupancy(k_pr_warp<false, false>));
-    low(pr_occupancy(k_pr_warp<false, true>));
-    low(pr_occupancy(k_pr_hub_chunks<true>));
-    low(pr_occupancy(k_pr_hub_chunks<false>));
+    low(pr_occupancy(k_pr_step<true, false>));
+    low(pr_occupancy(k_pr_step<true, true>));
+    low(pr_occupancy(k_pr_step<false, false>));
+    low(pr_occupancy(k_pr_step<false, true>));
     return n;
 }
 
@@ -503,55 +526,69 @@ extern "C" int ipg_pr_plan_create(ipg_graph* g, ipg_pr_plan** out)
                 break;
             }
         }
-        // classes over the gather lists (builds the in-lists of a directed graph)
-        if ((r = ipg_graph_bins(gw, 1, t0, t1, &p->bins)) != IPG_OK) break;
         if ((r = ipg_graph_view_get(gw, &p->gv)) != IPG_OK) break;
         p->grid = (uint32_t)p->sms * (uint32_t)pr_min_occupancy();
-        const uint64_t V = p->gv.V, nh = p->bins.count[2];
+        p->grid_flat = (uint32_t)p->sms * (uint32_t)pr_occupancy(k_pr_init);
+        // hub chunks: at most PR_CHUNK edges, fewer on a small graph so that
+        // every resident warp gets several (a quarter of its share); rows
+        // above a chunk (or t1) are hubs
+        const uint64_t share = p->gv.E / ((uint64_t)p->grid * (PR_THREADS / 32) * 4);
+        p->chunk = 256;
+        while (p->chunk < PR_CHUNK && p->chunk * 2 <= share) p->chunk *= 2;
+        p->hub_min = t1 < p->chunk ? t1 : p->chunk;
+        const uint64_t ts = t0 < p->hub_min ? t0 : p->hub_min;
+        const uint64_t mid = PR_MID < p->hub_min ? PR_MID : p->hub_min;
+        // classes over the gather lists (builds the in-lists of a directed graph)
+        if ((r = ipg_graph_bins(gw, 1, ts, mid > ts ? mid : ts, &p->bins)) != IPG_OK) break;
+        if ((r = ipg_graph_hubs(gw, 1, p->hub_min, p->chunk, &p->hubs)) != IPG_OK) break;
+        if ((r = ipg_graph_view_get(gw, &p->gv)) != IPG_OK) break;
+        const uint64_t V = p->gv.V;
         if ((r = pr_alloc(p, &p->b[0], V)) != IPG_OK) break;
         if ((r = pr_alloc(p, &p->b[1], V)) != IPG_OK) break;
         if ((r = pr_alloc(p, &p->xs, V)) != IPG_OK) break;
         if (p->new_of_old && (r = pr_alloc(p, &p->xs2, V)) != IPG_OK) break;
-        if ((r = pr_alloc(p, &p->hub_prefix, nh + 1)) != IPG_OK) break;
-        std::vector<uint32_t> cnt(nh + 1, 0);
-        if (nh) {
-            k_pr_hub_chunk_counts<<<(uint32_t)((nh + 255) / 256), 256>>>(p->bins.d_list[2], nh, p->gv.d_in_row,
-                                                                       p->hub_prefix);
-            cudaError_t e = cudaMemcpy(cnt.data(), p->hub_prefix, nh * 4, cudaMemcpyDeviceToHost);
-            if (e != cudaSuccess) {
-                r = ipg_internal_fail(IPG_ECUDA, cudaGetErrorString(e));
-                break;
-            }
-        }
-        uint64_t total = 0;
-        for (uint64_t i = 0; i < nh; i++) {
-            const uint32_t c = cnt[i];
-            cnt[i] = (uint32_t)total;
-            total += c;
-        }
-        cnt[nh] = (uint32_t)total;
-        if (total >= (1ULL << 32)) {
-            r = ipg_internal_fail(IPG_EINVAL, "ipg_pr_plan_create: too many hub chunks");
-            break;
-        }
-        p->chunks = total;
-        cudaError_t e = cudaMemcpy(p->hub_prefix, cnt.data(), (nh + 1) * 4, cudaMemcpyHostToDevice);
+        if ((r = pr_alloc(p, &p->partial, p->hubs.chunks)) != IPG_OK) break;
+        if ((r = pr_alloc(p, &p->arrived, p->hubs.hubs)) != IPG_OK) break;
+        cudaError_t e = cudaMemset(p->arrived, 0, (p->hubs.hubs ? p->hubs.hubs : 1) * 4);
         if (e != cudaSuccess) {
             r = ipg_internal_fail(IPG_ECUDA, cudaGetErrorString(e));
             break;
         }
-        if ((r = pr_alloc(p, &p->partial, total)) != IPG_OK) break;
-        std::vector<uint32_t> owner(total);
-        for (uint64_t i = 0; i < nh; i++)
-            for (uint32_t ch = cnt[i]; ch < cnt[i + 1]; ch++) owner[ch] = (uint32_t)i;
-        if ((r = pr_alloc(p, &p->hub_owner, total + 1)) != IPG_OK) break;
-        if (total) {
-            e = cudaMemcpy(p->hub_owner, owner.data(), total * 4, cudaMemcpyHostToDevice);
+        // the short class, vertices without in-edges behind the others
+        const uint64_t ns = p->bins.count[0];
+        if ((r = pr_alloc(p, &p->shorts, ns)) != IPG_OK) break;
+        if (ns) {
+            const PrHasEdges has{p->gv.d_in_row};
+            size_t tb = 0;
+            void* temp = nullptr;
+            e = cub::DevicePartition::If(nullptr, tb, p->bins.d_list[0], p->shorts, (uint32_t*)nullptr, (int64_t)ns, has);
+            const uint64_t bytes = ((uint64_t)tb + 15) / 16 * 16 + 16;
+            if (e == cudaSuccess && (r = ipg_dev_alloc(&temp, bytes)) != IPG_OK) break;
+            unsigned long long* cnt = (unsigned long long*)((char*)temp + bytes - 16);  // {with in-edges, dangling}
+            unsigned long long h[2] = {0, 0};
+            if (e == cudaSuccess) e = cudaMemset(cnt, 0, 16);
+            if (e == cudaSuccess)
+                e = cub::DevicePartition::If(temp, tb, p->bins.d_list[0], p->shorts, (uint32_t*)cnt, (int64_t)ns, has);
+            if (e == cudaSuccess) e = cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
+            if (e == cudaSuccess && h[0] < ns) {
+                k_pr_count_dangling<<<p->grid_flat, PR_THREADS>>>(p->shorts + h[0], ns - h[0], p->gv.d_row, cnt + 1);
+                e = cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
+            }
+            ipg_dev_free(temp, bytes);
             if (e != cudaSuccess) {
                 r = ipg_internal_fail(IPG_ECUDA, cudaGetErrorString(e));
                 break;
             }
+            p->empty = ns - h[0];
+            p->empty_dangling = h[1];
         }
+        // the classes as the plan's user knows them: thread, lanes, hubs
+        p->class_count[0] = p->bins.count[0];
+        p->class_edges[0] = p->bins.edges[0];
+        p->class_count[2] = p->hubs.hubs;
+        p->class_edges[2] = p->hubs.edges;
+        p->class_count[1] = p->bins.count[1] + p->bins.count[2] - p->hubs.hubs;
+        p->class_edges[1] = p->bins.edges[1] + p->bins.edges[2] - p->hubs.edges;
     } while (0);
     if (r != IPG_OK) {
         ipg_pr_plan_free(p);
@@ -581,6 +618,22 @@ extern "C" int ipg_pr_run_f32(ipg_pr_plan* p, uint32_t rounds, double damping, i
     a.row = p->gv.d_row;
     a.in_row = p->gv.d_in_row;
     a.in_adj = (const uint32_t*)p->gv.d_in_adj;
+    a.quads = ((uintptr_t)a.in_adj & 15) == 0 && p->hubs.ids_readable >= 4 && (p->hubs.ids_readable & 3) == 0;
+    for (int k = 0; k < 3; k++) {
+        a.list[k] = p->bins.d_list[k];
+        a.n[k] = p->bins.count[k];
+    }
+    a.list[0] = p->shorts;
+    a.n[0] -= p->empty;
+    a.empty = p->empty;
+    a.empty_dangling = p->empty_dangling;
+    a.hub = (const uint4*)p->hubs.d_hub;
+    a.owner = p->hubs.d_owner;
+    a.partial = p->partial;
+    a.arrived = p->arrived;
+    a.chunks = p->hubs.chunks;
+    a.chunk = p->chunk;
+    a.hub_min = p->hub_min;
     // superstep s writes its values to xbuf(s), so that the last one lands in
     // d_values (on the renamed copy: in xs2, gathered into d_values at the end)
     float* last = p->new_of_old ? p->xs2 : d_values;
@@ -590,23 +643,28 @@ extern "C" int ipg_pr_run_f32(ipg_pr_plan* p, uint32_t rounds, double damping, i
     a.b_cur = nullptr;
     a.b_next = p->b[0];
     a.x_out = xbuf(0);
-    k_pr_init<<<p->grid, PR_THREADS, 0, st>>>(a, V, (float)(1.0 / (double)V));  // pagerank.c:99
-    k_pr_diag<<<p->grid, PR_THREADS, 0, st>>>(a.x_out, nullptr, a.row, V, d_diag);
+    a.x_prev = nullptr;
+    a.diag = d_diag;
+    a.x0 = (float)(1.0 / (double)V);  // pagerank.c:99
+    k_pr_init<<<p->grid_flat, PR_THREADS, 0, st>>>(a, V, a.x0);
     PR_CUDA(cudaGetLastError());
     for (uint32_t s = 1; s <= rounds; s++) {
         a.b_cur = p->b[(s - 1) & 1];
         a.b_next = p->b[s & 1];
+        a.x_prev = xbuf(s - 1);
         a.x_out = xbuf(s);
+        a.diag = d_diag + (uint64_t)s * 3;
+        a.first = s == 1;
+        if (s <= 2 && a.empty) k_pr_empty<<<p->grid_flat, PR_THREADS, 0, st>>>(a, p->shorts + a.n[0]);
         const bool last = s == rounds;
-        int r;
-        if (compensated) r = last ? pr_superstep<true, true>(p, a, st) : pr_superstep<true, false>(p, a, st);
-        else r = last ? pr_superstep<false, true>(p, a, st) : pr_superstep<false, false>(p, a, st);
-        PR_TRY(r);
-        k_pr_diag<<<p->grid, PR_THREADS, 0, st>>>(a.x_out, xbuf(s - 1), a.row, V, d_diag + (uint64_t)s * 3);
+        if (compensated && last) k_pr_step<true, true><<<p->grid, PR_THREADS, 0, st>>>(a);
+        else if (compensated) k_pr_step<true, false><<<p->grid, PR_THREADS, 0, st>>>(a);
+        else if (last) k_pr_step<false, true><<<p->grid, PR_THREADS, 0, st>>>(a);
+        else k_pr_step<false, false><<<p->grid, PR_THREADS, 0, st>>>(a);
         PR_CUDA(cudaGetLastError());
     }
     if (p->new_of_old) {
-        k_pr_by_id<<<p->grid, PR_THREADS, 0, st>>>(last, p->new_of_old, V, d_values);
+        k_pr_by_id<<<p->grid_flat, PR_THREADS, 0, st>>>(last, p->new_of_old, V, d_values);
         PR_CUDA(cudaGetLastError());
     }
     return IPG_OK;
@@ -617,10 +675,10 @@ extern "C" int ipg_pr_plan_info(const ipg_pr_plan* p, uint64_t* class_counts, ui
 {
     if (!p) return ipg_internal_fail(IPG_EINVAL, "ipg_pr_plan_info: null plan");
     for (int k = 0; k < 3; k++) {
-        if (class_counts) class_counts[k] = p->bins.count[k];
-        if (class_edges) class_edges[k] = p->bins.edges[k];
+        if (class_counts) class_counts[k] = p->class_count[k];
+        if (class_edges) class_edges[k] = p->class_edges[k];
     }
-    if (hub_chunks) *hub_chunks = p->chunks;
+    if (hub_chunks) *hub_chunks = p->hubs.chunks;
     return IPG_OK;
 }
 

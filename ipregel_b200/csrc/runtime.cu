@@ -289,6 +289,10 @@ struct ipg_graph {
     }
 };
 
+// Ids of an array of E edges the runtime allocates: whole groups of four, so
+// that 128-bit loads of aligned groups stay inside.
+static uint64_t padded_ids(uint64_t E) { return E ? (E + 3) & ~3ULL : 4; }
+
 static uint32_t grid_for(uint64_t n, int threads, int per_sm = 8)
 {
     uint64_t blocks = (n + threads - 1) / threads;
@@ -633,8 +637,8 @@ extern "C" int ipg_graph_build_in(ipg_graph* g)
     cudaStream_t st = 0;
     IPG_TRY(ipg_dev_alloc(&g->in_row, (V + 1) * 8));
     g->in_row_bytes = (V + 1) * 8;
-    IPG_TRY(ipg_dev_alloc(&g->in_adj, (E ? E : 1) * (uint64_t)g->v.id_bytes));
-    g->in_adj_bytes = (E ? E : 1) * (uint64_t)g->v.id_bytes;
+    IPG_TRY(ipg_dev_alloc(&g->in_adj, padded_ids(E) * (uint64_t)g->v.id_bytes));
+    g->in_adj_bytes = padded_ids(E) * (uint64_t)g->v.id_bytes;
     if (g->v.d_wgt) {
         IPG_TRY(ipg_dev_alloc(&g->in_wgt, (E ? E : 1) * (uint64_t)g->v.weight_bytes));
         g->in_wgt_bytes = (E ? E : 1) * (uint64_t)g->v.weight_bytes;
@@ -687,7 +691,7 @@ extern "C" int ipg_graph_build_in(ipg_graph* g)
 static int alloc_out(ipg_graph* g, uint64_t V, uint64_t E, int id_bytes, int weight_bytes)
 {
     g->row_bytes = (V + 1) * 8;
-    g->adj_bytes = (E ? E : 1) * (uint64_t)id_bytes;
+    g->adj_bytes = padded_ids(E) * (uint64_t)id_bytes;
     IPG_TRY(ipg_dev_alloc(&g->row, g->row_bytes));
     IPG_TRY(ipg_dev_alloc(&g->adj, g->adj_bytes));
     if (weight_bytes) {
@@ -853,7 +857,7 @@ extern "C" int ipg_graph_degree_order(ipg_graph* g, int need_in, ipg_order* out)
     if (with_in && !in_alias && !o->in_row) {
         int r = IPG_OK;
         o->in_row_bytes = (V + 1) * 8;
-        o->in_adj_bytes = (E ? E : 1) * (uint64_t)g->v.id_bytes;
+        o->in_adj_bytes = padded_ids(E) * (uint64_t)g->v.id_bytes;
         r = ipg_dev_alloc(&o->in_row, o->in_row_bytes);
         if (r == IPG_OK) r = ipg_dev_alloc(&o->in_adj, o->in_adj_bytes);
         if (r == IPG_OK && g->v.d_in_wgt) {
@@ -1915,7 +1919,8 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
 // Hub rows cut into chunks (cached per direction).
 // ---------------------------------------------------------------------------
 __global__ void k_hub_chunks(const uint64_t* __restrict__ row, uint64_t V, uint64_t hub_min, uint64_t chunk,
-                             uint4* __restrict__ hub, uint32_t* __restrict__ owner, uint32_t* __restrict__ cnt)
+                             uint4* __restrict__ hub, uint32_t* __restrict__ owner, uint32_t* __restrict__ cnt,
+                             unsigned long long* __restrict__ edges)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t d = row[i + 1] - row[i];
@@ -1923,6 +1928,7 @@ __global__ void k_hub_chunks(const uint64_t* __restrict__ row, uint64_t V, uint6
             const uint32_t n = (uint32_t)((d + chunk - 1) / chunk);
             const uint32_t h = atomicAdd(&cnt[0], 1u), c0 = atomicAdd(&cnt[1], n);
             hub[h] = make_uint4((uint32_t)i, c0, n, 0u);
+            atomicAdd(edges, (unsigned long long)d);
             for (uint32_t k = 0; k < n; k++) owner[c0 + k] = h;
         }
     }
@@ -1951,17 +1957,26 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     uint4* hub = (uint4*)c.mem;
     uint32_t* owner = (uint32_t*)((char*)c.mem + hub_b);
     uint32_t* cnt = (uint32_t*)((char*)c.mem + hub_b + own_b);
-    uint32_t h[2] = {0, 0};
+    struct {
+        uint32_t hubs, chunks;
+        unsigned long long edges;
+    } h = {0, 0, 0};
     if (V) {
-        IPG_CUDA(cudaMemsetAsync(cnt, 0, 8, 0));
-        k_hub_chunks<<<grid_for(V, 256), 256>>>(use_in ? g->v.d_in_row : g->v.d_row, V, hub_min, chunk, hub, owner, cnt);
+        IPG_CUDA(cudaMemsetAsync(cnt, 0, sizeof h, 0));
+        k_hub_chunks<<<grid_for(V, 256), 256>>>(use_in ? g->v.d_in_row : g->v.d_row, V, hub_min, chunk, hub, owner, cnt,
+                                                (unsigned long long*)(cnt + 2));
         IPG_CUDA(cudaGetLastError());
-        IPG_CUDA(cudaMemcpy(h, cnt, 8, cudaMemcpyDeviceToHost));
+        IPG_CUDA(cudaMemcpy(&h, cnt, sizeof h, cudaMemcpyDeviceToHost));
     }
     c.hubs.d_hub = (const uint32_t*)hub;
-    c.hubs.hubs = h[0];
+    c.hubs.hubs = h.hubs;
+    c.hubs.edges = h.edges;
     c.hubs.d_owner = owner;
-    c.hubs.chunks = h[1];
+    c.hubs.chunks = h.chunks;
+    // a list array the runtime allocated is padded; a caller's ends at E
+    const void* ids = use_in ? g->v.d_in_adj : g->v.d_adj;
+    const bool own = (ids == g->adj && g->owns_out) || (ids == g->in_adj && ids);
+    c.hubs.ids_readable = own ? padded_ids(E) : E;
     c.hub_min = hub_min;
     c.chunk = chunk;
     c.valid = true;

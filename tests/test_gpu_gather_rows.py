@@ -27,6 +27,30 @@ def _graph(tail):
 
 
 @pytest.mark.parametrize("tail", [0, 1, 2, 3])
+@pytest.mark.parametrize("rounds", [1, 2, 3, 10])
+@pytest.mark.parametrize("directed", [False, True])
+def test_f32_rows_of_every_length(directed, rounds, tail):
+    """PageRank's precision split over the same rows; supersteps 1 and 2 write the vertices without in-edges.
+    Tolerances: a few FP32 roundings a superstep against FP64 (as the split's other tests), and the FP64 diagnostics
+    against sums of the returned values."""
+    import ipregel_b200 as ip
+    g = _graph(tail)
+    want, _, _ = O.run(g, "pagerank", "single_broadcast", rounds=rounds, directed=directed)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, g.adj, directed=directed)
+    pr = ip.PageRankF32(graph)
+    try:
+        x, diag = pr.run(rounds=rounds)
+        prev, _ = pr.run(rounds=rounds - 1)
+    finally:
+        pr.free()
+        graph.free()
+    assert np.max(np.abs(x - want) / want) <= 1e-5
+    x, prev = x.astype(np.float64), prev.astype(np.float64)
+    deg = np.diff(g.idx.astype(np.int64), append=g.E)
+    np.testing.assert_allclose(diag[-1], [x.sum(), x[deg == 0].sum(), np.abs(x - prev).sum()], rtol=1e-12)
+
+
+@pytest.mark.parametrize("tail", [0, 1, 2, 3])
 @pytest.mark.parametrize("app,version,id_bits,variant", [
     ("pagerank", "single_broadcast", 32, ""), ("pagerank", "single_broadcast", 32, "staged"),
     ("cc", "single_broadcast", 32, ""), ("cc", "single_broadcast", 64, "")])
