@@ -669,7 +669,10 @@ def stored_traffic(name, bytes_per_launch):
 
 
 NCU_KERNEL_NAMES = (("ipx_k_push<0>", "push_thread"), ("ipx_k_push<1>", "push_warp"), ("ipx_k_push<2>", "push_block"),
-                    ("ipx_k_compute_spread", "compute"))
+                    ("ipx_k_compute_spread", "compute"), ("ipx_k_front", "compute"), ("ipx_k_push(", "push"),
+                    ("ipx_k_count(", "count_active"))
+# a superstep's first launch
+NCU_SUPERSTEP_OPENERS = ("ipx_k_begin_superstep", "ipx_k_front")
 
 
 def write_traffic(csv_path, line_path, out_path=TRAFFIC_PATH):
@@ -678,7 +681,7 @@ def write_traffic(csv_path, line_path, out_path=TRAFFIC_PATH):
     of `bench.py --steps 1 --warmup 1 --no-e2e --no-cpu-baseline --no-extra
     --no-parity` and the JSON line of the same command run without ncu (its
     `kernels` give the algorithmic bytes).  The profiled step runs CC, then
-    SSSP, each superstep opening with ipx_k_begin_superstep; k_compact
+    SSSP, each superstep opening with one of NCU_SUPERSTEP_OPENERS; k_compact
     launches alternate broadcasters / next frontier within a superstep."""
     import csv
     line = json.loads(open(line_path).read().strip().splitlines()[-1])
@@ -689,8 +692,8 @@ def write_traffic(csv_path, line_path, out_path=TRAFFIC_PATH):
         launches.setdefault(r["ID"], {"name": r["Kernel Name"]})[r["Metric Name"]] = float(r["Metric Value"].replace(",", ""))
     order = [launches[k] for k in sorted(launches, key=int)]
     # the profiled step: the last 2 runs' host-loop launches, from the first
-    # begin_superstep of its CC run
-    begins = [i for i, x in enumerate(order) if x["name"].startswith("ipx_k_begin_superstep")]
+    # superstep of its CC run
+    begins = [i for i, x in enumerate(order) if x["name"].startswith(NCU_SUPERSTEP_OPENERS)]
     steps_sp = line["kernels"]["sssp:compute"]["launches"]
     begins = begins[-(steps_cc + steps_sp):]
     dram, seen = {}, {}

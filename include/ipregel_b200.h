@@ -237,11 +237,14 @@ typedef struct ipg_hubs {
     const uint32_t* d_owner;
     uint64_t chunks;
     uint64_t edges;          /* of all hubs */
-    uint64_t ids_readable;   /* ids of the list array that may be read: E, or E
-                              * rounded up to a multiple of 4 */
 } ipg_hubs;
 int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64_t chunk,
                    ipg_hubs* hubs);
+
+/* *quads = 1 when the rows' (or in-lists') 32-bit ids, and 4-byte weights if
+ * there are any, can be read in aligned groups of four up to the group that
+ * holds the last one: always for arrays the runtime allocated. */
+int ipg_graph_quads(const ipg_graph* g, int use_in, int* quads);
 
 /* The same degree classes without allocating anything -- no counterpart in
  * the reference.  Meant for callers that must not call cudaMalloc: code

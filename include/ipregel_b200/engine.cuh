@@ -86,12 +86,18 @@ static_assert(sizeof(ipx_msg) <= 8, "iPregel-B200: IP_MESSAGE_TYPE must be at mo
 #ifndef IPX_EDGE_CTAS
 #define IPX_EDGE_CTAS 6
 #endif
+/* CTA of the target marking kernel: one per SM, its shared memory the bits
+ * of the most often visited targets. */
+#define IPX_MARK_THREADS 1024
+#define IPX_MARK_WORDS 40960 /* most of them: 160 KiB */
 #define IPX_ERR_SEND_IN_BROADCAST 1u
 #define IPX_ERR_COMBINE_HINT 2u
 #define IPX_ERR_SUPERSTEP_LIMIT 4u
 #define IPX_ERR_COPY_TIMEOUT 8u
 #define IPX_ERR_RESERVED_MESSAGE 16u
 #define IPX_HIST 65536
+/* Supersteps the host-driven loop enqueues before it waits for the device. */
+#define IPX_BATCH 8
 
 /* Default degree-class thresholds for the thread / warp / block kernels
  * (runtime tuning parameters). */
@@ -107,7 +113,10 @@ static_assert(sizeof(ipx_msg) <= 8, "iPregel-B200: IP_MESSAGE_TYPE must be at mo
 /* deliver() returns true when the received bit of w may still be clear      */
 /* (the CAS policies know exactly: this call filled an empty mailbox; the    */
 /* hardware-atomic ones return true whenever they issued an update), and the */
-/* caller then sets the bit with a fire-and-forget atomic OR.                */
+/* caller then sets the bit with a fire-and-forget atomic OR.  Policies with */
+/* kPeek let a push look at the slot first: a message that does not win is   */
+/* dropped, and only a push that saw the slot empty sets the bit (the first  */
+/* to deliver in a superstep always does).                                   */
 /* ------------------------------------------------------------------------ */
 template <class T>
 struct ipx_word {
@@ -260,17 +269,11 @@ struct ipx_mailbox;
  * (V x 4 bytes per parity), which then stay in L2 at larger scales. */
 struct ipx_mailbox_min {
     typedef ipx_msg slot;
+    static constexpr bool kPeek = true;
     __device__ static slot empty() { return std::numeric_limits<ipx_msg>::max(); }
-    __device__ static bool precheck(slot* s, ipx_msg m)
-    {
-        const ipx_msg c = ipx_peek(s);
-        return m < c || (m == c && c == empty());
-    }
-    __device__ static bool commit(slot* s, ipx_msg m)
-    {
-        ipx_atomic_min(s, m);
-        return true;
-    }
+    __device__ static bool fresh(slot c) { return c == empty(); }
+    __device__ static bool wins(slot c, ipx_msg m) { return m < c || (m == c && fresh(c)); }
+    __device__ static void commit(slot* s, ipx_msg m) { ipx_atomic_min(s, m); }
     __device__ static bool deliver(slot* s, ipx_msg m)
     {
         if (m < __ldcg(s)) ipx_atomic_min(s, m);
@@ -281,27 +284,16 @@ struct ipx_mailbox_min {
         if (m < *s) *s = m;
         return true;
     }
-    __device__ static ipx_msg take(slot* s)
-    {
-        ipx_msg m = *s;
-        *s = empty();
-        return m;
-    }
+    __device__ static ipx_msg message(const slot& c) { return c; }
 };
 
 struct ipx_mailbox_max {
     typedef ipx_msg slot;
+    static constexpr bool kPeek = true;
     __device__ static slot empty() { return std::numeric_limits<ipx_msg>::lowest(); }
-    __device__ static bool precheck(slot* s, ipx_msg m)
-    {
-        const ipx_msg c = ipx_peek(s);
-        return m > c || (m == c && c == empty());
-    }
-    __device__ static bool commit(slot* s, ipx_msg m)
-    {
-        ipx_atomic_max(s, m);
-        return true;
-    }
+    __device__ static bool fresh(slot c) { return c == empty(); }
+    __device__ static bool wins(slot c, ipx_msg m) { return m > c || (m == c && fresh(c)); }
+    __device__ static void commit(slot* s, ipx_msg m) { ipx_atomic_max(s, m); }
     __device__ static bool deliver(slot* s, ipx_msg m)
     {
         if (m > __ldcg(s)) ipx_atomic_max(s, m);
@@ -312,12 +304,7 @@ struct ipx_mailbox_max {
         if (m > *s) *s = m;
         return true;
     }
-    __device__ static ipx_msg take(slot* s)
-    {
-        ipx_msg m = *s;
-        *s = empty();
-        return m;
-    }
+    __device__ static ipx_msg message(const slot& c) { return c; }
 };
 
 template <>
@@ -332,25 +319,19 @@ struct ipx_mailbox<IP_COMBINE_MAX, 8> : ipx_mailbox_max {};
 template <int MSGBYTES>
 struct ipx_mailbox<IP_COMBINE_SUM, MSGBYTES> {
     typedef ipx_msg slot;
+    static constexpr bool kPeek = false;
     __device__ static slot empty() { return (ipx_msg)0; }
-    __device__ static bool precheck(slot*, ipx_msg) { return true; }
     __device__ static bool deliver(slot* s, ipx_msg m)
     {
         ipx_atomic_add(s, m);
         return true;
     }
-    __device__ static bool commit(slot* s, ipx_msg m) { return deliver(s, m); }
     __device__ static bool merge(slot* s, ipx_msg m)
     {
         *s = *s + m;
         return true;
     }
-    __device__ static ipx_msg take(slot* s)
-    {
-        ipx_msg m = *s;
-        *s = (ipx_msg)0;
-        return m;
-    }
+    __device__ static ipx_msg message(const slot& c) { return c; }
 };
 
 /* Generic, up to 4 bytes: {flag, bits} in one 64-bit word, CAS loop around
@@ -359,9 +340,8 @@ struct ipx_mailbox<IP_COMBINE_SUM, MSGBYTES> {
 template <int MSGBYTES>
 struct ipx_mailbox_generic32 {
     typedef unsigned long long slot;
+    static constexpr bool kPeek = false;
     __device__ static slot empty() { return 0ULL; }
-    __device__ static bool precheck(slot*, ipx_msg) { return true; }
-    __device__ static bool commit(slot* s, ipx_msg m) { return deliver(s, m); }
     __device__ static bool deliver(slot* s, ipx_msg m)
     {
         unsigned long long old = __ldcg(s);
@@ -393,12 +373,7 @@ struct ipx_mailbox_generic32 {
         *s = (1ULL << 32) | ipx_to_word(v);
         return true;
     }
-    __device__ static ipx_msg take(slot* s)
-    {
-        unsigned long long w = *s;
-        *s = 0ULL;
-        return ipx_from_word<ipx_msg>((unsigned int)w);
-    }
+    __device__ static ipx_msg message(const slot& c) { return ipx_from_word<ipx_msg>((unsigned int)c); }
 };
 
 template <>
@@ -412,9 +387,8 @@ struct ipx_mailbox<IP_COMBINE_GENERIC, 4> : ipx_mailbox_generic32<4> {};
 template <>
 struct ipx_mailbox<IP_COMBINE_GENERIC, 8> {
     typedef ipx_slot128 slot;
+    static constexpr bool kPeek = false;
     __device__ static slot empty() { return slot{0ULL, 0ULL}; }
-    __device__ static bool precheck(slot*, ipx_msg) { return true; }
-    __device__ static bool commit(slot* s, ipx_msg m) { return deliver(s, m); }
     __device__ static bool deliver(slot* s, ipx_msg m)
     {
         unsigned long long of = __ldcg(&s->flag), ob = __ldcg(&s->bits);
@@ -447,12 +421,7 @@ struct ipx_mailbox<IP_COMBINE_GENERIC, 8> {
         s->flag = 1ULL;
         return true;
     }
-    __device__ static ipx_msg take(slot* s)
-    {
-        slot w = *s;
-        *s = slot{0ULL, 0ULL};
-        return ipx_from_word<ipx_msg>(w.bits);
-    }
+    __device__ static ipx_msg message(const slot& c) { return ipx_from_word<ipx_msg>(c.bits); }
 };
 
 template <>
@@ -600,6 +569,18 @@ __device__ __forceinline__ S ipx_slot_ld(const S* __restrict__ bs, uint64_t w)
 /* ------------------------------------------------------------------------ */
 /* Device-resident engine state, read through the constant bank.            */
 /* ------------------------------------------------------------------------ */
+/* What a superstep's kernels count: zeroed by the superstep's end.  n:
+ * broadcasters listed in the three row classes and the chunks of the hubs;
+ * tn: spread+single_broadcast's targets by class; edges / tedges: the degree
+ * sums (hubs last). */
+struct ipx_stat {
+    unsigned long long count;
+    unsigned long long edges[4];
+    unsigned long long tedges[3];
+    uint32_t n[4];
+    uint32_t tn[4];
+};
+
 struct ipx_consts {
     uint64_t V, E, W;  /* W = bitmap words */
     const uint64_t* row;
@@ -620,22 +601,36 @@ struct ipx_consts {
     ipx_slot* mbox[2];
     uint32_t* recv[2];
     ipx_msg* outbox;
-    uint32_t* bcaster;
+    uint32_t* bcaster; /* pulling push versions only */
     /* pull broadcast slots: single_broadcast alternates bslot[s & 1] (its
      * fused kernel reads superstep s's slots while writing s+1's);
      * spread+single_broadcast uses bslot[0] */
     ipx_bslot* bslot[2];
     ipx_sbslot* sbslot[2];
     uint32_t* bt;
-    /* counters: [0..3] active counts ring, [4] edges, [5] error word */
-    unsigned long long* ctr;
+    /* this superstep's counts, and a copy of the last one's */
+    ipx_stat* stat;
+    ipx_stat* last;
+    /* control words (IPX_CTL_*) */
+    unsigned long long* ctl;
     uint32_t* err;
-    /* direction optimisation (push versions on symmetric graphs) */
+    /* direction optimisation (push versions on symmetric graphs): pull when
+     * the broadcasters' out-edges exceed pull_threshold */
     int pull_ok;
-    /* list sizes ([0..2] broadcaster classes, [4..6] targets) and the
-     * per-superstep history of a captured loop: hist[s % IPX_HIST][0..3] =
-     * active count, edges traversed, direction, unused */
-    uint32_t* lcnt;
+    unsigned long long pull_threshold;
+    /* broadcasters by row length, and the hubs' chunks {vertex, chunk}: rows
+     * up to push_t[0] take a thread, up to push_t[1] 8 lanes, up to push_t[2]
+     * 16 lanes, longer ones a warp per push_chunk edges */
+    uint32_t* blist[3];
+    uint2* bchunk;
+    uint64_t push_t[3];
+    uint32_t push_chunk;
+    /* ids (and 4-byte weights) can be read in whole aligned groups of four */
+    int out_quads, in_quads;
+    /* spread+single_broadcast: targets by in-degree class */
+    uint32_t* tlist[3];
+    /* per superstep a record of hist[s % IPX_HIST]: active count, edges
+     * traversed, direction | error word << 32, nanoseconds */
     unsigned long long* hist;
     /* single_broadcast: the vertices by degree class (short, middle and
      * long rows, the hubs among the long ones; their numbers in class_n),
@@ -655,9 +650,6 @@ struct ipx_consts {
     const uint32_t* hub_owner;
     /* the in-lists with the flag of the most gathered vertices (null: none) */
     const uint32_t* in_adj_hot;
-    /* push / mark: chunk -> index of its hub in this superstep's hub list
-     * (null: found by a binary search over the prefix) */
-    const uint32_t* push_owner;
     /* The kernels run on a degree-ordered copy of the graph: vid_of[v] is
      * the id of vertex v in the caller's numbering, vindex_of its inverse
      * (both null when the graph is not renamed). */
@@ -680,46 +672,34 @@ __device__ __forceinline__ ipx_vid ipx_user_id(uint64_t v)
     return (ipx_vid)(ipx_c.vid_of ? (uint64_t)__ldg(&ipx_c.vid_of[v]) : v);
 }
 
-/* The current superstep, from device memory: the host writes it before each
- * superstep (host loop), or the previous superstep's last kernel advances it
- * (captured loop), so every kernel of a superstep reads the same value. */
+/* The current superstep, from device memory: each superstep's last kernel
+ * advances it, so every kernel of a superstep reads the same value. */
 __device__ __forceinline__ uint64_t ipx_step() { return (uint64_t)__ldg((const unsigned long long*)&ipd_superstep); }
 __device__ __forceinline__ int ipx_parity() { return (int)(ipx_step() & 1); }
 
-/* ctr layout (u64): [0..3] active-count ring, [5] error word (low half),
- * [8..10] degree sums of the broadcaster classes, [11..13] of the target
- * classes, both reset every superstep. */
-#define IPX_NCTR 16
-#define IPX_CTR_ERR 5
-/* [6]: delivery direction of the current superstep (0 push, 1 pull). */
-#define IPX_CTR_MODE 6
+/* Control words: the error word, "the program has ended" (the kernels of
+ * supersteps enqueued beyond it return at once), CTAs of the last kernel
+ * that are done, and the time stamp of the last superstep's end. */
+enum { IPX_CTL_ERR, IPX_CTL_DONE, IPX_CTL_ARRIVED, IPX_CTL_STAMP, IPX_NCTL };
+__device__ __forceinline__ bool ipx_done() { return __ldcg(&ipx_c.ctl[IPX_CTL_DONE]) != 0ULL; }
 
 /* Kernel ids for launch counting and per-kernel profiling. */
 enum {
     IPX_K_COMPUTE,
-    IPX_K_COMPACT_B,
-    IPX_K_PUSH0,
-    IPX_K_PUSH1,
-    IPX_K_PUSH2,
+    IPX_K_PUSH,
     IPX_K_COMPACT_T,
-    IPX_K_GATHER0,
-    IPX_K_GATHER1,
-    IPX_K_GATHER2,
-    IPX_K_MARK0,
-    IPX_K_MARK1,
-    IPX_K_MARK2,
+    IPX_K_GATHER,
+    IPX_K_GATHER_HUBS,
+    IPX_K_MARK,
     IPX_K_COUNT,
     IPX_K_PULLD0,
     IPX_K_PULLD1,
     IPX_K_PULLD2,
-    IPX_K_CTRL,
     IPX_K_N
 };
 static const char* const ipx_kname[IPX_K_N] = {
-    "compute", "compact_broadcasters", "push_thread", "push_warp", "push_block", "compact_targets",
-    "gather_thread", "gather_warp", "gather_block", "mark_thread", "mark_warp", "mark_block", "count_active",
-    "pull_deliver_thread", "pull_deliver_warp", "pull_deliver_block",
-    "superstep_control"};
+    "compute", "push", "compact_targets", "gather", "gather_hubs", "mark", "count_active",
+    "pull_deliver_thread", "pull_deliver_warp", "pull_deliver_block"};
 
 __device__ __forceinline__ uint64_t ipx_gtid() { return blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint64_t ipx_gstride() { return (uint64_t)gridDim.x * blockDim.x; }
@@ -772,13 +752,6 @@ __device__ __forceinline__ void ipx_set_bit_agg(uint32_t* bm, uint64_t v)
     if ((threadIdx.x & 31) == (unsigned)(__ffs(peers) - 1)) atomicOr(&bm[word], bits);
 }
 
-/* Sets bit v if it is clear; returns nothing (idempotent). */
-__device__ __forceinline__ void ipx_mark(uint32_t* bm, uint64_t v)
-{
-    const uint32_t bit = 1u << (v & 31);
-    if (!(__ldcg(&bm[v >> 5]) & bit)) atomicOr(&bm[v >> 5], bit);
-}
-
 /* Warp + block sum into a global counter (all threads of the block call). */
 __device__ __forceinline__ void ipx_block_count(unsigned long long c, unsigned long long* dst)
 {
@@ -793,17 +766,121 @@ __device__ __forceinline__ void ipx_block_count(unsigned long long c, unsigned l
     }
 }
 
+/* The loop the kernels run in: a captured one continues by its condition. */
+struct ipx_loop {
+    cudaGraphConditionalHandle handle;
+    int captured;
+    unsigned long long max_supersteps;
+};
+
+/* True in one CTA, the last of the grid to get here, with every other CTA's
+ * writes visible (all threads of every CTA call it, after their last write). */
+__device__ __forceinline__ bool ipx_last_cta()
+{
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned int n = atomicInc((unsigned int*)&ipx_c.ctl[IPX_CTL_ARRIVED], gridDim.x - 1);
+        s_last = n == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last;
+}
+
+__device__ __forceinline__ unsigned long long ipx_now()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+/* Direction of the superstep's delivery (push versions). */
+__device__ __forceinline__ bool ipx_pulls()
+{
+    if (!ipx_c.pull_ok) return false;
+    unsigned long long m = 0;
+    for (int k = 0; k < 4; k++) m += __ldcg(&ipx_c.stat->edges[k]);
+    return m > ipx_c.pull_threshold;
+}
+
+/* End of a superstep, by one thread after everything else of it: records
+ * the superstep in the history, advances to the next and decides whether
+ * the program goes on: while the count is nonzero (combiner_postamble.h:134;
+ * spread versions test it after superstep 0, combiner_spread_postamble.h:
+ * 212), no kernel reported an error and the superstep bound is not reached. */
+__device__ __forceinline__ void ipx_end_of_superstep(const ipx_loop& loop, unsigned long long count)
+{
+    const uint64_t s = ipx_step();
+    ipx_stat* st = ipx_c.stat;
+    ipx_stat x;
+    x.count = count;
+    unsigned long long edges = 0;
+    for (int k = 0; k < 4; k++) edges += x.edges[k] = __ldcg(&st->edges[k]);
+    bool pulled = false;
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+    edges = ipx_c.E;
+#else
+    pulled = ipx_c.pull_ok && edges > ipx_c.pull_threshold;
+    if (pulled) edges = ipx_c.E; /* a pulled superstep reads every row */
+#endif
+    for (int k = 0; k < 3; k++) edges += x.tedges[k] = __ldcg(&st->tedges[k]);
+    for (int k = 0; k < 4; k++) {
+        x.n[k] = __ldcg(&st->n[k]);
+        x.tn[k] = __ldcg(&st->tn[k]);
+    }
+    *ipx_c.last = x;
+    memset(st, 0, sizeof *st);
+    bool go = count != 0 && __ldcg(ipx_c.err) == 0;
+    if (go && s + 1 >= loop.max_supersteps) {
+        atomicOr(ipx_c.err, IPX_ERR_SUPERSTEP_LIMIT);
+        go = false;
+    }
+    const unsigned long long now = ipx_now(), then = __ldcg(&ipx_c.ctl[IPX_CTL_STAMP]);
+    ipx_c.ctl[IPX_CTL_STAMP] = now;
+    unsigned long long* h = ipx_c.hist + (s % IPX_HIST) * 4;
+    h[0] = count;
+    h[1] = edges;
+    h[2] = (pulled ? 1ULL : 0ULL) | ((unsigned long long)__ldcg(ipx_c.err) << 32);
+    h[3] = now > then ? now - then : 0ULL;
+    ipd_superstep = s + 1;
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+    /* the fused kernel of superstep s + 1 runs the compute phase of s + 2 */
+    ipd_compute_superstep = s + 2;
+#else
+    ipd_compute_superstep = s + 1;
+#endif
+    if (!go) ipx_c.ctl[IPX_CTL_DONE] = 1ULL;
+    if (loop.captured) cudaGraphSetConditional(loop.handle, go ? 1u : 0u);
+}
+
 /* Delivery of one message into mailbox parity p of vertex w. */
 __device__ __forceinline__ void ipx_deliver(int p, uint64_t w, ipx_msg m)
 {
     if (ipx_mb::deliver(&ipx_c.mbox[p][w], m)) atomicOr(&ipx_c.recv[p][w >> 5], 1u << (w & 31));
 }
 
-/* Edges per chunk of a high-degree vertex: the block class is split into
- * chunks that all CTAs share, so one hub does not leave a single CTA working
- * after the others have finished. */
+/* Edges per chunk of a hub's row in the static pull delivery of the push
+ * versions, and at most (fewer on small graphs) in push and mark, where a
+ * warp takes a chunk: one hub does not leave a single warp working after the
+ * others have finished. */
 #ifndef IPX_HUB_CHUNK
 #define IPX_HUB_CHUNK 2048
+#endif
+/* Lanes per row of the middle and the long class of push and mark, and the
+ * longest middle row.  CC / weighted SSSP, undirected R-MAT scale 24, ms of
+ * push a run: 8 and 32 lanes 4.6 / 6.9, 8 and 16 5.0 / 8.0, 16 and 32 4.5 / 6.6
+ * against 4.4 / 6.4 for 8 and 32 with the compute kernel's later lists; middle
+ * rows up to 32 or 128 edges within 2 % of 64. */
+#ifndef IPX_PUSH_GROUP
+#define IPX_PUSH_GROUP 8
+#endif
+#ifndef IPX_PUSH_LONG
+#define IPX_PUSH_LONG 32
+#endif
+#ifndef IPX_PUSH_MID
+#define IPX_PUSH_MID 64
 #endif
 /* 1: the hub class of the fused pull kernel takes a warp per chunk instead
  * of a CTA (no CTA-wide barriers per chunk); 0: a CTA per chunk, its ids
@@ -827,23 +904,6 @@ __device__ __forceinline__ void ipx_deliver(int p, uint64_t w, ipx_msg m)
 #ifndef IPX_UNROLL
 #define IPX_UNROLL 4
 #endif
-/* 1: sources of the thread and warp classes go through the warp-cooperative
- * expansion; 0: a thread per source (degree <= IPX_T0), a warp per source. */
-#ifndef IPX_PUSH_EXPAND
-#define IPX_PUSH_EXPAND 0
-#endif
-/* Lanes per source in the warp class of push and mark (8, 16 or 32).  On
- * the degree-ordered copy of undirected R-MAT scale 24 (most sources of the
- * class have a few dozen out-edges), CC + SSSP ran at 63.7 - 63.9 GTEPS with
- * 16, 62.0 with 8 and 61.5 - 61.6 with 32. */
-#ifndef IPX_PUSH_GROUP
-#define IPX_PUSH_GROUP 16
-#endif
-/* Lanes per source in the thread class of push and mark (1, 2, 4 or 8). */
-#ifndef IPX_PUSH_Q
-#define IPX_PUSH_Q 1
-#endif
-
 template <class T>
 __device__ __forceinline__ T ipx_shfl_idx(T x, int src)
 {
@@ -853,222 +913,260 @@ __device__ __forceinline__ T ipx_shfl_idx(T x, int src)
     return ipx_from_word<T>(w);
 }
 
-/* A visitor gets batches of U edges: edge index e[k], target w[k], the
- * source's message m[k] (outbox value) and ok[k] (lane holds an edge). */
+/* ------------------------------------------------------------------------ */
+/* Row walks: G lanes per row, each lane four consecutive edges per step.    */
+/* ------------------------------------------------------------------------ */
 
-/* Push visitor: prechecks a batch of mailboxes first, then commits. */
+/* Edges of a row; no row but a hub's comes near the limit. */
+__device__ __forceinline__ uint32_t ipx_row_edges(uint64_t r0, uint64_t r1)
+{
+    return r1 - r0 < 0x7fffffffull ? (uint32_t)(r1 - r0) : 0x7fffffffu;
+}
+
+/* The aligned four words at position rel (a multiple of 4) from row start r0
+ * rounded down to one: which of them belong to the row of deg edges is
+ * decided when they are used, so that nothing waits for the load before. */
+__device__ __forceinline__ uint4 ipx_ld_quad(const uint32_t* __restrict__ a, uint64_t r0, uint32_t deg, uint32_t rel)
+{
+    const uint32_t off = (uint32_t)r0 & 3u;
+    return __ldcs(reinterpret_cast<const uint4*>(a + (rel < off + deg ? r0 - off + rel : 0)));
+}
+
+/* A visitor gets up to four edges at once: edge index e + k, target w[k],
+ * ok[k] (the lane holds an edge), the source's message m. */
+
+/* Push: looks at four mailboxes before committing to any. */
 struct ipx_push_visit {
     static constexpr bool kNeedsMessage = true;
     int p;
-    bool warp_wide; /* a warp or CTA walks each source's edges (weights loaded evict-first) */
-    template <int U>
-    __device__ __forceinline__ void batch(const uint64_t* e, const ipx_vid* w, const ipx_msg* m, const bool* ok) const
+    template <class MB = ipx_mb>
+    __device__ __forceinline__ void deliver(const ipx_vid* w, const bool* ok, const ipx_msg* mk) const
     {
-        ipx_msg mk[U];
-        bool go[U];
+        ipx_slot* __restrict__ box = ipx_c.mbox[p];
+        if constexpr (MB::kPeek) {
+            ipx_slot c[4];
 #pragma unroll
-        for (int k = 0; k < U; k++) {
-            go[k] = false;
-            if (ok[k]) {
-#if IPX_EDGE_MSG
-                mk[k] = IP_BROADCAST_EDGE_MESSAGE(m[k], warp_wide ? ipx_ld_stream(&ipx_c.wgt[e[k]]) : ipx_c.wgt[e[k]]);
-#else
-                mk[k] = m[k];
-#endif
-                go[k] = ipx_mb::precheck(&ipx_c.mbox[p][(uint64_t)w[k]], mk[k]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            const uint64_t t = (uint64_t)w[k];
-            if (go[k] && ipx_mb::commit(&ipx_c.mbox[p][t], mk[k])) atomicOr(&ipx_c.recv[p][t >> 5], 1u << (t & 31));
-        }
-    }
-    /* Four consecutive edges e0 .. e0+3 (e0 a multiple of 4) whose ids one
-     * 128-bit load gave; 4-byte weights come the same way. */
-    __device__ __forceinline__ void batch_v4(uint64_t e0, const uint4& id, const ipx_msg& m) const
-    {
-        const uint32_t w[4] = {id.x, id.y, id.z, id.w};
-        ipx_msg mk[4];
-#if IPX_EDGE_MSG
-        if constexpr (sizeof(ipx_wgt) == 4) {
-            const uint4 ww = __ldcs(reinterpret_cast<const uint4*>(ipx_c.wgt + e0));
-            const uint32_t wk[4] = {ww.x, ww.y, ww.z, ww.w};
+            for (int k = 0; k < 4; k++) c[k] = ok[k] ? ipx_peek(&box[(uint64_t)w[k]]) : MB::empty();
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                ipx_wgt x;
-                memcpy(&x, &wk[k], 4);
-                mk[k] = IP_BROADCAST_EDGE_MESSAGE(m, x);
+                if (ok[k] && MB::wins(c[k], mk[k])) {
+                    const uint64_t t = (uint64_t)w[k];
+                    MB::commit(&box[t], mk[k]);
+                    if (MB::fresh(c[k])) atomicOr(&ipx_c.recv[p][t >> 5], 1u << (t & 31));
+                }
             }
         } else {
 #pragma unroll
-            for (int k = 0; k < 4; k++) mk[k] = IP_BROADCAST_EDGE_MESSAGE(m, ipx_ld_stream(&ipx_c.wgt[e0 + k]));
-        }
-#else
-        (void)e0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) mk[k] = m;
-#endif
-        bool go[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) go[k] = ipx_mb::precheck(&ipx_c.mbox[p][w[k]], mk[k]);
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (go[k] && ipx_mb::commit(&ipx_c.mbox[p][w[k]], mk[k])) atomicOr(&ipx_c.recv[p][w[k] >> 5], 1u << (w[k] & 31));
-    }
-};
-
-/* Target-marking visitor (spread+single_broadcast). */
-struct ipx_mark_visit {
-    static constexpr bool kNeedsMessage = false;
-    template <int U>
-    __device__ __forceinline__ void batch(const uint64_t* e, const ipx_vid* w, const ipx_msg* m, const bool* ok) const
-    {
-        (void)e;
-        (void)m;
-        uint32_t cur[U];
-#pragma unroll
-        for (int k = 0; k < U; k++) cur[k] = ok[k] ? __ldcg(&ipx_c.bt[(uint64_t)w[k] >> 5]) : IPX_FULL;
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            const uint32_t bit = 1u << ((uint64_t)w[k] & 31);
-            if (!(cur[k] & bit)) atomicOr(&ipx_c.bt[(uint64_t)w[k] >> 5], bit);
+            for (int k = 0; k < 4; k++) {
+                const uint64_t t = (uint64_t)w[k];
+                if (ok[k] && MB::deliver(&box[t], mk[k])) atomicOr(&ipx_c.recv[p][t >> 5], 1u << (t & 31));
+            }
         }
     }
-    __device__ __forceinline__ void batch_v4(uint64_t e0, const uint4& id, const ipx_msg& m) const
+    /* Weighted broadcasts take the quad's weights the way its ids came. */
+    __device__ __forceinline__ void unpack(const uint4& q, uint64_t r0, uint32_t deg, uint32_t rel, const ipx_msg& m,
+                                           ipx_vid* w, bool* ok, ipx_msg* mk) const
     {
-        const uint64_t e[4] = {e0, e0 + 1, e0 + 2, e0 + 3};
-        const ipx_vid w[4] = {(ipx_vid)id.x, (ipx_vid)id.y, (ipx_vid)id.z, (ipx_vid)id.w};
-        const ipx_msg mk[4] = {m, m, m, m};
-        const bool ok[4] = {true, true, true, true};
-        batch<4>(e, w, mk, ok);
-    }
-};
-
-/* Edges [e0, e1) of one source visited by a warp or block (lanes >= 32)
- * with 32-bit ids: the ids of four consecutive edges per lane come from one
- * 128-bit load (the weights too, when the visitor needs 4-byte weights),
- * the up to 3 edges before the first 16-byte boundary and after the last one
- * take a lane each. */
-template <class Visit>
-__device__ __forceinline__ void ipx_edges_v4(const uint32_t* __restrict__ adj, uint64_t e0, uint64_t e1,
-                                             uint64_t lane, uint64_t lanes, ipx_msg m, const Visit& visit)
-{
-    uint64_t a = (e0 + 3) & ~3ULL;
-    if (a > e1) a = e1;
-    const uint64_t b = a + ((e1 - a) & ~3ULL);
-    {
-        const uint64_t nh = a - e0, nt = e1 - b;
-        uint64_t e = e1;
-        if (lane < nh) e = e0 + lane;
-        else if (lane < nh + nt) e = b + (lane - nh);
-        const uint64_t ek[1] = {e};
-        const bool ok[1] = {e < e1};
-        const ipx_vid w[1] = {ok[0] ? (ipx_vid)ipx_ld_stream(&adj[e]) : (ipx_vid)0};
-        const ipx_msg mk[1] = {m};
-        visit.template batch<1>(ek, w, mk, ok);
-    }
-    const uint4* __restrict__ q = reinterpret_cast<const uint4*>(adj + a);
-    const uint64_t groups = (b - a) >> 2;
-    for (uint64_t g = lane; g < groups; g += lanes) visit.batch_v4(a + 4 * g, __ldcs(q + g), m);
-}
-
-/* The 128-bit path needs 16-byte aligned id and weight arrays (always so for
- * arrays the runtime allocates; a caller's array may not be). */
-__device__ __forceinline__ bool ipx_v4_ok(const void* adj)
-{
-    if constexpr (sizeof(ipx_vid) != 4) return false;
-    if ((reinterpret_cast<uintptr_t>(adj) & 15) != 0) return false;
-#if IPX_EDGE_MSG
-    if ((reinterpret_cast<uintptr_t>(ipx_c.wgt) & 15) != 0) return false;
-#endif
-    return true;
-}
-
-/* Visits edges [e0, e1) of one source lane-strided, IPX_UNROLL edges a lane
- * at a time, loading the ids of a batch before visiting any of it (warps and
- * blocks over 32-bit ids: ipx_edges_v4). */
-template <class Visit>
-__device__ __forceinline__ void ipx_edges_strided(const ipx_vid* __restrict__ adj, uint64_t e0, uint64_t e1,
-                                                  uint64_t lane, uint64_t lanes, ipx_msg m, const Visit& visit)
-{
-    if constexpr (sizeof(ipx_vid) == 4) {
-        if (lanes >= 8 && ipx_v4_ok(adj)) {
-            ipx_edges_v4(reinterpret_cast<const uint32_t*>(adj), e0, e1, lane, lanes, m, visit);
-            return;
-        }
-    }
-    for (uint64_t e = e0 + lane; e < e1; e += IPX_UNROLL * lanes) {
-        uint64_t ek[IPX_UNROLL];
-        ipx_vid w[IPX_UNROLL];
-        ipx_msg mk[IPX_UNROLL];
-        bool ok[IPX_UNROLL];
+        const uint32_t t = rel - ((uint32_t)r0 & 3u); /* edge of the row; before its first: wraps */
+        const uint32_t id[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int k = 0; k < IPX_UNROLL; k++) {
-            ek[k] = e + k * lanes;
-            ok[k] = ek[k] < e1;
-            w[k] = ok[k] ? ipx_ld_edge(&adj[ek[k]], lanes) : (ipx_vid)0;
+        for (int k = 0; k < 4; k++) {
+            w[k] = (ipx_vid)id[k];
+            ok[k] = t + k < deg;
             mk[k] = m;
         }
-        visit.template batch<IPX_UNROLL>(ek, w, mk, ok);
+#if IPX_EDGE_MSG
+        if constexpr (sizeof(ipx_wgt) == 4) {
+            const uint4 x = ipx_ld_quad(reinterpret_cast<const uint32_t*>(ipx_c.wgt), r0, deg, rel);
+            const uint32_t xk[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                ipx_wgt y;
+                memcpy(&y, &xk[k], 4);
+                mk[k] = IP_BROADCAST_EDGE_MESSAGE(m, y);
+            }
+        } else {
+            const uint64_t e = r0 - ((uint32_t)r0 & 3u) + rel;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (ok[k]) mk[k] = IP_BROADCAST_EDGE_MESSAGE(m, ipx_ld_stream(&ipx_c.wgt[e + k]));
+        }
+#endif
+    }
+    __device__ __forceinline__ void quad(const uint4& q, uint64_t r0, uint32_t deg, uint32_t rel, const ipx_msg& m) const
+    {
+        ipx_vid w[4];
+        bool ok[4];
+        ipx_msg mk[4];
+        unpack(q, r0, deg, rel, m, w, ok, mk);
+        deliver(w, ok, mk);
+    }
+    __device__ __forceinline__ void edges(const ipx_vid* w, const bool* ok, uint64_t e, uint64_t lanes, const ipx_msg& m) const
+    {
+        ipx_msg mk[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+#if IPX_EDGE_MSG
+            mk[k] = ok[k] ? IP_BROADCAST_EDGE_MESSAGE(m, ipx_ld_edge(&ipx_c.wgt[e + k * lanes], lanes)) : m;
+#else
+            (void)e;
+            (void)lanes;
+            mk[k] = m;
+#endif
+        }
+        deliver(w, ok, mk);
+    }
+};
+
+/* Target marking (spread+single_broadcast).  Targets below `bits` have a bit
+ * in the CTA's shared memory too, set at the CTA's first visit: a hub is hit
+ * by a large part of all edges, and without it every hit would read (or, from
+ * a stale L1 line, set) the same word of the L2. */
+struct ipx_mark_visit {
+    static constexpr bool kNeedsMessage = false;
+    uint32_t* seen;
+    uint64_t bits;
+    __device__ __forceinline__ void four(const ipx_vid* w, const bool* ok) const
+    {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!ok[k]) continue;
+            const uint64_t t = (uint64_t)w[k];
+            const uint32_t bit = 1u << (t & 31);
+            if (t < bits) {
+                if (seen[t >> 5] & bit) continue;
+                if (atomicOr(&seen[t >> 5], bit) & bit) continue;
+            }
+            if (!(ipx_c.bt[t >> 5] & bit)) atomicOr(&ipx_c.bt[t >> 5], bit);
+        }
+    }
+    __device__ __forceinline__ void quad(const uint4& q, uint64_t r0, uint32_t deg, uint32_t rel, const ipx_msg&) const
+    {
+        const uint32_t t = rel - ((uint32_t)r0 & 3u);
+        const ipx_vid w[4] = {(ipx_vid)q.x, (ipx_vid)q.y, (ipx_vid)q.z, (ipx_vid)q.w};
+        const bool ok[4] = {t < deg, t + 1 < deg, t + 2 < deg, t + 3 < deg};
+        four(w, ok);
+    }
+    __device__ __forceinline__ void edges(const ipx_vid* w, const bool* ok, uint64_t, uint64_t, const ipx_msg&) const
+    {
+        four(w, ok);
+    }
+};
+
+/* Edges [e0, e1) of one source, lane-strided: ids without 128-bit loads
+ * (64-bit ids; a caller's unaligned or unpadded array). */
+template <class Visit>
+__device__ __forceinline__ void ipx_edges_strided(const ipx_vid* __restrict__ adj, uint64_t e0, uint64_t e1,
+                                                  uint64_t lane, uint64_t lanes, const ipx_msg& m, const Visit& visit)
+{
+    for (uint64_t e = e0 + lane; e < e1; e += 4 * lanes) {
+        ipx_vid w[4];
+        bool ok[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            ok[k] = e + k * lanes < e1;
+            w[k] = ok[k] ? ipx_ld_edge(&adj[e + k * lanes], lanes) : (ipx_vid)0;
+        }
+        visit.edges(w, ok, e, lanes, m);
     }
 }
 
-/* Warp-cooperative expansion: a warp takes 32 sources of a list at once
- * (one coalesced read of their ids, row bounds and messages), scans their
- * degrees, and spreads the concatenated edges over its lanes, so every lane
- * has work whatever the degrees and the per-source load latency is paid once
- * per 32 sources.  Each lane finds its source by a 5-step search over the
- * warp's exclusive degree prefix (shuffles). */
-template <class Visit>
-__device__ __forceinline__ void ipx_warp_expand(const uint32_t* __restrict__ list, uint64_t n, const Visit& visit)
+/* The out-edges of a list's sources, G lanes each.  The chain list entry ->
+ * row bounds and message -> ids -> mailboxes is pipelined over the group's
+ * next sources, as in the pull gather. */
+template <int G, class Visit>
+__device__ __forceinline__ void ipx_walk_rows(const uint32_t* __restrict__ list, uint32_t n, const Visit& visit)
 {
-    const ipx_vid* __restrict__ adj = ipx_c.adj;
+    const uint32_t gl = threadIdx.x & (G - 1);
     const uint64_t* __restrict__ row = ipx_c.row;
-    const int lane = threadIdx.x & 31;
-    const uint64_t nwarps = ipx_gstride() >> 5;
-    for (uint64_t base = (ipx_gtid() >> 5) * 32; base < n; base += nwarps * 32) {
-        uint64_t r0 = 0;
-        uint32_t deg = 0;
-        ipx_msg m = ipx_msg();
-        if (base + lane < n) {
-            const uint64_t u = list[base + lane];
-            r0 = row[u];
-            deg = (uint32_t)(row[u + 1] - r0);
+    const uint64_t step = ipx_gstride() / G;
+    uint64_t i = ipx_gtid() / G;
+    if (i >= n) return;
+    if (!ipx_c.out_quads) {
+        for (; i < n; i += step) {
+            const uint64_t u = list[i];
+            ipx_msg m = ipx_msg();
             if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[u];
+            ipx_edges_strided(ipx_c.adj, row[u], row[u + 1], gl, G, m, visit);
         }
-        uint32_t inc = deg;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(IPX_FULL, inc, o);
-            if (lane >= o) inc += t;
+        return;
+    }
+    if constexpr (sizeof(ipx_vid) == 4) {
+        const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ipx_c.adj);
+        /* a: the row being walked, b: the next, c: the one after it; past the
+         * list's end vertex 0 stands in: loaded, never walked */
+        uint32_t ua = list[i], ub = i + step < n ? list[i + step] : 0u, uc = i + 2 * step < n ? list[i + 2 * step] : 0u;
+        uint64_t a0 = row[ua], b0 = row[ub];
+        uint32_t ad = ipx_row_edges(a0, row[ua + 1]), bd = ipx_row_edges(b0, row[ub + 1]);
+        ipx_msg ma = ipx_msg(), mb = ipx_msg(), mc = ipx_msg();
+        if constexpr (Visit::kNeedsMessage) {
+            ma = ipx_c.outbox[ua];
+            mb = ipx_c.outbox[ub];
         }
-        const uint32_t excl = inc - deg;
-        const uint32_t total = __shfl_sync(IPX_FULL, inc, 31);
-        for (uint32_t t0 = 0; t0 < total; t0 += 32 * IPX_UNROLL) {
-            uint64_t ek[IPX_UNROLL];
-            ipx_vid w[IPX_UNROLL];
-            ipx_msg mk[IPX_UNROLL];
-            bool ok[IPX_UNROLL];
-#pragma unroll
-            for (int k = 0; k < IPX_UNROLL; k++) {
-                const uint32_t pos = t0 + (uint32_t)(k * 32 + lane);
-                int j = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const uint32_t ex = __shfl_sync(IPX_FULL, excl, j + step);
-                    if (ex <= pos) j += step;
-                }
-                const uint64_t rj = __shfl_sync(IPX_FULL, r0, j);
-                const uint32_t xj = __shfl_sync(IPX_FULL, excl, j);
-                mk[k] = ipx_shfl_idx(m, j);
-                ok[k] = pos < total;
-                ek[k] = rj + (pos - xj);
-                w[k] = ok[k] ? ipx_ld_stream(&adj[ek[k]]) : (ipx_vid)0;
+        uint4 qa = ipx_ld_quad(adj, a0, ad, 4 * gl);
+        for (; i < n; i += step) {
+            const uint32_t ud = i + 3 * step < n ? list[i + 3 * step] : 0u;
+            const uint64_t c0 = row[uc], c1 = row[uc + 1];
+            if constexpr (Visit::kNeedsMessage) mc = ipx_c.outbox[uc];
+            const uint4 qb = ipx_ld_quad(adj, b0, bd, 4 * gl);
+            const uint32_t len = ((uint32_t)a0 & 3u) + ad;
+            for (uint32_t rel = 4 * gl;;) {
+                const uint4 next = ipx_ld_quad(adj, a0, ad, rel + 4 * G);
+                visit.quad(qa, a0, ad, rel, ma);
+                rel += 4 * G;
+                if (rel >= len) break;
+                qa = next;
             }
-            visit.template batch<IPX_UNROLL>(ek, w, mk, ok);
+            uc = ud;
+            a0 = b0;
+            ad = bd;
+            ma = mb;
+            b0 = c0;
+            bd = ipx_row_edges(c0, c1);
+            mb = mc;
+            qa = qb;
         }
     }
+}
+
+/* The chunks of the hubs among the sources, a warp each. */
+template <class Visit>
+__device__ __forceinline__ void ipx_walk_chunks(uint32_t n, const Visit& visit)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = ipx_gstride() >> 5, chunk = ipx_c.push_chunk;
+    for (uint64_t c = ipx_gtid() >> 5; c < n; c += warps) {
+        const uint2 h = ipx_c.bchunk[c];
+        const uint64_t e0 = ipx_c.row[h.x] + h.y * chunk, end = ipx_c.row[h.x + 1];
+        const uint64_t e1 = e0 + chunk < end ? e0 + chunk : end;
+        ipx_msg m = ipx_msg();
+        if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[h.x];
+        if (!ipx_c.out_quads) {
+            ipx_edges_strided(ipx_c.adj, e0, e1, lane, 32, m, visit);
+            continue;
+        }
+        if constexpr (sizeof(ipx_vid) == 4) {
+            const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ipx_c.adj);
+            const uint32_t deg = (uint32_t)(e1 - e0), len = ((uint32_t)e0 & 3u) + deg;
+            uint4 q = ipx_ld_quad(adj, e0, deg, 4 * lane);
+            for (uint32_t rel = 4 * lane; rel < len; rel += 128) {
+                const uint4 next = ipx_ld_quad(adj, e0, deg, rel + 128);
+                visit.quad(q, e0, deg, rel, m);
+                q = next;
+            }
+        }
+    }
+}
+
+/* All of a superstep's broadcasters, the longest work items first. */
+template <class Visit>
+__device__ __forceinline__ void ipx_walk_broadcasters(const Visit& visit)
+{
+    const ipx_stat* st = ipx_c.stat;
+    ipx_walk_chunks(__ldcg(&st->n[3]), visit);
+    ipx_walk_rows<IPX_PUSH_LONG>(ipx_c.blist[2], __ldcg(&st->n[2]), visit);
+    ipx_walk_rows<IPX_PUSH_GROUP>(ipx_c.blist[1], __ldcg(&st->n[1]), visit);
+    ipx_walk_rows<1>(ipx_c.blist[0], __ldcg(&st->n[0]), visit);
 }
 
 /* Chunk prefix of the high-degree class: prefix[i] = chunks of the hubs before
@@ -1233,124 +1331,36 @@ __device__ __forceinline__ void ipx_fill_topology(struct ip_vertex_t& x, uint64_
 }
 
 /* ------------------------------------------------------------------------ */
-/* Push delivery over degree-class lists of broadcasters.                   */
-/* MODE 0: a thread per broadcaster; 1: a warp; 2: a block.                 */
+/* Push delivery of the superstep's broadcasts.                             */
 /* ------------------------------------------------------------------------ */
-/* Runs a visitor over the out-edges of a degree-class list of sources:
- * MODE 0 and 1 by warp-cooperative expansion, MODE 2 (the hubs) a CTA per
- * IPX_HUB_CHUNK-edge chunk, chunks located through `prefix`. */
-template <int MODE, class Visit>
-__device__ __forceinline__ void ipx_over_sources(const uint32_t* __restrict__ list, uint64_t n,
-                                                 const uint32_t* __restrict__ prefix, const Visit& visit)
+/* Bound by the random mailbox reads: 283 G edges/s for CC, 226 for weighted
+ * SSSP (which reads weights and commits more) on undirected R-MAT scale 24,
+ * where the same ids gathered flat, without rows, messages or commits, reach
+ * 376 G/s from the L2.  A run's pushes took 5.1 / 7.6 ms with a launch per row
+ * class, sources by 1 and 16 lanes and hubs by a CTA per chunk, without the
+ * pipeline; 4.4 / 6.7 now.  64 registers: with 5 CTAs a few spills and the same
+ * time, with 6 5.8 / 8.6 (16 lanes), 8 mailbox reads in flight a lane instead
+ * of 4 no faster. */
+#ifndef IPX_PUSH_CTAS
+#define IPX_PUSH_CTAS 4
+#endif
+__global__ void __launch_bounds__(IPX_THREADS, IPX_PUSH_CTAS) ipx_k_push()
 {
-    if constexpr ((MODE == 0 || MODE == 1) && IPX_PUSH_EXPAND) {
-        ipx_warp_expand(list, n, visit);
-    } else if constexpr (MODE == 0 && sizeof(ipx_vid) == 8) {
-        /* 64-bit ids: the loop below would spill registers */
-        const ipx_vid* __restrict__ adj = ipx_c.adj;
-        const uint64_t* __restrict__ row = ipx_c.row;
-        for (uint64_t i = ipx_gtid(); i < n; i += ipx_gstride()) {
-            const uint64_t u = list[i];
-            ipx_msg m = ipx_msg();
-            if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[u];
-            ipx_edges_strided(adj, row[u], row[u + 1], 0, 1, m, visit);
-        }
-    } else if constexpr (MODE == 0 && IPX_PUSH_Q > 1) {
-        /* IPX_PUSH_Q consecutive lanes per source: a source's (at most
-         * IPX_T0) ids are read by the group's lanes together, sectors shared */
-        const ipx_vid* __restrict__ adj = ipx_c.adj;
-        const uint64_t* __restrict__ row = ipx_c.row;
-        const uint64_t q = threadIdx.x & (IPX_PUSH_Q - 1);
-        for (uint64_t i = ipx_gtid() / IPX_PUSH_Q; i < n; i += ipx_gstride() / IPX_PUSH_Q) {
-            const uint64_t u = list[i];
-            ipx_msg m = ipx_msg();
-            if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[u];
-            ipx_edges_strided(adj, row[u], row[u + 1], q, IPX_PUSH_Q, m, visit);
-        }
-    } else if constexpr (MODE == 0) {
-        /* the next source's list entry, row bounds and message are loaded
-         * while this source's edges are visited */
-        const ipx_vid* __restrict__ adj = ipx_c.adj;
-        const uint64_t* __restrict__ row = ipx_c.row;
-        const uint64_t stride = ipx_gstride();
-        uint64_t i = ipx_gtid(), r0 = 0, r1 = 0;
-        ipx_msg m = ipx_msg();
-        if (i < n) {
-            const uint64_t u = list[i];
-            r0 = row[u];
-            r1 = row[u + 1];
-            if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[u];
-        }
-        for (; i < n; i += stride) {
-            uint64_t r0n = 0, r1n = 0;
-            ipx_msg mn = ipx_msg();
-            if (i + stride < n) {
-                const uint64_t un = list[i + stride];
-                r0n = row[un];
-                r1n = row[un + 1];
-                if constexpr (Visit::kNeedsMessage) mn = ipx_c.outbox[un];
-            }
-            ipx_edges_strided(adj, r0, r1, 0, 1, m, visit);
-            r0 = r0n;
-            r1 = r1n;
-            m = mn;
-        }
-    } else if constexpr (MODE == 1) {
-        /* IPX_PUSH_GROUP lanes per source (a warp's worth, or fewer: most
-         * sources of the class have a few dozen out-edges) */
-        constexpr int G = IPX_PUSH_GROUP;
-        const ipx_vid* __restrict__ adj = ipx_c.adj;
-        const uint64_t* __restrict__ row = ipx_c.row;
-        const uint64_t lane = threadIdx.x & (G - 1);
-        for (uint64_t i = ipx_gtid() / G; i < n; i += ipx_gstride() / G) {
-            const uint64_t u = list[i];
-            ipx_msg m = ipx_msg();
-            if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[u];
-            ipx_edges_strided(adj, row[u], row[u + 1], lane, G, m, visit);
-        }
-    } else {
-        if (n == 0) return;
-        const ipx_vid* __restrict__ adj = ipx_c.adj;
-        const uint64_t* __restrict__ row = ipx_c.row;
-        const uint32_t chunks = prefix[n];
-        for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-            const uint64_t i = ipx_c.push_owner ? ipx_c.push_owner[c] : ipx_hub_of_chunk(prefix, n, c);
-            const uint64_t u = list[i];
-            const uint64_t e0 = row[u] + (uint64_t)(c - prefix[i]) * IPX_HUB_CHUNK;
-            const uint64_t end = row[u + 1];
-            const uint64_t e1 = (e0 + IPX_HUB_CHUNK < end) ? e0 + IPX_HUB_CHUNK : end;
-            ipx_msg m = ipx_msg();
-            if constexpr (Visit::kNeedsMessage) m = ipx_c.outbox[u];
-            ipx_edges_strided(adj, e0, e1, threadIdx.x, blockDim.x, m, visit);
-        }
-    }
+    if (ipx_done() || ipx_pulls()) return;
+    ipx_walk_broadcasters(ipx_push_visit{ipx_parity()});
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(IPX_THREADS, IPX_EDGE_CTAS) ipx_k_push(const uint32_t* __restrict__ list,
-                                                          const uint32_t* __restrict__ count,
-                                                          const uint32_t* __restrict__ prefix)
+#if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
+/* Marks the out-neighbours of broadcasters as targets. */
+extern __shared__ uint32_t ipx_seen[];
+__global__ void __launch_bounds__(IPX_MARK_THREADS, 1) ipx_k_mark(uint32_t words)
 {
-    if (ipx_c.pull_ok && __ldcg(&ipx_c.ctr[IPX_CTR_MODE])) return; /* this superstep pulls */
-    ipx_over_sources<MODE>(list, *count, prefix, ipx_push_visit{ipx_parity(), MODE != 0});
+    if (ipx_done()) return;
+    for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) ipx_seen[k] = 0u;
+    __syncthreads();
+    ipx_walk_broadcasters(ipx_mark_visit{ipx_seen, 32ULL * words});
 }
-
-/* Direction of the superstep's delivery: pull when the broadcasters' out-edges
- * (degree sums of the compaction) exceed `threshold`. */
-__global__ void ipx_k_decide(unsigned long long threshold)
-{
-    const unsigned long long m = ipx_c.ctr[8] + ipx_c.ctr[9] + ipx_c.ctr[10];
-    ipx_c.ctr[IPX_CTR_MODE] = (m > threshold) ? 1ULL : 0ULL;
-}
-
-/* Marks the out-neighbours of broadcasters as targets (spread+single_broadcast). */
-template <int MODE>
-__global__ void __launch_bounds__(IPX_THREADS, IPX_EDGE_CTAS) ipx_k_mark(const uint32_t* __restrict__ list,
-                                                          const uint32_t* __restrict__ count,
-                                                          const uint32_t* __restrict__ prefix)
-{
-    ipx_over_sources<MODE>(list, *count, prefix, ipx_mark_visit{});
-}
+#endif
 
 /* ------------------------------------------------------------------------ */
 /* Pull gather (ip_fetch_broadcast_messages, combiner_single_broadcast_      */
@@ -1459,97 +1469,6 @@ __device__ __forceinline__ void ipx_gather_fold_edges(const ipx_vid* __restrict_
     }
 }
 
-/* REACT: reactivate and count (single_broadcast) or not (spread+single_broadcast). */
-template <int MODE, bool REACT>
-__global__ void __launch_bounds__(IPX_THREADS, IPX_EDGE_CTAS) ipx_k_gather(const uint32_t* __restrict__ list,
-                                                            const uint32_t* __restrict__ count_dev,
-                                                            uint64_t count_host)
-{
-    const int ctr_slot = (int)(ipx_step() & 3);
-    const uint64_t n = count_dev ? (uint64_t)*count_dev : count_host;
-    const ipx_vid* __restrict__ adj = ipx_c.in_adj;
-    const uint64_t* __restrict__ row = ipx_c.in_row;
-    const ipx_bslot* __restrict__ bs = ipx_c.bslot[0];
-    const uint32_t stamp = (uint32_t)ipx_step();
-    unsigned long long react = 0;
-    if constexpr (MODE == 0) {
-        /* the next vertex's list entry is loaded while this vertex's
-         * in-edges are folded (its row bounds too would spill registers) */
-        const uint64_t stride = ipx_gstride();
-        uint64_t i = ipx_gtid(), v = (i < n) ? list[i] : 0;
-        for (; i < n; i += stride) {
-            const uint64_t vn = (i + stride < n) ? list[i + stride] : 0;
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges(adj, bs, stamp, row[v], row[v + 1], 0, 1, has, acc);
-            ipx_c.hasmsg_b[v] = has;
-            if (has) {
-                ipx_c.msg[v] = acc;
-                if constexpr (REACT) {
-                    if (!ipx_c.active_b[v]) {
-                        ipx_c.active_b[v] = 1;
-                        react++;
-                    }
-                }
-            }
-            v = vn;
-        }
-    } else if constexpr (MODE == 1) {
-        const int lane = threadIdx.x & 31;
-        for (uint64_t i = ipx_gtid() >> 5; i < n; i += ipx_gstride() >> 5) {
-            const uint64_t v = list[i];
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges(adj, bs, stamp, row[v], row[v + 1], lane, 32, has, acc);
-            ipx_warp_fold(has, acc);
-            if (lane == 0) {
-                ipx_c.hasmsg_b[v] = has;
-                if (has) {
-                    ipx_c.msg[v] = acc;
-                    if constexpr (REACT) {
-                        if (!ipx_c.active_b[v]) {
-                            ipx_c.active_b[v] = 1;
-                            react++;
-                        }
-                    }
-                }
-            }
-        }
-    } else {
-        __shared__ bool s_has[IPX_THREADS / 32];
-        __shared__ ipx_msg s_acc[IPX_THREADS / 32];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (uint64_t i = blockIdx.x; i < n; i += gridDim.x) {
-            const uint64_t v = list[i];
-            bool has = false;
-            ipx_msg acc;
-            ipx_gather_fold_edges(adj, bs, stamp, row[v], row[v + 1], threadIdx.x, blockDim.x, has, acc);
-            ipx_warp_fold(has, acc);
-            if (lane == 0) {
-                s_has[warp] = has;
-                s_acc[warp] = acc;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                has = false;
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) ipx_fold(has, acc, s_has[w], s_acc[w]);
-                ipx_c.hasmsg_b[v] = has;
-                if (has) {
-                    ipx_c.msg[v] = acc;
-                    if constexpr (REACT) {
-                        if (!ipx_c.active_b[v]) {
-                            ipx_c.active_b[v] = 1;
-                            react++;
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if constexpr (REACT) ipx_block_count(react, &ipx_c.ctr[ctr_slot]);
-}
-
 /* ------------------------------------------------------------------------ */
 /* Pull delivery for the push versions (direction optimisation).  On a       */
 /* symmetric graph a vertex's row lists exactly the vertices that would push */
@@ -1594,7 +1513,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_EDGE_CTAS) ipx_k_pull_deliver
                                                                                 uint64_t n,
                                                                                 const uint32_t* __restrict__ prefix)
 {
-    if (!__ldcg(&ipx_c.ctr[IPX_CTR_MODE])) return; /* this superstep pushes */
+    if (ipx_done() || !ipx_pulls()) return; /* this superstep pushes */
     const int p = ipx_parity();
     const uint64_t* __restrict__ row = ipx_c.in_row;
     if constexpr (MODE == 0) {
@@ -1650,96 +1569,266 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_EDGE_CTAS) ipx_k_pull_deliver
 /* ------------------------------------------------------------------------ */
 /* Compute kernels.                                                         */
 /* ------------------------------------------------------------------------ */
+#if IPX_VERSION != IPX_SINGLE_BROADCAST
+/* The compute phase of the push versions and of spread+single_broadcast, and
+ * the lists of this superstep's broadcasters, in one pass over the bitmaps.
+ *
+ * Combiner (push): src/combiner_postamble.h:151-183, vertices that are
+ * active, hold a message or received one; the mailbox swap of the previous
+ * superstep (:168-183) happens here, for the vertex about to run.  Spread
+ * (frontier push): src/combiner_spread_postamble.h:235-272 and the mailbox
+ * update :331-342, the vertices that received mail (all at superstep 0).
+ * Spread + single broadcast: combiner_spread_single_broadcast_postamble.h:
+ * 228-237, the targets of the last superstep.
+ *
+ * A warp takes `words` bitmap words at a time (8 on a large graph, fewer when
+ * that would leave warps with little to even out), a lane a word to load and write back
+ * and, of the nonzero ones, a vertex of each of FRONT_W words to compute: a
+ * dense frontier reads mailboxes, values and row bounds coalesced, a sparse
+ * one costs a scan of the bitmap, and there are no atomics and no list of the
+ * frontier.  Broadcasters go into the list of their row length through a
+ * buffer per warp in shared memory, emptied in long runs behind
+ * one reservation; hubs are listed by chunks.  No warp waits for another.
+ * Latency bound (half of the warps wait on loads, issue slots 43 % busy).
+ * Undirected R-MAT scale 24, CC / weighted SSSP, ms a run: 0.77 / 1.07 for what
+ * a compute kernel over a frontier list (0.93 / 1.42), the compaction of the
+ * broadcasters (0.35 / 0.48) and of the receivers (0.19 / 0.33) and the hubs'
+ * chunk prefix (0.1 / 0.2) took.  A reservation per CTA step behind barriers
+ * 0.82 / 1.33; 4, 16, 32 words a step 0.75 / 1.03, 0.84 / 1.16, 1.0 / 1.42;
+ * 3 CTAs per SM 1.1 / 1.7, 5 (it spills) 1.1 / 1.8. */
+#ifndef IPX_FRONT_CTAS
+#define IPX_FRONT_CTAS 4
+#endif
+#define IPX_FRONT_W 4
+#ifndef IPX_FRONT_BUF
+#define IPX_FRONT_BUF 512 /* entries a warp buffers; a step adds at most 128 */
+#endif
 
-/* Combiner (push): src/combiner_postamble.h:151-183.  One thread per vertex,
- * warp-aligned so that each warp owns whole bitmap words.  The mailbox swap
- * of the previous superstep (:168-183) happens here, for the vertex about to
- * run: a received message becomes the vertex's message and reactivates it. */
-__global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_combiner()
+struct ipx_front_buf {
+    uint32_t v[IPX_FRONT_BUF];
+    uint8_t cls[IPX_FRONT_BUF];
+};
+
+/* The warp's buffered broadcasters go to the ends of their classes' lists;
+ * n: how many of each class are among them. */
+__device__ __forceinline__ void ipx_front_flush(const ipx_front_buf& buf, const uint32_t* n)
 {
-    const uint64_t s = ipx_step();
-    const uint64_t V = ipx_c.V;
-    const uint64_t Vp = (V + 31) & ~31ULL;
-    const int pprev = (int)((s + 1) & 1);  /* parity of superstep s-1 */
     const int lane = threadIdx.x & 31;
-    for (uint64_t v = ipx_gtid(); v < Vp; v += ipx_gstride()) {
-        const uint64_t wi = v >> 5;
-        const uint32_t aw = ipx_c.active_bm[wi];
-        const uint32_t hw = ipx_c.hasmsg_bm[wi];
-        const uint32_t rw = s ? ipx_c.recv[pprev][wi] : 0u;
-        if ((aw | hw | rw) == 0u) continue; /* warp-uniform */
-        const uint32_t bit = 1u << lane;
-        bool a = aw & bit, h = hw & bit, out = false;
-        const bool r = rw & bit;
-        if (v < V && (a || h || r)) {
-            struct ip_vertex_t x;
-            x.id = ipx_user_id(v);
-            x.active = true;
-            if (r) {
-                x.has_message = true;
-                x.message = ipx_mb::take(&ipx_c.mbox[pprev][v]);
-            } else {
-                x.has_message = h;
-                if (h) x.message = ipx_c.msg[v];
-            }
-            const ipx_val v0 = ipx_c.value[v];
-            x.value = v0;
-            x.ipx_has_out = false;
-            ipx_fill_topology(x, v);
-            ip_compute(&x);
-            if (!ipx_same_bits(x.value, v0)) ipx_c.value[v] = x.value;
-            a = x.active;
-            h = x.has_message;
-            if (h) ipx_c.msg[v] = x.message;
-            if (x.ipx_has_out) {
-                ipx_c.outbox[v] = x.ipx_out;
-                out = true;
-            }
-        }
-        const uint32_t na = __ballot_sync(IPX_FULL, a), nh = __ballot_sync(IPX_FULL, h);
-        const uint32_t no = __ballot_sync(IPX_FULL, out);
-        if (lane == 0) {
-            if (na != aw) ipx_c.active_bm[wi] = na;
-            if (nh != hw) ipx_c.hasmsg_bm[wi] = nh;
-            if (no) ipx_c.bcaster[wi] = no;
-            if (rw) ipx_c.recv[pprev][wi] = 0u;
+    const uint32_t lt = (1u << lane) - 1u, total = n[0] + n[1] + n[2];
+    const uint32_t mine = lane == 0 ? n[0] : (lane == 1 ? n[1] : n[2]);
+    uint32_t at = 0;
+    if (lane < 3 && mine) at = atomicAdd(&ipx_c.stat->n[lane], mine);
+    uint32_t to[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) to[j] = __shfl_sync(IPX_FULL, at, j);
+    __syncwarp();
+    for (uint32_t q0 = 0; q0 < total; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        const int c = q < total ? (int)buf.cls[q] : 3;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const uint32_t b = __ballot_sync(IPX_FULL, c == j);
+            if (c == j) ipx_c.blist[j][to[j] + __popc(b & lt)] = buf.v[q];
+            to[j] += __popc(b);
         }
     }
+    __syncwarp();
 }
 
-/* Spread (frontier push): src/combiner_spread_postamble.h:235-272 and the
- * mailbox update :331-342.  Superstep 0 runs every vertex, later supersteps
- * the vertices that received mail; a frontier vertex always has a message. */
-__global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_spread(const uint32_t* __restrict__ frontier,
-                                                                    const uint32_t* __restrict__ fcount)
+__global__ void __launch_bounds__(IPX_THREADS, IPX_FRONT_CTAS) ipx_k_front(int words)
 {
+    if (ipx_done()) return;
+    __shared__ ipx_front_buf s_buf[IPX_THREADS / 32];
     const uint64_t s = ipx_step();
-    const uint64_t n = s ? (uint64_t)*fcount : ipx_c.V;
-    const int pprev = (int)((s + 1) & 1);
-    /* the next frontier entry is loaded while this vertex computes */
-    const uint64_t stride = ipx_gstride();
-    uint64_t i = ipx_gtid();
-    uint64_t vn = (i < n) ? (s ? frontier[i] : i) : 0;
-    for (; i < n; i += stride) {
-        const uint64_t v = vn;
-        vn = (i + stride < n) ? (s ? frontier[i + stride] : i + stride) : 0;
-        struct ip_vertex_t x;
-        x.id = ipx_user_id(v);
-        x.active = true;
-        x.has_message = s != 0;
-        if (s) x.message = ipx_mb::take(&ipx_c.mbox[pprev][v]);
-        const ipx_val v0 = ipx_c.value[v];
-        x.value = v0;
-        x.ipx_has_out = false;
-        ipx_fill_topology(x, v);
-        ip_compute(&x);
-        if (!ipx_same_bits(x.value, v0)) ipx_c.value[v] = x.value;
-        if (x.ipx_has_out) {
-            ipx_c.outbox[v] = x.ipx_out;
-            ipx_set_bit_agg(ipx_c.bcaster, v);
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    ipx_front_buf& buf = s_buf[threadIdx.x >> 5];
+    const uint64_t W = ipx_c.W, step = (ipx_gstride() >> 5) * (uint64_t)words;
+    [[maybe_unused]] const int pprev = (int)((s + 1) & 1); /* parity of superstep s-1 */
+    unsigned long long es[4] = {0, 0, 0, 0};
+    uint32_t n[3] = {0, 0, 0};
+    if (s == 0 && blockIdx.x == 0 && threadIdx.x == 0) ipx_c.ctl[IPX_CTL_STAMP] = ipx_now();
+    for (uint64_t base = (ipx_gtid() >> 5) * (uint64_t)words; base < W; base += step) {
+        /* this lane's word */
+        const uint64_t wl = base + lane;
+        const bool mine = lane < words && wl < W;
+        uint32_t word = 0;
+        [[maybe_unused]] uint32_t act = 0, has = 0, rec = 0, out_word = 0;
+        if (mine) {
+#if IPX_VERSION == IPX_COMBINER
+            act = ipx_c.active_bm[wl];
+            has = ipx_c.hasmsg_bm[wl];
+            rec = s ? ipx_c.recv[pprev][wl] : 0u;
+            word = act | has | rec;
+            if (rec) ipx_c.recv[pprev][wl] = 0u;
+#else
+#if IPX_VERSION == IPX_SPREAD
+            uint32_t* from = ipx_c.recv[pprev];
+#else
+            uint32_t* from = ipx_c.bt;
+#endif
+            if (s) {
+                word = from[wl];
+                if (word) from[wl] = 0u;
+            } else {
+                /* the vertex count ends inside the last word */
+                word = (wl == W - 1 && (ipx_c.V & 31)) ? (1u << (ipx_c.V & 31)) - 1u : IPX_FULL;
+            }
+#endif
+        }
+        [[maybe_unused]] const uint32_t act0 = act, has0 = has;
+        uint32_t todo = __ballot_sync(IPX_FULL, word != 0u);
+        while (todo) {
+            /* the next FRONT_W nonzero words */
+            int idx[IPX_FRONT_W];
+            uint32_t run[IPX_FRONT_W];
+            [[maybe_unused]] uint32_t hw[IPX_FRONT_W], rw[IPX_FRONT_W];
+#pragma unroll
+            for (int k = 0; k < IPX_FRONT_W; k++) {
+                idx[k] = todo ? __ffs(todo) - 1 : 0;
+                const uint32_t x = __shfl_sync(IPX_FULL, word, idx[k]);
+                run[k] = todo ? x : 0u;
+                todo &= todo - 1;
+#if IPX_VERSION == IPX_COMBINER
+                hw[k] = __shfl_sync(IPX_FULL, has0, idx[k]);
+                rw[k] = __shfl_sync(IPX_FULL, rec, idx[k]);
+#endif
+            }
+            /* every load of the warp's vertices before any of them computes */
+            ipx_val v0[IPX_FRONT_W];
+            [[maybe_unused]] ipx_slot box[IPX_FRONT_W];
+            [[maybe_unused]] bool hm[IPX_FRONT_W];
+            [[maybe_unused]] ipx_msg msg[IPX_FRONT_W];
+#pragma unroll
+            for (int k = 0; k < IPX_FRONT_W; k++) {
+                const uint64_t v = (base + idx[k]) * 32 + lane;
+                if ((run[k] >> lane) & 1u) {
+                    v0[k] = ipx_c.value[v];
+#if IPX_VERSION == IPX_COMBINER
+                    if ((rw[k] >> lane) & 1u) box[k] = ipx_c.mbox[pprev][v];
+                    else if ((hw[k] >> lane) & 1u) msg[k] = ipx_c.msg[v];
+#elif IPX_VERSION == IPX_SPREAD
+                    if (s) box[k] = ipx_c.mbox[pprev][v];
+#else
+                    hm[k] = ipx_c.hasmsg_b[v];
+                    if (hm[k]) msg[k] = ipx_c.msg[v];
+#endif
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < IPX_FRONT_W; k++) {
+                if (!run[k]) continue; /* warp-uniform */
+                const uint64_t v = (base + idx[k]) * 32 + lane;
+                uint64_t d = 0;
+                bool out = false;
+                [[maybe_unused]] bool na = false, nh = false;
+                if ((run[k] >> lane) & 1u) {
+                    struct ip_vertex_t x;
+                    x.id = ipx_user_id(v);
+                    x.active = true;
+#if IPX_VERSION == IPX_COMBINER
+                    const bool r = (rw[k] >> lane) & 1u;
+                    x.has_message = r || ((hw[k] >> lane) & 1u);
+                    if (r) {
+                        x.message = ipx_mb::message(box[k]);
+                        ipx_c.mbox[pprev][v] = ipx_mb::empty();
+                    } else if (x.has_message) {
+                        x.message = msg[k];
+                    }
+#elif IPX_VERSION == IPX_SPREAD
+                    x.has_message = s != 0; /* a frontier vertex always has one */
+                    if (s) {
+                        x.message = ipx_mb::message(box[k]);
+                        ipx_c.mbox[pprev][v] = ipx_mb::empty();
+                    }
+#else
+                    x.has_message = hm[k];
+                    if (hm[k]) x.message = msg[k];
+#endif
+                    x.value = v0[k];
+                    x.ipx_has_out = false;
+                    ipx_fill_topology(x, v);
+                    ip_compute(&x);
+                    if (!ipx_same_bits(x.value, v0[k])) ipx_c.value[v] = x.value;
+                    out = x.ipx_has_out;
+#if IPX_VERSION == IPX_COMBINER
+                    na = x.active;
+                    nh = x.has_message;
+                    if (nh) ipx_c.msg[v] = x.message;
+#endif
+                    if (out) {
+#if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
+                        ipx_bslot_put(&ipx_c.bslot[0][v], x.ipx_out, (uint32_t)s);
+#else
+                        ipx_c.outbox[v] = x.ipx_out;
+#endif
+                        d = ipx_c.row[v + 1] - ipx_c.row[v];
+                    }
+                }
+                const uint32_t nout = __ballot_sync(IPX_FULL, out);
+                if (lane == idx[k]) out_word = nout;
+#if IPX_VERSION == IPX_COMBINER
+                const uint32_t aw = __ballot_sync(IPX_FULL, na), mw = __ballot_sync(IPX_FULL, nh);
+                if (lane == idx[k]) {
+                    act = aw;
+                    has = mw;
+                }
+#endif
+                if (!nout) continue;
+                const int c = d == 0 ? -1 : (d <= ipx_c.push_t[0] ? 0 : (d <= ipx_c.push_t[1] ? 1 : (d <= ipx_c.push_t[2] ? 2 : 3)));
+                const uint32_t in = __ballot_sync(IPX_FULL, c >= 0 && c < 3);
+                if (c >= 0 && c < 3) {
+                    const uint32_t q = n[0] + n[1] + n[2] + __popc(in & lt);
+                    buf.v[q] = (uint32_t)v;
+                    buf.cls[q] = (uint8_t)c;
+                }
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    n[j] += __popc(__ballot_sync(IPX_FULL, c == j));
+                    if (c == j) es[j] += d;
+                }
+                uint32_t hubs = __ballot_sync(IPX_FULL, c == 3);
+                if (hubs) {
+                    const uint32_t ch = c == 3 ? (uint32_t)((d + ipx_c.push_chunk - 1) / ipx_c.push_chunk) : 0u;
+                    if (c == 3) es[3] += d;
+                    uint32_t at = 0;
+                    if (c == 3) at = atomicAdd(&ipx_c.stat->n[3], ch);
+                    while (hubs) {
+                        const int j = __ffs(hubs) - 1;
+                        hubs &= hubs - 1;
+                        const uint32_t aj = __shfl_sync(IPX_FULL, at, j), cj = __shfl_sync(IPX_FULL, ch, j);
+                        const uint32_t u = __shfl_sync(IPX_FULL, (uint32_t)v, j);
+                        for (uint32_t q = lane; q < cj; q += 32) ipx_c.bchunk[aj + q] = make_uint2(u, q);
+                    }
+                }
+            }
+            if (n[0] + n[1] + n[2] > IPX_FRONT_BUF - 32 * IPX_FRONT_W) {
+                ipx_front_flush(buf, n);
+                n[0] = n[1] = n[2] = 0;
+            }
+        }
+        if (mine) {
+#if IPX_VERSION == IPX_COMBINER
+            if (act != act0) ipx_c.active_bm[wl] = act;
+            if (has != has0) ipx_c.hasmsg_bm[wl] = has;
+#endif
+            if (ipx_c.pull_ok) ipx_c.bcaster[wl] = out_word;
         }
     }
+    if (n[0] + n[1] + n[2]) ipx_front_flush(buf, n);
+    __shared__ unsigned long long s_edges[4];
+    if (threadIdx.x < 4) s_edges[threadIdx.x] = 0ULL;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        unsigned long long e = es[j];
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(IPX_FULL, e, o);
+        if (lane == 0 && e) atomicAdd(&s_edges[j], e);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 && s_edges[threadIdx.x]) atomicAdd(&ipx_c.stat->edges[threadIdx.x], s_edges[threadIdx.x]);
 }
+#endif
 
 /* The single_broadcast version's record of a vertex's broadcast (or of
  * none) for the superstep `stamp`: a stamped slot is written only for a
@@ -1768,6 +1857,7 @@ __device__ __forceinline__ void ipx_sb_put(unsigned long long* p, bool out, cons
 __global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_sb0()
 {
     if (ipx_step() != 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ipx_c.ctl[IPX_CTL_STAMP] = ipx_now();
     const uint64_t V = ipx_c.V;
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[0];
     for (uint64_t v = ipx_gtid(); v < V; v += ipx_gstride()) {
@@ -1788,6 +1878,8 @@ __global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_sb0()
         if (!x.active) ipx_c.active_b[v] = 0;
         ipx_sb_put(&out[v], x.ipx_has_out, x.ipx_out, 0u);
     }
+    /* the fused kernel of superstep 0 runs the compute phase of superstep 1 */
+    if (ipx_last_cta() && threadIdx.x == 0) ipd_compute_superstep = 1;
 }
 
 /* After vertex v's gather of superstep s: whether v is active (it was after
@@ -2077,33 +2169,16 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
  * 17 and more edges go from 203 to 263 G edges/s; the same ids gathered flat,
  * without rows, reach 314 G/s, which the L2 bounds. */
 
-/* Edges p .. p+3 as loaded (p a multiple of 4): which of them belong to the
- * row is decided when they are used, so that nothing waits for the load
- * before. */
-__device__ __forceinline__ uint4 ipx_ld_quad(const uint32_t* __restrict__ adj, uint64_t p, uint64_t e1, uint64_t E)
+/* Folds the broadcasts of the row's edges among a quad's ids, in order. */
+template <bool HOT, class S>
+__device__ __forceinline__ void ipx_fold_quad(const S* __restrict__ bs, uint32_t stamp, const uint4& q, uint64_t r0,
+                                              uint32_t deg, uint32_t rel, bool& has, ipx_msg& acc)
 {
-    return __ldcs(reinterpret_cast<const uint4*>(adj + ((p < e1 && p + 4 <= E) ? p : 0)));
-}
-
-/* Folds the broadcasts of edges p .. p+3 that lie in [e0, e1), in order; q:
- * ipx_ld_quad of p.  The array's last, incomplete quad is read here. */
-template <bool HOT>
-__device__ __forceinline__ void ipx_fold_quad(const uint32_t* __restrict__ adj, const ipx_sbslot* __restrict__ bs,
-                                              uint32_t stamp, uint4 q, uint64_t p, uint64_t e0, uint64_t e1, uint64_t E,
-                                              bool& has, ipx_msg& acc)
-{
-    const int lo = p < e0 ? (int)(e0 - p) : 0;
-    const int hi = p < e1 ? (e1 - p < 4 ? (int)(e1 - p) : 4) : 0;
-    if (p + 4 > E && hi > 0) {
-        q.x = adj[p];
-        if (hi > 1) q.y = adj[p + 1];
-        if (hi > 2) q.z = adj[p + 2];
-    }
+    const uint32_t t = rel - ((uint32_t)r0 & 3u); /* edge of the row; before its first: wraps */
     const uint32_t id[4] = {q.x, q.y, q.z, q.w};
-    ipx_sbslot w[4];
+    S w[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++)
-        w[k] = (k >= lo && k < hi) ? ipx_slot_ld<HOT>(bs, (uint64_t)id[k]) : ipx_no_slot<ipx_sbslot>();
+    for (int k = 0; k < 4; k++) w[k] = t + k < deg ? ipx_slot_ld<HOT>(bs, (uint64_t)id[k]) : ipx_no_slot<S>();
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         ipx_msg m;
@@ -2125,21 +2200,75 @@ __device__ __forceinline__ void ipx_group_fold(bool& has, ipx_msg& acc, unsigned
     }
 }
 
-/* Gather + next compute phase of the list's vertices, G lanes each; SKIP:
- * hubs are passed over. */
+/* Lanes per row of the middle and the long class, and the longest middle
+ * row (rows up to t0 take a thread each): about as many lanes as a row has
+ * quads.  PageRank at scale 25 / personalised PageRank at 4 M vertices took
+ * 74.1 / 9.8 ms with 8 lanes up to 64 edges and 16 beyond, 77.6 / 10.3 with 16
+ * for both, 73.5 / 10.9 with 8 for both, 75.9 / 10.2 with 32 beyond 64. */
+#ifndef IPX_GATHER_GROUP
+#define IPX_GATHER_GROUP 8
+#endif
+#ifndef IPX_GATHER_LONG
+#define IPX_GATHER_LONG 16
+#endif
+#ifndef IPX_GATHER_MID
+#define IPX_GATHER_MID 64
+#endif
+
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+typedef ipx_sbslot ipx_gslot;
+#else
+typedef ipx_bslot ipx_gslot;
+#endif
+
+/* What becomes of vertex v's fold: single_broadcast runs its compute phase
+ * of the next superstep (with its activity and value, loaded before the
+ * fold) and returns the activity that this superstep counts;
+ * spread+single_broadcast stores it for the next superstep's. */
+struct ipx_vertex_state {
+    bool active;
+    ipx_val value;
+};
+__device__ __forceinline__ void ipx_gather_ahead(uint64_t v, bool mine, ipx_vertex_state& x)
+{
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+    x.active = mine ? ipx_c.active_b[v] != 0 : false;
+    x.value = mine ? ipx_c.value[v] : ipx_val();
+#else
+    (void)v;
+    (void)mine;
+    (void)x;
+#endif
+}
+__device__ __forceinline__ bool ipx_gather_done(uint64_t v, bool has, const ipx_msg& acc, const ipx_vertex_state& x,
+                                                ipx_gslot* out, uint32_t stamp)
+{
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+    return ipx_sb_compute_next(v, has, acc, x.active, x.value, out, stamp + 1);
+#else
+    (void)x;
+    (void)out;
+    (void)stamp;
+    ipx_c.hasmsg_b[v] = has;
+    if (has) ipx_c.msg[v] = acc;
+    return false;
+#endif
+}
+
+/* Gathers the list's vertices, G lanes each; SKIP: hubs are passed over. */
 template <int G, bool SKIP, bool HOT>
 __device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* __restrict__ list, uint32_t n,
-                                                              const ipx_vid* __restrict__ ids, bool quads,
+                                                              const ipx_vid* __restrict__ ids,
                                                               const uint64_t* __restrict__ row,
-                                                              const ipx_sbslot* __restrict__ bs, uint32_t stamp,
-                                                              ipx_sbslot* __restrict__ out)
+                                                              const ipx_gslot* __restrict__ bs, uint32_t stamp,
+                                                              ipx_gslot* __restrict__ out)
 {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const unsigned mask = (G == 32) ? IPX_FULL : (((1u << (G & 31)) - 1u) << (lane & ~(G - 1)));
     const uint64_t step = ipx_gstride() / G;
     uint64_t i = ipx_gtid() / G;
     unsigned long long cnt = 0;
-    if (!quads) {
+    if (!ipx_c.in_quads) {
         for (; i < n; i += step) {
             const uint64_t v = list[i];
             if (SKIP && row[v + 1] - row[v] > ipx_c.hub_min) continue;
@@ -2147,57 +2276,59 @@ __device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* __
             ipx_msg acc;
             ipx_gather_fold_edges<HOT>(ids, bs, stamp, row[v], row[v + 1], gl, G, has, acc);
             if (G > 1) ipx_group_fold<G>(has, acc, mask);
-            if (gl == 0) cnt += ipx_sb_compute_next(v, has, acc, ipx_c.active_b[v] != 0, ipx_c.value[v], out, stamp + 1);
+            ipx_vertex_state x;
+            ipx_gather_ahead(v, gl == 0, x);
+            if (gl == 0) cnt += ipx_gather_done(v, has, acc, x, out, stamp);
         }
         return cnt;
     }
     const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ids);
-    const uint64_t E = ipx_c.E;
     if (i >= n) return cnt;
     /* a: the row being folded, b: the next, c: the one after it.  Past the
      * list's end vertex 0 stands in: loaded, never folded. */
     uint32_t va = list[i], vb = i + step < n ? list[i + step] : 0u, vc = i + 2 * step < n ? list[i + 2 * step] : 0u;
-    uint64_t a0 = row[va], a1 = row[va + 1], b0 = row[vb], b1 = row[vb + 1];
-    uint4 qa = ipx_ld_quad(adj, (a0 & ~3ULL) + 4 * gl, a1, E);
+    uint64_t a0 = row[va], b0 = row[vb];
+    uint32_t ad = ipx_row_edges(a0, row[va + 1]), bd = ipx_row_edges(b0, row[vb + 1]);
+    uint4 qa = ipx_ld_quad(adj, a0, ad, 4 * gl);
     for (; i < n; i += step) {
-        const bool act = gl == 0 ? ipx_c.active_b[va] != 0 : false;
-        const ipx_val v0 = gl == 0 ? ipx_c.value[va] : ipx_val();
+        ipx_vertex_state x;
+        ipx_gather_ahead(va, gl == 0, x);
         const uint32_t vd = i + 3 * step < n ? list[i + 3 * step] : 0u;
         const uint64_t c0 = row[vc], c1 = row[vc + 1];
-        const uint4 qb = ipx_ld_quad(adj, (b0 & ~3ULL) + 4 * gl, b1, E);
+        const uint4 qb = ipx_ld_quad(adj, b0, bd, 4 * gl);
         bool has = false;
         ipx_msg acc;
-        const bool skip = SKIP && a1 - a0 > ipx_c.hub_min;
-        if (skip) a1 = a0;
-        uint64_t p = (a0 & ~3ULL) + 4 * gl;
-        ipx_fold_quad<HOT>(adj, bs, stamp, qa, p, a0, a1, E, has, acc);
-        for (p += 4 * G; p < a1; p += 4 * G)
-            ipx_fold_quad<HOT>(adj, bs, stamp, ipx_ld_quad(adj, p, a1, E), p, a0, a1, E, has, acc);
+        const bool skip = SKIP && ad > ipx_c.hub_min;
+        if (skip) ad = 0;
+        ipx_fold_quad<HOT>(bs, stamp, qa, a0, ad, 4 * gl, has, acc);
+        const uint32_t len = ((uint32_t)a0 & 3u) + ad;
+        for (uint32_t rel = 4 * gl + 4 * G; rel < len; rel += 4 * G)
+            ipx_fold_quad<HOT>(bs, stamp, ipx_ld_quad(adj, a0, ad, rel), a0, ad, rel, has, acc);
         if (G > 1) ipx_group_fold<G>(has, acc, mask);
-        if (gl == 0 && !skip) cnt += ipx_sb_compute_next(va, has, acc, act, v0, out, stamp + 1);
+        if (gl == 0 && !skip) cnt += ipx_gather_done(va, has, acc, x, out, stamp);
         va = vb;
         vb = vc;
         vc = vd;
         a0 = b0;
-        a1 = b1;
+        ad = bd;
         b0 = c0;
-        b1 = c1;
+        bd = ipx_row_edges(c0, c1);
         qa = qb;
     }
     return cnt;
 }
 
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
 /* The hub class with a warp per chunk: the warp folds its chunk, lane 0
  * stores the fold, and the warp whose chunk arrives last folds the hub's
  * partials -- each lane a contiguous run of them, then the runs in order by
  * shuffles -- and lane 0 runs the vertex's compute phase. */
 template <bool HOT>
 __device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
-    const ipx_vid* __restrict__ ids, bool quads, const uint64_t* __restrict__ row, const ipx_sbslot* __restrict__ bs,
+    const ipx_vid* __restrict__ ids, const uint64_t* __restrict__ row, const ipx_sbslot* __restrict__ bs,
     uint32_t stamp, ipx_sbslot* __restrict__ out)
 {
     const int lane = threadIdx.x & 31;
-    const uint64_t E = ipx_c.E;
     const uint64_t nwarps = ipx_gstride() >> 5;
     unsigned long long cnt = 0;
     for (uint64_t c = ipx_gtid() >> 5; c < ipx_c.chunks; c += nwarps) {
@@ -2205,13 +2336,13 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
         ipx_locate_chunk(row, (uint32_t)c, h);
         bool has = false;
         ipx_msg acc;
-        if (quads) {
+        if (ipx_c.in_quads) {
             const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ids);
-            uint64_t p = (h.e0 & ~3ULL) + 4 * lane;
-            uint4 q = ipx_ld_quad(adj, p, h.e1, E);
-            for (; p < h.e1; p += 128) {
-                const uint4 next = ipx_ld_quad(adj, p + 128, h.e1, E);
-                ipx_fold_quad<HOT>(adj, bs, stamp, q, p, h.e0, h.e1, E, has, acc);
+            const uint32_t deg = (uint32_t)(h.e1 - h.e0), len = ((uint32_t)h.e0 & 3u) + deg;
+            uint4 q = ipx_ld_quad(adj, h.e0, deg, 4 * lane);
+            for (uint32_t rel = 4 * lane; rel < len; rel += 128) {
+                const uint4 next = ipx_ld_quad(adj, h.e0, deg, rel + 128);
+                ipx_fold_quad<HOT>(bs, stamp, q, h.e0, deg, rel, has, acc);
                 q = next;
             }
         } else {
@@ -2244,21 +2375,6 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
     return cnt;
 }
 
-/* Lanes per row of the middle and the long class, and the longest middle
- * row (rows up to t0 take a thread each): about as many lanes as a row has
- * quads.  PageRank at scale 25 / personalised PageRank at 4 M vertices took
- * 74.1 / 9.8 ms with 8 lanes up to 64 edges and 16 beyond, 77.6 / 10.3 with 16
- * for both, 73.5 / 10.9 with 8 for both, 75.9 / 10.2 with 32 beyond 64. */
-#ifndef IPX_GATHER_GROUP
-#define IPX_GATHER_GROUP 8
-#endif
-#ifndef IPX_GATHER_LONG
-#define IPX_GATHER_LONG 16
-#endif
-#ifndef IPX_GATHER_MID
-#define IPX_GATHER_MID 64
-#endif
-
 /* Resident CTAs per SM the fused pull kernel is compiled for: it carries
  * ip_compute and the pipeline's registers besides the gather (64 a thread;
  * with 48 or 40 it spills: PageRank at scale 25 78.0 ms with 4 CTAs, 83.4
@@ -2280,8 +2396,9 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
  * 16 k to 500 k threads each end in a tail of their own, which on a graph of
  * 65,536 vertices was half of the superstep. */
 template <bool HOT>
-__global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_compute()
+__global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_compute(ipx_loop loop)
 {
+    if (ipx_done()) return;
     const uint64_t s = ipx_step();
     const uint32_t stamp = (uint32_t)s;
     /* HOT: ids of the in-lists carry the flag of the most gathered vertices */
@@ -2289,18 +2406,16 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_com
     const uint64_t* __restrict__ row = ipx_c.in_row;
     const ipx_sbslot* __restrict__ bs = ipx_c.sbslot[s & 1];
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[(s + 1) & 1];
-    /* 128-bit id loads need 32-bit ids and a 16-byte aligned array (a
-     * caller's may not be) of one load at least */
-    const bool quads = sizeof(ipx_vid) == 4 && (reinterpret_cast<uintptr_t>(adj) & 15) == 0 && ipx_c.E >= 4;
     unsigned long long cnt = 0;
     /* the longest work items first */
-    if constexpr (IPX_HUB_WARP) cnt += ipx_gather_hubs_warp<HOT>(adj, quads, row, bs, stamp, out);
-    cnt += ipx_gather_rows<IPX_GATHER_LONG, true, HOT>(ipx_c.class_list[2], ipx_c.class_n[2], adj, quads, row, bs,
-                                                       stamp, out);
-    cnt += ipx_gather_rows<IPX_GATHER_GROUP, false, HOT>(ipx_c.class_list[1], ipx_c.class_n[1], adj, quads, row, bs,
-                                                         stamp, out);
-    cnt += ipx_gather_rows<1, false, HOT>(ipx_c.class_list[0], ipx_c.class_n[0], adj, quads, row, bs, stamp, out);
-    ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
+    if constexpr (IPX_HUB_WARP) cnt += ipx_gather_hubs_warp<HOT>(adj, row, bs, stamp, out);
+    cnt += ipx_gather_rows<IPX_GATHER_LONG, true, HOT>(ipx_c.class_list[2], ipx_c.class_n[2], adj, row, bs, stamp,
+                                                       out);
+    cnt += ipx_gather_rows<IPX_GATHER_GROUP, false, HOT>(ipx_c.class_list[1], ipx_c.class_n[1], adj, row, bs, stamp,
+                                                         out);
+    cnt += ipx_gather_rows<1, false, HOT>(ipx_c.class_list[0], ipx_c.class_n[0], adj, row, bs, stamp, out);
+    ipx_block_count(cnt, &ipx_c.stat->count);
+    if (ipx_last_cta() && threadIdx.x == 0) ipx_end_of_superstep(loop, __ldcg(&ipx_c.stat->count));
 }
 
 #if !IPX_HUB_WARP
@@ -2315,6 +2430,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_com
 template <bool HOT>
 __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hubs()
 {
+    if (ipx_done()) return;
     const uint64_t s = ipx_step();
     const uint32_t stamp = (uint32_t)s;
     const ipx_vid* __restrict__ adj = HOT ? reinterpret_cast<const ipx_vid*>(ipx_c.in_adj_hot) : ipx_c.in_adj;
@@ -2325,7 +2441,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hub
     if constexpr (sizeof(ipx_vid) == 4 && IPX_HUB_SMEM) {
         if ((reinterpret_cast<uintptr_t>(adj) & 15) == 0) {
             cnt += ipx_gather_hubs_staged<HOT>(reinterpret_cast<const uint32_t*>(adj), row, bs, stamp, out);
-            ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
+            ipx_block_count(cnt, &ipx_c.stat->count);
             return;
         }
     }
@@ -2353,39 +2469,56 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hub
         cnt += ipx_hub_chunk_done(h, has, acc, out, stamp + 1, s_has, s_acc);
         __syncthreads();
     }
-    ipx_block_count(cnt, &ipx_c.ctr[s & 3]);
+    ipx_block_count(cnt, &ipx_c.stat->count);
 }
 #endif /* !IPX_HUB_WARP */
+#endif /* IPX_SINGLE_BROADCAST */
 
-/* Spread + single broadcast compute phase: combiner_spread_single_broadcast_
- * postamble.h:228-237, over the targets (all vertices at superstep 0). */
-__global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_ssb(const uint32_t* __restrict__ l0,
-                                                                 const uint32_t* __restrict__ l1,
-                                                                 const uint32_t* __restrict__ l2,
-                                                                 const uint32_t* __restrict__ cnt)
+#if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
+/* Spread + single broadcast: the targets' fetch (combiner_spread_single_
+ * broadcast_postamble.h:249-309), rows by length as in the fused pull kernel,
+ * those above t1 a CTA each; then the end of the superstep. */
+#ifndef IPX_TARGET_CTAS
+#define IPX_TARGET_CTAS 4
+#endif
+__global__ void __launch_bounds__(IPX_THREADS, IPX_TARGET_CTAS) ipx_k_gather_targets(ipx_loop loop)
 {
-    const uint64_t s = ipx_step();
-    const uint64_t c0 = s ? cnt[0] : ipx_c.V, c1 = s ? cnt[1] : 0, c2 = s ? cnt[2] : 0;
-    const uint64_t n = c0 + c1 + c2;
-    for (uint64_t i = ipx_gtid(); i < n; i += ipx_gstride()) {
-        const uint64_t v = !s ? i : (i < c0 ? l0[i] : (i < c0 + c1 ? l1[i - c0] : l2[i - c0 - c1]));
-        struct ip_vertex_t x;
-        x.id = ipx_user_id(v);
-        x.active = true;
-        x.has_message = ipx_c.hasmsg_b[v];
-        if (x.has_message) x.message = ipx_c.msg[v];
-        const ipx_val v0 = ipx_c.value[v];
-        x.value = v0;
-        x.ipx_has_out = false;
-        ipx_fill_topology(x, v);
-        ip_compute(&x);
-        if (!ipx_same_bits(x.value, v0)) ipx_c.value[v] = x.value;
-        if (x.ipx_has_out) {
-            ipx_bslot_put(&ipx_c.bslot[0][v], x.ipx_out, (uint32_t)s);
-            ipx_set_bit_agg(ipx_c.bcaster, v);
+    if (ipx_done()) return;
+    __shared__ bool s_has[IPX_THREADS / 32];
+    __shared__ ipx_msg s_acc[IPX_THREADS / 32];
+    const uint32_t stamp = (uint32_t)ipx_step();
+    const ipx_vid* __restrict__ adj = ipx_c.in_adj;
+    const uint64_t* __restrict__ row = ipx_c.in_row;
+    const ipx_bslot* __restrict__ bs = ipx_c.bslot[0];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t n2 = __ldcg(&ipx_c.stat->tn[2]);
+    for (uint32_t i = blockIdx.x; i < n2; i += gridDim.x) {
+        const uint64_t v = ipx_c.tlist[2][i];
+        bool has = false;
+        ipx_msg acc;
+        ipx_gather_fold_edges(adj, bs, stamp, row[v], row[v + 1], threadIdx.x, blockDim.x, has, acc);
+        ipx_warp_fold(has, acc);
+        if (lane == 0) {
+            s_has[warp] = has;
+            s_acc[warp] = acc;
         }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            has = false;
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) ipx_fold(has, acc, s_has[w], s_acc[w]);
+            ipx_gather_done(v, has, acc, ipx_vertex_state(), nullptr, stamp);
+        }
+        __syncthreads();
+    }
+    ipx_gather_rows<IPX_GATHER_LONG, false, false>(ipx_c.tlist[1], __ldcg(&ipx_c.stat->tn[1]), adj, row, bs, stamp, nullptr);
+    ipx_gather_rows<1, false, false>(ipx_c.tlist[0], __ldcg(&ipx_c.stat->tn[0]), adj, row, bs, stamp, nullptr);
+    if (ipx_last_cta() && threadIdx.x == 0) {
+        unsigned long long n = 0;
+        for (int k = 0; k < 3; k++) n += __ldcg(&ipx_c.stat->tn[k]);
+        ipx_end_of_superstep(loop, n);
     }
 }
+#endif
 
 /* ------------------------------------------------------------------------ */
 /* Initialisation kernels (ip_init_vertex_range of each version).           */
@@ -2427,80 +2560,30 @@ __global__ void ipx_k_fill_bits(uint32_t* bm, uint64_t V, uint64_t W)
     }
 }
 
-/* ------------------------------------------------------------------------ */
-/* Superstep control on the device.                                         */
-/* ------------------------------------------------------------------------ */
-
-/* Zeroes the counters a superstep accumulates into. */
-__global__ void ipx_k_begin_superstep()
+#if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SPREAD
+/* Active count of the superstep and its end: the vertices that received mail
+ * (spread), or that are active or did (combiner_postamble.h:151-183). */
+__global__ void __launch_bounds__(IPX_THREADS) ipx_k_count(ipx_loop loop)
 {
-    const uint64_t s = ipx_step();
-    ipx_c.ctr[s & 3] = 0ULL;
-    for (int k = 8; k < 14; k++) ipx_c.ctr[k] = 0ULL;
-#if IPX_VERSION == IPX_SINGLE_BROADCAST
-    /* the fused kernels of superstep s run the compute phase of s + 1
-     * (superstep 0's own compute phase, ipx_k_compute_sb0, ran before) */
-    ipd_compute_superstep = s + 1;
-#endif
-}
-
-/* Combiner: active count of the superstep = |active or received|
- * (combiner_postamble.h:151-183), parity read on the device. */
-__global__ void __launch_bounds__(IPX_THREADS) ipx_k_count_combiner()
-{
-    const uint64_t s = ipx_step();
-    const uint32_t* __restrict__ a = ipx_c.active_bm;
-    const uint32_t* __restrict__ r = ipx_c.recv[s & 1];
+    if (ipx_done()) return;
+    /* four words at a time: the bitmaps' last words of four are padding */
+    const uint4* __restrict__ r = reinterpret_cast<const uint4*>(ipx_c.recv[ipx_parity()]);
     unsigned long long c = 0;
-    for (uint64_t i = ipx_gtid(); i < ipx_c.W; i += ipx_gstride()) c += __popc(a[i] | r[i]);
-    ipx_block_count(c, &ipx_c.ctr[s & 3]);
-}
-
-/* Active count the reference prints for the superstep just run and tests in
- * its loop condition (each version's ip_run). */
-__device__ __forceinline__ unsigned long long ipx_superstep_count(uint64_t s)
-{
-#if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SINGLE_BROADCAST
-    return ipx_c.ctr[s & 3];
-#elif IPX_VERSION == IPX_SPREAD
-    (void)s;
-    return ipx_c.lcnt[4];
-#else
-    (void)s;
-    return (unsigned long long)ipx_c.lcnt[4] + ipx_c.lcnt[5] + ipx_c.lcnt[6];
+    for (uint64_t i = ipx_gtid(); i < (ipx_c.W + 3) / 4; i += ipx_gstride()) {
+        uint4 x = r[i];
+#if IPX_VERSION == IPX_COMBINER
+        const uint4 a = reinterpret_cast<const uint4*>(ipx_c.active_bm)[i];
+        x.x |= a.x;
+        x.y |= a.y;
+        x.z |= a.z;
+        x.w |= a.w;
 #endif
-}
-
-/* Last kernel of a captured superstep: records the superstep in the history,
- * advances the superstep and sets the loop's condition: continue while the
- * count is nonzero (combiner_postamble.h:134; spread versions test it after
- * superstep 0, combiner_spread_postamble.h:212), no kernel reported an error
- * and the superstep bound is not reached. */
-__global__ void ipx_k_advance(cudaGraphConditionalHandle loop, unsigned long long max_supersteps)
-{
-    const uint64_t s = ipx_step();
-    const unsigned long long count = ipx_superstep_count(s);
-    unsigned long long edges = 0;
-#if IPX_VERSION == IPX_SINGLE_BROADCAST
-    edges = ipx_c.E;
-#else
-    const bool pulled = ipx_c.pull_ok && ipx_c.ctr[IPX_CTR_MODE];
-    edges = pulled ? ipx_c.E : ipx_c.ctr[8] + ipx_c.ctr[9] + ipx_c.ctr[10];
-    edges += ipx_c.ctr[11] + ipx_c.ctr[12] + ipx_c.ctr[13];
-#endif
-    unsigned long long* h = ipx_c.hist + (s % IPX_HIST) * 4;
-    h[0] = count;
-    h[1] = edges;
-    h[2] = ipx_c.pull_ok ? ipx_c.ctr[IPX_CTR_MODE] : 0ULL;
-    bool go = count != 0 && *ipx_c.err == 0;
-    if (go && s + 1 >= max_supersteps) {
-        atomicOr(ipx_c.err, IPX_ERR_SUPERSTEP_LIMIT);
-        go = false;
+        c += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
     }
-    ipd_superstep = s + 1;
-    ipd_compute_superstep = s + 1;
-    cudaGraphSetConditional(loop, go ? 1u : 0u);
+    ipx_block_count(c, &ipx_c.stat->count);
+    if (ipx_last_cta() && threadIdx.x == 0) ipx_end_of_superstep(loop, __ldcg(&ipx_c.stat->count));
 }
+#endif
 
 /* Checks an IP_COMBINE_KIND hint against the user's ip_combine on sample
  * pairs before the hint is trusted. */

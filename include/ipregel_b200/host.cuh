@@ -74,14 +74,12 @@ struct ipx_host_state {
      * re-attaching a graph of about the same shape allocates and frees
      * nothing (cudaFree synchronises the whole device) */
     std::vector<std::pair<void*, uint64_t>> spare;
-    uint32_t* blist[3] = {nullptr, nullptr, nullptr};  /* broadcaster classes */
-    uint32_t* tlist[3] = {nullptr, nullptr, nullptr};  /* frontier / target classes */
-    uint32_t* lcnt = nullptr;                          /* [0..2] broadcaster, [4..6] targets */
-    uint32_t* hub_prefix = nullptr;                    /* chunk prefix of the broadcaster hubs */
-    uint32_t* pull_prefix = nullptr;                   /* chunk prefix of the static in-degree hubs */
-    unsigned long long pull_threshold = 0;             /* pull when broadcaster edges exceed this */
-    unsigned long long* h_ctr = nullptr;               /* pinned mirror of ctr */
-    uint32_t* h_lcnt = nullptr;                        /* pinned mirror of lcnt */
+    uint32_t* pull_prefix = nullptr; /* chunk prefix of the static in-degree hubs (pulling push versions) */
+    /* pinned: the records of a batch of supersteps, the last one's counts */
+    struct ipx_pinned {
+        unsigned long long hist[IPX_BATCH][4];
+        ipx_stat last;
+    }* pin = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     ipg_bins gbins;                                    /* static in-degree classes (pulling push versions) */
@@ -105,6 +103,10 @@ struct ipx_host_state {
     int tb = IPX_THREADS;      /* CTA size in use */
     uint32_t grid_compute = 0; /* resident CTAs of the compute kernel */
     uint32_t grid_edge = 0;    /* resident CTAs of the edge kernels */
+    uint32_t grid_count = 0;   /* CTAs of the counting kernel */
+    uint32_t grid_pull = 0;    /* resident CTAs of the pull delivery */
+    uint32_t mark_words = 0;   /* spread+single_broadcast: bits of the marking kernel in shared memory */
+    int front_words = 1;       /* bitmap words a warp of the compute kernel takes at a time */
     uint32_t grid_hubs = 0;    /* single_broadcast, a CTA per hub chunk: of the hub kernel */
     std::vector<struct ip_vertex_t> host_vertices;
     bool host_valid = false;
@@ -206,10 +208,8 @@ static void ipx_release_state(bool keep = false)
     if (ipx_h.gexec) cudaGraphExecDestroy(ipx_h.gexec);
     ipx_h.gexec = nullptr;
     if (!keep) { /* a re-attach keeps the stream, events and pinned words too */
-        if (ipx_h.h_ctr) cudaFreeHost(ipx_h.h_ctr);
-        if (ipx_h.h_lcnt) cudaFreeHost(ipx_h.h_lcnt);
-        ipx_h.h_ctr = nullptr;
-        ipx_h.h_lcnt = nullptr;
+        if (ipx_h.pin) cudaFreeHost(ipx_h.pin);
+        ipx_h.pin = nullptr;
         if (ipx_h.ev0) cudaEventDestroy(ipx_h.ev0);
         if (ipx_h.ev1) cudaEventDestroy(ipx_h.ev1);
         if (ipx_h.st) cudaStreamDestroy(ipx_h.st);
@@ -240,8 +240,8 @@ static uint32_t ipx_resident_grid(K kernel, int block, int per_sm)
     return ipx_grid(n < per_sm ? n : per_sm);
 }
 
-/* First degree threshold of the broadcaster classes. */
-static uint64_t ipx_push_t0() { return IPX_PUSH_EXPAND ? ipx_h.tune.t1 : ipx_h.tune.t0; }
+/* Words of a bitmap: whole groups of four, the rest zero (ipx_k_count). */
+static uint64_t ipx_bitmap_words(uint64_t W) { return (W + 4) & ~3ULL; }
 
 /* ip_init_vertex_range (combiner_postamble.h:89-117 and the other versions):
  * every per-vertex flag back to its initial value. */
@@ -256,15 +256,14 @@ static int ipx_reset_vertex_state()
         IPX_CU(cudaGetLastError());
     }
 #if IPX_VERSION == IPX_COMBINER
+    IPX_CU(cudaMemsetAsync(c.active_bm, 0, ipx_bitmap_words(W) * 4, st));
     if (W) ipx_k_fill_bits<<<ipx_grid(), IPX_THREADS, 0, st>>>(c.active_bm, V, W);
-    IPX_CU(cudaMemsetAsync(c.hasmsg_bm, 0, W * 4 + 4, st));
-    IPX_CU(cudaMemsetAsync(c.recv[0], 0, W * 4 + 4, st));
-    IPX_CU(cudaMemsetAsync(c.recv[1], 0, W * 4 + 4, st));
-    IPX_CU(cudaMemsetAsync(c.bcaster, 0, W * 4 + 4, st));
+    IPX_CU(cudaMemsetAsync(c.hasmsg_bm, 0, ipx_bitmap_words(W) * 4, st));
+    IPX_CU(cudaMemsetAsync(c.recv[0], 0, ipx_bitmap_words(W) * 4, st));
+    IPX_CU(cudaMemsetAsync(c.recv[1], 0, ipx_bitmap_words(W) * 4, st));
 #elif IPX_VERSION == IPX_SPREAD
-    IPX_CU(cudaMemsetAsync(c.recv[0], 0, W * 4 + 4, st));
-    IPX_CU(cudaMemsetAsync(c.recv[1], 0, W * 4 + 4, st));
-    IPX_CU(cudaMemsetAsync(c.bcaster, 0, W * 4 + 4, st));
+    IPX_CU(cudaMemsetAsync(c.recv[0], 0, ipx_bitmap_words(W) * 4, st));
+    IPX_CU(cudaMemsetAsync(c.recv[1], 0, ipx_bitmap_words(W) * 4, st));
 #elif IPX_VERSION == IPX_SINGLE_BROADCAST
     /* every stamp IPX_NO_STAMP: no slot counts in any superstep */
     IPX_CU(cudaMemsetAsync(c.sbslot[0], 0xff, (V ? V : 1) * sizeof(ipx_sbslot), st));
@@ -274,10 +273,9 @@ static int ipx_reset_vertex_state()
     IPX_CU(cudaMemsetAsync(c.hasmsg_b, 0, V + 1, st));
     IPX_CU(cudaMemsetAsync(c.bslot[0], 0xff, (V ? V : 1) * sizeof(ipx_bslot), st));
     IPX_CU(cudaMemsetAsync(c.bt, 0, W * 4 + 4, st));
-    IPX_CU(cudaMemsetAsync(c.bcaster, 0, W * 4 + 4, st));
 #endif
-    IPX_CU(cudaMemsetAsync(c.ctr, 0, IPX_NCTR * sizeof(unsigned long long), st));
-    IPX_CU(cudaMemsetAsync(ipx_h.lcnt, 0, 8 * sizeof(uint32_t), st));
+    IPX_CU(cudaMemsetAsync(c.ctl, 0, IPX_NCTL * sizeof(unsigned long long), st));
+    IPX_CU(cudaMemsetAsync(c.stat, 0, sizeof(ipx_stat), st));
     IPX_CU(cudaStreamSynchronize(st));
     ip_superstep = 0;
     ip_active_vertices = V;
@@ -389,46 +387,52 @@ static int ipx_setup_state()
     if (!ipx_h.st) IPX_CU(cudaStreamCreateWithFlags(&ipx_h.st, cudaStreamNonBlocking));
     if (!ipx_h.ev0) IPX_CU(cudaEventCreate(&ipx_h.ev0));
     if (!ipx_h.ev1) IPX_CU(cudaEventCreate(&ipx_h.ev1));
-    if (!ipx_h.h_ctr)
-        IPX_CU(cudaHostAlloc((void**)&ipx_h.h_ctr, IPX_NCTR * sizeof(unsigned long long), cudaHostAllocDefault));
-    if (!ipx_h.h_lcnt) IPX_CU(cudaHostAlloc((void**)&ipx_h.h_lcnt, 8 * sizeof(uint32_t), cudaHostAllocDefault));
+    if (!ipx_h.pin) IPX_CU(cudaHostAlloc((void**)&ipx_h.pin, sizeof(*ipx_h.pin), cudaHostAllocDefault));
     IPX_OK(ipx_alloc(&c.value, V));
     if (ipx_h.vindex_of) IPX_OK(ipx_alloc(&ipx_h.values_by_id, V));
-    IPX_OK(ipx_alloc(&c.ctr, IPX_NCTR));
-    c.err = (uint32_t*)(c.ctr + IPX_CTR_ERR);
-    IPX_OK(ipx_alloc(&ipx_h.lcnt, 8));
-    c.lcnt = ipx_h.lcnt;
+    IPX_OK(ipx_alloc(&c.ctl, IPX_NCTL));
+    c.err = (uint32_t*)(c.ctl + IPX_CTL_ERR);
+    IPX_OK(ipx_alloc(&c.stat, 1));
+    IPX_OK(ipx_alloc(&c.last, 1));
     IPX_OK(ipx_alloc(&c.hist, (uint64_t)IPX_HIST * 4));
-    IPX_OK(ipx_alloc(&ipx_h.hub_prefix, gv.E / (ipx_h.tune.t1 + 1) + 2));
-#if !IPX_PULL || IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
     {
-        /* the chunks of this superstep's broadcaster hubs: at most E / chunk
-         * + one partial chunk per hub */
-        uint32_t* owner = nullptr;
-        IPX_OK(ipx_alloc(&owner, gv.E / IPX_HUB_CHUNK + gv.E / (ipx_h.tune.t1 + 1) + 2));
-        c.push_owner = owner;
+        int q = 0;
+        IPX_OK(ipg_graph_quads(ipx_h.gw, 0, &q));
+        c.out_quads = q;
+        c.in_quads = 0;
+        if (gv.has_in) {
+            IPX_OK(ipg_graph_quads(ipx_h.gw, 1, &q));
+            c.in_quads = q;
+        }
+    }
+#if IPX_VERSION != IPX_SINGLE_BROADCAST
+    {
+        /* rows of this superstep's broadcasters by class; hubs above a chunk
+         * (a quarter of a resident warp's share of the edges, so that every
+         * warp gets several) or the tuned t1 */
+        const uint64_t share = gv.E / ((uint64_t)ipg_sm_count() * IPX_PUSH_CTAS * (IPX_THREADS / 32) * 4);
+        uint64_t chunk = 256;
+        while (chunk < IPX_HUB_CHUNK && chunk * 2 <= share) chunk *= 2;
+        c.push_chunk = (uint32_t)chunk;
+        c.push_t[2] = chunk == IPX_HUB_CHUNK || ipx_h.tune.t1 < chunk ? ipx_h.tune.t1 : chunk;
+        c.push_t[0] = ipx_h.tune.t0 < c.push_t[2] ? ipx_h.tune.t0 : c.push_t[2];
+        c.push_t[1] = IPX_PUSH_MID < c.push_t[2] ? IPX_PUSH_MID : c.push_t[2];
+        if (c.push_t[1] < c.push_t[0]) c.push_t[1] = c.push_t[0];
+        for (int k = 0; k < 3; k++) IPX_OK(ipx_alloc(&c.blist[k], V));
+        IPX_OK(ipx_alloc(&c.bchunk, gv.E / chunk + gv.E / (c.push_t[2] + 1) + 2));
     }
 #endif
 #if IPX_VERSION == IPX_COMBINER
-    IPX_OK(ipx_alloc(&c.active_bm, W + 1));
-    IPX_OK(ipx_alloc(&c.hasmsg_bm, W + 1));
+    IPX_OK(ipx_alloc(&c.active_bm, ipx_bitmap_words(W)));
+    IPX_OK(ipx_alloc(&c.hasmsg_bm, ipx_bitmap_words(W)));
     IPX_OK(ipx_alloc(&c.msg, V));
 #endif
 #if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SPREAD
     IPX_OK(ipx_alloc(&c.mbox[0], V));
     IPX_OK(ipx_alloc(&c.mbox[1], V));
-    IPX_OK(ipx_alloc(&c.recv[0], W + 1));
-#if IPX_VERSION == IPX_COMBINER
-    IPX_OK(ipx_alloc(&c.recv[1], W + 1));
-#else
-    c.recv[1] = c.recv[0]; /* compacted (and cleared) every superstep */
-#endif
+    IPX_OK(ipx_alloc(&c.recv[0], ipx_bitmap_words(W)));
+    IPX_OK(ipx_alloc(&c.recv[1], ipx_bitmap_words(W)));
     IPX_OK(ipx_alloc(&c.outbox, V));
-    IPX_OK(ipx_alloc(&c.bcaster, W + 1));
-    for (int k = 0; k < 3; k++) IPX_OK(ipx_alloc(&ipx_h.blist[k], V));
-#endif
-#if IPX_VERSION == IPX_SPREAD
-    IPX_OK(ipx_alloc(&ipx_h.tlist[0], V));
 #endif
 #if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SPREAD
     /* Direction optimisation: a dense superstep may deliver by pulling over
@@ -443,9 +447,10 @@ static int ipx_setup_state()
         const unsigned long long div = ipx_h.tune.pull_div;
         const bool in_exact = gv.symmetric || (gv.directed && gv.has_in);
         c.pull_ok = (in_exact && div > 0 && V > 0) ? 1 : 0;
-        ipx_h.pull_threshold = div ? gv.E / div : ~0ULL;
+        c.pull_threshold = div ? gv.E / div : ~0ULL;
     }
     if (c.pull_ok) {
+        IPX_OK(ipx_alloc(&c.bcaster, W + 1));
         IPX_OK(ipg_graph_bins(ipx_h.gw, gv.directed ? 1 : 0, ipx_h.tune.t0, ipx_h.tune.t1, &ipx_h.gbins));
         IPX_OK(ipx_alloc(&ipx_h.pull_prefix, ipx_h.gbins.count[2] + 2));
         uint32_t* dcount = nullptr;
@@ -496,9 +501,7 @@ static int ipx_setup_state()
 #endif
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
     IPX_OK(ipx_alloc(&c.bt, W + 1));
-    IPX_OK(ipx_alloc(&c.bcaster, W + 1));
-    for (int k = 0; k < 3; k++) IPX_OK(ipx_alloc(&ipx_h.blist[k], V));
-    for (int k = 0; k < 3; k++) IPX_OK(ipx_alloc(&ipx_h.tlist[k], V));
+    for (int k = 0; k < 3; k++) IPX_OK(ipx_alloc(&c.tlist[k], V));
 #endif
     IPX_CU(cudaMemcpyToSymbol(ipx_c, &c, sizeof c));
     size_t vc = V, ec = gv.E;
@@ -516,13 +519,7 @@ static int ipx_setup_state()
     {
         const int tb = ipx_h.tb;
         const int per_sm = 2048 / tb;
-#if IPX_VERSION == IPX_COMBINER
-        ipx_h.grid_compute = ipx_resident_grid(ipx_k_compute_combiner, tb, per_sm);
-        ipx_h.grid_edge = ipx_resident_grid(ipx_k_push<1>, tb, per_sm);
-#elif IPX_VERSION == IPX_SPREAD
-        ipx_h.grid_compute = ipx_resident_grid(ipx_k_compute_spread, tb, per_sm);
-        ipx_h.grid_edge = ipx_resident_grid(ipx_k_push<1>, tb, per_sm);
-#elif IPX_VERSION == IPX_SINGLE_BROADCAST
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
         ipx_h.grid_compute = ipx_resident_grid(ipx_k_compute_sb0, tb, per_sm);
         ipx_h.grid_edge = c.in_adj_hot ? ipx_resident_grid(ipx_k_gather_compute<true>, tb, per_sm)
                                        : ipx_resident_grid(ipx_k_gather_compute<false>, tb, per_sm);
@@ -531,8 +528,24 @@ static int ipx_setup_state()
                                        : ipx_resident_grid(ipx_k_gather_hubs<false>, tb, per_sm);
 #endif
 #else
-        ipx_h.grid_compute = ipx_resident_grid(ipx_k_compute_ssb, tb, per_sm);
-        ipx_h.grid_edge = ipx_resident_grid(ipx_k_gather<1, false>, tb, per_sm);
+        /* a warp's words per step: as many as leave every resident warp eight
+         * steps (they even out), at most 8 */
+        ipx_h.grid_compute = ipx_resident_grid(ipx_k_front, tb, per_sm);
+        const uint64_t warps = (uint64_t)ipx_h.grid_compute * (tb / 32);
+        ipx_h.front_words = 1;
+        while (ipx_h.front_words < 8 && W >= warps * 16 * ipx_h.front_words) ipx_h.front_words *= 2;
+        const uint64_t per_cta = (uint64_t)(tb / 32) * ipx_h.front_words, ctas_front = (W + per_cta - 1) / per_cta;
+        if (ctas_front < ipx_h.grid_compute) ipx_h.grid_compute = ctas_front ? (uint32_t)ctas_front : 1u;
+        const uint64_t ctas = (W / 4 + IPX_THREADS) / IPX_THREADS, most = (uint64_t)ipg_sm_count();
+        ipx_h.grid_count = (uint32_t)(ctas < most ? (ctas ? ctas : 1) : most);
+#if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
+        ipx_h.grid_edge = ipx_resident_grid(ipx_k_gather_targets, tb, per_sm);
+        ipx_h.mark_words = (uint32_t)(W < IPX_MARK_WORDS ? W : IPX_MARK_WORDS);
+        IPX_CU(cudaFuncSetAttribute(ipx_k_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, IPX_MARK_WORDS * 4));
+#else
+        ipx_h.grid_edge = ipx_resident_grid(ipx_k_push, tb, per_sm);
+        ipx_h.grid_pull = ipx_resident_grid(ipx_k_pull_deliver<1>, tb, per_sm);
+#endif
 #endif
     }
     ipx_h.ready = true;
@@ -596,9 +609,6 @@ static int ipx_set_superstep(uint64_t s)
     return IPG_OK;
 }
 
-static int ipx_push_class(int k, uint32_t g);
-static int ipx_deliver_superstep(uint32_t ge);
-
 /* ---- per-kernel profiling (the role of IP_ENABLE_THREAD_PROFILING in the
  * reference, e.g. combiner_spread_postamble.h:166-178, :353-401): every
  * launch is counted; with profiling on, each is bracketed by events and its
@@ -627,54 +637,6 @@ static void ipx_k_end()
         ipx_k_end();               \
     } while (0)
 
-static int ipx_push_class(int k, uint32_t g)
-{
-    cudaStream_t st = ipx_h.st;
-    uint32_t* pre = ipx_h.hub_prefix;
-    if (k == 0) IPX_LAUNCH(IPX_K_PUSH0, ipx_k_push<0><<<g, ipx_h.tb, 0, st>>>(ipx_h.blist[0], ipx_h.lcnt + 0, pre));
-    if (k == 1) IPX_LAUNCH(IPX_K_PUSH1, ipx_k_push<1><<<g, ipx_h.tb, 0, st>>>(ipx_h.blist[1], ipx_h.lcnt + 1, pre));
-    if (k == 2) {
-        IPX_LAUNCH(IPX_K_CTRL, ipx_k_hub_prefix<><<<1, 1024, 0, st>>>(ipx_h.blist[2], ipx_h.lcnt + 2, ipx_h.c.row, pre,
-                                                                       (uint32_t*)ipx_h.c.push_owner));
-        IPX_LAUNCH(IPX_K_PUSH2, ipx_k_push<2><<<g, ipx_h.tb, 0, st>>>(ipx_h.blist[2], ipx_h.lcnt + 2, pre));
-    }
-    IPX_CU(cudaGetLastError());
-    return IPG_OK;
-}
-
-/* Delivery of the superstep's broadcasts (push versions): compact the
- * broadcasters into degree classes, then push along their rows, or, on a
- * symmetric graph when their out-edges pass the threshold, pull over every
- * row.  The direction is chosen on the device (ipx_k_decide); the kernels of
- * the other direction return at once. */
-static int ipx_deliver_superstep(uint32_t ge)
-{
-#if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SPREAD
-    const ipx_consts& c = ipx_h.c;
-    cudaStream_t st = ipx_h.st;
-    uint64_t* edges_b = (uint64_t*)(c.ctr + 8);
-    IPX_LAUNCH(IPX_K_COMPACT_B, IPX_OK(ipg_compact(c.bcaster, c.V, c.row, ipx_push_t0(), ipx_h.tune.t1, ipx_h.blist[0],
-                                                   ipx_h.blist[1], ipx_h.blist[2], ipx_h.lcnt, edges_b,
-                                                   c.pull_ok ? 0 : 1, st)));
-    if (c.pull_ok) IPX_LAUNCH(IPX_K_CTRL, ipx_k_decide<<<1, 1, 0, st>>>(ipx_h.pull_threshold));
-    for (int k = 0; k < 3; k++) IPX_OK(ipx_push_class(k, ge));
-    if (c.pull_ok) {
-        const ipg_bins& b = ipx_h.gbins;
-        IPX_LAUNCH(IPX_K_PULLD0, ipx_k_pull_deliver<0><<<ge, ipx_h.tb, 0, st>>>(b.d_list[0], b.count[0],
-                                                                                   ipx_h.pull_prefix));
-        IPX_LAUNCH(IPX_K_PULLD1, ipx_k_pull_deliver<1><<<ge, ipx_h.tb, 0, st>>>(b.d_list[1], b.count[1],
-                                                                                   ipx_h.pull_prefix));
-        IPX_LAUNCH(IPX_K_PULLD2, ipx_k_pull_deliver<2><<<ge, ipx_h.tb, 0, st>>>(b.d_list[2], b.count[2],
-                                                                                   ipx_h.pull_prefix));
-        IPX_CU(cudaMemsetAsync(c.bcaster, 0, c.W * 4 + 4, st));
-    }
-    IPX_CU(cudaGetLastError());
-#else
-    (void)ge;
-#endif
-    return IPG_OK;
-}
-
 /* Algorithmic bytes of the superstep's kernels: the data each must move once
  * (ids, row offsets, values, messages, mailbox read-modify-writes, bitmap
  * bits), from the list sizes and degree sums of this superstep. */
@@ -683,181 +645,117 @@ static void ipx_account_bytes(uint64_t s, uint64_t frontier)
     const double V = (double)ipx_h.c.V;
     const double ib = sizeof(ipx_vid), vb = sizeof(ipx_val), mb = sizeof(ipx_msg), sb = sizeof(ipx_slot);
     const double wb = IPX_EDGE_MSG ? (double)IPX_WEIGHT_BYTES : 0.0;
-    [[maybe_unused]] const unsigned long long* ctr = ipx_h.h_ctr;
-    [[maybe_unused]] const uint32_t* l = ipx_h.h_lcnt;
+    const ipx_stat& x = ipx_h.pin->last;
     double* B = ipx_h.prof_bytes;
     double* N = ipx_h.prof_edges;
     (void)s;
     (void)sb;
     (void)wb;
-    (void)N;
-#if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SPREAD
-    const double nb = (double)l[0] + l[1] + l[2];
-    B[IPX_K_COMPUTE] += (IPX_VERSION == IPX_COMBINER ? V * 3.0 / 8.0 : frontier * 4.0) +
-                        frontier * (2 * vb + sb) + nb * mb;
-    B[IPX_K_COMPACT_B] += V / 8.0 + nb * 20.0;
-    if (ipx_h.c.pull_ok && ctr[IPX_CTR_MODE]) {
+    (void)frontier;
+#if IPX_VERSION == IPX_SINGLE_BROADCAST
+    /* superstep 0's compute: activity, value read and write, broadcast;
+     * the fused kernel: per vertex its in-row bounds, activity, value read
+     * and write and a broadcast (the compute phase of the next superstep);
+     * per in-edge its id and the gathered message */
+    (void)x;
+    if (s == 0) B[IPX_K_COMPUTE] += V * (1.0 + 2 * vb + 16.0 + mb);
+    B[IPX_K_GATHER] += V * (16.0 + 1.0 + 2 * vb + mb) + (double)ipx_h.c.E * (ib + mb);
+    N[IPX_K_GATHER] += (double)ipx_h.c.E;
+#else
+    /* the compute kernel: the bitmap, the frontier's values and messages,
+     * per broadcaster its row bounds, list entry and message */
+    const double nb = (double)x.n[0] + x.n[1] + x.n[2] + x.n[3];
+    const double bedges = (double)x.edges[0] + x.edges[1] + x.edges[2] + x.edges[3];
+    B[IPX_K_COMPUTE] += V * (IPX_VERSION == IPX_COMBINER ? 3.0 : 1.0) / 8.0 + frontier * (2 * vb + sb) + nb * (20.0 + mb);
+#if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
+    const double nt = (double)x.tn[0] + x.tn[1] + x.tn[2];
+    const double tedges = (double)x.tedges[0] + x.tedges[1] + x.tedges[2];
+    B[IPX_K_MARK] += nb * 20.0 + bedges * (ib + 0.125);
+    N[IPX_K_MARK] += bedges;
+    B[IPX_K_COMPACT_T] += V / 8.0 + nt * 20.0;
+    B[IPX_K_GATHER] += nt * (4.0 + 16.0 + 1.0 + mb) + tedges * (ib + mb);
+    N[IPX_K_GATHER] += tedges;
+#else
+    if (ipx_h.c.pull_ok && bedges > (double)ipx_h.c.pull_threshold) {
         /* pulled: every row once, messages of the broadcasting neighbours */
         const ipg_bins& b = ipx_h.gbins;
-        const double bedges = (double)ctr[8] + ctr[9] + ctr[10];
         const double E = ipx_h.c.E ? (double)ipx_h.c.E : 1.0;
         for (int k = 0; k < 3; k++)
             B[IPX_K_PULLD0 + k] +=
                 b.count[k] * (4.0 + 16.0 + sb) + b.edges[k] * (ib + 0.125) + bedges * (mb + wb) * (b.edges[k] / E);
         for (int k = 0; k < 3; k++) N[IPX_K_PULLD0 + k] += b.edges[k];
     } else {
-        for (int k = 0; k < 3; k++) B[IPX_K_PUSH0 + k] += l[k] * (20.0 + mb) + ctr[8 + k] * (ib + sb + wb);
-        for (int k = 0; k < 3; k++) N[IPX_K_PUSH0 + k] += ctr[8 + k];
+        B[IPX_K_PUSH] += nb * (20.0 + mb) + bedges * (ib + sb + wb);
+        N[IPX_K_PUSH] += bedges;
     }
-#if IPX_VERSION == IPX_COMBINER
-    B[IPX_K_COUNT] += V / 4.0;
-#else
-    B[IPX_K_COMPACT_T] += V / 8.0 + l[4] * 4.0;
+    B[IPX_K_COUNT] += V * (IPX_VERSION == IPX_COMBINER ? 2.0 : 1.0) / 8.0;
 #endif
-#elif IPX_VERSION == IPX_SINGLE_BROADCAST
-    /* superstep 0's compute: activity, value read and write, broadcast;
-     * the fused kernel: per vertex its in-row bounds, activity, value read
-     * and write and a broadcast (the compute phase of the next superstep);
-     * per in-edge its id and the gathered message */
-    (void)frontier;
-    if (s == 0) B[IPX_K_COMPUTE] += V * (1.0 + 2 * vb + 16.0 + mb);
-    B[IPX_K_GATHER1] += V * (16.0 + 1.0 + 2 * vb + mb) + (double)ipx_h.c.E * (ib + mb);
-    N[IPX_K_GATHER1] += (double)ipx_h.c.E;
-#else
-    const double nb = (double)l[0] + l[1] + l[2];
-    B[IPX_K_COMPUTE] += frontier * (4.0 + 2 * vb + 1 + mb) + nb * mb;
-    B[IPX_K_COMPACT_B] += V / 8.0 + nb * 20.0;
-    for (int k = 0; k < 3; k++) B[IPX_K_MARK0 + k] += l[k] * 20.0 + ctr[8 + k] * (ib + 0.125);
-    for (int k = 0; k < 3; k++) N[IPX_K_MARK0 + k] += ctr[8 + k];
-    B[IPX_K_COMPACT_T] += V / 8.0 + ((double)l[4] + l[5] + l[6]) * 20.0;
-    for (int k = 0; k < 3; k++)
-        B[IPX_K_GATHER0 + k] += l[4 + k] * (4.0 + 16.0 + 1.0 + mb) + ctr[11 + k] * (ib + mb + 0.125);
-    for (int k = 0; k < 3; k++) N[IPX_K_GATHER0 + k] += ctr[11 + k];
 #endif
 }
 
-static int ipx_end_superstep(uint64_t s, uint64_t* count, uint64_t frontier)
+/* The message of a kernel's error word. */
+static int ipx_fail_device(uint32_t err)
 {
-    cudaStream_t st = ipx_h.st;
-    IPX_CU(cudaMemcpyAsync(ipx_h.h_ctr, ipx_h.c.ctr, IPX_NCTR * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    IPX_CU(cudaMemcpyAsync(ipx_h.h_lcnt, ipx_h.lcnt, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    IPX_CU(cudaEventRecord(ipx_h.ev1, st));
-    IPX_CU(cudaEventSynchronize(ipx_h.ev1));
-    IPX_CU(cudaGetLastError());
-    uint32_t err = (uint32_t)(ipx_h.h_ctr[IPX_CTR_ERR] & 0xffffffffu);
     if (err & IPX_ERR_SEND_IN_BROADCAST)
         return ipx_fail(IPG_EDEVICE,
                         "The function send_message should not be used in the SINGLE_BROADCAST version; only "
                         "broadcast() should be called, and once per superstep maximum.");
+    if (err & IPX_ERR_SUPERSTEP_LIMIT) return ipx_fail(IPG_EDEVICE, "superstep limit (IPG_MAX_SUPERSTEPS) reached");
     if (err & IPX_ERR_COPY_TIMEOUT)
         return ipx_fail(IPG_EDEVICE, "a bulk copy into shared memory did not complete in time (results kept exact)");
     if (err & IPX_ERR_RESERVED_MESSAGE)
         return ipx_fail(IPG_EDEVICE, "a broadcast FP64 message had all 64 bits set, the pattern the single_broadcast "
                                      "engine reserves for 'no broadcast' (build with -DIPX_SB_DENSE=0 to allow it)");
-    if (err) return ipx_fail(IPG_EDEVICE, "a kernel reported an error");
-#if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SINGLE_BROADCAST
-    *count = ipx_h.h_ctr[s & 3];
-#elif IPX_VERSION == IPX_SPREAD
-    *count = ipx_h.h_lcnt[4];
-#else
-    *count = (uint64_t)ipx_h.h_lcnt[4] + ipx_h.h_lcnt[5] + ipx_h.h_lcnt[6];
-#endif
-#if IPX_VERSION == IPX_SINGLE_BROADCAST
-    ipx_h.edges += ipx_h.c.E;
-#else
-    if (ipx_h.c.pull_ok && ipx_h.h_ctr[IPX_CTR_MODE]) {
-        ipx_h.edges += ipx_h.c.E; /* a pulled superstep reads every row */
-        ipx_h.pulled_supersteps++;
-    } else {
-        for (int k = 8; k < 11; k++) ipx_h.edges += ipx_h.h_ctr[k];
-    }
-    for (int k = 11; k < 14; k++) ipx_h.edges += ipx_h.h_ctr[k];
-#endif
-    if (ipx_h.profile) {
-        for (int i = 0; i < ipx_h.npev; i++) {
-            float kms = 0.f;
-            IPX_CU(cudaEventElapsedTime(&kms, ipx_h.pev[0][i], ipx_h.pev[1][i]));
-            ipx_h.prof_ms[ipx_h.pkid[i]] += kms;
-            ipx_h.prof_timed[ipx_h.pkid[i]]++;
-        }
-        ipx_h.npev = 0;
-        ipx_account_bytes(s, frontier);
-    }
-    float ms = 0.f;
-    IPX_CU(cudaEventElapsedTime(&ms, ipx_h.ev0, ipx_h.ev1));
-    double sec = ms * 1e-3;
-    ipx_h.total_seconds += sec;
-    ipx_h.counts.push_back(*count);
-    ip_active_vertices = *count;
-    if (!ipx_h.quiet) {
-        printf("Superstep%zuDuration:%f\n", (size_t)s, sec);
-        printf("Superstep%zuActiveVertexCount:%zu\n", (size_t)s, (size_t)*count);
-    }
-    return IPG_OK;
+    return ipx_fail(IPG_EDEVICE, "a kernel reported an error");
 }
 
 /* Enqueues one superstep's kernels on the engine stream.  Nothing here
  * depends on host-side values of the superstep: kernels read it (and the
- * mailbox parity) from device memory, so the same sequence serves the host
- * loop and the captured loop. */
-static int ipx_enqueue_superstep()
+ * mailbox parity) from device memory, the last one advances it, and a kernel
+ * enqueued beyond the program's end returns at once, so the same sequence
+ * serves the host loop and the captured loop.  first: superstep 0 may be
+ * among those the sequence serves. */
+static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
 {
     const ipx_consts& c = ipx_h.c;
     cudaStream_t st = ipx_h.st;
     const uint32_t g = ipx_h.grid_compute;
     const uint32_t ge = ipx_h.grid_edge;
-    const uint64_t V = c.V;
-    (void)V;
+    (void)first;
     (void)ge;
 #if IPX_VERSION == IPX_SINGLE_BROADCAST
-    /* superstep 0's compute phase (returns at once later), before
-     * ipx_k_begin_superstep moves ip_get_superstep() to the next superstep */
-    IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_compute_sb0<<<g, ipx_h.tb, 0, st>>>());
-#endif
-    IPX_LAUNCH(IPX_K_CTRL, ipx_k_begin_superstep<<<1, 1, 0, st>>>());
-#if IPX_VERSION == IPX_COMBINER
-    IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_compute_combiner<<<g, ipx_h.tb, 0, st>>>());
-    IPX_CU(cudaMemsetAsync(ipx_h.lcnt, 0, 4 * sizeof(uint32_t), st));
-    IPX_OK(ipx_deliver_superstep(ge));
-    IPX_LAUNCH(IPX_K_COUNT, ipx_k_count_combiner<<<ipx_grid(4), 256, 0, st>>>());
-#elif IPX_VERSION == IPX_SPREAD
-    IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_compute_spread<<<g, ipx_h.tb, 0, st>>>(ipx_h.tlist[0], ipx_h.lcnt + 4));
-    IPX_CU(cudaMemsetAsync(ipx_h.lcnt, 0, 8 * sizeof(uint32_t), st));
-    IPX_OK(ipx_deliver_superstep(ge));
-    /* spread keeps one received bitmap (recv[0] == recv[1]): its compaction
-     * clears it before the next superstep's sends */
-    IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.recv[0], V, nullptr, 0, 0, ipx_h.tlist[0], nullptr, nullptr,
-                                                   ipx_h.lcnt + 4, nullptr, 1, st)));
-#elif IPX_VERSION == IPX_SINGLE_BROADCAST
-    {
-        /* gather of this superstep fused with the next one's compute phase */
-        const bool hot = c.in_adj_hot != nullptr;
+    /* superstep 0's compute phase (returns at once later) */
+    if (first) IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_compute_sb0<<<g, ipx_h.tb, 0, st>>>());
+    /* gather of this superstep fused with the next one's compute phase */
+    const bool hot = c.in_adj_hot != nullptr;
 #if !IPX_HUB_WARP
-        if (c.chunks)
-            IPX_LAUNCH(IPX_K_GATHER2, hot ? ipx_k_gather_hubs<true><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>()
+    if (c.chunks)
+        IPX_LAUNCH(IPX_K_GATHER_HUBS, hot ? ipx_k_gather_hubs<true><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>()
                                           : ipx_k_gather_hubs<false><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>());
 #endif
-        IPX_LAUNCH(IPX_K_GATHER1, hot ? ipx_k_gather_compute<true><<<ge, ipx_h.tb, 0, st>>>()
-                                      : ipx_k_gather_compute<false><<<ge, ipx_h.tb, 0, st>>>());
-    }
+    IPX_LAUNCH(IPX_K_GATHER, hot ? ipx_k_gather_compute<true><<<ge, ipx_h.tb, 0, st>>>(loop)
+                                 : ipx_k_gather_compute<false><<<ge, ipx_h.tb, 0, st>>>(loop));
 #else
-    uint64_t* edges_b = (uint64_t*)(c.ctr + 8);
-    uint64_t* edges_t = (uint64_t*)(c.ctr + 11);
-    IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_compute_ssb<<<g, ipx_h.tb, 0, st>>>(ipx_h.tlist[0], ipx_h.tlist[1],
-                                                                            ipx_h.tlist[2], ipx_h.lcnt + 4));
-    IPX_CU(cudaMemsetAsync(ipx_h.lcnt, 0, 8 * sizeof(uint32_t), st));
-    IPX_LAUNCH(IPX_K_COMPACT_B, IPX_OK(ipg_compact(c.bcaster, V, c.row, ipx_push_t0(), ipx_h.tune.t1, ipx_h.blist[0],
-                                                   ipx_h.blist[1], ipx_h.blist[2], ipx_h.lcnt, edges_b, 1, st)));
-    IPX_LAUNCH(IPX_K_MARK0, ipx_k_mark<0><<<ge, ipx_h.tb, 0, st>>>(ipx_h.blist[0], ipx_h.lcnt + 0, ipx_h.hub_prefix));
-    IPX_LAUNCH(IPX_K_MARK1, ipx_k_mark<1><<<ge, ipx_h.tb, 0, st>>>(ipx_h.blist[1], ipx_h.lcnt + 1, ipx_h.hub_prefix));
-    IPX_LAUNCH(IPX_K_CTRL, ipx_k_hub_prefix<><<<1, 1024, 0, st>>>(ipx_h.blist[2], ipx_h.lcnt + 2, c.row, ipx_h.hub_prefix,
-                                                                   (uint32_t*)c.push_owner));
-    IPX_LAUNCH(IPX_K_MARK2, ipx_k_mark<2><<<ge, ipx_h.tb, 0, st>>>(ipx_h.blist[2], ipx_h.lcnt + 2, ipx_h.hub_prefix));
-    IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.bt, V, c.in_row, ipx_h.tune.t0, ipx_h.tune.t1, ipx_h.tlist[0], ipx_h.tlist[1],
-                                                   ipx_h.tlist[2], ipx_h.lcnt + 4, edges_t, 1, st)));
-    IPX_LAUNCH(IPX_K_GATHER0, ipx_k_gather<0, false><<<ge, ipx_h.tb, 0, st>>>(ipx_h.tlist[0], ipx_h.lcnt + 4, 0));
-    IPX_LAUNCH(IPX_K_GATHER1, ipx_k_gather<1, false><<<ge, ipx_h.tb, 0, st>>>(ipx_h.tlist[1], ipx_h.lcnt + 5, 0));
-    IPX_LAUNCH(IPX_K_GATHER2, ipx_k_gather<2, false><<<ge, ipx_h.tb, 0, st>>>(ipx_h.tlist[2], ipx_h.lcnt + 6, 0));
+    IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_front<<<g, ipx_h.tb, 0, st>>>(ipx_h.front_words));
+#if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
+    IPX_LAUNCH(IPX_K_MARK, ipx_k_mark<<<ipg_sm_count(), IPX_MARK_THREADS, ipx_h.mark_words * 4, st>>>(ipx_h.mark_words));
+    IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.bt, c.V, c.in_row, ipx_h.tune.t0, ipx_h.tune.t1, c.tlist[0],
+                                                   c.tlist[1], c.tlist[2], c.stat->tn, (uint64_t*)c.stat->tedges, 0, st)));
+    IPX_LAUNCH(IPX_K_GATHER, ipx_k_gather_targets<<<ge, ipx_h.tb, 0, st>>>(loop));
+#else
+    /* delivery: push along the broadcasters' rows, or, on a symmetric graph
+     * when their out-edges pass the threshold, pull over every row; the
+     * kernels of the other direction return at once */
+    IPX_LAUNCH(IPX_K_PUSH, ipx_k_push<<<ge, ipx_h.tb, 0, st>>>());
+    if (c.pull_ok) {
+        const ipg_bins& b = ipx_h.gbins;
+        const uint32_t gp = ipx_h.grid_pull;
+        IPX_LAUNCH(IPX_K_PULLD0, ipx_k_pull_deliver<0><<<gp, ipx_h.tb, 0, st>>>(b.d_list[0], b.count[0], ipx_h.pull_prefix));
+        IPX_LAUNCH(IPX_K_PULLD1, ipx_k_pull_deliver<1><<<gp, ipx_h.tb, 0, st>>>(b.d_list[1], b.count[1], ipx_h.pull_prefix));
+        IPX_LAUNCH(IPX_K_PULLD2, ipx_k_pull_deliver<2><<<gp, ipx_h.tb, 0, st>>>(b.d_list[2], b.count[2], ipx_h.pull_prefix));
+    }
+    IPX_LAUNCH(IPX_K_COUNT, ipx_k_count<<<ipx_h.grid_count, IPX_THREADS, 0, st>>>(loop));
+#endif
 #endif
     IPX_CU(cudaGetLastError());
     return IPG_OK;
@@ -873,39 +771,72 @@ static uint64_t ipx_max_supersteps()
     return (IPX_PULL && n > (uint64_t)IPX_NO_STAMP - 1) ? (uint64_t)IPX_NO_STAMP - 1 : n;
 }
 
-/* Host-driven loop: one synchronisation per superstep, which gives the
- * reference's per-superstep log lines with their durations. */
+/* Host-driven loop: IPX_BATCH supersteps are enqueued before the host waits
+ * for their records (one at a time while profiling); those beyond the
+ * program's end do nothing.  Gives the reference's per-superstep log lines
+ * with their durations. */
 static int ipx_run_host_loop()
 {
-    const uint64_t V = ipx_h.c.V;
-    uint64_t count = ip_active_vertices;
-    const uint64_t max_supersteps = ipx_max_supersteps();
-    for (uint64_t s = 0;; s++) {
 #if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SINGLE_BROADCAST
-        if (count == 0) break; /* while(ip_active_vertices != 0), combiner_postamble.h:134 */
-#else
-        if (s > 0 && count == 0) break; /* while(first || count > 0), combiner_spread_postamble.h:212 */
+    if (ip_active_vertices == 0) return IPG_OK; /* while(ip_active_vertices != 0), combiner_postamble.h:134 */
 #endif
-        if (s >= max_supersteps) return ipx_fail(IPG_EDEVICE, "superstep limit (IPG_MAX_SUPERSTEPS) reached");
-        /* vertices the compute kernel runs: the frontier (spread versions) or
-         * the active ones of the previous superstep */
-        const uint64_t frontier = (s == 0) ? V : count;
-        IPX_OK(ipx_set_superstep(s));
-        IPX_CU(cudaEventRecord(ipx_h.ev0, ipx_h.st));
-        IPX_OK(ipx_enqueue_superstep());
-        IPX_OK(ipx_end_superstep(s, &count, frontier));
-        ip_superstep = s + 1;
+    cudaStream_t st = ipx_h.st;
+    const ipx_consts& c = ipx_h.c;
+    const ipx_loop loop = {0, 0, (unsigned long long)ipx_max_supersteps()};
+    uint64_t count = ip_active_vertices;
+    IPX_OK(ipx_set_superstep(0));
+    for (uint64_t s = 0;;) {
+        const int batch = ipx_h.profile ? 1 : IPX_BATCH;
+        IPX_CU(cudaEventRecord(ipx_h.ev0, st));
+        for (int k = 0; k < batch; k++) IPX_OK(ipx_enqueue_superstep(loop, s + k == 0));
+        IPX_CU(cudaEventRecord(ipx_h.ev1, st));
+        IPX_CU(cudaMemcpyAsync(ipx_h.pin->hist, c.hist + (s % IPX_HIST) * 4, (size_t)batch * 32, cudaMemcpyDeviceToHost, st));
+        if (ipx_h.profile)
+            IPX_CU(cudaMemcpyAsync(&ipx_h.pin->last, c.last, sizeof(ipx_stat), cudaMemcpyDeviceToHost, st));
+        IPX_CU(cudaStreamSynchronize(st));
+        IPX_CU(cudaGetLastError());
+        float ms = 0.f;
+        IPX_CU(cudaEventElapsedTime(&ms, ipx_h.ev0, ipx_h.ev1));
+        ipx_h.total_seconds += ms * 1e-3;
+        for (int k = 0; k < batch; k++, s++) {
+            const unsigned long long* h = ipx_h.pin->hist[k];
+            const uint64_t frontier = (s == 0) ? c.V : count; /* vertices the compute kernel ran */
+            const uint32_t err = (uint32_t)(h[2] >> 32);
+            /* a program at the superstep bound has run it */
+            if (err & ~IPX_ERR_SUPERSTEP_LIMIT) return ipx_fail_device(err);
+            count = h[0];
+            ipx_h.edges += h[1];
+            if (h[2] & 1) ipx_h.pulled_supersteps++;
+            if (ipx_h.profile) {
+                for (int i = 0; i < ipx_h.npev; i++) {
+                    float kms = 0.f;
+                    IPX_CU(cudaEventElapsedTime(&kms, ipx_h.pev[0][i], ipx_h.pev[1][i]));
+                    ipx_h.prof_ms[ipx_h.pkid[i]] += kms;
+                    ipx_h.prof_timed[ipx_h.pkid[i]]++;
+                }
+                ipx_h.npev = 0;
+                ipx_account_bytes(s, frontier);
+            }
+            ipx_h.counts.push_back(count);
+            ip_active_vertices = count;
+            ip_superstep = s + 1;
+            if (!ipx_h.quiet) {
+                printf("Superstep%zuDuration:%f\n", (size_t)s, (double)h[3] * 1e-9);
+                printf("Superstep%zuActiveVertexCount:%zu\n", (size_t)s, (size_t)count);
+            }
+            if (err) return ipx_fail_device(err);
+            if (count == 0) return IPG_OK;
+        }
     }
-    return IPG_OK;
 }
 
-/* Captured loop: the superstep's kernels, then ipx_k_advance, as the body of
- * a CUDA-graph while node; one launch runs the program to quiescence with no
+/* Captured loop: the superstep's kernels as the body of a CUDA-graph while
+ * node, whose condition the last of them sets; one launch runs the program to quiescence with no
  * host synchronisation between supersteps.  The graph is built once per
  * attached graph and reused by later runs. */
 /* Adds the superstep loop as a root node of `graph`: a while node whose
- * body is one superstep's kernels followed by ipx_k_advance, which records
- * the superstep and sets the condition on the device. */
+ * body is one superstep's kernels, the last of which records the superstep
+ * and sets the condition on the device. */
 static int ipx_add_loop_node(cudaGraph_t graph)
 {
     cudaGraphConditionalHandle handle;
@@ -923,8 +854,8 @@ static int ipx_add_loop_node(cudaGraph_t graph)
     uint64_t before[IPX_K_N];
     memcpy(before, ipx_h.prof_launches, sizeof before);
     IPX_CU(cudaStreamBeginCaptureToGraph(ipx_h.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    int r = ipx_enqueue_superstep();
-    IPX_LAUNCH(IPX_K_CTRL, ipx_k_advance<<<1, 1, 0, ipx_h.st>>>(handle, (unsigned long long)ipx_max_supersteps()));
+    const ipx_loop loop = {handle, 1, (unsigned long long)ipx_max_supersteps()};
+    int r = ipx_enqueue_superstep(loop, true);
     cudaGraph_t captured = nullptr;
     cudaError_t e = cudaStreamEndCapture(ipx_h.st, &captured);
     ipx_h.profile = prof;
@@ -1003,7 +934,7 @@ static int ipx_loop_collect(double seconds)
         const unsigned long long* h = S <= IPX_HIST ? &hist[s * 4] : nullptr;
         const uint64_t count = h ? h[0] : 0;
         if (h) ipx_h.edges += h[1];
-        if (h && h[2]) ipx_h.pulled_supersteps++;
+        if (h && (h[2] & 1)) ipx_h.pulled_supersteps++;
         ipx_h.counts.push_back(count);
         if (!ipx_h.quiet) {
             /* one launch for all supersteps: durations are the loop's average */
@@ -1016,17 +947,7 @@ static int ipx_loop_collect(double seconds)
     ip_superstep = S;
     ip_active_vertices = ipx_h.counts.empty() ? 0 : ipx_h.counts.back();
     ipx_h.host_valid = false;
-    if (err & IPX_ERR_SEND_IN_BROADCAST)
-        return ipx_fail(IPG_EDEVICE,
-                        "The function send_message should not be used in the SINGLE_BROADCAST version; only "
-                        "broadcast() should be called, and once per superstep maximum.");
-    if (err & IPX_ERR_SUPERSTEP_LIMIT) return ipx_fail(IPG_EDEVICE, "superstep limit (IPG_MAX_SUPERSTEPS) reached");
-    if (err & IPX_ERR_COPY_TIMEOUT)
-        return ipx_fail(IPG_EDEVICE, "a bulk copy into shared memory did not complete in time (results kept exact)");
-    if (err & IPX_ERR_RESERVED_MESSAGE)
-        return ipx_fail(IPG_EDEVICE, "a broadcast FP64 message had all 64 bits set, the pattern the single_broadcast "
-                                     "engine reserves for 'no broadcast' (build with -DIPX_SB_DENSE=0 to allow it)");
-    if (err) return ipx_fail(IPG_EDEVICE, "a kernel reported an error");
+    if (err) return ipx_fail_device(err);
     return IPG_OK;
 }
 

@@ -81,6 +81,7 @@ struct ipg_pr_plan {
     float* xs2 = nullptr;
     ipg_hubs hubs{};                   // rows above hub_min in chunks
     uint64_t hub_min = 0, chunk = 0;
+    bool quads = false;                // the gather lists take 128-bit loads
     float2* partial = nullptr;         // (sum, compensation) of every hub chunk
     uint32_t* arrived = nullptr;       // per hub the chunks arrived (0 between supersteps)
     uint32_t* shorts = nullptr;        // the short class: first the vertices with in-edges
@@ -542,6 +543,9 @@ extern "C" int ipg_pr_plan_create(ipg_graph* g, ipg_pr_plan** out)
         if ((r = ipg_graph_bins(gw, 1, ts, mid > ts ? mid : ts, &p->bins)) != IPG_OK) break;
         if ((r = ipg_graph_hubs(gw, 1, p->hub_min, p->chunk, &p->hubs)) != IPG_OK) break;
         if ((r = ipg_graph_view_get(gw, &p->gv)) != IPG_OK) break;
+        int quads = 0;
+        if ((r = ipg_graph_quads(gw, 1, &quads)) != IPG_OK) break;
+        p->quads = quads != 0;
         const uint64_t V = p->gv.V;
         if ((r = pr_alloc(p, &p->b[0], V)) != IPG_OK) break;
         if ((r = pr_alloc(p, &p->b[1], V)) != IPG_OK) break;
@@ -618,7 +622,7 @@ extern "C" int ipg_pr_run_f32(ipg_pr_plan* p, uint32_t rounds, double damping, i
     a.row = p->gv.d_row;
     a.in_row = p->gv.d_in_row;
     a.in_adj = (const uint32_t*)p->gv.d_in_adj;
-    a.quads = ((uintptr_t)a.in_adj & 15) == 0 && p->hubs.ids_readable >= 4 && (p->hubs.ids_readable & 3) == 0;
+    a.quads = p->quads;
     for (int k = 0; k < 3; k++) {
         a.list[k] = p->bins.d_list[k];
         a.n[k] = p->bins.count[k];

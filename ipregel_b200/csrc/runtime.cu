@@ -640,8 +640,8 @@ extern "C" int ipg_graph_build_in(ipg_graph* g)
     IPG_TRY(ipg_dev_alloc(&g->in_adj, padded_ids(E) * (uint64_t)g->v.id_bytes));
     g->in_adj_bytes = padded_ids(E) * (uint64_t)g->v.id_bytes;
     if (g->v.d_wgt) {
-        IPG_TRY(ipg_dev_alloc(&g->in_wgt, (E ? E : 1) * (uint64_t)g->v.weight_bytes));
-        g->in_wgt_bytes = (E ? E : 1) * (uint64_t)g->v.weight_bytes;
+        IPG_TRY(ipg_dev_alloc(&g->in_wgt, padded_ids(E) * (uint64_t)g->v.weight_bytes));
+        g->in_wgt_bytes = padded_ids(E) * (uint64_t)g->v.weight_bytes;
     }
     k_fill_u64<<<grid_for(V + 1, 256), 256, 0, st>>>((uint64_t*)g->in_row, V + 1, E);
     if (E) {
@@ -695,7 +695,7 @@ static int alloc_out(ipg_graph* g, uint64_t V, uint64_t E, int id_bytes, int wei
     IPG_TRY(ipg_dev_alloc(&g->row, g->row_bytes));
     IPG_TRY(ipg_dev_alloc(&g->adj, g->adj_bytes));
     if (weight_bytes) {
-        g->wgt_bytes = (E ? E : 1) * (uint64_t)weight_bytes;
+        g->wgt_bytes = padded_ids(E) * (uint64_t)weight_bytes;
         IPG_TRY(ipg_dev_alloc(&g->wgt, g->wgt_bytes));
     }
     g->v.V = V;
@@ -861,7 +861,7 @@ extern "C" int ipg_graph_degree_order(ipg_graph* g, int need_in, ipg_order* out)
         r = ipg_dev_alloc(&o->in_row, o->in_row_bytes);
         if (r == IPG_OK) r = ipg_dev_alloc(&o->in_adj, o->in_adj_bytes);
         if (r == IPG_OK && g->v.d_in_wgt) {
-            o->in_wgt_bytes = (E ? E : 1) * (uint64_t)g->v.weight_bytes;
+            o->in_wgt_bytes = padded_ids(E) * (uint64_t)g->v.weight_bytes;
             r = ipg_dev_alloc(&o->in_wgt, o->in_wgt_bytes);
         }
         if (r != IPG_OK) {  // the copy stays as it was, without in-lists
@@ -1546,7 +1546,7 @@ __global__ void k_weights(const uint64_t* __restrict__ row, uint64_t V, uint64_t
 static int attach_weights(ipg_graph* g, uint32_t wmax, uint64_t seed)
 {
     if (g->wgt) return IPG_OK;
-    g->wgt_bytes = (g->v.E ? g->v.E : 1) * 4;
+    g->wgt_bytes = padded_ids(g->v.E) * 4;
     IPG_TRY(ipg_dev_alloc(&g->wgt, g->wgt_bytes));
     g->v.weight_bytes = 4;
     g->v.d_wgt = g->wgt;
@@ -1973,13 +1973,25 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     c.hubs.edges = h.edges;
     c.hubs.d_owner = owner;
     c.hubs.chunks = h.chunks;
-    // a list array the runtime allocated is padded; a caller's ends at E
-    const void* ids = use_in ? g->v.d_in_adj : g->v.d_adj;
-    const bool own = (ids == g->adj && g->owns_out) || (ids == g->in_adj && ids);
-    c.hubs.ids_readable = own ? padded_ids(E) : E;
     c.hub_min = hub_min;
     c.chunk = chunk;
     c.valid = true;
     *hubs = c.hubs;
+    return IPG_OK;
+}
+
+extern "C" int ipg_graph_quads(const ipg_graph* g, int use_in, int* quads)
+{
+    if (!g || !quads) return fail(IPG_EINVAL, "ipg_graph_quads: null argument");
+    *quads = 0;
+    if (use_in && !g->v.has_in) return fail(IPG_EINVAL, "ipg_graph_quads: the graph has no in-lists");
+    const void* ids = use_in ? g->v.d_in_adj : g->v.d_adj;
+    const void* wgt = use_in ? g->v.d_in_wgt : g->v.d_wgt;
+    // arrays the runtime allocated are padded; a caller's end at E
+    const bool own = (ids == g->adj && g->owns_out) || (ids == g->in_adj && ids);
+    const uint64_t E = g->v.E;
+    const bool whole = own || (E >= 4 && (E & 3) == 0);
+    const bool aligned = ((uintptr_t)ids & 15) == 0 && (g->v.weight_bytes != 4 || ((uintptr_t)wgt & 15) == 0);
+    *quads = (g->v.id_bytes == 4 && ids && whole && aligned) ? 1 : 0;
     return IPG_OK;
 }

@@ -1,6 +1,7 @@
-"""The single_broadcast gather at the sizes where its rows change hands: row
-lengths around the 128-bit id loads, the lanes per row, the degree classes and
-the hub chunks, with the edge array ending at every position of a load."""
+"""The row walks (pull gather, push, target marking) at the sizes where rows
+change hands: lengths around the 128-bit id loads, the lanes per row, the
+degree classes and the hub chunks, with the edge array ending at every
+position of a load; and the compute kernel's bitmaps at their edges."""
 import numpy as np
 import pytest
 
@@ -80,5 +81,76 @@ def test_rows_of_every_length(app, version, id_bits, variant, tail):
     finally:
         eng.set_tuning()
         eng.set_order(True)
+        eng.release()
+        graph.free()
+
+
+@pytest.mark.parametrize("tail", [0, 1, 2, 3])
+@pytest.mark.parametrize("app,version,id_bits,generic", [
+    ("cc", "combiner", 32, False), ("cc", "spread", 32, False), ("cc", "single_broadcast_spread", 32, False),
+    ("cc", "spread", 64, False), ("cc", "single_broadcast_spread", 64, False), ("cc", "spread", 32, True),
+    ("sssp_weighted", "combiner", 32, False), ("sssp_weighted", "spread", 32, False), ("pagerank", "combiner", 32, False),
+    ("pagerank", "spread", 32, True)])
+def test_pushed_rows_of_every_length(app, version, id_bits, generic, tail):
+    import ipregel_b200 as ip
+    g = _graph(tail)
+    rng = np.random.default_rng(tail)
+    wgt = rng.integers(1, 256, g.E).astype(np.uint32) if app == "sssp_weighted" else None
+    g = O.CSR(g.V, g.E, g.idx, g.adj, wgt)
+    want, counts, _ = O.run(g, app, version, id_bytes=id_bits // 8)
+    adj = g.adj if id_bits == 32 else g.adj.astype(np.uint64)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, adj, wgt=wgt, id_bytes=id_bits // 8)
+    eng = ip.Engine(app, version, id_bits, generic)
+    eng.set_quiet(True)
+    try:
+        if app == "pagerank":
+            eng.set_param("rounds", 10)
+        if app == "sssp_weighted":
+            eng.set_param("source", 0)
+        for tune in (dict(), dict(t0=4, t1=4096), dict(t0=2, t1=3), dict(block=64, t0=64, t1=200)):
+            for order in (True, False):
+                eng.set_order(order)
+                eng.set_tuning(**tune)
+                eng.attach(graph)
+                res = eng.run()
+                assert res.counts == [int(c) for c in counts], (tune, order)
+                if app == "pagerank":
+                    assert float(np.max(np.abs(res.values - want))) <= PR_TOL, (tune, order)
+                else:
+                    np.testing.assert_array_equal(res.values.astype(np.uint64), want.astype(np.uint64))
+    finally:
+        eng.set_tuning()
+        eng.set_order(True)
+        eng.release()
+        graph.free()
+
+
+@pytest.mark.parametrize("V", [1, 31, 32, 33, 127, 128, 129, 4095, 4097, 40_001, 700_001])
+@pytest.mark.parametrize("app,version", [("cc", "combiner"), ("cc", "spread"), ("cc", "single_broadcast_spread"),
+                                         ("sssp", "spread"), ("cc", "single_broadcast")])
+def test_bitmap_edges(app, version, V):
+    """Vertex counts around the words of the bitmaps, the steps of a warp and the batches of supersteps: a ring (the
+    frontier of two vertices crosses every word) for the small ones, a random graph for the others."""
+    import ipregel_b200 as ip
+    if V <= 129:
+        g = O.from_edges(V, [(i, (i + 1) % V) for i in range(V) if V > 1] + [((i + 1) % V, i) for i in range(V) if V > 2])
+    else:
+        g = O.gen_er(V, 3 * V, seed=V, undirected=True)
+    want, counts, _ = O.run(g, app, version)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, g.adj)
+    eng = ip.Engine(app, version)
+    eng.set_quiet(True)
+    try:
+        if app == "sssp":
+            eng.set_param("source", 0)
+        for loop in (False, True):
+            eng.set_graph_loop(loop)
+            eng.attach(graph)
+            for _ in range(2):
+                res = eng.run()
+                assert res.counts == [int(c) for c in counts]
+                np.testing.assert_array_equal(res.values.astype(np.uint64), want.astype(np.uint64))
+    finally:
+        eng.set_graph_loop(False)
         eng.release()
         graph.free()
