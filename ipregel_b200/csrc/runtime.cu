@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <atomic>
 #include <cerrno>
 #include <cstdarg>
@@ -212,29 +213,65 @@ struct ipg_graph {
     void* in_row = nullptr; uint64_t in_row_bytes = 0;
     void* in_adj = nullptr; uint64_t in_adj_bytes = 0;
     void* in_wgt = nullptr; uint64_t in_wgt_bytes = 0;
+    // Degree classes and hub tables, per direction, least recently asked for
+    // first.  Users of one graph (engines, split plans, servers) ask with
+    // thresholds of their own and hold what they got, so a set stays until
+    // the contents change; past DERIVED_MAX sets, or when memory is short,
+    // the least recently asked for goes.
+    template <class S>
+    struct Sets {
+        static constexpr size_t DERIVED_MAX = 16;
+        S set[DERIVED_MAX];
+        size_t n = 0;
+        void drop(size_t keep)
+        {
+            for (; n > keep; n--) {
+                ipg_dev_free(set[0].mem, set[0].bytes);
+                std::rotate(set, set + 1, set + n);
+            }
+        }
+        template <class F>
+        S* find(F is)
+        {
+            S* e = std::find_if(set, set + n, is);
+            if (e == set + n) return nullptr;
+            std::rotate(e, e + 1, set + n);
+            return set + n - 1;
+        }
+        // memory of a new set, which its maker adds or gives back
+        int alloc(void** p, uint64_t bytes)
+        {
+            drop(DERIVED_MAX - 1);
+            int r = ipg_dev_alloc(p, bytes);
+            while (r != IPG_OK && n) {
+                drop(n - 1);
+                r = ipg_dev_alloc(p, bytes);
+            }
+            return r;
+        }
+        void add(const S& s) { set[n++] = s; }
+    };
     struct BinCache {
-        bool valid = false;
         uint64_t t0 = 0, t1 = 0;
-        void* lists = nullptr;
+        void* mem = nullptr;
         uint64_t bytes = 0;
-        ipg_bins bins;
-    } bins[2];
+        ipg_bins bins = {};
+    };
     struct HubCache {
-        bool valid = false;
         uint64_t hub_min = 0, chunk = 0;
         void* mem = nullptr;
         uint64_t bytes = 0;
         ipg_hubs hubs = {};
-    } hubs[2];
+    };
+    Sets<BinCache> bins[2];
+    Sets<HubCache> hubs[2];
     // what was derived from the rows (which = 0), the in-lists (1) or both (-1)
     void drop_derived(int which = -1)
     {
         for (int k = 0; k < 2; k++) {
             if (which >= 0 && which != k) continue;
-            ipg_dev_free(bins[k].lists, bins[k].bytes);
-            bins[k] = BinCache();
-            ipg_dev_free(hubs[k].mem, hubs[k].bytes);
-            hubs[k] = HubCache();
+            bins[k].drop(0);
+            hubs[k].drop(0);
         }
     }
     // ipg_graph_refill_host's own stream, device words (check bits, degree
@@ -1847,6 +1884,14 @@ extern "C" int ipg_bitmap_popc_or(const uint32_t* d_a, const uint32_t* d_b, uint
     return IPG_OK;
 }
 
+// Memory of a set being made, given back when the set does not come to be added.
+struct SetMem {
+    void* p = nullptr;
+    uint64_t bytes;
+    explicit SetMem(uint64_t b) : bytes(b) {}
+    ~SetMem() { ipg_dev_free(p, bytes); }
+};
+
 // ---------------------------------------------------------------------------
 // Static degree bins of all vertices (cached per direction).
 // ---------------------------------------------------------------------------
@@ -1854,17 +1899,17 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
 {
     if (!g || !bins) return fail(IPG_EINVAL, "ipg_graph_bins: null argument");
     if (use_in && !g->v.has_in) IPG_TRY(ipg_graph_build_in(g));
-    auto& c = g->bins[use_in ? 1 : 0];
-    if (c.valid && c.t0 == t0 && c.t1 == t1) {
-        *bins = c.bins;
+    auto& sets = g->bins[use_in ? 1 : 0];
+    if (const auto* had = sets.find([&](const ipg_graph::BinCache& b) { return b.t0 == t0 && b.t1 == t1; })) {
+        *bins = had->bins;
         return IPG_OK;
     }
-    ipg_dev_free(c.lists, c.bytes);
-    c.lists = nullptr;
-    c.valid = false;
     const uint64_t V = g->v.V;
+    ipg_graph::BinCache c;
     c.bytes = (V ? V : 1) * 4 + 64;
-    IPG_TRY(ipg_dev_alloc(&c.lists, c.bytes));
+    SetMem mem(c.bytes);
+    IPG_TRY(sets.alloc(&mem.p, mem.bytes));
+    c.mem = mem.p;
     DevBuf cnt, l1, l2;
     IPG_TRY(cnt.alloc(64));
     IPG_TRY(l1.alloc((V ? V : 1) * 4));
@@ -1872,14 +1917,14 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
     IPG_CUDA(cudaMemset(cnt.p, 0, 64));
     const uint64_t* row = use_in ? g->v.d_in_row : g->v.d_row;
     uint64_t* d_esum = (uint64_t*)((char*)cnt.p + 32);
-    IPG_TRY(ipg_compact(nullptr, V, row, t0, t1, (uint32_t*)c.lists, l1.as<uint32_t>(), l2.as<uint32_t>(),
+    IPG_TRY(ipg_compact(nullptr, V, row, t0, t1, (uint32_t*)c.mem, l1.as<uint32_t>(), l2.as<uint32_t>(),
                         cnt.as<uint32_t>(), d_esum, 0, nullptr));
     uint32_t h[3] = {0, 0, 0};
     uint64_t esum[3] = {0, 0, 0};
     IPG_CUDA(cudaMemcpy(h, cnt.p, 12, cudaMemcpyDeviceToHost));
     IPG_CUDA(cudaMemcpy(esum, d_esum, 24, cudaMemcpyDeviceToHost));
     // Pack the three lists back to back in one allocation.
-    uint32_t* base = (uint32_t*)c.lists;
+    uint32_t* base = (uint32_t*)c.mem;
     if (h[1]) IPG_CUDA(cudaMemcpy(base + h[0], l1.p, (uint64_t)h[1] * 4, cudaMemcpyDeviceToDevice));
     if (h[2]) IPG_CUDA(cudaMemcpy(base + h[0] + h[1], l2.p, (uint64_t)h[2] * 4, cudaMemcpyDeviceToDevice));
     // Lists within a class come out tile-ordered, which is id order, since
@@ -1910,7 +1955,8 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
     c.bins.t1 = t1;
     c.t0 = t0;
     c.t1 = t1;
-    c.valid = true;
+    sets.add(c);
+    mem.p = nullptr;
     *bins = c.bins;
     return IPG_OK;
 }
@@ -1939,9 +1985,10 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     if (!g || !hubs) return fail(IPG_EINVAL, "ipg_graph_hubs: null argument");
     if (chunk < 1) return fail(IPG_EINVAL, "ipg_graph_hubs: chunks hold at least one edge");
     if (use_in && !g->v.has_in) IPG_TRY(ipg_graph_build_in(g));
-    auto& c = g->hubs[use_in ? 1 : 0];
-    if (c.valid && c.hub_min == hub_min && c.chunk == chunk) {
-        *hubs = c.hubs;
+    auto& sets = g->hubs[use_in ? 1 : 0];
+    if (const auto* had =
+            sets.find([&](const ipg_graph::HubCache& h) { return h.hub_min == hub_min && h.chunk == chunk; })) {
+        *hubs = had->hubs;
         return IPG_OK;
     }
     const uint64_t V = g->v.V, E = g->v.E;
@@ -1949,11 +1996,12 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     if (hubs_max > V) hubs_max = V;
     const uint64_t chunks_max = E / chunk + hubs_max + 1;
     if (chunks_max >= (1ULL << 32)) return fail(IPG_EINVAL, "ipg_graph_hubs: too many chunks for 32-bit indices");
-    ipg_dev_free(c.mem, c.bytes);
-    c = ipg_graph::HubCache();
     const uint64_t hub_b = align256((hubs_max + 1) * 16), own_b = align256(chunks_max * 4);
-    IPG_TRY(ipg_dev_alloc(&c.mem, hub_b + own_b + 256));
+    ipg_graph::HubCache c;
     c.bytes = hub_b + own_b + 256;
+    SetMem mem(c.bytes);
+    IPG_TRY(sets.alloc(&mem.p, mem.bytes));
+    c.mem = mem.p;
     uint4* hub = (uint4*)c.mem;
     uint32_t* owner = (uint32_t*)((char*)c.mem + hub_b);
     uint32_t* cnt = (uint32_t*)((char*)c.mem + hub_b + own_b);
@@ -1975,7 +2023,8 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     c.hubs.chunks = h.chunks;
     c.hub_min = hub_min;
     c.chunk = chunk;
-    c.valid = true;
+    sets.add(c);
+    mem.p = nullptr;
     *hubs = c.hubs;
     return IPG_OK;
 }

@@ -154,3 +154,32 @@ def test_bitmap_edges(app, version, V):
         eng.set_graph_loop(False)
         eng.release()
         graph.free()
+
+
+def test_users_of_one_graph_keep_their_classes(monkeypatch):
+    """An engine and precision-split plans with other thresholds hold classes and hub tables of the same graph at
+    the same time; running one after another has been made leaves its results bitwise as they were."""
+    import ipregel_b200 as ip
+    g = _graph(1)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, g.adj)
+    eng = ip.Engine("pagerank", "single_broadcast")
+    eng.set_quiet(True)
+    plans = []
+    try:
+        eng.set_param("rounds", 10)
+        eng.attach(graph)
+        first = eng.run().values.copy()
+        runs = []
+        for t0, t1 in ((16, 4096), (4, 100), (8, 40)):
+            monkeypatch.setenv("IPG_PR_T0", str(t0))
+            monkeypatch.setenv("IPG_PR_T1", str(t1))
+            plans.append(ip.PageRankF32(graph))
+            runs.append(plans[-1].run(rounds=10)[0].copy())
+        np.testing.assert_array_equal(eng.run().values, first)
+        for plan, x in zip(plans, runs):
+            np.testing.assert_array_equal(plan.run(rounds=10)[0], x)
+    finally:
+        for plan in plans:
+            plan.free()
+        eng.release()
+        graph.free()
