@@ -56,6 +56,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 extern "C" int ipg_internal_fail(int code, const char* msg);
@@ -65,11 +66,12 @@ namespace {
 constexpr int MP_K = 64;
 constexpr int PP_K = 32;           // PPR lanes: a row of 32 FP32 quotients is one 128-byte line
 constexpr int PP_Q = PP_K / 4;     // float4 quads per row
-constexpr int PP_SLOTS = 32 / PP_Q;  // rows per warp load instruction
-static_assert(PP_K <= 64 && PP_Q <= 16 && PP_K % 16 == 0, "PPR lanes: a warp covers whole rows");
+constexpr int PP_SLOTS = 4;        // edge streams of a row above PP_T0
+static_assert(PP_Q == 8, "PPR lanes: a superstep walks 1, 2, 4 or 8 quads of a row");
 constexpr int SRV_THREADS = 256;
 constexpr uint64_t MP_T0 = 8, MP_T1 = 4096;
-constexpr uint64_t PP_T0 = 64;                      // PPR: quads up to this degree, then warps
+constexpr uint64_t PP_T0 = 64;                      // PPR: quads up to this degree, then several streams a row,
+constexpr uint64_t PP_T1 = 512, PP_CHUNK = 512;     // and above this one chunks of as many edges
 constexpr uint64_t PP_NOALLOC_MAX_V = 67108864ull;  // ipg_degree_classes_noalloc's vertex limit
 constexpr uint32_t HUB_CHUNK = 1024;
 constexpr uint32_t SRV_INF = 0xffffffffu;
@@ -897,7 +899,19 @@ struct PpLanes {
     float* out[PP_K];       // result buffer of a lane in its last gather, else null
     uint32_t seed[PP_K];
     unsigned long long active;  // lanes gathering this superstep
+    // The quads of lanes the superstep walks (bit per quad): those with a
+    // gathering lane, and those whose next row holds values of lanes that
+    // have left.  Thread q of a group takes quad (map >> 4q) & 15; 15: none.
+    uint32_t quads, map;
 };
+
+// The quad of thread q of a group; whether any of its lanes gathers.
+__device__ __forceinline__ int pp_quad(const PpLanes& L, int q, bool& on)
+{
+    const int Q = (int)((L.map >> (4 * q)) & 15u);
+    on = Q < PP_Q && ((L.active >> (4 * (Q & 7))) & 0xFULL) != 0;
+    return Q;
+}
 
 struct PpArgs {
     const uint64_t* __restrict__ row;
@@ -905,6 +919,9 @@ struct PpArgs {
     const float* __restrict__ b_cur;
     float* __restrict__ b_next;
     float2* __restrict__ partial;  // (sum, compensation) per hub chunk and lane
+    const uint4* __restrict__ hub;       // {vertex, first chunk, chunks}
+    const uint32_t* __restrict__ owner;  // chunk -> hub
+    uint64_t hubs, chunks;
 };
 
 // Compensated summation; the value of a pair is s + c.  Per term, Kahan's
@@ -962,9 +979,9 @@ __device__ __forceinline__ float4 pp_row(const PpArgs& a, uint32_t u, int q)
     return reinterpret_cast<const float4*>(a.b_cur + (uint64_t)u * PP_K)[q];
 }
 
-// Threads q < PP_Q of a group finish lanes 4q..4q+3 of vertex v from their
-// compensated sums: x to the result buffer of a lane in its last gather,
-// else the quotient x / deg into the next row.
+// Finishes lanes 4q..4q+3 of vertex v from their compensated sums: x to the
+// result buffer of a lane in its last gather, else the quotient x / deg into
+// the next row.
 __device__ __forceinline__ void pp_finish_quad(const PpArgs& a, const PpLanes& L, uint64_t v, uint64_t deg, int q,
                                                const float* s, const float* c)
 {
@@ -984,175 +1001,206 @@ __device__ __forceinline__ void pp_finish_quad(const PpArgs& a, const PpLanes& L
     if (deg) reinterpret_cast<float4*>(a.b_next + v * PP_K)[q] = make_float4(bn[0], bn[1], bn[2], bn[3]);
 }
 
-// A warp gathers [e0, e1): thread t takes lane quad t % PP_Q and edge slot
-// t / PP_Q (PP_SLOTS slots), reading the neighbour's quad as one float4, so
-// each load instruction reads PP_SLOTS whole rows.  Every 4 rows of a thread
-// are summed pairwise and added compensated; the next 32 ids are loaded while
-// the current rows are in flight.  Then the slots of each quad merge (TwoSum),
-// and threads 0..PP_Q-1 hold the totals of their quads.  The order of a
-// lane's terms depends on the edge list only, not on which lanes are active.
-__device__ __forceinline__ void pp_gather_warp(const PpArgs& a, uint64_t e0, uint64_t e1, bool quad_on, float* s,
-                                               float* c)
+// A group of PP_SLOTS * NQ threads gathers [e0, e1): thread t takes lane quad
+// t % NQ and edge slot t / NQ, reading the neighbour's quad as one float4, so
+// each load instruction reads 4 (rows) x NQ quads of every group in the warp.
+// Every 4 rows of a thread are summed pairwise and added compensated; the next
+// 32 ids are loaded while the current rows are in flight.  Then the slots of
+// each quad merge (TwoSum), and threads 0..NQ-1 hold the totals of their
+// quads.  The order of a lane's terms depends on the edge list only, not on
+// which lanes are active or how many quads are walked.
+template <int NQ>
+__device__ __forceinline__ void pp_gather_group(const PpArgs& a, uint64_t e0, uint64_t e1, int Q, bool on, float* s,
+                                                float* c)
 {
-    const int lane = threadIdx.x & 31, slot = lane / PP_Q, q = lane % PP_Q;
+    constexpr int GS = PP_SLOTS * NQ, IPT = 32 / GS;  // threads, ids a thread loads per 32 edges
+    const int lane = threadIdx.x & 31, t = lane & (GS - 1), gb = lane - t, slot = t / NQ;
+    const unsigned mask = GS == 32 ? FULL : ((1u << (GS & 31)) - 1u) << gb;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 4; i++) s[i] = c[i] = 0.0f;
-    uint32_t uj = (e0 + lane < e1) ? ld_edge(&a.adj[e0 + lane]) : 0u;
+    uint32_t uj[IPT], un[IPT];
+#pragma unroll
+    for (int i = 0; i < IPT; i++) uj[i] = (e0 + i * GS + t < e1) ? ld_edge(&a.adj[e0 + i * GS + t]) : 0u;
     for (uint64_t e = e0; e < e1; e += 32) {
-        const uint32_t un = (e + 32 + lane < e1) ? ld_edge(&a.adj[e + 32 + lane]) : 0u;
+#pragma unroll
+        for (int i = 0; i < IPT; i++)
+            un[i] = (e + 32 + i * GS + t < e1) ? ld_edge(&a.adj[e + 32 + i * GS + t]) : 0u;
         const int nj = (int)((e1 - e) < 32 ? (e1 - e) : 32);
 #pragma unroll
-        for (int h = 0; h < 32 / PP_SLOTS; h += 4) {
+        for (int h = 0; h < 8; h += 4) {
             float4 x[4];
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const int jj = (h + r) * PP_SLOTS + slot;
-                const uint32_t u = __shfl_sync(FULL, uj, jj);
-                x[r] = (quad_on && jj < nj) ? pp_row(a, u, q) : z;
+                const uint32_t u = __shfl_sync(mask, uj[(h + r) / NQ], gb + ((h + r) % NQ) * PP_SLOTS + slot);
+                x[r] = (on && jj < nj) ? pp_row(a, u, Q) : z;
             }
-            if (quad_on) pp_add4(s, c, pp_sum4(x[0], x[1], x[2], x[3]));
+            if (on) pp_add4(s, c, pp_sum4(x[0], x[1], x[2], x[3]));
         }
-        uj = un;
+#pragma unroll
+        for (int i = 0; i < IPT; i++) uj[i] = un[i];
     }
 #pragma unroll
-    for (int off = PP_Q; off < 32; off <<= 1)
+    for (int off = NQ; off < GS; off <<= 1)
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const float s2 = __shfl_xor_sync(FULL, s[i], off), c2 = __shfl_xor_sync(FULL, c[i], off);
+            const float s2 = __shfl_xor_sync(mask, s[i], off), c2 = __shfl_xor_sync(mask, c[i], off);
             pp_merge(s[i], c[i], s2, c2);
         }
 }
 
-// PP_Q threads per low-degree vertex (degree <= PP_T0): thread q of the group
-// takes lane quad q of every in-neighbour's row, so a warp reads 32 / PP_Q
-// whole rows per load instruction and no partial sums need merging.  Four
-// threads of the group load four consecutive ids at a time and the group
-// shares them by shuffle; the four rows are summed pairwise and added
-// compensated, in edge order.
+// NQ threads per low-degree vertex (degree <= PP_T0): thread q of the group
+// takes one walked quad of every in-neighbour's row, so a warp reads 32 / NQ
+// rows per load instruction and no partial sums need merging.  The group's
+// first threads load four consecutive ids at a time and share them by
+// shuffle; the four rows are summed pairwise and added compensated, in edge
+// order.
+//
+// The walk is bound by the latency of the rows, whatever part of them is
+// used: with a thread for each of the 8 quads a superstep took the same time
+// for 1 busy lane as for 32, because the threads of idle quads waited along.
+// With threads for the walked quads only, and rows above 512 edges in chunks
+// (a warp on up to 4,096 edges was the tail of a superstep), 20 supersteps at
+// undirected R-MAT scale 20 went from 19.4 to 6.0 ms for 1 lane, 20.5 to 6.9
+// for 7 (2 quads), 20.9 to 10.3 for 16 and 21.1 to 14.6 for 32; with narrow
+// groups alone 13.4, 17.0, 19.1 and 22.0.
+template <int NQ>
 __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_rows(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
                                                          uint64_t n)
 {
-    const int lane = threadIdx.x & 31, q = lane % PP_Q, gb = lane - q;
-    const unsigned gmask = ((1u << PP_Q) - 1u) << gb;
-    const bool quad_on = (L.active >> (4 * q)) & 0xFULL;
+    constexpr int IPT = NQ < 4 ? 4 / NQ : 1;  // ids a thread loads per four edges
+    const int lane = threadIdx.x & 31, q = lane % NQ, gb = lane - q;
+    const unsigned gmask = ((1u << NQ) - 1u) << gb;
+    bool on;
+    const int Q = pp_quad(L, q, on);
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / PP_Q;
+    const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / NQ;
+    auto load_ids = [&](uint64_t e, uint64_t e1, uint32_t* u) {
+#pragma unroll
+        for (int i = 0; i < IPT; i++) {
+            const int j = q * IPT + i;
+            u[i] = (j < 4 && e + j < e1) ? a.adj[e + j] : 0u;
+        }
+    };
     // The next vertex's list entry, row bounds and first four ids are loaded
     // while this vertex's rows are gathered, and the next four ids of a row
     // while its current four rows are: the chain list -> offsets -> ids ->
     // rows leaves the critical path except for its last link.  The threads
     // of a group share i, so they leave the loop together.
-    uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / PP_Q;
+    uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / NQ;
     uint64_t v = 0, e0 = 0, e1 = 0;
-    uint32_t u0 = 0;
+    uint32_t u0[IPT] = {}, u0n[IPT] = {};
     if (i < n) {
         v = list[i];
         e0 = a.row[v];
         e1 = a.row[v + 1];
-        u0 = (q < 4 && e0 + q < e1) ? a.adj[e0 + q] : 0u;
+        load_ids(e0, e1, u0);
     }
     for (; i < n; i += groups) {
         const uint64_t in = i + groups;
         uint64_t vn = 0, e0n = 0, e1n = 0;
-        uint32_t u0n = 0;
         if (in < n) {
             vn = list[in];
             e0n = a.row[vn];
             e1n = a.row[vn + 1];
-            u0n = (q < 4 && e0n + q < e1n) ? a.adj[e0n + q] : 0u;
+            load_ids(e0n, e1n, u0n);
         }
         float s[4], c[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) s[k] = c[k] = 0.0f;
-        uint32_t uj = u0;
         for (uint64_t e = e0; e < e1; e += 4) {
-            const uint32_t un = (q < 4 && e + 4 + q < e1) ? a.adj[e + 4 + q] : 0u;
+            uint32_t un[IPT];
+            load_ids(e + 4, e1, un);
             const int ne = (int)((e1 - e) < 4 ? (e1 - e) : 4);
             float4 x[4];
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                const uint32_t u = __shfl_sync(gmask, uj, gb + r);
-                x[r] = (quad_on && r < ne) ? pp_row(a, u, q) : z;
+                const uint32_t u = __shfl_sync(gmask, u0[r % IPT], gb + r / IPT);
+                x[r] = (on && r < ne) ? pp_row(a, u, Q) : z;
             }
-            if (quad_on) pp_add4(s, c, pp_sum4(x[0], x[1], x[2], x[3]));
-            uj = un;
+            if (on) pp_add4(s, c, pp_sum4(x[0], x[1], x[2], x[3]));
+#pragma unroll
+            for (int k = 0; k < IPT; k++) u0[k] = un[k];
         }
-        pp_finish_quad(a, L, v, e1 - e0, q, s, c);
+        if (Q < PP_Q) pp_finish_quad(a, L, v, e1 - e0, Q, s, c);
         v = vn;
         e0 = e0n;
         e1 = e1n;
-        u0 = u0n;
+#pragma unroll
+        for (int k = 0; k < IPT; k++) u0[k] = u0n[k];
     }
 }
 
-// A warp per vertex of higher degree (up to MP_T1).
-__global__ void __launch_bounds__(SRV_THREADS) k_pp_vertices(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
+// PP_SLOTS * NQ threads per vertex of higher degree (up to PP_T1; hubs are
+// passed over).
+template <int NQ>
+__global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_vertices(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
                                                              uint64_t n)
 {
-    const int lane = threadIdx.x & 31;
-    const bool quad_on = (L.active >> (4 * (lane % PP_Q))) & 0xFULL;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    constexpr int GS = PP_SLOTS * NQ;
+    const int t = threadIdx.x & (GS - 1);
+    bool on;
+    const int Q = pp_quad(L, t % NQ, on);
+    const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / GS;
+    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / GS; i < n; i += groups) {
         const uint64_t v = list[i];
         const uint64_t e0 = a.row[v], e1 = a.row[v + 1];
+        if (e1 - e0 > PP_T1) continue;  // the group's threads share v
         float s[4], c[4];
-        pp_gather_warp(a, e0, e1, quad_on, s, c);
-        if (lane < PP_Q) pp_finish_quad(a, L, v, e1 - e0, lane, s, c);
+        pp_gather_group<NQ>(a, e0, e1, Q, on, s, c);
+        if (t < NQ && Q < PP_Q) pp_finish_quad(a, L, v, e1 - e0, Q, s, c);
     }
 }
 
-// Hubs: a warp per HUB_CHUNK edges, partial sums per chunk and lane...
-__global__ void __launch_bounds__(SRV_THREADS) k_pp_hub_chunks(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
-                                                               uint32_t n, const uint32_t* __restrict__ prefix)
+// Hubs: as many threads per PP_CHUNK edges, partial sums per chunk and lane...
+template <int NQ>
+__global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_hub_chunks(PpArgs a, PpLanes L)
 {
-    if (!n) return;
-    const int lane = threadIdx.x & 31;
-    const bool quad_on = (L.active >> (4 * (lane % PP_Q))) & 0xFULL;
-    const uint32_t chunks = prefix[n];
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
-        const uint32_t i = hub_of_chunk(prefix, n, (uint32_t)c);
-        const uint64_t v = list[i];
-        const uint64_t e0 = a.row[v] + (uint64_t)((uint32_t)c - prefix[i]) * HUB_CHUNK;
-        const uint64_t end = a.row[v + 1];
+    constexpr int GS = PP_SLOTS * NQ;
+    const int t = threadIdx.x & (GS - 1);
+    bool on;
+    const int Q = pp_quad(L, t % NQ, on);
+    const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / GS;
+    for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / GS; c < a.chunks; c += groups) {
+        const uint4 hub = a.hub[a.owner[c]];
+        const uint64_t e0 = a.row[hub.x] + ((uint32_t)c - hub.y) * PP_CHUNK, end = a.row[hub.x + 1];
         float s[4], cc[4];
-        pp_gather_warp(a, e0, e0 + HUB_CHUNK < end ? e0 + HUB_CHUNK : end, quad_on, s, cc);
-        if (lane < PP_Q)
+        pp_gather_group<NQ>(a, e0, e0 + PP_CHUNK < end ? e0 + PP_CHUNK : end, Q, on, s, cc);
+        if (t < NQ && Q < PP_Q)
 #pragma unroll
-            for (int j = 0; j < 4; j++) a.partial[c * PP_K + 4 * lane + j] = make_float2(s[j], cc[j]);
+            for (int j = 0; j < 4; j++) a.partial[c * PP_K + 4 * Q + j] = make_float2(s[j], cc[j]);
     }
 }
 
-// ...then a warp per hub merges its chunks' partials in chunk order (a
-// thread per lane) and threads 0..PP_Q-1 finish the hub's quads.
-__global__ void __launch_bounds__(SRV_THREADS) k_pp_hub_finish(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
-                                                               uint32_t n, const uint32_t* __restrict__ prefix)
+// ...then a warp per hub and walked quad merges the hub's chunks: a thread per
+// lane of the quad and eighth of the chunks, in chunk order, then the eighths.
+__global__ void __launch_bounds__(SRV_THREADS) k_pp_hub_finish(PpArgs a, PpLanes L, int nq)
 {
-    __shared__ float2 sh[SRV_THREADS / 32][PP_K];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, j = lane & 3, part = lane >> 2;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const uint64_t v = list[i];
-        for (int k = lane; k < PP_K; k += 32) {
-            float s = 0.0f, c = 0.0f;
-            for (uint32_t ch = prefix[i]; ch < prefix[i + 1]; ch++) {
-                const float2 p = a.partial[(uint64_t)ch * PP_K + k];
-                pp_merge(s, c, p.x, p.y);
-            }
-            sh[w][k] = make_float2(s, c);
+    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < a.hubs * nq; i += warps) {
+        const uint4 hub = a.hub[i / nq];
+        bool on;
+        const int Q = pp_quad(L, (int)(i % nq), on);
+        const uint32_t per = (hub.z + 7) / 8, c0 = part * per, c1 = c0 + per < hub.z ? c0 + per : hub.z;
+        float s = 0.0f, c = 0.0f;
+        for (uint32_t k = c0; k < c1; k++) {
+            const float2 p = a.partial[(uint64_t)(hub.y + k) * PP_K + 4 * Q + j];
+            pp_merge(s, c, p.x, p.y);
         }
-        __syncwarp();
-        if (lane < PP_Q) {
-            float s4[4], c4[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                s4[j] = sh[w][4 * lane + j].x;
-                c4[j] = sh[w][4 * lane + j].y;
-            }
-            pp_finish_quad(a, L, v, a.row[v + 1] - a.row[v], lane, s4, c4);
+        for (int off = 4; off < 32; off <<= 1) {
+            const float s2 = __shfl_xor_sync(FULL, s, off), c2 = __shfl_xor_sync(FULL, c, off);
+            pp_merge(s, c, s2, c2);
         }
-        __syncwarp();
+        float s4[4], c4[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            s4[k] = __shfl_sync(FULL, s, k);
+            c4[k] = __shfl_sync(FULL, c, k);
+        }
+        if (lane == 0) pp_finish_quad(a, L, hub.x, a.row[hub.x + 1] - a.row[hub.x], Q, s4, c4);
     }
 }
 
@@ -1190,6 +1238,7 @@ struct Graph {
     ipg_bins bins{};
     uint32_t* hub_prefix = nullptr;  // nh + 1 entries, then the hub count and the union-find error word
     uint64_t hub_chunks = 0;
+    uint64_t pp_hubs = 0, pp_chunks = 0;  // rows above PP_T1 and their chunks
     uint32_t* cc_err = nullptr;
     uint32_t* cc_giant = nullptr;
     bool classes = false;
@@ -1228,9 +1277,14 @@ struct Group {
     int cc_lane = -1;  // label-propagation CC lane admitted in this admission pass
     // PPR
     float* b[2] = {nullptr, nullptr};
+    uint32_t dirty[2] = {0, 0};  // quads of each buffer that may hold nonzero quotients
     float2* partial = nullptr;
-    // gather classes: quads for degree <= PP_T0, warps up to MP_T1 (hubs
-    // above, from the graph's classes); null when the graph is too large for
+    // the hubs (rows above PP_T1) and their chunks
+    uint4* hub = nullptr;
+    uint32_t* owner = nullptr;
+    uint64_t hubs = 0, chunks = 0;
+    // gather classes: quads for degree <= PP_T0, streams up to PP_T1 (hubs
+    // above); null when the graph is too large for
     // ipg_degree_classes_noalloc, and then the graph's classes serve
     uint32_t* pp_list = nullptr;
     uint64_t* pp_tot = nullptr;
@@ -1308,7 +1362,7 @@ uint64_t group_bytes(const Graph* G, int kind)
 {
     const uint64_t V = G->gv.V, E = G->gv.E;
     if (kind == 0) return V * (MP_K * 4 + 16 + 12) + V / 4 + (E / (MP_T1 + 1) + 2) * 4 + 4096;
-    return V * (PP_K * 4 * 2 + 4) + (E / HUB_CHUNK + V / MP_T1 + 2) * (PP_K * 8) + 4096;
+    return V * (PP_K * 4 * 2 + 4) + G->pp_chunks * (PP_K * 8 + 4) + G->pp_hubs * 16 + 4096;
 }
 
 // Frees idle groups (least recently used first) until `need` more bytes fit
@@ -1350,6 +1404,10 @@ int graph_classes(Graph* Gr, cudaStream_t st)
     cudaMemcpyAsync(&chunks, Gr->hub_prefix + nh, 4, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return ipg_internal_fail(IPG_ECUDA, "serve: hub prefix failed");
     Gr->hub_chunks = chunks;
+    ipg_hubs H{};
+    if ((r = ipg_graph_hubs(Gr->g, 0, PP_T1, PP_CHUNK, &H)) != IPG_OK) return r;
+    Gr->pp_hubs = H.hubs;
+    Gr->pp_chunks = H.chunks;
     Gr->classes = true;
     return IPG_OK;
 }
@@ -1428,7 +1486,21 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
         if (r == IPG_OK) r = graph_classes(Gr, G->st);
         if (r == IPG_OK) r = galloc(G, &G->b[0], V * PP_K);
         if (r == IPG_OK) r = galloc(G, &G->b[1], V * PP_K);
-        if (r == IPG_OK) r = galloc(G, &G->partial, Gr->hub_chunks * PP_K);
+        ipg_hubs H{};
+        if (r == IPG_OK) r = ipg_graph_hubs(Gr->g, 0, PP_T1, PP_CHUNK, &H);
+        if (r == IPG_OK) r = galloc(G, &G->partial, H.chunks * PP_K);
+        // copies of its own, counted in the group's bytes
+        if (r == IPG_OK) r = galloc(G, &G->hub, H.hubs);
+        if (r == IPG_OK) r = galloc(G, &G->owner, H.chunks);
+        if (r == IPG_OK) {
+            G->hubs = H.hubs;
+            G->chunks = H.chunks;
+            if ((H.hubs && cudaMemcpyAsync(G->hub, H.d_hub, H.hubs * 16, cudaMemcpyDeviceToDevice, G->st) != cudaSuccess) ||
+                (H.chunks &&
+                 cudaMemcpyAsync(G->owner, H.d_owner, H.chunks * 4, cudaMemcpyDeviceToDevice, G->st) != cudaSuccess) ||
+                cudaStreamSynchronize(G->st) != cudaSuccess)
+                r = ipg_internal_fail(IPG_ECUDA, "serve: PPR hub table failed");
+        }
         if (r == IPG_OK) {
             // quotients of idle lanes are 0: an admitted lane sets its seed only
             cudaMemsetAsync(G->b[0], 0, V * PP_K * 4, G->st);
@@ -1440,11 +1512,11 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
             // the server's calls of ipg_degree_classes_noalloc are serialised
             // by this synchronisation (its scratch is shared)
             uint64_t tot[6] = {0, 0, 0, 0, 0, 0};
-            if (r == IPG_OK) r = ipg_degree_classes_noalloc(V, Gr->gv.d_row, PP_T0, MP_T1, G->pp_list, G->pp_tot, G->st);
+            if (r == IPG_OK) r = ipg_degree_classes_noalloc(V, Gr->gv.d_row, PP_T0, PP_T1, G->pp_list, G->pp_tot, G->st);
             if (r == IPG_OK && (cudaMemcpyAsync(tot, G->pp_tot, sizeof tot, cudaMemcpyDeviceToHost, G->st) != cudaSuccess ||
                                 cudaStreamSynchronize(G->st) != cudaSuccess))
                 r = ipg_internal_fail(IPG_ECUDA, "serve: PPR degree classes failed");
-            if (r == IPG_OK && tot[2] != Gr->bins.count[2])
+            if (r == IPG_OK && tot[2] != G->hubs)
                 r = ipg_internal_fail(IPG_EINVAL, "serve: PPR hub class differs from the graph's");
             G->pp_n[0] = tot[0];
             G->pp_n[1] = tot[1];
@@ -1564,6 +1636,7 @@ void admit(ipg_server* S, Group* G, double now)
             const uint32_t g = resident_cap(k_mp_init_lane, thread_grid(V));
             if (q.kind == IPG_QUERY_PPR) {
                 k_pp_admit<<<1, 1, 0, G->st>>>(G->b[G->cur], G->G->gv.d_row, q.src, k);
+                G->dirty[G->cur] |= 1u << (k / 4);
                 G->it[k] = 0;
                 G->seed[k] = (uint32_t)q.src;
             } else if (q.kind == IPG_QUERY_CC) {
@@ -1681,6 +1754,10 @@ int launch_superstep(ipg_server* S, Group* G)
         a.b_cur = G->b[G->cur];
         a.b_next = G->b[G->cur ^ 1];
         a.partial = G->partial;
+        a.hub = G->hub;
+        a.owner = G->owner;
+        a.hubs = G->hubs;
+        a.chunks = G->chunks;
         PpLanes L;
         L.active = G->busy;
         for (int k = 0; k < PP_K; k++) {
@@ -1699,16 +1776,37 @@ int launch_superstep(ipg_server* S, Group* G)
         const uint64_t n0 = G->pp_list ? G->pp_n[0] : B.count[0];
         const uint32_t* l1 = G->pp_list ? G->pp_list + n0 : B.d_list[1];
         const uint64_t n1 = G->pp_list ? G->pp_n[1] : B.count[1];
-        if (n0)
-            k_pp_rows<<<resident_cap(k_pp_rows, thread_grid(n0 * PP_Q)), SRV_THREADS, 0, G->st>>>(a, L, l0, n0);
-        if (n1)
-            k_pp_vertices<<<resident_cap(k_pp_vertices, warp_grid(n1)), SRV_THREADS, 0, G->st>>>(a, L, l1, n1);
-        if (B.count[2]) {
-            k_pp_hub_chunks<<<resident_cap(k_pp_hub_chunks, warp_grid(Gr->hub_chunks)), SRV_THREADS, 0, G->st>>>(
-                a, L, B.d_list[2], (uint32_t)B.count[2], Gr->hub_prefix);
-            k_pp_hub_finish<<<resident_cap(k_pp_hub_finish, warp_grid(B.count[2])), SRV_THREADS, 0, G->st>>>(
-                a, L, B.d_list[2], (uint32_t)B.count[2], Gr->hub_prefix);
-        }
+        // the quads walked: those with a busy lane, and those whose next row
+        // still holds quotients of lanes that have left (written as 0 now)
+        uint32_t busy_quads = 0;
+        for (int q = 0; q < PP_Q; q++)
+            if ((G->busy >> (4 * q)) & 0xFULL) busy_quads |= 1u << q;
+        L.quads = busy_quads | G->dirty[G->cur ^ 1];
+        L.map = 0xffffffffu;
+        int nq = 0;
+        for (int q = 0; q < PP_Q; q++)
+            if ((L.quads >> q) & 1u) {
+                L.map = (L.map & ~(15u << (4 * nq))) | ((uint32_t)q << (4 * nq));
+                nq++;
+            }
+        G->dirty[G->cur ^ 1] = busy_quads;
+        auto launch = [&](auto width) {
+            constexpr int NQ = decltype(width)::value;
+            if (n0)
+                k_pp_rows<NQ><<<resident_cap(k_pp_rows<NQ>, thread_grid(n0 * NQ)), SRV_THREADS, 0, G->st>>>(a, L, l0, n0);
+            if (n1)
+                k_pp_vertices<NQ><<<resident_cap(k_pp_vertices<NQ>, thread_grid(n1 * PP_SLOTS * NQ)), SRV_THREADS, 0,
+                                    G->st>>>(a, L, l1, n1);
+            if (a.chunks)
+                k_pp_hub_chunks<NQ><<<resident_cap(k_pp_hub_chunks<NQ>, thread_grid(a.chunks * PP_SLOTS * NQ)),
+                                      SRV_THREADS, 0, G->st>>>(a, L);
+        };
+        if (nq <= 1) launch(std::integral_constant<int, 1>());
+        else if (nq <= 2) launch(std::integral_constant<int, 2>());
+        else if (nq <= 4) launch(std::integral_constant<int, 4>());
+        else launch(std::integral_constant<int, 8>());
+        if (a.hubs)
+            k_pp_hub_finish<<<resident_cap(k_pp_hub_finish, warp_grid(a.hubs * nq)), SRV_THREADS, 0, G->st>>>(a, L, nq);
         G->cur ^= 1;
         S->stats.kernel_launches += 4;
     }
