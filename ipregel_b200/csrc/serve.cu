@@ -69,21 +69,29 @@ constexpr int PP_Q = PP_K / 4;     // float4 quads per row
 constexpr int PP_SLOTS = 4;        // edge streams of a row above PP_T0
 static_assert(PP_Q == 8, "PPR lanes: a superstep walks 1, 2, 4 or 8 quads of a row");
 constexpr int SRV_THREADS = 256;
-constexpr uint64_t MP_T0 = 8, MP_T1 = 4096;
-constexpr uint64_t PP_T0 = 64;                      // PPR: quads up to this degree, then several streams a row,
-constexpr uint64_t PP_T1 = 512, PP_CHUNK = 512;     // and above this one chunks of as many edges
+constexpr uint64_t MP_T0 = 8;       // min-plus: a thread a vertex up to this degree, then a warp
+// Rows above MP_T1 edges are hubs: HUB_CHUNK edges a warp.  A warp alone on a
+// row of up to 4,096 edges was the tail of every superstep: with 4096 / 1024 /
+// 512 / 256 / 128, 14 SSSP queries at undirected R-MAT scale 20 took 7.9 / 6.0
+// / 5.8 / 5.4 / 5.8 ms and 40 took 21.6 / 17.6 / 16.8 / 15.7 / 15.2.
+constexpr uint64_t MP_T1 = 256;
+constexpr uint32_t HUB_CHUNK = 256;
+constexpr uint64_t PP_T0 = 64;    // PPR: quads up to this degree, then several streams a row up to MP_T1
 constexpr uint64_t PP_NOALLOC_MAX_V = 67108864ull;  // ipg_degree_classes_noalloc's vertex limit
-constexpr uint32_t HUB_CHUNK = 1024;
 constexpr uint32_t SRV_INF = 0xffffffffu;
 constexpr unsigned FULL = 0xffffffffu;
-// Up to MP_SPARSE lanes of a vertex: a thread per edge, each relaxing all.
-constexpr int MP_SPARSE = 8;
+// Up to MP_SPARSE lanes of a vertex: a thread per edge, each relaxing all (2,
+// 4 and 8 took 4.80, 4.75 and 5.3 ms for 14 queries, 15.1, 14.7 and 14.9 for 40).
+constexpr int MP_SPARSE = 4;
 // A min-plus superstep pulls (symmetric graphs) when its frontier holds at
-// least E / MP_PULL_DIV edges and at least MP_PULL_LANES lanes are busy.  On
-// R-MAT graphs of scale 22 and 25 with 32 busy lanes, the dense supersteps
-// took 15-40 % less time pulled than pushed; with 5 lanes, 3-4 times more.
+// least E / MP_PULL_DIV edges and at least MP_PULL_LANES lanes are busy.  A
+// pull reads a neighbour's whole 256-byte row, a push the quads of its lanes
+// in use, so a pull pays only where most are: dense supersteps pulled against
+// pushed took, for all queries, 13.0 / 8.1 ms with 32 lanes, 13.6 / 13.5 with
+// 40 and 15.3 / 15.4 with 64 at R-MAT scale 20, 5.5 / 5.8 with 40 and 6.2 /
+// 6.7 with 64 at scale 18, 50 / 47 and 53.6 / 53.6 at scale 22.
 constexpr uint64_t MP_PULL_DIV = 4;
-constexpr int MP_PULL_LANES = 16;
+constexpr int MP_PULL_LANES = 40;
 // Resident CTAs per SM the min-plus kernels are compiled for (64 registers).
 #define MP_CTAS 4
 
@@ -102,14 +110,12 @@ double now_s()
 __device__ __forceinline__ uint32_t ld_edge(const uint32_t* p) { return __ldcs(p); }
 
 // Status of a min-plus group after a superstep, copied to the host in one
-// transfer: lane flags, list sizes, hub chunks of list 2, least deferred
-// distance of each lane.
+// transfer: lane flags, list sizes, least deferred distance of each lane.
 struct MpStatus {
     unsigned long long any;   // lanes that improved a distance
     unsigned long long near;  // lanes that relaxed a vertex below their threshold
     unsigned long long far;   // lanes that deferred a vertex
     uint32_t cnt[3];
-    uint32_t chunks;
     uint32_t far_min[64];     // least deferred distance per lane
     unsigned long long work;  // lane-edge relaxations examined (edges x lanes relaxing them)
     unsigned long long esum[3];  // degree sums of the next frontier's classes
@@ -144,53 +150,20 @@ uint32_t resident_cap(K kernel, uint32_t want)
     return std::min(want, it->second);
 }
 
-// prefix[i] = sum over j < i of ceil(deg(list[j]) / HUB_CHUNK); prefix[n] =
-// total, also written to *total when given.
-__global__ void __launch_bounds__(1024) k_chunk_prefix(const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                                                       const uint64_t* __restrict__ row, uint32_t* __restrict__ prefix,
-                                                       uint32_t* __restrict__ total)
-{
-    __shared__ uint32_t s[1024];
-    __shared__ uint32_t carry;
-    const uint32_t n = *count;
-    const int t = threadIdx.x;
-    if (t == 0) carry = 0;
-    __syncthreads();
-    for (uint32_t base = 0; base < n; base += 1024) {
-        const uint32_t i = base + t;
-        uint32_t c = 0;
-        if (i < n) {
-            const uint64_t v = list[i];
-            c = (uint32_t)((row[v + 1] - row[v] + HUB_CHUNK - 1) / HUB_CHUNK);
-        }
-        s[t] = c;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            const uint32_t x = t >= off ? s[t - off] : 0;
-            __syncthreads();
-            s[t] += x;
-            __syncthreads();
-        }
-        if (i < n) prefix[i] = carry + s[t] - c;
-        __syncthreads();
-        if (t == 1023) carry += s[1023];
-        __syncthreads();
-    }
-    if (t == 0) {
-        prefix[n] = carry;
-        if (total) *total = carry;
-    }
-}
+// The hubs of a graph (rows above MP_T1) in chunks of HUB_CHUNK edges.
+struct Hubs {
+    const uint4* __restrict__ hub;       // {vertex, first chunk, chunks}
+    const uint32_t* __restrict__ owner;  // chunk -> hub
+    uint64_t hubs, chunks;
+};
 
-__device__ __forceinline__ uint32_t hub_of_chunk(const uint32_t* __restrict__ prefix, uint32_t n, uint32_t c)
+// Edges [e0, e1) of chunk c of a hub.
+__device__ __forceinline__ void hub_chunk(const uint64_t* __restrict__ row, const uint4& hub, uint32_t c, uint64_t& e0,
+                                          uint64_t& e1)
 {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (prefix[mid] <= c) lo = mid;
-        else hi = mid;
-    }
-    return lo;
+    const uint64_t end = row[hub.x + 1];
+    e0 = row[hub.x] + (uint64_t)(c - hub.y) * HUB_CHUNK;
+    e1 = e0 + HUB_CHUNK < end ? e0 + HUB_CHUNK : end;
 }
 
 // ---------------------------------------------------------------------------
@@ -209,6 +182,7 @@ struct MpArgs {
     MpStatus* __restrict__ st;
     uint64_t wmask;                    // lanes whose edges carry their weight (SSSP)
     uint64_t busy;                     // lanes holding a query
+    Hubs hubs;
 };
 
 // Per-thread flags of a superstep, reduced per CTA into the status.
@@ -251,16 +225,24 @@ __device__ __forceinline__ void mp_mark(const MpArgs& a, uint32_t u, unsigned lo
 }
 
 // Edges e0 + lane, e0 + lane + stride, ... of v for its m <= L lanes; L is
-// the smallest of 1, 2, 4, 8 holding m, so no instruction is issued for
+// the smallest of 1, 2, 4 holding m, so no instruction is issued for
 // lanes v does not have.
 template <int L>
 __device__ __forceinline__ void mp_edges_sparse(const MpArgs& a, uint64_t e0, uint64_t e1, uint64_t lane,
                                                 uint64_t stride, int m, const int* ks, const uint32_t* ds,
                                                 MpAcc& acc)
 {
+    uint32_t un = 0, tn = 0;
+    if (e0 + lane < e1) {
+        un = ld_edge(&a.adj[e0 + lane]);
+        tn = a.wgt ? ld_edge(&a.wgt[e0 + lane]) : 0u;
+    }
     for (uint64_t e = e0 + lane; e < e1; e += stride) {
-        const uint32_t u = ld_edge(&a.adj[e]);
-        const uint32_t t = a.wgt ? ld_edge(&a.wgt[e]) : 0u;
+        const uint32_t u = un, t = tn;
+        if (e + stride < e1) {
+            un = ld_edge(&a.adj[e + stride]);
+            tn = a.wgt ? ld_edge(&a.wgt[e + stride]) : 0u;
+        }
         acc.work += (unsigned)m;
         const unsigned long long bits = mp_relax_edge<L>(a, u, t, m, ks, ds);
         if (bits) {
@@ -276,8 +258,68 @@ __device__ __forceinline__ void mp_edges_sparse_any(const MpArgs& a, uint64_t e0
 {
     if (m == 1) mp_edges_sparse<1>(a, e0, e1, lane, stride, m, ks, ds, acc);
     else if (m == 2) mp_edges_sparse<2>(a, e0, e1, lane, stride, m, ks, ds, acc);
-    else if (m <= 4) mp_edges_sparse<4>(a, e0, e1, lane, stride, m, ks, ds, acc);
     else mp_edges_sparse<MP_SPARSE>(a, e0, e1, lane, stride, m, ks, ds, acc);
+}
+
+// Edges [e0, e1) of v for the lanes R, by a warp: thread t takes quad t % NQ of
+// the lanes (all of R lie in the first NQ quads) and edge slot t / NQ, reading
+// four lanes of the neighbour's row as one 16-byte load, so an instruction
+// reads 32 / NQ rows and up to four such rows are in flight per thread; the
+// next 32 ids and weights are loaded meanwhile.  A superstep is bound by the
+// rows' latency and the L2's sectors: a thread per lane, one row an instruction
+// and half of the threads idle with up to 32 lanes in use, shared the chip
+// badly with the PPR supersteps beside it (a mix of 14 SSSP, 7 PPR and 3 CC
+// queries at scale 20: 17.1 ms, and 11.2 with quads; 14 SSSP alone 8.2 and 7.9).
+template <int NQ>
+__device__ __forceinline__ void mp_edges_quads(const MpArgs& a, uint64_t v, uint64_t e0, uint64_t e1,
+                                               unsigned long long R, MpAcc& acc)
+{
+    constexpr int S = 32 / NQ, U = NQ < 4 ? NQ : 4;  // edges an instruction, instructions in flight
+    const int lane = threadIdx.x & 31, q = lane % NQ, slot = lane / NQ;
+    const uint32_t act = (uint32_t)(R >> (4 * q)) & 15u, wm = (uint32_t)(a.wmask >> (4 * q)) & 15u;
+    const uint4 dv = reinterpret_cast<const uint4*>(a.dist + v * MP_K)[q];
+    const uint32_t d[4] = {dv.x, dv.y, dv.z, dv.w};
+    uint32_t wn = e0 + lane < e1 ? ld_edge(&a.adj[e0 + lane]) : 0u;
+    uint32_t tn = (e0 + lane < e1 && a.wgt) ? ld_edge(&a.wgt[e0 + lane]) : 0u;
+    for (uint64_t e = e0; e < e1; e += 32) {
+        const uint64_t ee = e + 32 + lane;
+        const uint32_t wj = wn, tj = tn;
+        wn = ee < e1 ? ld_edge(&a.adj[ee]) : 0u;
+        tn = (ee < e1 && a.wgt) ? ld_edge(&a.wgt[ee]) : 0u;
+        const int nj = (int)((e1 - e) < 32 ? (e1 - e) : 32);
+#pragma unroll
+        for (int h = 0; h < NQ; h += U) {
+            if (h * S >= nj) break;
+            uint32_t u[U], t[U];
+            uint4 c[U];
+#pragma unroll
+            for (int r = 0; r < U; r++) {
+                const int j = (h + r) * S + slot;
+                u[r] = __shfl_sync(FULL, wj, j);
+                t[r] = __shfl_sync(FULL, tj, j);
+                c[r] = make_uint4(0u, 0u, 0u, 0u);
+                if (j < nj && act) c[r] = reinterpret_cast<const uint4*>(a.dist + (uint64_t)u[r] * MP_K)[q];
+            }
+#pragma unroll
+            for (int r = 0; r < U; r++) {
+                const uint32_t cr[4] = {c[r].x, c[r].y, c[r].z, c[r].w};
+                uint32_t* du = a.dist + (uint64_t)u[r] * MP_K + 4 * q;
+                uint32_t bits = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t nd = d[k] + (((wm >> k) & 1u) ? t[r] : 0u);
+                    if (((act >> k) & 1u) && nd < cr[k]) {
+                        atomicMin(du + k, nd);
+                        bits |= 1u << k;
+                    }
+                }
+                if (bits) {
+                    mp_mark(a, u[r], (unsigned long long)bits << (4 * q));
+                    acc.any |= (unsigned long long)bits << (4 * q);
+                }
+            }
+        }
+    }
 }
 
 // Near-far ordering per lane.  A frontier lane whose distance at v is below
@@ -295,7 +337,7 @@ __device__ __forceinline__ void mp_defer(const MpArgs& a, uint32_t v, unsigned l
 
 // One warp relaxes the edges [e0, e1) of v for all of v's frontier lanes
 // below their thresholds: a thread per edge when few lanes remain, else a
-// thread per lane.  The warp classifies the lanes itself (a lane each).
+// thread per quad of lanes.  The warp classifies the lanes itself (a lane each).
 __device__ __forceinline__ void mp_relax(const MpArgs& a, uint64_t v, uint64_t e0, uint64_t e1, bool mark_deferred,
                                          MpAcc& acc, uint32_t* s_fmin)
 {
@@ -335,53 +377,12 @@ __device__ __forceinline__ void mp_relax(const MpArgs& a, uint64_t v, uint64_t e
         mp_edges_sparse_any(a, e0, e1, lane, 32, m, ks, ds, acc);
         return;
     }
-    const bool w0 = ((uint32_t)a.wmask >> lane) & 1u, w1 = ((uint32_t)(a.wmask >> 32) >> lane) & 1u;
-    for (uint64_t e = e0; e < e1; e += 32) {
-        const uint64_t ee = e + lane;
-        const uint32_t wj = ee < e1 ? ld_edge(&a.adj[ee]) : 0u;
-        const uint32_t tj = (ee < e1 && a.wgt) ? ld_edge(&a.wgt[ee]) : 0u;
-        const int nj = (int)((e1 - e) < 32 ? (e1 - e) : 32);
-        for (int j0 = 0; j0 < nj; j0 += 4) {
-            uint32_t u[4], t[4], c0[4], c1[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                u[q] = __shfl_sync(FULL, wj, (j0 + q) & 31);
-                t[q] = __shfl_sync(FULL, tj, (j0 + q) & 31);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const bool ok = j0 + q < nj;
-                c0[q] = (ok && act0) ? a.dist[(uint64_t)u[q] * MP_K + lane] : 0u;
-                c1[q] = (ok && act1) ? a.dist[(uint64_t)u[q] * MP_K + 32 + lane] : 0u;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if (j0 + q >= nj) break;
-                bool i0 = false, i1 = false;
-                if (act0) {
-                    const uint32_t nd = d0 + (w0 ? t[q] : 0u);
-                    if (nd < c0[q]) {
-                        atomicMin(&a.dist[(uint64_t)u[q] * MP_K + lane], nd);
-                        i0 = true;
-                    }
-                }
-                if (act1) {
-                    const uint32_t nd = d1 + (w1 ? t[q] : 0u);
-                    if (nd < c1[q]) {
-                        atomicMin(&a.dist[(uint64_t)u[q] * MP_K + 32 + lane], nd);
-                        i1 = true;
-                    }
-                }
-                const uint32_t b0 = Mlo ? __ballot_sync(FULL, i0) : 0u;
-                const uint32_t b1 = Mhi ? __ballot_sync(FULL, i1) : 0u;
-                if ((b0 | b1) && lane == 0) {
-                    const unsigned long long bits = (unsigned long long)b0 | ((unsigned long long)b1 << 32);
-                    mp_mark(a, u[q], bits);
-                    acc.any |= bits;
-                }
-            }
-        }
-    }
+    const int top = (63 - __clzll((long long)R)) / 4;  // highest quad with a relaxing lane
+    if (top < 1) mp_edges_quads<1>(a, v, e0, e1, R, acc);
+    else if (top < 2) mp_edges_quads<2>(a, v, e0, e1, R, acc);
+    else if (top < 4) mp_edges_quads<4>(a, v, e0, e1, R, acc);
+    else if (top < 8) mp_edges_quads<8>(a, v, e0, e1, R, acc);
+    else mp_edges_quads<16>(a, v, e0, e1, R, acc);
 }
 
 // The CTA's flags and least deferred distances into the status.
@@ -481,25 +482,35 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_vertices(MpArgs a, 
     mp_block_flush(acc, a, s_fmin);
 }
 
-// A warp per HUB_CHUNK edges of a frontier hub (class 2); the chunk holding
-// the hub's first edge marks its deferred lanes.
-__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_hubs(MpArgs a, const uint32_t* __restrict__ list,
-                                                                   const uint32_t* __restrict__ count,
-                                                                   const uint32_t* __restrict__ prefix)
+// A warp per HUB_CHUNK edges of a frontier hub; the hub's first chunk marks its
+// deferred lanes.  All chunks of the graph are looked at, those of hubs outside
+// the frontier left out by a ballot: `per` chunks a warp (as many as give every
+// resident warp work, at most 32), taken `groups` apart, since the chunks of one
+// hub lie together.
+__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_hubs(MpArgs a, uint32_t per, uint32_t groups)
 {
     __shared__ uint32_t s_fmin[MP_K];
     mp_fmin_init(s_fmin);
-    const uint32_t n = *count;
     MpAcc acc;
-    if (n) {
-        const uint32_t chunks = prefix[n];
-        const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-        for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
-            const uint32_t i = hub_of_chunk(prefix, n, (uint32_t)c);
-            const uint64_t v = list[i];
-            const uint64_t e0 = a.row[v] + (uint64_t)((uint32_t)c - prefix[i]) * HUB_CHUNK;
-            const uint64_t end = a.row[v + 1];
-            mp_relax(a, v, e0, e0 + HUB_CHUNK < end ? e0 + HUB_CHUNK : end, (uint32_t)c == prefix[i], acc, s_fmin);
+    const int lane = threadIdx.x & 31;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
+        const uint64_t mine = g + (uint64_t)lane * groups;
+        uint32_t v = 0;
+        bool fr = false;
+        if (lane < per && mine < a.hubs.chunks) {
+            v = a.hubs.hub[a.hubs.owner[mine]].x;
+            fr = (a.fcur[v >> 5] >> (v & 31)) & 1u;
+        }
+        uint32_t todo = __ballot_sync(FULL, fr);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t c = (uint32_t)(g + (uint64_t)j * groups);
+            const uint4 hub = a.hubs.hub[a.hubs.owner[c]];
+            uint64_t e0, e1;
+            hub_chunk(a.row, hub, c, e0, e1);
+            mp_relax(a, hub.x, e0, e1, c == hub.y, acc, s_fmin);
         }
     }
     __syncthreads();
@@ -629,8 +640,7 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_pull(MpArgs a, cons
 // A warp per HUB_CHUNK in-edges of a hub (degree > MP_T1): candidates lower
 // dist[u] by atomicMin (several chunks per hub); the hub's first chunk
 // classifies its own frontier lanes.
-__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_pull_hubs(MpArgs a, const uint32_t* __restrict__ list,
-                                                                        uint32_t n, const uint32_t* __restrict__ prefix)
+__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_pull_hubs(MpArgs a)
 {
     __shared__ uint32_t s_fmin[MP_K];
     mp_fmin_init(s_fmin);
@@ -638,32 +648,29 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_pull_hubs(MpArgs a,
     const int lane = threadIdx.x & 31;
     const uint32_t thr0 = __ldg(&a.thr[lane]), thr1 = __ldg(&a.thr[lane + 32]);
     const bool w0 = (a.wmask >> lane) & 1ULL, w1 = (a.wmask >> (lane + 32)) & 1ULL;
-    if (n) {
-        const uint32_t chunks = prefix[n];
-        const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-        for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
-            const uint32_t i = hub_of_chunk(prefix, n, (uint32_t)c);
-            const uint32_t u = list[i];
-            const uint64_t e0 = a.row[u] + (uint64_t)((uint32_t)c - prefix[i]) * HUB_CHUNK;
-            const uint64_t end = a.row[u + 1];
-            uint32_t b0 = SRV_INF, b1 = SRV_INF;
-            mp_pull_edges(a, e0, e0 + HUB_CHUNK < end ? e0 + HUB_CHUNK : end, thr0, thr1, w0, w1, b0, b1, acc);
-            unsigned long long D = 0;
-            if ((uint32_t)c == prefix[i]) {
-                const unsigned long long fu = ((a.fcur[u >> 5] >> (u & 31)) & 1u) ? a.front[u] : 0ULL;
-                if (fu)
-                    D = mp_pull_own(fu, a.dist[(uint64_t)u * MP_K + lane], a.dist[(uint64_t)u * MP_K + 32 + lane], thr0,
-                                    thr1, acc, s_fmin);
-            }
-            const bool i0 = b0 != SRV_INF && b0 < atomicMin(&a.dist[(uint64_t)u * MP_K + lane], b0);
-            const bool i1 = b1 != SRV_INF && b1 < atomicMin(&a.dist[(uint64_t)u * MP_K + 32 + lane], b1);
-            const unsigned long long I = (unsigned long long)__ballot_sync(FULL, i0) |
-                                         ((unsigned long long)__ballot_sync(FULL, i1) << 32);
-            if (lane == 0 && (I | D)) {
-                acc.any |= I;
-                atomicOr((unsigned long long*)&a.next[u], I | D);
-                atomicOr(&a.fbm[u >> 5], 1u << (u & 31));
-            }
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < a.hubs.chunks; c += warps) {
+        const uint4 hub = a.hubs.hub[a.hubs.owner[c]];
+        const uint32_t u = hub.x;
+        uint64_t e0, e1;
+        hub_chunk(a.row, hub, (uint32_t)c, e0, e1);
+        uint32_t b0 = SRV_INF, b1 = SRV_INF;
+        mp_pull_edges(a, e0, e1, thr0, thr1, w0, w1, b0, b1, acc);
+        unsigned long long D = 0;
+        if ((uint32_t)c == hub.y) {
+            const unsigned long long fu = ((a.fcur[u >> 5] >> (u & 31)) & 1u) ? a.front[u] : 0ULL;
+            if (fu)
+                D = mp_pull_own(fu, a.dist[(uint64_t)u * MP_K + lane], a.dist[(uint64_t)u * MP_K + 32 + lane], thr0,
+                                thr1, acc, s_fmin);
+        }
+        const bool i0 = b0 != SRV_INF && b0 < atomicMin(&a.dist[(uint64_t)u * MP_K + lane], b0);
+        const bool i1 = b1 != SRV_INF && b1 < atomicMin(&a.dist[(uint64_t)u * MP_K + 32 + lane], b1);
+        const unsigned long long I = (unsigned long long)__ballot_sync(FULL, i0) |
+                                     ((unsigned long long)__ballot_sync(FULL, i1) << 32);
+        if (lane == 0 && (I | D)) {
+            acc.any |= I;
+            atomicOr((unsigned long long*)&a.next[u], I | D);
+            atomicOr(&a.fbm[u >> 5], 1u << (u & 31));
         }
     }
     __syncthreads();
@@ -723,13 +730,26 @@ __global__ void k_mp_mark_all(const uint64_t* __restrict__ front, uint64_t V, ui
     }
 }
 
-// Lane k's values out, and the lane back to INF for its next query (so an
-// SSSP admission writes only its source).
-__global__ void k_mp_extract(uint32_t* __restrict__ dist, uint64_t V, int k, uint32_t* __restrict__ out)
+// The values of the lanes of quad q that are done out, and those lanes back to
+// INF for their next query (so an SSSP admission writes only its source).  A
+// lane lies one word in every 256 bytes, so reading it reads a 32-byte sector
+// per vertex: lanes done together share that read, up to a quad's four.
+// (14 queries at scale 20: 0.45 ms of extraction one lane at a time, 4.9 -> 4.75
+// ms in all.)
+struct MpOut {
+    uint32_t* out[4];  // null: the lane is not done
+};
+
+__global__ void k_mp_extract(uint32_t* __restrict__ dist, uint64_t V, int q, MpOut o)
 {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
-        out[v] = dist[v * MP_K + k];
-        dist[v * MP_K + k] = SRV_INF;
+        uint4* p = reinterpret_cast<uint4*>(dist + v * MP_K) + q;
+        uint4 d = *p;
+        if (o.out[0]) { o.out[0][v] = d.x; d.x = SRV_INF; }
+        if (o.out[1]) { o.out[1][v] = d.y; d.y = SRV_INF; }
+        if (o.out[2]) { o.out[2][v] = d.z; d.z = SRV_INF; }
+        if (o.out[3]) { o.out[3][v] = d.w; d.w = SRV_INF; }
+        *p = d;
     }
 }
 
@@ -860,28 +880,31 @@ __global__ void k_cc_hook_warp(const uint64_t* __restrict__ row, const uint32_t*
     }
 }
 
-__global__ void k_cc_hook_hub(const uint64_t* __restrict__ row, const uint32_t* __restrict__ adj,
-                              const uint32_t* __restrict__ list, uint32_t n, const uint32_t* __restrict__ prefix,
+__global__ void k_cc_hook_hub(const uint64_t* __restrict__ row, const uint32_t* __restrict__ adj, Hubs H,
                               uint32_t* p, uint32_t* err, const uint32_t* __restrict__ giant, uint32_t skip)
 {
-    if (!n) return;
     const int lane = threadIdx.x & 31;
-    const uint32_t chunks = prefix[n];
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
-        const uint32_t i = hub_of_chunk(prefix, n, (uint32_t)c);
-        const uint32_t v = list[i];
-        if (giant) {
-            const uint32_t root = __shfl_sync(FULL, lane == 0 ? cc_find(p, v) : 0u, 0);
-            if (root == *giant) continue;
-        }
-        const uint64_t first = row[v] + skip;
-        uint64_t e0 = row[v] + (uint64_t)((uint32_t)c - prefix[i]) * HUB_CHUNK;
-        const uint64_t e1 = e0 + HUB_CHUNK < row[v + 1] ? e0 + HUB_CHUNK : row[v + 1];
-        if (e0 < first) e0 = first;
-        for (uint64_t e = e0 + lane; e < e1; e += 32) {
-            const uint32_t u = adj[e];
-            if (cc_wanted(v, u, giant != nullptr)) cc_hook(p, v, u, err);
+    const uint64_t per = min((uint64_t)32, (H.chunks + warps - 1) / warps), groups = (H.chunks + per - 1) / per;
+    for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
+        const uint64_t mine = g + (uint64_t)lane * groups;
+        bool want = lane < per && mine < H.chunks;
+        if (want && giant) want = cc_find(p, H.hub[H.owner[mine]].x) != *giant;
+        uint32_t todo = __ballot_sync(FULL, want);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t c = (uint32_t)(g + (uint64_t)j * groups);
+            const uint4 hub = H.hub[H.owner[c]];
+            const uint32_t v = hub.x;
+            const uint64_t first = row[v] + skip;
+            uint64_t e0, e1;
+            hub_chunk(row, hub, c, e0, e1);
+            if (e0 < first) e0 = first;
+            for (uint64_t e = e0 + lane; e < e1; e += 32) {
+                const uint32_t u = adj[e];
+                if (cc_wanted(v, u, giant != nullptr)) cc_hook(p, v, u, err);
+            }
         }
     }
 }
@@ -919,9 +942,7 @@ struct PpArgs {
     const float* __restrict__ b_cur;
     float* __restrict__ b_next;
     float2* __restrict__ partial;  // (sum, compensation) per hub chunk and lane
-    const uint4* __restrict__ hub;       // {vertex, first chunk, chunks}
-    const uint32_t* __restrict__ owner;  // chunk -> hub
-    uint64_t hubs, chunks;
+    Hubs H;
 };
 
 // Compensated summation; the value of a pair is s + c.  Per term, Kahan's
@@ -1060,11 +1081,11 @@ __device__ __forceinline__ void pp_gather_group(const PpArgs& a, uint64_t e0, ui
 // The walk is bound by the latency of the rows, whatever part of them is
 // used: with a thread for each of the 8 quads a superstep took the same time
 // for 1 busy lane as for 32, because the threads of idle quads waited along.
-// With threads for the walked quads only, and rows above 512 edges in chunks
+// With threads for the walked quads only, and rows above MP_T1 edges in chunks
 // (a warp on up to 4,096 edges was the tail of a superstep), 20 supersteps at
-// undirected R-MAT scale 20 went from 19.4 to 6.0 ms for 1 lane, 20.5 to 6.9
-// for 7 (2 quads), 20.9 to 10.3 for 16 and 21.1 to 14.6 for 32; with narrow
-// groups alone 13.4, 17.0, 19.1 and 22.0.
+// undirected R-MAT scale 20 went from 19.4 to 5.8 ms for 1 lane, 20.5 to 6.8
+// for 7 (2 quads) and 21.1 to 14.6 for 32; with narrow groups alone 13.4, 17.0
+// and 22.0, with rows to 512 in one piece 6.0, 6.9 and 14.6.
 template <int NQ>
 __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_rows(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
                                                          uint64_t n)
@@ -1132,7 +1153,7 @@ __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_rows(PpArgs a, PpLanes L,
     }
 }
 
-// PP_SLOTS * NQ threads per vertex of higher degree (up to PP_T1; hubs are
+// PP_SLOTS * NQ threads per vertex of higher degree (up to MP_T1; hubs are
 // passed over).
 template <int NQ>
 __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_vertices(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
@@ -1146,14 +1167,14 @@ __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_vertices(PpArgs a, PpLane
     for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / GS; i < n; i += groups) {
         const uint64_t v = list[i];
         const uint64_t e0 = a.row[v], e1 = a.row[v + 1];
-        if (e1 - e0 > PP_T1) continue;  // the group's threads share v
+        if (e1 - e0 > MP_T1) continue;  // the group's threads share v
         float s[4], c[4];
         pp_gather_group<NQ>(a, e0, e1, Q, on, s, c);
         if (t < NQ && Q < PP_Q) pp_finish_quad(a, L, v, e1 - e0, Q, s, c);
     }
 }
 
-// Hubs: as many threads per PP_CHUNK edges, partial sums per chunk and lane...
+// Hubs: as many threads per HUB_CHUNK edges, partial sums per chunk and lane...
 template <int NQ>
 __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_hub_chunks(PpArgs a, PpLanes L)
 {
@@ -1162,11 +1183,12 @@ __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_hub_chunks(PpArgs a, PpLa
     bool on;
     const int Q = pp_quad(L, t % NQ, on);
     const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / GS;
-    for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / GS; c < a.chunks; c += groups) {
-        const uint4 hub = a.hub[a.owner[c]];
-        const uint64_t e0 = a.row[hub.x] + ((uint32_t)c - hub.y) * PP_CHUNK, end = a.row[hub.x + 1];
+    for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / GS; c < a.H.chunks; c += groups) {
+        const uint4 hub = a.H.hub[a.H.owner[c]];
+        uint64_t e0, e1;
+        hub_chunk(a.row, hub, (uint32_t)c, e0, e1);
         float s[4], cc[4];
-        pp_gather_group<NQ>(a, e0, e0 + PP_CHUNK < end ? e0 + PP_CHUNK : end, Q, on, s, cc);
+        pp_gather_group<NQ>(a, e0, e1, Q, on, s, cc);
         if (t < NQ && Q < PP_Q)
 #pragma unroll
             for (int j = 0; j < 4; j++) a.partial[c * PP_K + 4 * Q + j] = make_float2(s[j], cc[j]);
@@ -1179,8 +1201,8 @@ __global__ void __launch_bounds__(SRV_THREADS) k_pp_hub_finish(PpArgs a, PpLanes
 {
     const int lane = threadIdx.x & 31, j = lane & 3, part = lane >> 2;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < a.hubs * nq; i += warps) {
-        const uint4 hub = a.hub[i / nq];
+    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < a.H.hubs * nq; i += warps) {
+        const uint4 hub = a.H.hub[i / nq];
         bool on;
         const int Q = pp_quad(L, (int)(i % nq), on);
         const uint32_t per = (hub.z + 7) / 8, c0 = part * per, c1 = c0 + per < hub.z ? c0 + per : hub.z;
@@ -1233,12 +1255,12 @@ struct Graph {
     ipg_graph_view gv{};
     Group* mp = nullptr;
     Group* pp = nullptr;
-    // degree classes over all vertices and the chunk prefix of their hubs,
-    // built at first use by the PPR gathers and the union-find pass
+    // degree classes over all vertices
     ipg_bins bins{};
-    uint32_t* hub_prefix = nullptr;  // nh + 1 entries, then the hub count and the union-find error word
-    uint64_t hub_chunks = 0;
-    uint64_t pp_hubs = 0, pp_chunks = 0;  // rows above PP_T1 and their chunks
+    // the hubs' table (the graph's own may be replaced) and the union-find's words
+    void* cls = nullptr;
+    uint64_t cls_bytes = 0;
+    Hubs hubs{};
     uint32_t* cc_err = nullptr;
     uint32_t* cc_giant = nullptr;
     bool classes = false;
@@ -1264,14 +1286,12 @@ struct Group {
     uint32_t* list[3] = {nullptr, nullptr, nullptr};
     uint64_t hesum = 0;                   // frontier edges of the next superstep (last status)
     uint32_t* cnt = nullptr;              // into stat_d
-    uint32_t* prefix = nullptr;
     uint32_t* thr_d = nullptr;            // lane thresholds of the next superstep
     uint32_t* thr_pin = nullptr;          // their pinned staging copy
     uint32_t thr_h[MP_K];
     MpStatus* stat_d = nullptr;
     MpStatus* stat_h = nullptr;           // pinned copy after each superstep
     uint32_t hn[3] = {0, 0, 0};           // list sizes the host knows of
-    uint32_t hchunks = 0;                 // hub chunks of list 2
     uint32_t appended = 0;                // sources appended since
     uint64_t wmask = 0;
     int cc_lane = -1;  // label-propagation CC lane admitted in this admission pass
@@ -1279,11 +1299,7 @@ struct Group {
     float* b[2] = {nullptr, nullptr};
     uint32_t dirty[2] = {0, 0};  // quads of each buffer that may hold nonzero quotients
     float2* partial = nullptr;
-    // the hubs (rows above PP_T1) and their chunks
-    uint4* hub = nullptr;
-    uint32_t* owner = nullptr;
-    uint64_t hubs = 0, chunks = 0;
-    // gather classes: quads for degree <= PP_T0, streams up to PP_T1 (hubs
+    // gather classes: quads for degree <= PP_T0, streams up to MP_T1 (hubs
     // above); null when the graph is too large for
     // ipg_degree_classes_noalloc, and then the graph's classes serve
     uint32_t* pp_list = nullptr;
@@ -1360,9 +1376,9 @@ void free_group(ipg_server* S, Group* G)
 
 uint64_t group_bytes(const Graph* G, int kind)
 {
-    const uint64_t V = G->gv.V, E = G->gv.E;
-    if (kind == 0) return V * (MP_K * 4 + 16 + 12) + V / 4 + (E / (MP_T1 + 1) + 2) * 4 + 4096;
-    return V * (PP_K * 4 * 2 + 4) + G->pp_chunks * (PP_K * 8 + 4) + G->pp_hubs * 16 + 4096;
+    const uint64_t V = G->gv.V;
+    if (kind == 0) return V * (MP_K * 4 + 16 + 12) + V / 4 + 4096;
+    return V * (PP_K * 4 * 2 + 4) + G->hubs.chunks * (PP_K * 8) + 4096;
 }
 
 // Frees idle groups (least recently used first) until `need` more bytes fit
@@ -1383,31 +1399,30 @@ bool make_room(ipg_server* S, uint64_t need)
     return true;
 }
 
-// Degree classes of all vertices of a graph and the chunk prefix of its hubs
-// (built once; the PPR gathers and the union-find pass use them).
+// Degree classes of all vertices of a graph and its hubs in chunks (built once;
+// the min-plus and PPR groups and the union-find pass use them).
 int graph_classes(Graph* Gr, cudaStream_t st)
 {
     if (Gr->classes) return IPG_OK;
     int r = ipg_graph_bins(Gr->g, 0, MP_T0, MP_T1, &Gr->bins);
     if (r != IPG_OK) return r;
-    const uint64_t nh = Gr->bins.count[2];
-    void* p = nullptr;
-    if ((r = ipg_dev_alloc(&p, (nh + 5) * 4)) != IPG_OK) return r;
-    Gr->hub_prefix = (uint32_t*)p;
-    uint32_t* count = Gr->hub_prefix + nh + 2;
-    Gr->cc_err = count + 1;
-    Gr->cc_giant = count + 2;
-    const uint32_t n2 = (uint32_t)nh;
-    uint32_t chunks = 0;
-    cudaMemcpyAsync(count, &n2, 4, cudaMemcpyHostToDevice, st);
-    k_chunk_prefix<<<1, 1024, 0, st>>>(Gr->bins.d_list[2], count, Gr->gv.d_row, Gr->hub_prefix, nullptr);
-    cudaMemcpyAsync(&chunks, Gr->hub_prefix + nh, 4, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return ipg_internal_fail(IPG_ECUDA, "serve: hub prefix failed");
-    Gr->hub_chunks = chunks;
-    ipg_hubs H{};
-    if ((r = ipg_graph_hubs(Gr->g, 0, PP_T1, PP_CHUNK, &H)) != IPG_OK) return r;
-    Gr->pp_hubs = H.hubs;
-    Gr->pp_chunks = H.chunks;
+    ipg_hubs N{};
+    if ((r = ipg_graph_hubs(Gr->g, 0, MP_T1, HUB_CHUNK, &N)) != IPG_OK) return r;
+    const uint64_t bytes = N.hubs * 16 + (N.chunks + 2) * 4;
+    if ((r = ipg_dev_alloc(&Gr->cls, bytes)) != IPG_OK) return r;
+    Gr->cls_bytes = bytes;
+    uint4* hub = (uint4*)Gr->cls;
+    uint32_t* owner = (uint32_t*)(hub + N.hubs);
+    Gr->cc_err = owner + N.chunks;
+    Gr->cc_giant = Gr->cc_err + 1;
+    if ((N.hubs && cudaMemcpyAsync(hub, N.d_hub, N.hubs * 16, cudaMemcpyDeviceToDevice, st) != cudaSuccess) ||
+        (N.chunks && cudaMemcpyAsync(owner, N.d_owner, N.chunks * 4, cudaMemcpyDeviceToDevice, st) != cudaSuccess) ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return ipg_internal_fail(IPG_ECUDA, "serve: hub table failed");
+    Gr->hubs.hub = hub;
+    Gr->hubs.owner = owner;
+    Gr->hubs.chunks = N.chunks;
+    Gr->hubs.hubs = N.hubs;
     Gr->classes = true;
     return IPG_OK;
 }
@@ -1430,10 +1445,9 @@ void run_union_find(Graph* Gr, uint32_t* p, cudaStream_t st)
     if (B.count[1])
         k_cc_hook_warp<<<resident_cap(k_cc_hook_warp, warp_grid(B.count[1])), SRV_THREADS, 0, st>>>(
             gv.d_row, adj, B.d_list[1], B.count[1], p, Gr->cc_err, Gr->cc_giant, CC_SAMPLE);
-    if (B.count[2])
-        k_cc_hook_hub<<<resident_cap(k_cc_hook_hub, warp_grid(Gr->hub_chunks)), SRV_THREADS, 0, st>>>(
-            gv.d_row, adj, B.d_list[2], (uint32_t)B.count[2], Gr->hub_prefix, p, Gr->cc_err, Gr->cc_giant,
-            CC_SAMPLE);
+    if (Gr->hubs.chunks)
+        k_cc_hook_hub<<<resident_cap(k_cc_hook_hub, warp_grid(Gr->hubs.chunks)), SRV_THREADS, 0, st>>>(
+            gv.d_row, adj, Gr->hubs, p, Gr->cc_err, Gr->cc_giant, CC_SAMPLE);
     k_cc_compress<<<resident_cap(k_cc_compress, thread_grid(gv.V)), SRV_THREADS, 0, st>>>(p, gv.V);
 }
 
@@ -1445,7 +1459,7 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
     G->kind = kind;
     G->G = Gr;
     G->lane_q.resize(kind == 0 ? MP_K : PP_K);
-    const uint64_t V = Gr->gv.V, E = Gr->gv.E;
+    const uint64_t V = Gr->gv.V;
     int r = IPG_OK;
     // smaller graphs get higher-priority streams: their supersteps are short,
     // and their CTAs go first whenever SMs free up
@@ -1470,7 +1484,6 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
         if (r == IPG_OK) r = galloc(G, &G->thr_d, MP_K);
         if (r == IPG_OK && cudaHostAlloc((void**)&G->thr_pin, MP_K * 4, cudaHostAllocDefault) != cudaSuccess)
             r = ipg_internal_fail(IPG_ENOMEM, "serve: pinned allocation failed");
-        if (r == IPG_OK) r = galloc(G, &G->prefix, E / (MP_T1 + 1) + 2);
         if (r == IPG_OK && cudaHostAlloc((void**)&G->stat_h, sizeof(MpStatus), cudaHostAllocDefault) != cudaSuccess)
             r = ipg_internal_fail(IPG_ENOMEM, "serve: pinned allocation failed");
         if (r == IPG_OK) {
@@ -1480,27 +1493,12 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
             cudaMemsetAsync(G->fbm[0], 0, ((V + 31) / 32 + 1) * 4, G->st);
             cudaMemsetAsync(G->fbm[1], 0, ((V + 31) / 32 + 1) * 4, G->st);
             cudaMemsetAsync(G->stat_d, 0, sizeof(MpStatus), G->st);
-            cudaMemsetAsync(G->prefix, 0, 8, G->st);
         }
     } else {
         if (r == IPG_OK) r = graph_classes(Gr, G->st);
         if (r == IPG_OK) r = galloc(G, &G->b[0], V * PP_K);
         if (r == IPG_OK) r = galloc(G, &G->b[1], V * PP_K);
-        ipg_hubs H{};
-        if (r == IPG_OK) r = ipg_graph_hubs(Gr->g, 0, PP_T1, PP_CHUNK, &H);
-        if (r == IPG_OK) r = galloc(G, &G->partial, H.chunks * PP_K);
-        // copies of its own, counted in the group's bytes
-        if (r == IPG_OK) r = galloc(G, &G->hub, H.hubs);
-        if (r == IPG_OK) r = galloc(G, &G->owner, H.chunks);
-        if (r == IPG_OK) {
-            G->hubs = H.hubs;
-            G->chunks = H.chunks;
-            if ((H.hubs && cudaMemcpyAsync(G->hub, H.d_hub, H.hubs * 16, cudaMemcpyDeviceToDevice, G->st) != cudaSuccess) ||
-                (H.chunks &&
-                 cudaMemcpyAsync(G->owner, H.d_owner, H.chunks * 4, cudaMemcpyDeviceToDevice, G->st) != cudaSuccess) ||
-                cudaStreamSynchronize(G->st) != cudaSuccess)
-                r = ipg_internal_fail(IPG_ECUDA, "serve: PPR hub table failed");
-        }
+        if (r == IPG_OK) r = galloc(G, &G->partial, Gr->hubs.chunks * PP_K);
         if (r == IPG_OK) {
             // quotients of idle lanes are 0: an admitted lane sets its seed only
             cudaMemsetAsync(G->b[0], 0, V * PP_K * 4, G->st);
@@ -1512,11 +1510,11 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
             // the server's calls of ipg_degree_classes_noalloc are serialised
             // by this synchronisation (its scratch is shared)
             uint64_t tot[6] = {0, 0, 0, 0, 0, 0};
-            if (r == IPG_OK) r = ipg_degree_classes_noalloc(V, Gr->gv.d_row, PP_T0, PP_T1, G->pp_list, G->pp_tot, G->st);
+            if (r == IPG_OK) r = ipg_degree_classes_noalloc(V, Gr->gv.d_row, PP_T0, MP_T1, G->pp_list, G->pp_tot, G->st);
             if (r == IPG_OK && (cudaMemcpyAsync(tot, G->pp_tot, sizeof tot, cudaMemcpyDeviceToHost, G->st) != cudaSuccess ||
                                 cudaStreamSynchronize(G->st) != cudaSuccess))
                 r = ipg_internal_fail(IPG_ECUDA, "serve: PPR degree classes failed");
-            if (r == IPG_OK && tot[2] != G->hubs)
+            if (r == IPG_OK && tot[2] != Gr->hubs.hubs)
                 r = ipg_internal_fail(IPG_EINVAL, "serve: PPR hub class differs from the graph's");
             G->pp_n[0] = tot[0];
             G->pp_n[1] = tot[1];
@@ -1669,11 +1667,9 @@ void admit(ipg_server* S, Group* G, double now)
         cudaMemsetAsync(G->stat_d->esum, 0, sizeof G->stat_d->esum, G->st);
         ipg_compact(G->fbm[G->cur], V, G->G->gv.d_row, MP_T0, MP_T1, G->list[0], G->list[1], G->list[2], G->cnt,
                     (uint64_t*)G->stat_d->esum, 0, G->st);
-        k_chunk_prefix<<<1, 1024, 0, G->st>>>(G->list[2], G->cnt + 2, G->G->gv.d_row, G->prefix, &G->stat_d->chunks);
         cudaMemcpyAsync(G->stat_h, G->stat_d, sizeof(MpStatus), cudaMemcpyDeviceToHost, G->st);
         cudaStreamSynchronize(G->st);
         for (int c = 0; c < 3; c++) G->hn[c] = G->stat_h->cnt[c];
-        G->hchunks = G->stat_h->chunks;
         G->hesum = G->stat_h->esum[0] + G->stat_h->esum[1] + G->stat_h->esum[2];
         G->appended = 0;
     }
@@ -1698,11 +1694,9 @@ int launch_superstep(ipg_server* S, Group* G)
         a.wmask = G->wmask;
         a.busy = G->busy;
         // grids from the list sizes of the last status plus the sources
-        // appended since (each in some list; a hub one adds its chunks)
+        // appended since (each in some list)
         const uint64_t add = G->appended;
-        const uint64_t hub_chunks_max = (gv.max_out_degree + HUB_CHUNK - 1) / HUB_CHUNK;
         const uint64_t n0 = G->hn[0] + add, n1 = G->hn[1] + add;
-        const uint64_t chunks = G->hchunks + add * hub_chunks_max;
         memcpy(G->thr_pin, G->thr_h, sizeof G->thr_h);  // the last copy finished with the last superstep
         cudaMemcpyAsync(G->thr_d, G->thr_pin, sizeof G->thr_h, cudaMemcpyHostToDevice, G->st);
         cudaMemsetAsync(G->stat_d, 0, 3 * sizeof(unsigned long long), G->st);
@@ -1712,6 +1706,8 @@ int launch_superstep(ipg_server* S, Group* G)
         // direction: pull when the frontier's edges are a large part of the
         // graph and enough lanes are busy to share each row read
         const Graph* Gr = G->G;
+        a.hubs = Gr->hubs;
+        const uint64_t chunks = Gr->hubs.chunks;
         const bool pull = S->pull && gv.symmetric && Gr->classes && __builtin_popcountll(G->busy) >= MP_PULL_LANES &&
                           G->hesum * MP_PULL_DIV >= gv.E;
         if (pull) {
@@ -1719,19 +1715,22 @@ int launch_superstep(ipg_server* S, Group* G)
             const uint64_t n01 = B.count[0] + B.count[1];
             if (n01)
                 k_mp_pull<<<resident_cap(k_mp_pull, warp_grid(n01)), SRV_THREADS, 0, G->st>>>(a, B.d_list[0], n01);
-            if (B.count[2])
-                k_mp_pull_hubs<<<resident_cap(k_mp_pull_hubs, warp_grid(Gr->hub_chunks)), SRV_THREADS, 0, G->st>>>(
-                    a, B.d_list[2], (uint32_t)B.count[2], Gr->hub_prefix);
-            S->stats.kernel_launches += (n01 ? 1 : 0) + (B.count[2] ? 1 : 0);
+            if (chunks)
+                k_mp_pull_hubs<<<resident_cap(k_mp_pull_hubs, warp_grid(chunks)), SRV_THREADS, 0, G->st>>>(a);
+            S->stats.kernel_launches += (n01 ? 1 : 0) + (chunks ? 1 : 0);
         } else {
-            if (add) k_chunk_prefix<<<1, 1024, 0, G->st>>>(G->list[2], G->cnt + 2, gv.d_row, G->prefix, nullptr);
             k_mp_thread<<<resident_cap(k_mp_thread, thread_grid(n0)), SRV_THREADS, 0, G->st>>>(a, G->list[0],
                                                                                             G->cnt + 0);
             k_mp_vertices<<<resident_cap(k_mp_vertices, warp_grid(n1)), SRV_THREADS, 0, G->st>>>(a, G->list[1],
                                                                                               G->cnt + 1);
-            k_mp_hubs<<<resident_cap(k_mp_hubs, warp_grid(chunks)), SRV_THREADS, 0, G->st>>>(a, G->list[2],
-                                                                                          G->cnt + 2, G->prefix);
-            S->stats.kernel_launches += 3 + (add ? 1 : 0);
+            const bool hubs = chunks && G->hn[2] + add;
+            if (hubs) {
+                const uint64_t warps = (uint64_t)resident_cap(k_mp_hubs, warp_grid(chunks)) * (SRV_THREADS / 32);
+                const uint32_t per = (uint32_t)std::min<uint64_t>(32, (chunks + warps - 1) / warps);
+                const uint32_t groups = (uint32_t)((chunks + per - 1) / per);
+                k_mp_hubs<<<resident_cap(k_mp_hubs, warp_grid(groups)), SRV_THREADS, 0, G->st>>>(a, per, groups);
+            }
+            S->stats.kernel_launches += hubs ? 3 : 2;
         }
         S->stats.pull_supersteps += pull ? 1 : 0;
         k_mp_clear<<<resident_cap(k_mp_clear, thread_grid(G->hn[0] + G->hn[1] + G->hn[2] + add)), SRV_THREADS, 0,
@@ -1742,10 +1741,9 @@ int launch_superstep(ipg_server* S, Group* G)
         ipg_compact(G->fbm[G->cur ^ 1], gv.V, gv.d_row, MP_T0, MP_T1, G->list[0], G->list[1], G->list[2], G->cnt,
                     (uint64_t*)G->stat_d->esum, 0, G->st);
         cudaMemsetAsync(G->fbm[G->cur], 0, ((gv.V + 31) / 32 + 1) * 4, G->st);
-        k_chunk_prefix<<<1, 1024, 0, G->st>>>(G->list[2], G->cnt + 2, gv.d_row, G->prefix, &G->stat_d->chunks);
         cudaMemcpyAsync(G->stat_h, G->stat_d, sizeof(MpStatus), cudaMemcpyDeviceToHost, G->st);
         G->cur ^= 1;
-        S->stats.kernel_launches += 4;
+        S->stats.kernel_launches += 3;
     } else {
         const Graph* Gr = G->G;
         PpArgs a;
@@ -1754,10 +1752,7 @@ int launch_superstep(ipg_server* S, Group* G)
         a.b_cur = G->b[G->cur];
         a.b_next = G->b[G->cur ^ 1];
         a.partial = G->partial;
-        a.hub = G->hub;
-        a.owner = G->owner;
-        a.hubs = G->hubs;
-        a.chunks = G->chunks;
+        a.H = Gr->hubs;
         PpLanes L;
         L.active = G->busy;
         for (int k = 0; k < PP_K; k++) {
@@ -1797,16 +1792,16 @@ int launch_superstep(ipg_server* S, Group* G)
             if (n1)
                 k_pp_vertices<NQ><<<resident_cap(k_pp_vertices<NQ>, thread_grid(n1 * PP_SLOTS * NQ)), SRV_THREADS, 0,
                                     G->st>>>(a, L, l1, n1);
-            if (a.chunks)
-                k_pp_hub_chunks<NQ><<<resident_cap(k_pp_hub_chunks<NQ>, thread_grid(a.chunks * PP_SLOTS * NQ)),
+            if (a.H.chunks)
+                k_pp_hub_chunks<NQ><<<resident_cap(k_pp_hub_chunks<NQ>, thread_grid(a.H.chunks * PP_SLOTS * NQ)),
                                       SRV_THREADS, 0, G->st>>>(a, L);
         };
         if (nq <= 1) launch(std::integral_constant<int, 1>());
         else if (nq <= 2) launch(std::integral_constant<int, 2>());
         else if (nq <= 4) launch(std::integral_constant<int, 4>());
         else launch(std::integral_constant<int, 8>());
-        if (a.hubs)
-            k_pp_hub_finish<<<resident_cap(k_pp_hub_finish, warp_grid(a.hubs * nq)), SRV_THREADS, 0, G->st>>>(a, L, nq);
+        if (a.H.hubs)
+            k_pp_hub_finish<<<resident_cap(k_pp_hub_finish, warp_grid(a.H.hubs * nq)), SRV_THREADS, 0, G->st>>>(a, L, nq);
         G->cur ^= 1;
         S->stats.kernel_launches += 4;
     }
@@ -1825,7 +1820,6 @@ void retire(ipg_server* S, Group* G, double now)
     if (G->kind == 0) {
         const MpStatus& st = *G->stat_h;
         for (int c = 0; c < 3; c++) G->hn[c] = st.cnt[c];
-        G->hchunks = st.chunks;
         S->work[(size_t)G->G->gid * 2] += st.work;
         G->hesum = st.esum[0] + st.esum[1] + st.esum[2];
         G->appended = 0;
@@ -1850,22 +1844,27 @@ void retire(ipg_server* S, Group* G, double now)
                 Query& q = S->queries[qid];
                 if (alloc_result(S, q, G->st) != IPG_OK) ok = false;
             }
-            if (!ok) continue;
-            const void* first = nullptr;
+            if (ok) extracted |= 1ULL << k;
+        }
+        for (int q4 = 0; q4 < MP_K / 4; q4++) {
+            MpOut o{};
+            for (int j = 0; j < 4; j++)
+                if ((extracted >> (4 * q4 + j)) & 1) o.out[j] = (uint32_t*)S->queries[G->lane_q[4 * q4 + j][0]].result;
+            if ((extracted >> (4 * q4)) & 0xFULL)
+                k_mp_extract<<<resident_cap(k_mp_extract, thread_grid(G->G->gv.V)), SRV_THREADS, 0, G->st>>>(
+                    G->dist, G->G->gv.V, q4, o);
+        }
+        for (int k = 0; k < MP_K; k++) {
+            if (!((extracted >> k) & 1)) continue;
+            const void* first = S->queries[G->lane_q[k][0]].result;
             for (uint64_t qid : G->lane_q[k]) {
                 Query& q = S->queries[qid];
-                if (!first) {
-                    k_mp_extract<<<resident_cap(k_mp_extract, thread_grid(G->G->gv.V)), SRV_THREADS, 0, G->st>>>(
-                        G->dist, G->G->gv.V, k, (uint32_t*)q.result);
-                    first = q.result;
-                } else {
+                if (q.result != first)
                     cudaMemcpyAsync(q.result, first, q.result_bytes, cudaMemcpyDeviceToDevice, G->st);
-                }
                 finishing(S, q, G->st);
             }
             G->lane_q[k].clear();
             if (G->cc_lane == k) G->cc_lane = -1;
-            extracted |= 1ULL << k;
         }
         G->busy &= ~extracted;
     } else {
@@ -1931,7 +1930,7 @@ extern "C" void ipg_server_free(ipg_server* S)
     cudaStreamDestroy(S->rel_st);
     cudaMemPoolDestroy(S->rpool);
     for (auto& g : S->graphs)
-        if (g->hub_prefix) ipg_dev_free(g->hub_prefix, (g->bins.count[2] + 5) * 4);
+        ipg_dev_free(g->cls, g->cls_bytes);
     delete S;
 }
 
@@ -1950,7 +1949,7 @@ extern "C" int ipg_server_add_graph(ipg_server* S, ipg_graph* g, int* gid)
     // the pull supersteps walk them) are built now, before queries arrive:
     // building them synchronises the device
     if ((r = graph_classes(G.get(), nullptr)) != IPG_OK) {
-        if (G->hub_prefix) ipg_dev_free(G->hub_prefix, (G->bins.count[2] + 5) * 4);
+        ipg_dev_free(G->cls, G->cls_bytes);
         return r;
     }
     *gid = (int)S->graphs.size();

@@ -1,5 +1,5 @@
 """The server's gathers at their edges: numbers of lanes around the quads a superstep walks, rows around the thread,
-stream and hub-chunk classes, and lanes that leave while others gather and join again later."""
+stream and hub-chunk classes (256 edges), and lanes that leave while others gather and join again later."""
 import numpy as np
 import pytest
 
@@ -8,8 +8,8 @@ import oracle as O
 pytestmark = pytest.mark.gpu
 
 PPR_TOL = 2e-6  # FP32 lanes against the FP64 oracle, max abs per vertex
-# around four ids (4), 32 edges of a stream, the classes (8, 64, 512) and hub chunks of 512 and 1,024 edges
-LENGTHS = (1, 2, 3, 4, 5, 7, 8, 9, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 511, 512, 513, 1023, 1024, 1025,
+# around four ids (4), 32 edges of a stream, the classes (8, 64, 256) and hub chunks of 256 edges
+LENGTHS = (1, 2, 3, 4, 5, 7, 8, 9, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1025,
            1537, 4095, 4096, 4097, 4609)
 
 
@@ -58,6 +58,45 @@ def test_ppr_lanes_around_the_quads(ppr_case, first, later):
         for x, w in zip(got, want[:first + later] + want[:1]):
             assert np.max(np.abs(x.astype(np.float64) - w)) <= PPR_TOL
         np.testing.assert_array_equal(got[-1].view(np.uint32), got[0].view(np.uint32))
+    finally:
+        srv.free()
+        d.free()
+
+
+@pytest.fixture(scope="module")
+def sssp_case():
+    g = _graph()
+    srcs = [int(s) for s in np.random.default_rng(10).choice(np.flatnonzero(np.diff(g.idx.astype(np.int64), append=g.E)),
+                                                             66, replace=False)]
+    srcs[1] = len(LENGTHS) - 1
+    srcs[2] = g.V - 1
+    return g, srcs, [O.dijkstra(g, s) for s in srcs], O.run(g, "cc", "spread")[0]
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+@pytest.mark.parametrize("first,later", [(1, 1), (4, 3), (5, 4), (8, 1), (9, 8), (16, 1), (17, 16), (33, 3), (40, 2), (64, 2)])
+def test_sssp_lanes_around_the_quads(sssp_case, symmetric, first, later):
+    """`first` queries, `later` more after two supersteps, and a last one on cleared lanes; components beside them
+    (union-find on the symmetric graph, a label lane on the other)."""
+    import ipregel_b200 as ip
+    from ipregel_b200 import serve as S
+    g, srcs, want, comp = sssp_case
+    d = ip.Graph.from_csr(g.V, g.E, g.idx, g.adj, wgt=g.wgt)
+    d.set_symmetric(symmetric)
+    srv = S.Server()
+    try:
+        gid = srv.add_graph(d)
+        ids = [srv.submit(gid, S.SSSP, s) for s in srcs[:first]]
+        while srv.stats()["supersteps"] < 2:
+            srv.poll()
+        ids += [srv.submit(gid, S.SSSP, s) for s in srcs[first:first + later]]
+        cc = srv.submit(gid, S.CC, 0)
+        srv.drain()
+        ids.append(srv.submit(gid, S.SSSP, srcs[0]))
+        srv.drain()
+        for q, w in zip(ids, want[:first + later] + want[:1]):
+            np.testing.assert_array_equal(srv.result(q, S.SSSP, g.V), w)
+        np.testing.assert_array_equal(srv.result(cc, S.CC, g.V), comp)
     finally:
         srv.free()
         d.free()
