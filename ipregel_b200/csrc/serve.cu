@@ -76,7 +76,11 @@ constexpr uint64_t MP_T0 = 8;       // min-plus: a thread a vertex up to this de
 // / 5.8 / 5.4 / 5.8 ms and 40 took 21.6 / 17.6 / 16.8 / 15.7 / 15.2.
 constexpr uint64_t MP_T1 = 256;
 constexpr uint32_t HUB_CHUNK = 256;
-constexpr uint64_t PP_T0 = 64;    // PPR: quads up to this degree, then several streams a row up to MP_T1
+// PPR: a thread a quad up to this degree, then several streams a row up to
+// MP_T1.  Rows of up to 64 edges beside each other left narrow groups waiting
+// for the longest: with 64 / 32 / 16 / 8, 1 query took 5.8 / 5.2 / 5.15 / 5.1
+// ms, 7 took 6.9 / 6.2 / 6.4 / 6.7 and 32 took 14.7 / 14.8 / 14.9 / 15.9.
+constexpr uint64_t PP_T0 = 32;
 constexpr uint64_t PP_NOALLOC_MAX_V = 67108864ull;  // ipg_degree_classes_noalloc's vertex limit
 constexpr uint32_t SRV_INF = 0xffffffffu;
 constexpr unsigned FULL = 0xffffffffu;
@@ -1083,8 +1087,8 @@ __device__ __forceinline__ void pp_gather_group(const PpArgs& a, uint64_t e0, ui
 // for 1 busy lane as for 32, because the threads of idle quads waited along.
 // With threads for the walked quads only, and rows above MP_T1 edges in chunks
 // (a warp on up to 4,096 edges was the tail of a superstep), 20 supersteps at
-// undirected R-MAT scale 20 went from 19.4 to 5.8 ms for 1 lane, 20.5 to 6.8
-// for 7 (2 quads) and 21.1 to 14.6 for 32; with narrow groups alone 13.4, 17.0
+// undirected R-MAT scale 20 went from 19.4 to 5.2 ms for 1 lane, 20.5 to 6.2
+// for 7 (2 quads) and 21.1 to 14.8 for 32; with narrow groups alone 13.4, 17.0
 // and 22.0, with rows to 512 in one piece 6.0, 6.9 and 14.6.
 template <int NQ>
 __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_rows(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
