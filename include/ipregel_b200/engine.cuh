@@ -81,11 +81,6 @@ static_assert(sizeof(ipx_msg) <= 8, "iPregel-B200: IP_MESSAGE_TYPE must be at mo
 /* Largest CTA the kernels are compiled for; the launch size is a runtime
  * tuning parameter (a multiple of 32 up to this). */
 #define IPX_THREADS 256
-/* Resident CTAs per SM the edge kernels (push, mark, gather) are compiled
- * for: 6 x 256 threads keeps their ~40 registers without spilling. */
-#ifndef IPX_EDGE_CTAS
-#define IPX_EDGE_CTAS 6
-#endif
 /* CTA of the target marking kernel: one per SM, its shared memory the bits
  * of the most often visited targets. */
 #define IPX_MARK_THREADS 1024
@@ -632,12 +627,12 @@ struct ipx_consts {
     /* per superstep a record of hist[s % IPX_HIST]: active count, edges
      * traversed, direction | error word << 32, nanoseconds */
     unsigned long long* hist;
-    /* single_broadcast: the vertices by degree class (short, middle and
-     * long rows, the hubs among the long ones; their numbers in class_n),
-     * and the hubs (rows above hub_min, ipg_graph_hubs) {vertex, first
-     * chunk, chunks} with, per chunk, the index of its hub and the partial
-     * fold ({message, has} in a slot, has in the stamp word), per hub the
-     * chunks arrived */
+    /* single_broadcast, and pulling push versions: the vertices by in-degree
+     * class (short, middle and long rows, the hubs among the long ones; their
+     * numbers in class_n), and the hubs (rows above hub_min, ipg_graph_hubs)
+     * {vertex, first chunk, chunks} with, per chunk, the index of its hub;
+     * single_broadcast also per chunk the partial fold ({message, has} in a
+     * slot, has in the stamp word) and per hub the chunks arrived */
     const uint32_t* class_list[3];
     uint32_t class_n[3];
     const uint4* hub;
@@ -645,8 +640,6 @@ struct ipx_consts {
     uint32_t* hub_arrived;
     uint64_t hub_min;
     uint32_t chunks, hub_chunk;
-    /* chunk -> index of its hub: of those hubs, or of the static hub class
-     * of a pulling push version */
     const uint32_t* hub_owner;
     /* the in-lists with the flag of the most gathered vertices (null: none) */
     const uint32_t* in_adj_hot;
@@ -692,14 +685,12 @@ enum {
     IPX_K_GATHER_HUBS,
     IPX_K_MARK,
     IPX_K_COUNT,
-    IPX_K_PULLD0,
-    IPX_K_PULLD1,
-    IPX_K_PULLD2,
+    IPX_K_PULLD,
     IPX_K_N
 };
 static const char* const ipx_kname[IPX_K_N] = {
     "compute", "push", "compact_targets", "gather", "gather_hubs", "mark", "count_active",
-    "pull_deliver_thread", "pull_deliver_warp", "pull_deliver_block"};
+    "pull_deliver"};
 
 __device__ __forceinline__ uint64_t ipx_gtid() { return blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint64_t ipx_gstride() { return (uint64_t)gridDim.x * blockDim.x; }
@@ -861,9 +852,8 @@ __device__ __forceinline__ void ipx_deliver(int p, uint64_t w, ipx_msg m)
     if (ipx_mb::deliver(&ipx_c.mbox[p][w], m)) atomicOr(&ipx_c.recv[p][w >> 5], 1u << (w & 31));
 }
 
-/* Edges per chunk of a hub's row in the static pull delivery of the push
- * versions, and at most (fewer on small graphs) in push and mark, where a
- * warp takes a chunk: one hub does not leave a single warp working after the
+/* Edges per chunk of a hub's row at most (fewer on small graphs) in push, mark
+ * and pull delivery, where a warp takes a chunk: one hub does not leave a single warp working after the
  * others have finished. */
 #ifndef IPX_HUB_CHUNK
 #define IPX_HUB_CHUNK 2048
@@ -1169,46 +1159,6 @@ __device__ __forceinline__ void ipx_walk_broadcasters(const Visit& visit)
     ipx_walk_rows<1>(ipx_c.blist[0], __ldcg(&st->n[0]), visit);
 }
 
-/* Chunk prefix of the high-degree class: prefix[i] = chunks of the hubs before
- * i, prefix[n] = total (one block, a carried scan over tiles of its width).
- * With owner, also owner[c] = i for every chunk c of hub i, so that a chunk
- * finds its hub with one load instead of a binary search over the prefix. */
-template <uint32_t CHUNK = IPX_HUB_CHUNK>
-__global__ void __launch_bounds__(1024) ipx_k_hub_prefix(const uint32_t* __restrict__ list,
-                                                         const uint32_t* __restrict__ count,
-                                                         const uint64_t* __restrict__ row, uint32_t* __restrict__ prefix,
-                                                         uint32_t* __restrict__ owner = nullptr)
-{
-    __shared__ uint32_t s[1024];
-    const uint64_t n = *count;
-    uint32_t carry = 0;
-    for (uint64_t base = 0; base < n; base += 1024) {
-        const uint64_t i = base + threadIdx.x;
-        uint32_t c = 0;
-        if (i < n) {
-            const uint64_t u = list[i];
-            c = (uint32_t)((row[u + 1] - row[u] + CHUNK - 1) / CHUNK);
-        }
-        s[threadIdx.x] = c;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            const uint32_t x = (threadIdx.x >= (unsigned)o) ? s[threadIdx.x - o] : 0u;
-            __syncthreads();
-            s[threadIdx.x] += x;
-            __syncthreads();
-        }
-        if (i < n) {
-            const uint32_t p = carry + s[threadIdx.x] - c;
-            prefix[i] = p;
-            if (owner)
-                for (uint32_t k = 0; k < c; k++) owner[p + k] = (uint32_t)i;
-        }
-        carry += s[1023];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) prefix[n] = carry;
-}
-
 /* ---- the flagged in-lists of the single_broadcast gather (attach time) ---- */
 /* cnt[u] += 1 for every occurrence of u in the in-lists. */
 __global__ void ipx_k_count_occurrences(const uint32_t* __restrict__ adj, uint64_t E, uint32_t* __restrict__ cnt)
@@ -1238,18 +1188,6 @@ __global__ void ipx_k_flag_hot(const uint32_t* __restrict__ adj, uint64_t E, con
         const uint32_t u = adj[e];
         out[e] = u | (cnt[u] >= threshold ? IPX_HOT_BIT : 0u);
     }
-}
-
-/* Hub index of chunk c: the last i with prefix[i] <= c. */
-__device__ __forceinline__ uint64_t ipx_hub_of_chunk(const uint32_t* __restrict__ prefix, uint64_t n, uint32_t c)
-{
-    uint64_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint64_t mid = (lo + hi) >> 1;
-        if (prefix[mid] <= c) lo = mid;
-        else hi = mid;
-    }
-    return lo;
 }
 
 /* ---- the vertex functions that depend on the version ---- */
@@ -1469,6 +1407,20 @@ __device__ __forceinline__ void ipx_gather_fold_edges(const ipx_vid* __restrict_
     }
 }
 
+/* The tree over the G lanes of one group (G a power of two <= 32); `mask`
+ * holds the group's lanes. */
+template <int G>
+__device__ __forceinline__ void ipx_group_fold(bool& has, ipx_msg& acc, unsigned mask)
+{
+    typedef typename ipx_word<ipx_msg>::type W;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        const bool oh = __shfl_down_sync(mask, has, o, G);
+        const ipx_msg om = ipx_from_word<ipx_msg>(__shfl_down_sync(mask, ipx_to_word(acc), o, G));
+        ipx_fold(has, acc, oh, om);
+    }
+}
+
 /* ------------------------------------------------------------------------ */
 /* Pull delivery for the push versions (direction optimisation).  On a       */
 /* symmetric graph a vertex's row lists exactly the vertices that would push */
@@ -1476,95 +1428,187 @@ __device__ __forceinline__ void ipx_gather_fold_edges(const ipx_vid* __restrict_
 /* the message a push would have left in its mailbox (the fold order differs */
 /* only as ip_combine's contract allows).  Used in dense supersteps: it      */
 /* streams every row once and needs no atomics except for the hubs' chunks.  */
-/* MODE 0: thread per vertex, 1: warp per vertex, 2: CTA per 2048-edge chunk */
-/* of a high-degree vertex, committed with the mailbox's atomic.             */
+/* One launch, the longest work items first: a warp per chunk of a hub,      */
+/* committed with the mailbox's atomic, then groups of 32, 8 and 1 lanes per */
+/* row, pipelined over the group's next rows as in the push's walk.          */
 /* ------------------------------------------------------------------------ */
+#if IPX_VERSION == IPX_COMBINER || IPX_VERSION == IPX_SPREAD
+/* The messages of up to four edges' sources, in edge order; ok[k]: the lane
+ * holds an edge.  A source's bit is read first and its message only if it
+ * broadcast: below one in 20 most would be read for nothing.  Rate bound: 240
+ * G edges/s on random in-lists of 8 edges (256 graphs of 1,024 to 65,536
+ * vertices in one union of 4.3 M) against 275 G/s for random reads that hit
+ * the L2.  CC and weighted SSSP over that union took 2.26 and 3.93 ms with a
+ * launch per class (a thread, a warp, a CTA a row) and no pipeline, 1.95 and
+ * 3.39 now. */
+__device__ __forceinline__ void ipx_pull_fold4(const uint64_t* u, const bool* ok, const ipx_wgt* x, bool& has, ipx_msg& acc)
+{
+    const uint32_t* __restrict__ bc = ipx_c.bcaster;
+    const ipx_msg* __restrict__ ob = ipx_c.outbox;
+    bool on[4];
+    ipx_msg m[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) on[k] = ok[k] && ((__ldg(&bc[u[k] >> 5]) >> (u[k] & 31)) & 1u);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (on[k]) m[k] = __ldg(&ob[u[k]]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (!on[k]) continue;
+#if IPX_EDGE_MSG
+        ipx_fold(has, acc, true, IP_BROADCAST_EDGE_MESSAGE(m[k], x[k]));
+#else
+        (void)x;
+        ipx_fold(has, acc, true, m[k]);
+#endif
+    }
+}
+
+/* A quad of ids (and of weights) of the row [r0, r0 + deg). */
+__device__ __forceinline__ void ipx_pull_fold_quad(const uint4& q, uint64_t r0, uint32_t deg, uint32_t rel, bool& has,
+                                                   ipx_msg& acc)
+{
+    const uint32_t t = rel - ((uint32_t)r0 & 3u); /* edge of the row; before its first: wraps */
+    const uint64_t u[4] = {q.x, q.y, q.z, q.w};
+    const bool ok[4] = {t < deg, t + 1 < deg, t + 2 < deg, t + 3 < deg};
+    ipx_wgt x[4];
+#if IPX_EDGE_MSG
+    if constexpr (sizeof(ipx_wgt) == 4) {
+        const uint4 w = ipx_ld_quad(reinterpret_cast<const uint32_t*>(ipx_c.in_wgt), r0, deg, rel);
+        const uint32_t wk[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) memcpy(&x[k], &wk[k], 4);
+    } else {
+        const uint64_t e = r0 - ((uint32_t)r0 & 3u) + rel;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (ok[k]) x[k] = ipx_ld_stream(&ipx_c.in_wgt[e + k]);
+    }
+#endif
+    ipx_pull_fold4(u, ok, x, has, acc);
+}
+
+/* Edges [e0, e1) without 128-bit loads, lane-strided. */
 __device__ __forceinline__ void ipx_pull_fold_edges(uint64_t e0, uint64_t e1, uint64_t lane, uint64_t lanes, bool& has,
                                                     ipx_msg& acc)
 {
     const ipx_vid* __restrict__ adj = ipx_c.in_adj;
-    const uint32_t* __restrict__ bc = ipx_c.bcaster;
-    const ipx_msg* __restrict__ ob = ipx_c.outbox;
-    for (uint64_t e = e0 + lane; e < e1; e += IPX_UNROLL * lanes) {
-        uint64_t u[IPX_UNROLL];
-        uint32_t word[IPX_UNROLL];
+    for (uint64_t e = e0 + lane; e < e1; e += 4 * lanes) {
+        uint64_t u[4];
+        bool ok[4];
+        ipx_wgt x[4];
 #pragma unroll
-        for (int k = 0; k < IPX_UNROLL; k++) {
-            const uint64_t ek = e + k * lanes;
-            u[k] = (ek < e1) ? (uint64_t)ipx_ld_edge(&adj[ek], lanes) : 0;
-            word[k] = (ek < e1) ? __ldg(&bc[u[k] >> 5]) : 0u;
-        }
-#pragma unroll
-        for (int k = 0; k < IPX_UNROLL; k++) {
-            if ((word[k] >> (u[k] & 31)) & 1u) {
+        for (int k = 0; k < 4; k++) {
+            ok[k] = e + k * lanes < e1;
+            u[k] = ok[k] ? (uint64_t)ipx_ld_edge(&adj[e + k * lanes], lanes) : 0;
 #if IPX_EDGE_MSG
-                ipx_msg m = IP_BROADCAST_EDGE_MESSAGE(__ldg(&ob[u[k]]), ipx_ld_edge(&ipx_c.in_wgt[e + k * lanes], lanes));
-#else
-                ipx_msg m = __ldg(&ob[u[k]]);
+            if (ok[k]) x[k] = ipx_ld_edge(&ipx_c.in_wgt[e + k * lanes], lanes);
 #endif
-                ipx_fold(has, acc, true, m);
+        }
+        ipx_pull_fold4(u, ok, x, has, acc);
+    }
+}
+
+/* The list's rows, G lanes each; SKIP: hubs are passed over. */
+template <int G, bool SKIP>
+__device__ __forceinline__ void ipx_pull_rows(const uint32_t* __restrict__ list, uint32_t n, int p)
+{
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const unsigned mask = (G == 32) ? IPX_FULL : (((1u << (G & 31)) - 1u) << (lane & ~(G - 1)));
+    const uint64_t* __restrict__ row = ipx_c.in_row;
+    const uint64_t step = ipx_gstride() / G;
+    uint64_t i = ipx_gtid() / G;
+    auto done = [&](uint64_t v, bool has, ipx_msg acc) {
+        if (G > 1) ipx_group_fold<G>(has, acc, mask);
+        if (gl == 0 && has && ipx_mb::merge(&ipx_c.mbox[p][v], acc)) {
+            if (G == 1) ipx_set_bit_agg(ipx_c.recv[p], v);
+            else atomicOr(&ipx_c.recv[p][v >> 5], 1u << (v & 31));
+        }
+    };
+    if (!ipx_c.in_quads) {
+        for (; i < n; i += step) {
+            const uint64_t v = list[i];
+            if (SKIP && row[v + 1] - row[v] > ipx_c.hub_min) continue;
+            bool has = false;
+            ipx_msg acc;
+            ipx_pull_fold_edges(row[v], row[v + 1], gl, G, has, acc);
+            done(v, has, acc);
+        }
+        return;
+    }
+    if (i >= n) return;
+    if constexpr (sizeof(ipx_vid) == 4) {
+        const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ipx_c.in_adj);
+        /* a: the row being folded, b: the next, c: the one after it; past the
+         * list's end vertex 0 stands in: loaded, never folded */
+        uint32_t va = list[i], vb = i + step < n ? list[i + step] : 0u, vc = i + 2 * step < n ? list[i + 2 * step] : 0u;
+        uint64_t a0 = row[va], b0 = row[vb];
+        uint32_t ad = ipx_row_edges(a0, row[va + 1]), bd = ipx_row_edges(b0, row[vb + 1]);
+        uint4 qa = ipx_ld_quad(adj, a0, ad, 4 * gl);
+        for (; i < n; i += step) {
+            const uint32_t vd = i + 3 * step < n ? list[i + 3 * step] : 0u;
+            const uint64_t c0 = row[vc], c1 = row[vc + 1];
+            const uint4 qb = ipx_ld_quad(adj, b0, bd, 4 * gl);
+            if (!SKIP || ad <= ipx_c.hub_min) {
+                bool has = false;
+                ipx_msg acc;
+                const uint32_t len = ((uint32_t)a0 & 3u) + ad;
+                for (uint32_t rel = 4 * gl;;) {
+                    const uint4 next = ipx_ld_quad(adj, a0, ad, rel + 4 * G);
+                    ipx_pull_fold_quad(qa, a0, ad, rel, has, acc);
+                    rel += 4 * G;
+                    if (rel >= len) break;
+                    qa = next;
+                }
+                done(va, has, acc);
             }
+            va = vb;
+            vb = vc;
+            vc = vd;
+            a0 = b0;
+            ad = bd;
+            b0 = c0;
+            bd = ipx_row_edges(c0, c1);
+            qa = qb;
         }
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(IPX_THREADS, IPX_EDGE_CTAS) ipx_k_pull_deliver(const uint32_t* __restrict__ list,
-                                                                                uint64_t n,
-                                                                                const uint32_t* __restrict__ prefix)
+#ifndef IPX_PULL_CTAS
+#define IPX_PULL_CTAS 4
+#endif
+__global__ void __launch_bounds__(IPX_THREADS, IPX_PULL_CTAS) ipx_k_pull_deliver()
 {
     if (ipx_done() || !ipx_pulls()) return; /* this superstep pushes */
-    const int p = ipx_parity();
-    const uint64_t* __restrict__ row = ipx_c.in_row;
-    if constexpr (MODE == 0) {
-        for (uint64_t i = ipx_gtid(); i < n; i += ipx_gstride()) {
-            const uint64_t v = list[i];
-            bool has = false;
-            ipx_msg acc;
-            ipx_pull_fold_edges(row[v], row[v + 1], 0, 1, has, acc);
-            if (has && ipx_mb::merge(&ipx_c.mbox[p][v], acc)) ipx_set_bit_agg(ipx_c.recv[p], v);
-        }
-    } else if constexpr (MODE == 1) {
-        const int lane = threadIdx.x & 31;
-        for (uint64_t i = ipx_gtid() >> 5; i < n; i += ipx_gstride() >> 5) {
-            const uint64_t v = list[i];
-            bool has = false;
-            ipx_msg acc;
-            ipx_pull_fold_edges(row[v], row[v + 1], lane, 32, has, acc);
-            ipx_warp_fold(has, acc);
-            if (lane == 0 && has && ipx_mb::merge(&ipx_c.mbox[p][v], acc))
-                atomicOr(&ipx_c.recv[p][v >> 5], 1u << (v & 31));
-        }
-    } else {
-        __shared__ bool s_has[IPX_THREADS / 32];
-        __shared__ ipx_msg s_acc[IPX_THREADS / 32];
-        if (n == 0) return;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const uint32_t chunks = prefix[n];
-        for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-            const uint64_t i = ipx_c.hub_owner ? ipx_c.hub_owner[c] : ipx_hub_of_chunk(prefix, n, c);
-            const uint64_t v = list[i];
-            const uint64_t e0 = row[v] + (uint64_t)(c - prefix[i]) * IPX_HUB_CHUNK;
-            const uint64_t e1 = (e0 + IPX_HUB_CHUNK < row[v + 1]) ? e0 + IPX_HUB_CHUNK : row[v + 1];
-            bool has = false;
-            ipx_msg acc;
-            ipx_pull_fold_edges(e0, e1, threadIdx.x, blockDim.x, has, acc);
-            ipx_warp_fold(has, acc);
-            if (lane == 0) {
-                s_has[warp] = has;
-                s_acc[warp] = acc;
+    const int p = ipx_parity(), lane = threadIdx.x & 31;
+    const uint64_t warps = ipx_gstride() >> 5;
+    for (uint64_t c = ipx_gtid() >> 5; c < ipx_c.chunks; c += warps) {
+        const uint4 hub = ipx_c.hub[ipx_c.hub_owner[c]];
+        const uint64_t v = hub.x, e0 = ipx_c.in_row[v] + (c - hub.y) * ipx_c.hub_chunk, end = ipx_c.in_row[v + 1];
+        const uint64_t e1 = e0 + ipx_c.hub_chunk < end ? e0 + ipx_c.hub_chunk : end;
+        bool has = false;
+        ipx_msg acc;
+        if (sizeof(ipx_vid) == 4 && ipx_c.in_quads) {
+            const uint32_t* __restrict__ adj = reinterpret_cast<const uint32_t*>(ipx_c.in_adj);
+            const uint32_t deg = (uint32_t)(e1 - e0), len = ((uint32_t)e0 & 3u) + deg;
+            uint4 q = ipx_ld_quad(adj, e0, deg, 4 * lane);
+            for (uint32_t rel = 4 * lane; rel < len; rel += 128) {
+                const uint4 next = ipx_ld_quad(adj, e0, deg, rel + 128);
+                ipx_pull_fold_quad(q, e0, deg, rel, has, acc);
+                q = next;
             }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                has = false;
-                for (int w = 0; w < (int)(blockDim.x >> 5); w++) ipx_fold(has, acc, s_has[w], s_acc[w]);
-                /* chunks of one hub meet in its mailbox: the atomic delivery */
-                if (has && ipx_mb::deliver(&ipx_c.mbox[p][v], acc)) atomicOr(&ipx_c.recv[p][v >> 5], 1u << (v & 31));
-            }
-            __syncthreads();
+        } else {
+            ipx_pull_fold_edges(e0, e1, lane, 32, has, acc);
         }
+        ipx_warp_fold(has, acc);
+        /* chunks of one hub meet in its mailbox: the atomic delivery */
+        if (lane == 0 && has && ipx_mb::deliver(&ipx_c.mbox[p][v], acc)) atomicOr(&ipx_c.recv[p][v >> 5], 1u << (v & 31));
     }
+    ipx_pull_rows<IPX_PUSH_LONG, true>(ipx_c.class_list[2], ipx_c.class_n[2], p);
+    ipx_pull_rows<IPX_PUSH_GROUP, false>(ipx_c.class_list[1], ipx_c.class_n[1], p);
+    ipx_pull_rows<1, false>(ipx_c.class_list[0], ipx_c.class_n[0], p);
 }
+#endif
 
 /* ------------------------------------------------------------------------ */
 /* Compute kernels.                                                         */
@@ -2183,20 +2227,6 @@ __device__ __forceinline__ void ipx_fold_quad(const S* __restrict__ bs, uint32_t
     for (int k = 0; k < 4; k++) {
         ipx_msg m;
         if (ipx_slot_take(w[k], stamp, m)) ipx_fold(has, acc, true, m);
-    }
-}
-
-/* The tree over the G lanes of one group (G a power of two <= 32); `mask`
- * holds the group's lanes. */
-template <int G>
-__device__ __forceinline__ void ipx_group_fold(bool& has, ipx_msg& acc, unsigned mask)
-{
-    typedef typename ipx_word<ipx_msg>::type W;
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-        const bool oh = __shfl_down_sync(mask, has, o, G);
-        const ipx_msg om = ipx_from_word<ipx_msg>(__shfl_down_sync(mask, ipx_to_word(acc), o, G));
-        ipx_fold(has, acc, oh, om);
     }
 }
 

@@ -74,7 +74,6 @@ struct ipx_host_state {
      * re-attaching a graph of about the same shape allocates and frees
      * nothing (cudaFree synchronises the whole device) */
     std::vector<std::pair<void*, uint64_t>> spare;
-    uint32_t* pull_prefix = nullptr; /* chunk prefix of the static in-degree hubs (pulling push versions) */
     /* pinned: the records of a batch of supersteps, the last one's counts */
     struct ipx_pinned {
         unsigned long long hist[IPX_BATCH][4];
@@ -399,7 +398,7 @@ static int ipx_setup_state()
         int q = 0;
         IPX_OK(ipg_graph_quads(ipx_h.gw, 0, &q));
         c.out_quads = q;
-        c.in_quads = 0;
+        c.in_quads = q; /* the rows are the in-lists */
         if (gv.has_in) {
             IPX_OK(ipg_graph_quads(ipx_h.gw, 1, &q));
             c.in_quads = q;
@@ -451,18 +450,19 @@ static int ipx_setup_state()
     }
     if (c.pull_ok) {
         IPX_OK(ipx_alloc(&c.bcaster, W + 1));
-        IPX_OK(ipg_graph_bins(ipx_h.gw, gv.directed ? 1 : 0, ipx_h.tune.t0, ipx_h.tune.t1, &ipx_h.gbins));
-        IPX_OK(ipx_alloc(&ipx_h.pull_prefix, ipx_h.gbins.count[2] + 2));
-        uint32_t* dcount = nullptr;
-        IPX_OK(ipx_alloc(&dcount, 1));
-        const uint32_t n2 = (uint32_t)ipx_h.gbins.count[2];
-        IPX_CU(cudaMemcpy(dcount, &n2, 4, cudaMemcpyHostToDevice));
-        uint32_t* owner = nullptr;
-        IPX_OK(ipx_alloc(&owner, ipx_h.gbins.edges[2] / IPX_HUB_CHUNK + n2 + 1));
-        ipx_k_hub_prefix<><<<1, 1024>>>(ipx_h.gbins.d_list[2], dcount, c.in_row, ipx_h.pull_prefix, owner);
-        IPX_CU(cudaGetLastError());
-        IPX_CU(cudaDeviceSynchronize());
-        c.hub_owner = owner;
+        /* classes and chunks of the in-lists as of the push's rows */
+        const int in = gv.directed ? 1 : 0;
+        IPX_OK(ipg_graph_bins(ipx_h.gw, in, c.push_t[0], c.push_t[1], &ipx_h.gbins));
+        IPX_OK(ipg_graph_hubs(ipx_h.gw, in, c.push_t[2], c.push_chunk, &ipx_h.ghubs));
+        for (int k = 0; k < 3; k++) {
+            c.class_list[k] = ipx_h.gbins.d_list[k];
+            c.class_n[k] = (uint32_t)ipx_h.gbins.count[k];
+        }
+        c.hub = (const uint4*)ipx_h.ghubs.d_hub;
+        c.hub_owner = ipx_h.ghubs.d_owner;
+        c.hub_min = c.push_t[2];
+        c.chunks = (uint32_t)ipx_h.ghubs.chunks;
+        c.hub_chunk = c.push_chunk;
     }
 #endif
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
@@ -544,7 +544,7 @@ static int ipx_setup_state()
         IPX_CU(cudaFuncSetAttribute(ipx_k_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, IPX_MARK_WORDS * 4));
 #else
         ipx_h.grid_edge = ipx_resident_grid(ipx_k_push, tb, per_sm);
-        ipx_h.grid_pull = ipx_resident_grid(ipx_k_pull_deliver<1>, tb, per_sm);
+        ipx_h.grid_pull = ipx_resident_grid(ipx_k_pull_deliver, tb, per_sm);
 #endif
 #endif
     }
@@ -678,12 +678,9 @@ static void ipx_account_bytes(uint64_t s, uint64_t frontier)
 #else
     if (ipx_h.c.pull_ok && bedges > (double)ipx_h.c.pull_threshold) {
         /* pulled: every row once, messages of the broadcasting neighbours */
-        const ipg_bins& b = ipx_h.gbins;
-        const double E = ipx_h.c.E ? (double)ipx_h.c.E : 1.0;
-        for (int k = 0; k < 3; k++)
-            B[IPX_K_PULLD0 + k] +=
-                b.count[k] * (4.0 + 16.0 + sb) + b.edges[k] * (ib + 0.125) + bedges * (mb + wb) * (b.edges[k] / E);
-        for (int k = 0; k < 3; k++) N[IPX_K_PULLD0 + k] += b.edges[k];
+        const double E = (double)ipx_h.c.E;
+        B[IPX_K_PULLD] += ipx_h.c.V * (4.0 + 16.0 + sb) + E * (ib + 0.125) + bedges * (mb + wb);
+        N[IPX_K_PULLD] += E;
     } else {
         B[IPX_K_PUSH] += nb * (20.0 + mb) + bedges * (ib + sb + wb);
         N[IPX_K_PUSH] += bedges;
@@ -747,13 +744,7 @@ static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
      * when their out-edges pass the threshold, pull over every row; the
      * kernels of the other direction return at once */
     IPX_LAUNCH(IPX_K_PUSH, ipx_k_push<<<ge, ipx_h.tb, 0, st>>>());
-    if (c.pull_ok) {
-        const ipg_bins& b = ipx_h.gbins;
-        const uint32_t gp = ipx_h.grid_pull;
-        IPX_LAUNCH(IPX_K_PULLD0, ipx_k_pull_deliver<0><<<gp, ipx_h.tb, 0, st>>>(b.d_list[0], b.count[0], ipx_h.pull_prefix));
-        IPX_LAUNCH(IPX_K_PULLD1, ipx_k_pull_deliver<1><<<gp, ipx_h.tb, 0, st>>>(b.d_list[1], b.count[1], ipx_h.pull_prefix));
-        IPX_LAUNCH(IPX_K_PULLD2, ipx_k_pull_deliver<2><<<gp, ipx_h.tb, 0, st>>>(b.d_list[2], b.count[2], ipx_h.pull_prefix));
-    }
+    if (c.pull_ok) IPX_LAUNCH(IPX_K_PULLD, ipx_k_pull_deliver<<<ipx_h.grid_pull, ipx_h.tb, 0, st>>>());
     IPX_LAUNCH(IPX_K_COUNT, ipx_k_count<<<ipx_h.grid_count, IPX_THREADS, 0, st>>>(loop));
 #endif
 #endif

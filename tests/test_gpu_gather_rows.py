@@ -183,3 +183,53 @@ def test_users_of_one_graph_keep_their_classes(monkeypatch):
             plan.free()
         eng.release()
         graph.free()
+
+
+@pytest.mark.parametrize("tail", [0, 1, 2, 3])
+@pytest.mark.parametrize("app,version,id_bits,generic,symmetric", [
+    ("cc", "combiner", 32, False, False), ("cc", "spread", 32, False, True), ("cc", "spread", 64, False, False),
+    ("cc", "spread", 32, True, False), ("sssp_weighted", "combiner", 32, False, True),
+    ("sssp_weighted", "spread", 32, False, False), ("pagerank", "combiner", 32, False, False)])
+def test_pulled_rows_of_every_length(app, version, id_bits, generic, symmetric, tail):
+    """Every superstep with an edge to deliver pulls (over the transpose, or over the rows of a symmetric graph)."""
+    import ipregel_b200 as ip
+    g = _graph(tail)
+    rng = np.random.default_rng(tail)
+    # the in-lists get the lengths: edges reversed, and both ways on the symmetric graph
+    src, dst = g.adj.astype(np.int64), np.repeat(np.arange(g.V), np.diff(g.idx.astype(np.int64), append=g.E))
+    if symmetric:
+        src, dst = np.concatenate((src, dst)), np.concatenate((dst, src))
+    order = np.lexsort((dst, src))
+    src, dst = src[order], dst[order]
+    deg = np.bincount(src, minlength=g.V)
+    idx = np.concatenate(([0], np.cumsum(deg)[:-1])).astype(np.uint64)
+    wgt = (1 + (src * 31 + dst * 31 + src * dst) % 255).astype(np.uint32) if app == "sssp_weighted" else None
+    g = O.CSR(g.V, len(src), idx, dst.astype(np.uint32), wgt)
+    want, counts, _ = O.run(g, app, version, id_bytes=id_bits // 8)
+    adj = g.adj if id_bits == 32 else g.adj.astype(np.uint64)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, adj, wgt=wgt, id_bytes=id_bits // 8, directed=not symmetric)
+    if symmetric:
+        graph.set_symmetric(True)
+    eng = ip.Engine(app, version, id_bits, generic)
+    eng.set_quiet(True)
+    try:
+        if app == "pagerank":
+            eng.set_param("rounds", 10)
+        if app == "sssp_weighted":
+            eng.set_param("source", 0)
+        for tune in (dict(), dict(t0=4, t1=4096), dict(t0=2, t1=3), dict(block=64, t0=64, t1=200)):
+            for order in (True, False):
+                eng.set_order(order)
+                eng.set_tuning(pull_div=10 ** 9, **tune)
+                eng.attach(graph)
+                res = eng.run()
+                assert res.counts == [int(c) for c in counts], (tune, order)
+                if app == "pagerank":
+                    assert float(np.max(np.abs(res.values - want))) <= PR_TOL, (tune, order)
+                else:
+                    np.testing.assert_array_equal(res.values.astype(np.uint64), want.astype(np.uint64))
+    finally:
+        eng.set_tuning()
+        eng.set_order(True)
+        eng.release()
+        graph.free()
