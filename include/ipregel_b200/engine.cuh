@@ -674,7 +674,13 @@ __device__ __forceinline__ int ipx_parity() { return (int)(ipx_step() & 1); }
  * supersteps enqueued beyond it return at once), CTAs of the last kernel
  * that are done, and the time stamp of the last superstep's end. */
 enum { IPX_CTL_ERR, IPX_CTL_DONE, IPX_CTL_ARRIVED, IPX_CTL_STAMP, IPX_NCTL };
-__device__ __forceinline__ bool ipx_done() { return __ldcg(&ipx_c.ctl[IPX_CTL_DONE]) != 0ULL; }
+__device__ __forceinline__ bool ipx_done()
+{
+    /* lets the next kernel's CTAs onto the SMs as this one's leave them, and
+     * waits for the one before; each kernel of a superstep begins with it */
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+    return __ldcg(&ipx_c.ctl[IPX_CTL_DONE]) != 0ULL;
+}
 
 /* Kernel ids for launch counting and per-kernel profiling. */
 enum {

@@ -239,6 +239,15 @@ static uint32_t ipx_resident_grid(K kernel, int block, int per_sm)
     return ipx_grid(n < per_sm ? n : per_sm);
 }
 
+/* CTAs of an edge kernel: the resident ones, fewer when the graph has fewer
+ * rows and pairs of edges than threads (R-MAT scale 8 to 12: 3 to 8 % less per
+ * run; with groups of four instead of pairs scale 14 lost 2 %). */
+static uint32_t ipx_edge_grid(uint32_t resident, uint64_t V, uint64_t E, int block)
+{
+    const uint64_t ctas = (V + E / 2 + block - 1) / block;
+    return ctas < resident ? (ctas ? (uint32_t)ctas : 1u) : resident;
+}
+
 /* Words of a bitmap: whole groups of four, the rest zero (ipx_k_count). */
 static uint64_t ipx_bitmap_words(uint64_t W) { return (W + 4) & ~3ULL; }
 
@@ -548,6 +557,8 @@ static int ipx_setup_state()
 #endif
 #endif
     }
+    ipx_h.grid_edge = ipx_edge_grid(ipx_h.grid_edge, V, gv.E, ipx_h.tb);
+    if (ipx_h.grid_pull) ipx_h.grid_pull = ipx_edge_grid(ipx_h.grid_pull, V, gv.E, ipx_h.tb);
     ipx_h.ready = true;
     return ipx_reset_vertex_state();
 }
@@ -712,40 +723,74 @@ static int ipx_fail_device(uint32_t err)
  * enqueued beyond the program's end returns at once, so the same sequence
  * serves the host loop and the captured loop.  first: superstep 0 may be
  * among those the sequence serves. */
+/* A kernel of a superstep; early: its CTAs come onto the SMs while the kernel
+ * before it drains (programmatic dependent launch) and wait there for its end
+ * (ipx_done), so the launch is not in the chain of a superstep's three to
+ * five.  CC, weighted SSSP and PageRank on R-MAT of scale 8 to 18 take 10 to
+ * 30 % less; the compute and the counting kernel gain or lose nothing beyond.
+ * Not all do: the push, whose CTAs then sit on the SMs as the compute kernel
+ * left them and not in order, took 437 / 440 us at scale 18 (8 M edges; early /
+ * not), 547 / 544 at 19, 745 / 697 at 20, 6.9 / 5.45 ms at 24 (CC), so only
+ * graphs of fewer than IPX_EARLY_PUSH edges start it early.  The pull gather
+ * takes 1.72 / 1.82 ms at scale 20 (31 M edges, PageRank), 10.0 / 9.6 at 22,
+ * the target marking and its gather 1.27 / 1.30 at 20: IPX_EARLY_GATHER.  Not in
+ * captured loops, whose kernels are nodes of a graph. */
+#define IPX_EARLY_PUSH (1ULL << 23)
+#define IPX_EARLY_GATHER (1ULL << 25)
+template <class... P, class... A>
+static void ipx_start(bool early, void (*kernel)(P...), uint32_t grid, int block, size_t smem, A... args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ipx_h.st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
 {
+    const bool early = !loop.captured && !ipx_h.profile;
+    [[maybe_unused]] const bool early_push = early && ipx_h.c.E < IPX_EARLY_PUSH;
+    [[maybe_unused]] const bool early_gather = early && ipx_h.c.E < IPX_EARLY_GATHER;
     const ipx_consts& c = ipx_h.c;
     cudaStream_t st = ipx_h.st;
     const uint32_t g = ipx_h.grid_compute;
     const uint32_t ge = ipx_h.grid_edge;
     (void)first;
     (void)ge;
+    (void)st;
 #if IPX_VERSION == IPX_SINGLE_BROADCAST
     /* superstep 0's compute phase (returns at once later) */
-    if (first) IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_compute_sb0<<<g, ipx_h.tb, 0, st>>>());
+    if (first) IPX_LAUNCH(IPX_K_COMPUTE, ipx_start(false, ipx_k_compute_sb0, g, ipx_h.tb, 0));
     /* gather of this superstep fused with the next one's compute phase */
     const bool hot = c.in_adj_hot != nullptr;
 #if !IPX_HUB_WARP
     if (c.chunks)
-        IPX_LAUNCH(IPX_K_GATHER_HUBS, hot ? ipx_k_gather_hubs<true><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>()
-                                          : ipx_k_gather_hubs<false><<<ipx_h.grid_hubs, ipx_h.tb, 0, st>>>());
+        IPX_LAUNCH(IPX_K_GATHER_HUBS, hot ? ipx_start(early_gather, ipx_k_gather_hubs<true>, ipx_h.grid_hubs, ipx_h.tb, 0)
+                                          : ipx_start(early_gather, ipx_k_gather_hubs<false>, ipx_h.grid_hubs, ipx_h.tb, 0));
 #endif
-    IPX_LAUNCH(IPX_K_GATHER, hot ? ipx_k_gather_compute<true><<<ge, ipx_h.tb, 0, st>>>(loop)
-                                 : ipx_k_gather_compute<false><<<ge, ipx_h.tb, 0, st>>>(loop));
+    IPX_LAUNCH(IPX_K_GATHER, hot ? ipx_start(early_gather, ipx_k_gather_compute<true>, ge, ipx_h.tb, 0, loop)
+                                 : ipx_start(early_gather, ipx_k_gather_compute<false>, ge, ipx_h.tb, 0, loop));
 #else
-    IPX_LAUNCH(IPX_K_COMPUTE, ipx_k_front<<<g, ipx_h.tb, 0, st>>>(ipx_h.front_words));
+    IPX_LAUNCH(IPX_K_COMPUTE, ipx_start(early, ipx_k_front, g, ipx_h.tb, 0, ipx_h.front_words));
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
-    IPX_LAUNCH(IPX_K_MARK, ipx_k_mark<<<ipg_sm_count(), IPX_MARK_THREADS, ipx_h.mark_words * 4, st>>>(ipx_h.mark_words));
+    IPX_LAUNCH(IPX_K_MARK, ipx_start(early_gather, ipx_k_mark, ipg_sm_count(), IPX_MARK_THREADS, ipx_h.mark_words * 4, ipx_h.mark_words));
     IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.bt, c.V, c.in_row, ipx_h.tune.t0, ipx_h.tune.t1, c.tlist[0],
                                                    c.tlist[1], c.tlist[2], c.stat->tn, (uint64_t*)c.stat->tedges, 0, st)));
-    IPX_LAUNCH(IPX_K_GATHER, ipx_k_gather_targets<<<ge, ipx_h.tb, 0, st>>>(loop));
+    IPX_LAUNCH(IPX_K_GATHER, ipx_start(early_gather, ipx_k_gather_targets, ge, ipx_h.tb, 0, loop));
 #else
     /* delivery: push along the broadcasters' rows, or, on a symmetric graph
      * when their out-edges pass the threshold, pull over every row; the
      * kernels of the other direction return at once */
-    IPX_LAUNCH(IPX_K_PUSH, ipx_k_push<<<ge, ipx_h.tb, 0, st>>>());
-    if (c.pull_ok) IPX_LAUNCH(IPX_K_PULLD, ipx_k_pull_deliver<<<ipx_h.grid_pull, ipx_h.tb, 0, st>>>());
-    IPX_LAUNCH(IPX_K_COUNT, ipx_k_count<<<ipx_h.grid_count, IPX_THREADS, 0, st>>>(loop));
+    IPX_LAUNCH(IPX_K_PUSH, ipx_start(early_push, ipx_k_push, ge, ipx_h.tb, 0));
+    if (c.pull_ok) IPX_LAUNCH(IPX_K_PULLD, ipx_start(early_push, ipx_k_pull_deliver, ipx_h.grid_pull, ipx_h.tb, 0));
+    IPX_LAUNCH(IPX_K_COUNT, ipx_start(early, ipx_k_count, ipx_h.grid_count, IPX_THREADS, 0, loop));
 #endif
 #endif
     IPX_CU(cudaGetLastError());
