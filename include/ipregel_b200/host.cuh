@@ -759,12 +759,10 @@ static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
     [[maybe_unused]] const bool early_push = early && ipx_h.c.E < IPX_EARLY_PUSH;
     [[maybe_unused]] const bool early_gather = early && ipx_h.c.E < IPX_EARLY_GATHER;
     const ipx_consts& c = ipx_h.c;
-    cudaStream_t st = ipx_h.st;
     const uint32_t g = ipx_h.grid_compute;
     const uint32_t ge = ipx_h.grid_edge;
     (void)first;
     (void)ge;
-    (void)st;
 #if IPX_VERSION == IPX_SINGLE_BROADCAST
     /* superstep 0's compute phase (returns at once later) */
     if (first) IPX_LAUNCH(IPX_K_COMPUTE, ipx_start(false, ipx_k_compute_sb0, g, ipx_h.tb, 0));
@@ -782,7 +780,7 @@ static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
     IPX_LAUNCH(IPX_K_MARK, ipx_start(early_gather, ipx_k_mark, ipg_sm_count(), IPX_MARK_THREADS, ipx_h.mark_words * 4, ipx_h.mark_words));
     IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.bt, c.V, c.in_row, ipx_h.tune.t0, ipx_h.tune.t1, c.tlist[0],
-                                                   c.tlist[1], c.tlist[2], c.stat->tn, (uint64_t*)c.stat->tedges, 0, st)));
+                                                   c.tlist[1], c.tlist[2], c.stat->tn, (uint64_t*)c.stat->tedges, 0, ipx_h.st)));
     IPX_LAUNCH(IPX_K_GATHER, ipx_start(early_gather, ipx_k_gather_targets, ge, ipx_h.tb, 0, loop));
 #else
     /* delivery: push along the broadcasters' rows, or, on a symmetric graph
