@@ -427,13 +427,9 @@ __device__ __forceinline__ void mp_fmin_init(uint32_t* s_fmin)
 
 // A thread per low-degree frontier vertex (class 0): its lanes one at a
 // time, each over the vertex's few edges.
-__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_thread(MpArgs a, const uint32_t* __restrict__ list,
-                                                                     const uint32_t* __restrict__ count)
+__device__ __forceinline__ void mp_threads(const MpArgs& a, const uint32_t* __restrict__ list, uint32_t n, MpAcc& acc,
+                                           uint32_t* s_fmin)
 {
-    __shared__ uint32_t s_fmin[MP_K];
-    mp_fmin_init(s_fmin);
-    const uint32_t n = *count;
-    MpAcc acc;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t v = list[i];
         uint64_t M = a.front[v];
@@ -465,25 +461,17 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_thread(MpArgs a, co
         }
         if (deferred) mp_defer(a, v, deferred, acc);
     }
-    __syncthreads();
-    mp_block_flush(acc, a, s_fmin);
 }
 
 // A warp per frontier vertex (class 1).
-__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_vertices(MpArgs a, const uint32_t* __restrict__ list,
-                                                                       const uint32_t* __restrict__ count)
+__device__ __forceinline__ void mp_vertices(const MpArgs& a, const uint32_t* __restrict__ list, uint32_t n, MpAcc& acc,
+                                            uint32_t* s_fmin)
 {
-    __shared__ uint32_t s_fmin[MP_K];
-    mp_fmin_init(s_fmin);
-    const uint32_t n = *count;
-    MpAcc acc;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
         const uint64_t v = list[i];
         mp_relax(a, v, a.row[v], a.row[v + 1], true, acc, s_fmin);
     }
-    __syncthreads();
-    mp_block_flush(acc, a, s_fmin);
 }
 
 // A warp per HUB_CHUNK edges of a frontier hub; the hub's first chunk marks its
@@ -491,11 +479,8 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_vertices(MpArgs a, 
 // the frontier left out by a ballot: `per` chunks a warp (as many as give every
 // resident warp work, at most 32), taken `groups` apart, since the chunks of one
 // hub lie together.
-__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_hubs(MpArgs a, uint32_t per, uint32_t groups)
+__device__ __forceinline__ void mp_hubs(const MpArgs& a, uint32_t per, uint32_t groups, MpAcc& acc, uint32_t* s_fmin)
 {
-    __shared__ uint32_t s_fmin[MP_K];
-    mp_fmin_init(s_fmin);
-    MpAcc acc;
     const int lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
@@ -517,6 +502,24 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_hubs(MpArgs a, uint
             mp_relax(a, hub.x, e0, e1, c == hub.y, acc, s_fmin);
         }
     }
+}
+
+// A push superstep: the frontier hubs' chunks, then the rows a warp and those
+// a thread each, in one launch, so that the classes share one tail.
+// 14 queries took 4.73 ms with a launch a class and 4.28 so at undirected R-MAT
+// scale 20, 1.87 and 1.48 at 65,536 vertices (with k_mp_begin for four memsets
+// and a copy a superstep), 40 queries 13.3 and 13.6.
+__global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_push(MpArgs a, const uint32_t* __restrict__ l0,
+                                                                  const uint32_t* __restrict__ l1,
+                                                                  const uint32_t* __restrict__ cnt, uint32_t per,
+                                                                  uint32_t groups)
+{
+    __shared__ uint32_t s_fmin[MP_K];
+    mp_fmin_init(s_fmin);
+    MpAcc acc;
+    mp_hubs(a, per, groups, acc, s_fmin);
+    mp_vertices(a, l1, cnt[1], acc, s_fmin);
+    mp_threads(a, l0, cnt[0], acc, s_fmin);
     __syncthreads();
     mp_block_flush(acc, a, s_fmin);
 }
@@ -682,15 +685,31 @@ __global__ void __launch_bounds__(SRV_THREADS, MP_CTAS) k_mp_pull_hubs(MpArgs a)
 }
 
 // After a superstep: the consumed frontier masks back to zero.
-__global__ void k_mp_clear(uint64_t* __restrict__ front, const uint32_t* __restrict__ l0, const uint32_t* __restrict__ l1,
-                           const uint32_t* __restrict__ l2, const uint32_t* __restrict__ cnt)
+__global__ void k_mp_clear(uint64_t* __restrict__ front, uint32_t* __restrict__ fcur, const uint32_t* __restrict__ l0,
+                           const uint32_t* __restrict__ l1, const uint32_t* __restrict__ l2,
+                           const uint32_t* __restrict__ cnt)
 {
     const uint64_t n0 = cnt[0], n1 = cnt[1], n2 = cnt[2];
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n0 + n1 + n2;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t v = i < n0 ? l0[i] : (i < n0 + n1 ? l1[i - n0] : l2[i - n0 - n1]);
         front[v] = 0ULL;
+        fcur[v >> 5] = 0u;  // every bit of the word is a frontier vertex's
     }
+}
+
+// The status and the lanes' thresholds for the superstep about to run (the
+// list sizes stay: they are its frontier's).
+struct MpThr {
+    uint32_t t[MP_K];
+};
+__global__ void __launch_bounds__(MP_K) k_mp_begin(MpStatus* __restrict__ st, uint32_t* __restrict__ thr, MpThr t)
+{
+    const int k = threadIdx.x;
+    thr[k] = t.t[k];
+    st->far_min[k] = SRV_INF;
+    if (k < 3) st->esum[k] = 0ULL;
+    if (k == 3) st->any = st->near = st->far = st->work = 0ULL;
 }
 
 // Lane k of every vertex to the vertex id, every vertex in lane k's frontier
@@ -1091,8 +1110,7 @@ __device__ __forceinline__ void pp_gather_group(const PpArgs& a, uint64_t e0, ui
 // for 7 (2 quads) and 21.1 to 14.8 for 32; with narrow groups alone 13.4, 17.0
 // and 22.0, with rows to 512 in one piece 6.0, 6.9 and 14.6.
 template <int NQ>
-__global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_rows(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
-                                                         uint64_t n)
+__device__ __forceinline__ void pp_rows(const PpArgs& a, const PpLanes& L, const uint32_t* __restrict__ list, uint64_t n)
 {
     constexpr int IPT = NQ < 4 ? 4 / NQ : 1;  // ids a thread loads per four edges
     const int lane = threadIdx.x & 31, q = lane % NQ, gb = lane - q;
@@ -1160,8 +1178,8 @@ __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_rows(PpArgs a, PpLanes L,
 // PP_SLOTS * NQ threads per vertex of higher degree (up to MP_T1; hubs are
 // passed over).
 template <int NQ>
-__global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_vertices(PpArgs a, PpLanes L, const uint32_t* __restrict__ list,
-                                                             uint64_t n)
+__device__ __forceinline__ void pp_vertices(const PpArgs& a, const PpLanes& L, const uint32_t* __restrict__ list,
+                                            uint64_t n)
 {
     constexpr int GS = PP_SLOTS * NQ;
     const int t = threadIdx.x & (GS - 1);
@@ -1180,7 +1198,7 @@ __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_vertices(PpArgs a, PpLane
 
 // Hubs: as many threads per HUB_CHUNK edges, partial sums per chunk and lane...
 template <int NQ>
-__global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_hub_chunks(PpArgs a, PpLanes L)
+__device__ __forceinline__ void pp_hub_chunks(const PpArgs& a, const PpLanes& L)
 {
     constexpr int GS = PP_SLOTS * NQ;
     const int t = threadIdx.x & (GS - 1);
@@ -1197,6 +1215,19 @@ __global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_hub_chunks(PpArgs a, PpLa
 #pragma unroll
             for (int j = 0; j < 4; j++) a.partial[c * PP_K + 4 * Q + j] = make_float2(s[j], cc[j]);
     }
+}
+
+// All of a superstep's gathers but the hubs' last merge, the longest first, in
+// one launch: 20 rounds of 1 / 7 / 32 queries at scale 20 took 5.1 / 6.1 / 14.7
+// ms with a launch a class and 4.8 / 5.8 / 13.9 so.
+template <int NQ>
+__global__ void __launch_bounds__(SRV_THREADS, 4) k_pp_step(const PpArgs a, const PpLanes L,
+                                                            const uint32_t* __restrict__ l0, uint64_t n0,
+                                                            const uint32_t* __restrict__ l1, uint64_t n1)
+{
+    pp_hub_chunks<NQ>(a, L);
+    pp_vertices<NQ>(a, L, l1, n1);
+    pp_rows<NQ>(a, L, l0, n0);
 }
 
 // ...then a warp per hub and walked quad merges the hub's chunks: a thread per
@@ -1291,8 +1322,7 @@ struct Group {
     uint64_t hesum = 0;                   // frontier edges of the next superstep (last status)
     uint32_t* cnt = nullptr;              // into stat_d
     uint32_t* thr_d = nullptr;            // lane thresholds of the next superstep
-    uint32_t* thr_pin = nullptr;          // their pinned staging copy
-    uint32_t thr_h[MP_K];
+    MpThr thr_h{};
     MpStatus* stat_d = nullptr;
     MpStatus* stat_h = nullptr;           // pinned copy after each superstep
     uint32_t hn[3] = {0, 0, 0};           // list sizes the host knows of
@@ -1366,7 +1396,6 @@ void free_group(ipg_server* S, Group* G)
     if (G->st) cudaStreamSynchronize(G->st);
     for (auto& a : G->allocs) ipg_dev_free(a.first, a.second);
     if (G->stat_h) cudaFreeHost(G->stat_h);
-    if (G->thr_pin) cudaFreeHost(G->thr_pin);
     if (G->ev) cudaEventDestroy(G->ev);
     if (G->ev0) cudaEventDestroy(G->ev0);
     if (G->st) cudaStreamDestroy(G->st);
@@ -1486,8 +1515,6 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
         if (r == IPG_OK) r = galloc(G, &G->stat_d, 1);
         if (r == IPG_OK) G->cnt = G->stat_d->cnt;
         if (r == IPG_OK) r = galloc(G, &G->thr_d, MP_K);
-        if (r == IPG_OK && cudaHostAlloc((void**)&G->thr_pin, MP_K * 4, cudaHostAllocDefault) != cudaSuccess)
-            r = ipg_internal_fail(IPG_ENOMEM, "serve: pinned allocation failed");
         if (r == IPG_OK && cudaHostAlloc((void**)&G->stat_h, sizeof(MpStatus), cudaHostAllocDefault) != cudaSuccess)
             r = ipg_internal_fail(IPG_ENOMEM, "serve: pinned allocation failed");
         if (r == IPG_OK) {
@@ -1644,7 +1671,7 @@ void admit(ipg_server* S, Group* G, double now)
             } else if (q.kind == IPG_QUERY_CC) {
                 k_mp_init_lane<<<g, SRV_THREADS, 0, G->st>>>(G->dist, G->front[G->cur], V, k, 1);
                 G->wmask &= ~(1ULL << k);
-                G->thr_h[k] = SRV_INF;  // labels are no distances: never deferred
+                G->thr_h.t[k] = SRV_INF;  // labels are no distances: never deferred
                 G->cc_lane = k;
                 rebuild = true;
             } else {
@@ -1652,7 +1679,7 @@ void admit(ipg_server* S, Group* G, double now)
                 k_mp_admit_source<<<1, 1, 0, G->st>>>(G->dist, G->front[G->cur], G->fbm[G->cur], G->G->gv.d_row,
                                                        q.src, k, G->list[0], G->list[1], G->list[2], G->cnt);
                 G->wmask |= 1ULL << k;
-                G->thr_h[k] = S->delta;
+                G->thr_h.t[k] = S->delta;
                 G->appended++;
             }
             S->stats.lanes_admitted++;
@@ -1701,12 +1728,7 @@ int launch_superstep(ipg_server* S, Group* G)
         // appended since (each in some list)
         const uint64_t add = G->appended;
         const uint64_t n0 = G->hn[0] + add, n1 = G->hn[1] + add;
-        memcpy(G->thr_pin, G->thr_h, sizeof G->thr_h);  // the last copy finished with the last superstep
-        cudaMemcpyAsync(G->thr_d, G->thr_pin, sizeof G->thr_h, cudaMemcpyHostToDevice, G->st);
-        cudaMemsetAsync(G->stat_d, 0, 3 * sizeof(unsigned long long), G->st);
-        cudaMemsetAsync(G->stat_d->far_min, 0xff, sizeof G->stat_d->far_min, G->st);
-        cudaMemsetAsync(&G->stat_d->work, 0, sizeof G->stat_d->work, G->st);
-        cudaMemsetAsync(G->stat_d->esum, 0, sizeof G->stat_d->esum, G->st);
+        k_mp_begin<<<1, MP_K, 0, G->st>>>(G->stat_d, G->thr_d, G->thr_h);
         // direction: pull when the frontier's edges are a large part of the
         // graph and enough lanes are busy to share each row read
         const Graph* Gr = G->G;
@@ -1723,31 +1745,27 @@ int launch_superstep(ipg_server* S, Group* G)
                 k_mp_pull_hubs<<<resident_cap(k_mp_pull_hubs, warp_grid(chunks)), SRV_THREADS, 0, G->st>>>(a);
             S->stats.kernel_launches += (n01 ? 1 : 0) + (chunks ? 1 : 0);
         } else {
-            k_mp_thread<<<resident_cap(k_mp_thread, thread_grid(n0)), SRV_THREADS, 0, G->st>>>(a, G->list[0],
-                                                                                            G->cnt + 0);
-            k_mp_vertices<<<resident_cap(k_mp_vertices, warp_grid(n1)), SRV_THREADS, 0, G->st>>>(a, G->list[1],
-                                                                                              G->cnt + 1);
             const bool hubs = chunks && G->hn[2] + add;
-            if (hubs) {
-                const uint64_t warps = (uint64_t)resident_cap(k_mp_hubs, warp_grid(chunks)) * (SRV_THREADS / 32);
-                const uint32_t per = (uint32_t)std::min<uint64_t>(32, (chunks + warps - 1) / warps);
-                const uint32_t groups = (uint32_t)((chunks + per - 1) / per);
-                k_mp_hubs<<<resident_cap(k_mp_hubs, warp_grid(groups)), SRV_THREADS, 0, G->st>>>(a, per, groups);
-            }
-            S->stats.kernel_launches += hubs ? 3 : 2;
+            const uint32_t grid = resident_cap(
+                k_mp_push, (uint32_t)std::min<uint64_t>(0x7fffffffULL, (uint64_t)thread_grid(n0) + warp_grid(n1) +
+                                                                          (hubs ? warp_grid(chunks) : 0)));
+            const uint64_t warps = (uint64_t)grid * (SRV_THREADS / 32);
+            const uint32_t per = hubs ? (uint32_t)std::min<uint64_t>(32, (chunks + warps - 1) / warps) : 1;
+            const uint32_t groups = hubs ? (uint32_t)((chunks + per - 1) / per) : 0;
+            k_mp_push<<<grid, SRV_THREADS, 0, G->st>>>(a, G->list[0], G->list[1], G->cnt, per, groups);
+            S->stats.kernel_launches += 1;
         }
         S->stats.pull_supersteps += pull ? 1 : 0;
         k_mp_clear<<<resident_cap(k_mp_clear, thread_grid(G->hn[0] + G->hn[1] + G->hn[2] + add)), SRV_THREADS, 0,
-                     G->st>>>(G->front[G->cur], G->list[0], G->list[1], G->list[2], G->cnt);
+                     G->st>>>(G->front[G->cur], G->fbm[G->cur], G->list[0], G->list[1], G->list[2], G->cnt);
         cudaMemsetAsync(G->cnt, 0, 12, G->st);
         // the next bitmap is kept (it is the next superstep's frontier bitmap);
-        // this superstep's is cleared for reuse as the one after
+        // this superstep's was cleared for reuse as the one after
         ipg_compact(G->fbm[G->cur ^ 1], gv.V, gv.d_row, MP_T0, MP_T1, G->list[0], G->list[1], G->list[2], G->cnt,
                     (uint64_t*)G->stat_d->esum, 0, G->st);
-        cudaMemsetAsync(G->fbm[G->cur], 0, ((gv.V + 31) / 32 + 1) * 4, G->st);
         cudaMemcpyAsync(G->stat_h, G->stat_d, sizeof(MpStatus), cudaMemcpyDeviceToHost, G->st);
         G->cur ^= 1;
-        S->stats.kernel_launches += 3;
+        S->stats.kernel_launches += 4;
     } else {
         const Graph* Gr = G->G;
         PpArgs a;
@@ -1791,14 +1809,9 @@ int launch_superstep(ipg_server* S, Group* G)
         G->dirty[G->cur ^ 1] = busy_quads;
         auto launch = [&](auto width) {
             constexpr int NQ = decltype(width)::value;
-            if (n0)
-                k_pp_rows<NQ><<<resident_cap(k_pp_rows<NQ>, thread_grid(n0 * NQ)), SRV_THREADS, 0, G->st>>>(a, L, l0, n0);
-            if (n1)
-                k_pp_vertices<NQ><<<resident_cap(k_pp_vertices<NQ>, thread_grid(n1 * PP_SLOTS * NQ)), SRV_THREADS, 0,
-                                    G->st>>>(a, L, l1, n1);
-            if (a.H.chunks)
-                k_pp_hub_chunks<NQ><<<resident_cap(k_pp_hub_chunks<NQ>, thread_grid(a.H.chunks * PP_SLOTS * NQ)),
-                                      SRV_THREADS, 0, G->st>>>(a, L);
+            const uint64_t threads = (n0 + (n1 + a.H.chunks) * PP_SLOTS) * NQ;
+            k_pp_step<NQ><<<resident_cap(k_pp_step<NQ>, thread_grid(threads)), SRV_THREADS, 0, G->st>>>(a, L, l0, n0, l1,
+                                                                                                       n1);
         };
         if (nq <= 1) launch(std::integral_constant<int, 1>());
         else if (nq <= 2) launch(std::integral_constant<int, 2>());
@@ -1807,7 +1820,7 @@ int launch_superstep(ipg_server* S, Group* G)
         if (a.H.hubs)
             k_pp_hub_finish<<<resident_cap(k_pp_hub_finish, warp_grid(a.H.hubs * nq)), SRV_THREADS, 0, G->st>>>(a, L, nq);
         G->cur ^= 1;
-        S->stats.kernel_launches += 4;
+        S->stats.kernel_launches += a.H.hubs ? 2 : 1;
     }
     cudaEventRecord(G->ev, G->st);
     cudaError_t e = cudaGetLastError();
@@ -1834,8 +1847,8 @@ void retire(ipg_server* S, Group* G, double now)
         const uint64_t raise = G->busy & st.far & ~st.near;
         for (int k = 0; k < MP_K; k++)
             if ((raise >> k) & 1) {
-                const uint64_t base = st.far_min[k] != SRV_INF ? st.far_min[k] : G->thr_h[k];
-                G->thr_h[k] = (uint32_t)std::min<uint64_t>(base + S->delta, SRV_INF);
+                const uint64_t base = st.far_min[k] != SRV_INF ? st.far_min[k] : G->thr_h.t[k];
+                G->thr_h.t[k] = (uint32_t)std::min<uint64_t>(base + S->delta, SRV_INF);
             }
         uint64_t extracted = 0;
         for (int k = 0; k < MP_K; k++) {
