@@ -81,10 +81,13 @@ static_assert(sizeof(ipx_msg) <= 8, "iPregel-B200: IP_MESSAGE_TYPE must be at mo
 /* Largest CTA the kernels are compiled for; the launch size is a runtime
  * tuning parameter (a multiple of 32 up to this). */
 #define IPX_THREADS 256
-/* CTA of the target marking kernel: one per SM, its shared memory the bits
- * of the most often visited targets. */
+/* CTA of the target marking kernel, its shared memory the bits of the most
+ * often visited targets (bitmap words of the lowest, that is best connected,
+ * vertices). */
 #define IPX_MARK_THREADS 1024
-#define IPX_MARK_WORDS 40960 /* most of them: 160 KiB */
+#ifndef IPX_MARK_WORDS
+#define IPX_MARK_WORDS 1024
+#endif
 #define IPX_ERR_SEND_IN_BROADCAST 1u
 #define IPX_ERR_COMBINE_HINT 2u
 #define IPX_ERR_SUPERSTEP_LIMIT 4u
@@ -1017,7 +1020,12 @@ struct ipx_push_visit {
 /* Target marking (spread+single_broadcast).  Targets below `bits` have a bit
  * in the CTA's shared memory too, set at the CTA's first visit: a hub is hit
  * by a large part of all edges, and without it every hit would read (or, from
- * a stale L1 line, set) the same word of the L2. */
+ * a stale L1 line, set) the same word of the L2.  Few targets are hubs: with
+ * the bits of 1.3 M vertices (160 KiB, which leaves room for one CTA and little
+ * L1) CC at R-MAT scale 22 / 24 took 3.74 / 13.0 ms, with 512 k 3.67 / 12.9,
+ * with 32 k 3.50 / 12.7, and with 32 k and two CTAs per SM 3.13 / 10.8, the
+ * latency of the other targets' words being what is left.  16 k bits do as
+ * well; CTAs of 256 or 512 threads take 1 to 3 % more. */
 struct ipx_mark_visit {
     static constexpr bool kNeedsMessage = false;
     uint32_t* seen;
@@ -1295,9 +1303,12 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_PUSH_CTAS) ipx_k_push()
 }
 
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
-/* Marks the out-neighbours of broadcasters as targets. */
+/* Marks the out-neighbours of broadcasters as targets.  CTAS per SM: two on
+ * 2^23 edges and more; below, where there is less to wait for, one with twice
+ * the registers (561 against 575 us, SSSP at R-MAT scale 18). */
 extern __shared__ uint32_t ipx_seen[];
-__global__ void __launch_bounds__(IPX_MARK_THREADS, 1) ipx_k_mark(uint32_t words)
+template <int CTAS>
+__global__ void __launch_bounds__(IPX_MARK_THREADS, CTAS) ipx_k_mark(uint32_t words)
 {
     if (ipx_done()) return;
     for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) ipx_seen[k] = 0u;

@@ -104,6 +104,7 @@ struct ipx_host_state {
     uint32_t grid_edge = 0;    /* resident CTAs of the edge kernels */
     uint32_t grid_count = 0;   /* CTAs of the counting kernel */
     uint32_t grid_pull = 0;    /* resident CTAs of the pull delivery */
+    uint32_t mark_ctas = 1;    /* CTAs per SM of the marking kernel */
     uint32_t mark_words = 0;   /* spread+single_broadcast: bits of the marking kernel in shared memory */
     int front_words = 1;       /* bitmap words a warp of the compute kernel takes at a time */
     uint32_t grid_hubs = 0;    /* single_broadcast, a CTA per hub chunk: of the hub kernel */
@@ -550,7 +551,7 @@ static int ipx_setup_state()
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
         ipx_h.grid_edge = ipx_resident_grid(ipx_k_gather_targets, tb, per_sm);
         ipx_h.mark_words = (uint32_t)(W < IPX_MARK_WORDS ? W : IPX_MARK_WORDS);
-        IPX_CU(cudaFuncSetAttribute(ipx_k_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, IPX_MARK_WORDS * 4));
+        ipx_h.mark_ctas = gv.E < (1ULL << 23) ? 1 : 2;
 #else
         ipx_h.grid_edge = ipx_resident_grid(ipx_k_push, tb, per_sm);
         ipx_h.grid_pull = ipx_resident_grid(ipx_k_pull_deliver, tb, per_sm);
@@ -778,7 +779,9 @@ static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
 #else
     IPX_LAUNCH(IPX_K_COMPUTE, ipx_start(early, ipx_k_front, g, ipx_h.tb, 0, ipx_h.front_words));
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
-    IPX_LAUNCH(IPX_K_MARK, ipx_start(early_gather, ipx_k_mark, ipg_sm_count(), IPX_MARK_THREADS, ipx_h.mark_words * 4, ipx_h.mark_words));
+    IPX_LAUNCH(IPX_K_MARK, ipx_start(early_gather, ipx_h.mark_ctas == 2 ? ipx_k_mark<2> : ipx_k_mark<1>,
+                                     (uint32_t)ipg_sm_count() * ipx_h.mark_ctas, IPX_MARK_THREADS, ipx_h.mark_words * 4,
+                                     ipx_h.mark_words));
     IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.bt, c.V, c.in_row, ipx_h.tune.t0, ipx_h.tune.t1, c.tlist[0],
                                                    c.tlist[1], c.tlist[2], c.stat->tn, (uint64_t*)c.stat->tedges, 0, ipx_h.st)));
     IPX_LAUNCH(IPX_K_GATHER, ipx_start(early_gather, ipx_k_gather_targets, ge, ipx_h.tb, 0, loop));
