@@ -166,7 +166,7 @@ extern "C" {
 __host__ __device__ size_t ip_get_superstep()
 {
 #ifdef __CUDA_ARCH__
-    return __ldg((const unsigned long long*)&ipd_compute_superstep);
+    return ipd_compute_superstep; /* a plain load: a kernel may start before the value is written */
 #else
     return ip_superstep;
 #endif
