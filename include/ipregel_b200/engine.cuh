@@ -669,10 +669,11 @@ __device__ __forceinline__ ipx_vid ipx_user_id(uint64_t v)
 }
 
 /* The current superstep, from device memory: each superstep's last kernel
- * advances it, so every kernel of a superstep reads the same value.  Volatile,
- * like the end flag below: a kernel may have started before the value was
- * written (ipx_done), so the compiler must not move the read ahead of the wait. */
-__device__ __forceinline__ uint64_t ipx_step() { return (uint64_t)*(const volatile size_t*)&ipd_superstep; }
+ * advances it, so every kernel of a superstep reads the same value.  A plain
+ * load, like the end flag's below: a kernel may have started before the value
+ * was written (ipx_done), so the compiler must not move the read ahead of the wait,
+ * as it may __ldg's. */
+__device__ __forceinline__ uint64_t ipx_step() { return (uint64_t)ipd_superstep; }
 __device__ __forceinline__ int ipx_parity() { return (int)(ipx_step() & 1); }
 
 /* Control words: the error word, "the program has ended" (the kernels of
@@ -684,7 +685,7 @@ __device__ __forceinline__ bool ipx_done()
     /* lets the next kernel's CTAs onto the SMs as this one's leave them, and
      * waits for the one before; each kernel of a superstep begins with it */
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
-    return *(const volatile unsigned long long*)&ipx_c.ctl[IPX_CTL_DONE] != 0ULL;
+    return ipx_c.ctl[IPX_CTL_DONE] != 0ULL;
 }
 
 /* Kernel ids for launch counting and per-kernel profiling. */
