@@ -162,14 +162,25 @@ struct ip_vertex_t {
 extern "C" {
 #endif
 
+#ifdef __CUDACC__
+/* The superstep that ip_get_superstep reports on the device: a word of the CTA's
+ * shared memory, which every engine kernel that runs the application's functions
+ * fills at its start (ipx_done).  ipd_compute_superstep itself is written while
+ * the next kernel's CTAs wait on the SMs, so its load has to be ordered behind
+ * their wait and must not take the read-only path; such a load in the vertex
+ * loop cost 5.7 -> 6.8 ms for CC and SSSP over a union of 256 random graphs. */
+__device__ __forceinline__ size_t& ipx_step_word()
+{
+    __shared__ size_t s_step;
+    return s_step;
+}
+#endif
+
 /* ---- accessors (src/iPregel_preamble.h:66-103) ---- */
 __host__ __device__ size_t ip_get_superstep()
 {
 #ifdef __CUDA_ARCH__
-    /* through the read-only path, so that it leaves the vertex loop (a plain
-     * load stays in it: 5.7 -> 6.8 ms for CC and SSSP over a union of 256 random
-     * graphs); the loops lie behind the kernel's wait and its test of the end */
-    return __ldg((const unsigned long long*)&ipd_compute_superstep);
+    return ipx_step_word();
 #else
     return ip_superstep;
 #endif

@@ -536,31 +536,36 @@ __device__ __forceinline__ uint64_t ipx_policy(bool hot)
 __device__ __forceinline__ unsigned long long ipx_ld_policy(const unsigned long long* p, uint64_t pol)
 {
     unsigned long long r;
-    asm volatile("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(pol));
     return r;
 }
 __device__ __forceinline__ uint2 ipx_ld_policy(const uint2* p, uint64_t pol)
 {
     uint2 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(r.x), "=r"(r.y) : "l"(p), "l"(pol));
+    asm volatile("ld.global.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(r.x), "=r"(r.y) : "l"(p), "l"(pol));
     return r;
 }
 __device__ __forceinline__ uint4 ipx_ld_policy(const uint4* p, uint64_t pol)
 {
     uint4 r;
-    asm volatile("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+    asm volatile("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                  : "l"(p), "l"(pol));
     return r;
 }
-/* The slot of the in-neighbour whose id word is w: HOT ids carry the flag. */
+/* The slot of the in-neighbour whose id word is w: HOT ids carry the flag.
+ * Slots, mailboxes, messages, bitmaps and lists are written by the kernel before,
+ * which may still run when this one's CTAs come onto the SMs (ipx_done): they are
+ * read by ordinary loads, not through the read-only path (__ldg, ld.global.nc),
+ * which is for what nothing writes while the grid exists, and their pointers are
+ * not declared __restrict__. */
 template <bool HOT, class S>
-__device__ __forceinline__ S ipx_slot_ld(const S* __restrict__ bs, uint64_t w)
+__device__ __forceinline__ S ipx_slot_ld(const S* bs, uint64_t w)
 {
     if constexpr (HOT) {
         return ipx_ld_policy(&bs[w & (IPX_HOT_BIT - 1u)], ipx_policy((w & IPX_HOT_BIT) != 0));
     } else {
-        return __ldg(&bs[w]);
+        return bs[w];
     }
 }
 
@@ -671,8 +676,7 @@ __device__ __forceinline__ ipx_vid ipx_user_id(uint64_t v)
 /* The current superstep, from device memory: each superstep's last kernel
  * advances it, so every kernel of a superstep reads the same value.  A plain
  * load, like the end flag's below: a kernel may have started before the value
- * was written (ipx_done), so the compiler must not move the read ahead of the wait,
- * as it may __ldg's. */
+ * was written (ipx_done). */
 __device__ __forceinline__ uint64_t ipx_step() { return (uint64_t)ipd_superstep; }
 __device__ __forceinline__ int ipx_parity() { return (int)(ipx_step() & 1); }
 
@@ -680,12 +684,19 @@ __device__ __forceinline__ int ipx_parity() { return (int)(ipx_step() & 1); }
  * supersteps enqueued beyond it return at once), CTAs of the last kernel
  * that are done, and the time stamp of the last superstep's end. */
 enum { IPX_CTL_ERR, IPX_CTL_DONE, IPX_CTL_ARRIVED, IPX_CTL_STAMP, IPX_NCTL };
-__device__ __forceinline__ bool ipx_done()
+/* step: the kernel runs functions of the application (ip_compute, ip_combine,
+ * the edge's message), which may ask for the superstep. */
+__device__ __forceinline__ bool ipx_done(bool step = true)
 {
     /* lets the next kernel's CTAs onto the SMs as this one's leave them, and
      * waits for the one before; each kernel of a superstep begins with it */
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
-    return ipx_c.ctl[IPX_CTL_DONE] != 0ULL;
+    const bool done = ipx_c.ctl[IPX_CTL_DONE] != 0ULL;
+    if (step) {
+        if (threadIdx.x == 0) ipx_step_word() = ipd_compute_superstep;
+        __syncthreads();
+    }
+    return done;
 }
 
 /* Kernel ids for launch counting and per-kernel profiling. */
@@ -944,7 +955,7 @@ struct ipx_push_visit {
     template <class MB = ipx_mb>
     __device__ __forceinline__ void deliver(const ipx_vid* w, const bool* ok, const ipx_msg* mk) const
     {
-        ipx_slot* __restrict__ box = ipx_c.mbox[p];
+        ipx_slot* box = ipx_c.mbox[p];
         if constexpr (MB::kPeek) {
             ipx_slot c[4];
 #pragma unroll
@@ -1082,7 +1093,7 @@ __device__ __forceinline__ void ipx_edges_strided(const ipx_vid* __restrict__ ad
  * row bounds and message -> ids -> mailboxes is pipelined over the group's
  * next sources, as in the pull gather. */
 template <int G, class Visit>
-__device__ __forceinline__ void ipx_walk_rows(const uint32_t* __restrict__ list, uint32_t n, const Visit& visit)
+__device__ __forceinline__ void ipx_walk_rows(const uint32_t* list, uint32_t n, const Visit& visit)
 {
     const uint32_t gl = threadIdx.x & (G - 1);
     const uint64_t* __restrict__ row = ipx_c.row;
@@ -1313,7 +1324,7 @@ extern __shared__ uint32_t ipx_seen[];
 template <int CTAS>
 __global__ void __launch_bounds__(IPX_MARK_THREADS, CTAS) ipx_k_mark(uint32_t words)
 {
-    if (ipx_done()) return;
+    if (ipx_done(false)) return;
     for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) ipx_seen[k] = 0u;
     __syncthreads();
     ipx_walk_broadcasters(ipx_mark_visit{ipx_seen, 32ULL * words});
@@ -1357,7 +1368,7 @@ __device__ __forceinline__ void ipx_warp_fold(bool& has, ipx_msg& acc)
  * (ipx_gather_fold_edges_v4). */
 template <bool HOT = false, class S>
 __device__ __forceinline__ void ipx_gather_fold_edges_v4(const uint32_t* __restrict__ adj,
-                                                         const S* __restrict__ bs, uint32_t stamp,
+                                                         const S* bs, uint32_t stamp,
                                                          uint64_t e0, uint64_t e1, uint64_t lane, uint64_t lanes,
                                                          bool& has, ipx_msg& acc)
 {
@@ -1397,7 +1408,7 @@ __device__ __forceinline__ void ipx_gather_fold_edges_v4(const uint32_t* __restr
 
 template <bool HOT = false, class S>
 __device__ __forceinline__ void ipx_gather_fold_edges(const ipx_vid* __restrict__ adj,
-                                                      const S* __restrict__ bs, uint32_t stamp, uint64_t e0,
+                                                      const S* bs, uint32_t stamp, uint64_t e0,
                                                       uint64_t e1, uint64_t lane, uint64_t lanes, bool& has,
                                                       ipx_msg& acc)
 {
@@ -1463,15 +1474,15 @@ __device__ __forceinline__ void ipx_group_fold(bool& has, ipx_msg& acc, unsigned
  * 3.39 now. */
 __device__ __forceinline__ void ipx_pull_fold4(const uint64_t* u, const bool* ok, const ipx_wgt* x, bool& has, ipx_msg& acc)
 {
-    const uint32_t* __restrict__ bc = ipx_c.bcaster;
-    const ipx_msg* __restrict__ ob = ipx_c.outbox;
+    const uint32_t* bc = ipx_c.bcaster;
+    const ipx_msg* ob = ipx_c.outbox;
     bool on[4];
     ipx_msg m[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) on[k] = ok[k] && ((__ldg(&bc[u[k] >> 5]) >> (u[k] & 31)) & 1u);
+    for (int k = 0; k < 4; k++) on[k] = ok[k] && ((bc[u[k] >> 5] >> (u[k] & 31)) & 1u);
 #pragma unroll
     for (int k = 0; k < 4; k++)
-        if (on[k]) m[k] = __ldg(&ob[u[k]]);
+        if (on[k]) m[k] = ob[u[k]];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (!on[k]) continue;
@@ -1921,6 +1932,8 @@ __device__ __forceinline__ void ipx_sb_put(unsigned long long* p, bool out, cons
 __global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_sb0()
 {
     if (ipx_step() != 0) return;
+    if (threadIdx.x == 0) ipx_step_word() = ipd_compute_superstep;
+    __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) ipx_c.ctl[IPX_CTL_STAMP] = ipx_now();
     const uint64_t V = ipx_c.V;
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[0];
@@ -2118,7 +2131,7 @@ __device__ __forceinline__ unsigned long long ipx_hub_chunk_done(const ipx_hub_c
 #if !IPX_HUB_WARP
 template <bool HOT>
 __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
-    const uint32_t* __restrict__ adj, const uint64_t* __restrict__ row, const ipx_sbslot* __restrict__ bs,
+    const uint32_t* __restrict__ adj, const uint64_t* __restrict__ row, const ipx_sbslot* bs,
     uint32_t stamp, ipx_sbslot* __restrict__ out)
 {
     const uint32_t chunks = ipx_c.chunks;
@@ -2235,7 +2248,7 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
 
 /* Folds the broadcasts of the row's edges among a quad's ids, in order. */
 template <bool HOT, class S>
-__device__ __forceinline__ void ipx_fold_quad(const S* __restrict__ bs, uint32_t stamp, const uint4& q, uint64_t r0,
+__device__ __forceinline__ void ipx_fold_quad(const S* bs, uint32_t stamp, const uint4& q, uint64_t r0,
                                               uint32_t deg, uint32_t rel, bool& has, ipx_msg& acc)
 {
     const uint32_t t = rel - ((uint32_t)r0 & 3u); /* edge of the row; before its first: wraps */
@@ -2307,10 +2320,10 @@ __device__ __forceinline__ bool ipx_gather_done(uint64_t v, bool has, const ipx_
 
 /* Gathers the list's vertices, G lanes each; SKIP: hubs are passed over. */
 template <int G, bool SKIP, bool HOT>
-__device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* __restrict__ list, uint32_t n,
+__device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* list, uint32_t n,
                                                               const ipx_vid* __restrict__ ids,
                                                               const uint64_t* __restrict__ row,
-                                                              const ipx_gslot* __restrict__ bs, uint32_t stamp,
+                                                              const ipx_gslot* bs, uint32_t stamp,
                                                               ipx_gslot* __restrict__ out)
 {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
@@ -2375,7 +2388,7 @@ __device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* __
  * shuffles -- and lane 0 runs the vertex's compute phase. */
 template <bool HOT>
 __device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
-    const ipx_vid* __restrict__ ids, const uint64_t* __restrict__ row, const ipx_sbslot* __restrict__ bs,
+    const ipx_vid* __restrict__ ids, const uint64_t* __restrict__ row, const ipx_sbslot* bs,
     uint32_t stamp, ipx_sbslot* __restrict__ out)
 {
     const int lane = threadIdx.x & 31;
@@ -2454,7 +2467,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_com
     /* HOT: ids of the in-lists carry the flag of the most gathered vertices */
     const ipx_vid* __restrict__ adj = HOT ? reinterpret_cast<const ipx_vid*>(ipx_c.in_adj_hot) : ipx_c.in_adj;
     const uint64_t* __restrict__ row = ipx_c.in_row;
-    const ipx_sbslot* __restrict__ bs = ipx_c.sbslot[s & 1];
+    const ipx_sbslot* bs = ipx_c.sbslot[s & 1];
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[(s + 1) & 1];
     unsigned long long cnt = 0;
     /* the longest work items first */
@@ -2485,7 +2498,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hub
     const uint32_t stamp = (uint32_t)s;
     const ipx_vid* __restrict__ adj = HOT ? reinterpret_cast<const ipx_vid*>(ipx_c.in_adj_hot) : ipx_c.in_adj;
     const uint64_t* __restrict__ row = ipx_c.in_row;
-    const ipx_sbslot* __restrict__ bs = ipx_c.sbslot[s & 1];
+    const ipx_sbslot* bs = ipx_c.sbslot[s & 1];
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[(s + 1) & 1];
     unsigned long long cnt = 0;
     if constexpr (sizeof(ipx_vid) == 4 && IPX_HUB_SMEM) {
@@ -2539,7 +2552,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_TARGET_CTAS) ipx_k_gather_tar
     const uint32_t stamp = (uint32_t)ipx_step();
     const ipx_vid* __restrict__ adj = ipx_c.in_adj;
     const uint64_t* __restrict__ row = ipx_c.in_row;
-    const ipx_bslot* __restrict__ bs = ipx_c.bslot[0];
+    const ipx_bslot* bs = ipx_c.bslot[0];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t n2 = __ldcg(&ipx_c.stat->tn[2]);
     for (uint32_t i = blockIdx.x; i < n2; i += gridDim.x) {
@@ -2615,9 +2628,9 @@ __global__ void ipx_k_fill_bits(uint32_t* bm, uint64_t V, uint64_t W)
  * (spread), or that are active or did (combiner_postamble.h:151-183). */
 __global__ void __launch_bounds__(IPX_THREADS) ipx_k_count(ipx_loop loop)
 {
-    if (ipx_done()) return;
+    if (ipx_done(false)) return;
     /* four words at a time: the bitmaps' last words of four are padding */
-    const uint4* __restrict__ r = reinterpret_cast<const uint4*>(ipx_c.recv[ipx_parity()]);
+    const uint4* r = reinterpret_cast<const uint4*>(ipx_c.recv[ipx_parity()]);
     unsigned long long c = 0;
     for (uint64_t i = ipx_gtid(); i < (ipx_c.W + 3) / 4; i += ipx_gstride()) {
         uint4 x = r[i];
@@ -2639,6 +2652,8 @@ __global__ void __launch_bounds__(IPX_THREADS) ipx_k_count(ipx_loop loop)
  * pairs before the hint is trusted. */
 __global__ void ipx_k_check_hint(int kind)
 {
+    if (threadIdx.x == 0) ipx_step_word() = ipd_compute_superstep;
+    __syncthreads();
     for (uint64_t i = ipx_gtid(); i < 4096; i += ipx_gstride()) {
         unsigned long long ra = (i * 0x9E3779B97F4A7C15ULL) ^ (i >> 3), rb = (i * 0xC2B2AE3D27D4EB4FULL) + 7;
         ipx_msg a, b;

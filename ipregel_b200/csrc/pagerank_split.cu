@@ -134,18 +134,20 @@ struct PrStep {
     const uint64_t* __restrict__ row;     // out-rows: the degrees
     const uint64_t* __restrict__ in_row;  // gather lists (the rows themselves
     const uint32_t* __restrict__ in_adj;  // unless the graph is directed)
-    const float* __restrict__ b_cur;   // read by the gathers
-    float* __restrict__ b_next;        // written for the next superstep
-    float* __restrict__ x_out;         // this superstep's values
-    const float* __restrict__ x_prev;  // the last superstep's
-    double* __restrict__ diag;         // this superstep's mass, dangling mass, residual
+    // written by the superstep before, which may still run when this one's CTAs
+    // come onto the SMs (k_pr_step): ordinary loads, no __restrict__
+    const float* b_cur;   // read by the gathers
+    float* b_next;        // written for the next superstep
+    float* x_out;         // this superstep's values
+    const float* x_prev;  // the last superstep's
+    double* diag;         // this superstep's mass, dangling mass, residual
     float ratio, damping;
     const uint32_t* __restrict__ list[3];  // short, middle, long rows (hubs among the long)
     uint64_t n[3];
     const uint4* __restrict__ hub;         // {vertex, first chunk, chunks}
     const uint32_t* __restrict__ owner;    // chunk -> hub
-    float2* __restrict__ partial;
-    uint32_t* __restrict__ arrived;
+    float2* partial;
+    uint32_t* arrived;
     uint64_t chunks, chunk, hub_min;
     uint64_t empty, empty_dangling;  // vertices without in-edges; of those, without out-edges
     float x0;                        // superstep 0's value
@@ -220,7 +222,7 @@ __device__ __forceinline__ void pr_add_quad(const PrStep& a, const uint4& q, uin
     const uint32_t id[4] = {q.x, q.y, q.z, q.w};
     float w[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) w[k] = t + k < deg ? __ldg(&a.b_cur[id[k]]) : 0.0f;
+    for (int k = 0; k < 4; k++) w[k] = t + k < deg ? a.b_cur[id[k]] : 0.0f;
 #pragma unroll
     for (int k = 0; k < 4; k++) pr_add<COMP>(s, c, w[k]);  // 0 leaves the pair as it is
 }
@@ -230,7 +232,7 @@ template <bool COMP>
 __device__ __forceinline__ void pr_gather(const PrStep& a, uint64_t e0, uint64_t e1, uint64_t lane, uint64_t lanes,
                                           float& s, float& c)
 {
-    for (uint64_t e = e0 + lane; e < e1; e += lanes) pr_add<COMP>(s, c, __ldg(&a.b_cur[a.in_adj[e]]));
+    for (uint64_t e = e0 + lane; e < e1; e += lanes) pr_add<COMP>(s, c, a.b_cur[a.in_adj[e]]);
 }
 
 // Out-degree of v whose gather list holds n ids.
