@@ -281,6 +281,15 @@ int ipg_compact(uint32_t* d_bitmap, uint64_t V, const uint64_t* d_row,
                 uint32_t* d_list2, uint32_t* d_counts, uint64_t* d_edges,
                 int clear, void* stream);
 
+/* ipg_compact, which does nothing when *d_skip (u64, device, read when the
+ * kernel runs; NULL: never skipped) is not 0: for loops whose steps are
+ * enqueued before it is known which is the last, since lists appended to once
+ * more would grow past their end. */
+int ipg_compact_unless(const uint64_t* d_skip, uint32_t* d_bitmap, uint64_t V,
+                       const uint64_t* d_row, uint64_t t0, uint64_t t1,
+                       uint32_t* d_list0, uint32_t* d_list1, uint32_t* d_list2,
+                       uint32_t* d_counts, uint64_t* d_edges, int clear, void* stream);
+
 /* d_out (u64, device) += popcount(a | b) over nwords words (b nullable). */
 int ipg_bitmap_popc_or(const uint32_t* d_a, const uint32_t* d_b, uint64_t nwords,
                        uint64_t* d_out, void* stream);

@@ -782,8 +782,13 @@ static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
     IPX_LAUNCH(IPX_K_MARK, ipx_start(early_gather, ipx_h.mark_ctas == 2 ? ipx_k_mark<2> : ipx_k_mark<1>,
                                      (uint32_t)ipg_sm_count() * ipx_h.mark_ctas, IPX_MARK_THREADS, ipx_h.mark_words * 4,
                                      ipx_h.mark_words));
-    IPX_LAUNCH(IPX_K_COMPACT_T, IPX_OK(ipg_compact(c.bt, c.V, c.in_row, ipx_h.tune.t0, ipx_h.tune.t1, c.tlist[0],
-                                                   c.tlist[1], c.tlist[2], c.stat->tn, (uint64_t*)c.stat->tedges, 0, ipx_h.st)));
+    /* enqueued beyond the program's end it must list nothing, as the other
+     * kernels do: a run that ends by the superstep bound or an error leaves its
+     * last targets in the bitmap, and the lists hold V entries */
+    IPX_LAUNCH(IPX_K_COMPACT_T,
+               IPX_OK(ipg_compact_unless((const uint64_t*)&c.ctl[IPX_CTL_DONE], c.bt, c.V, c.in_row, ipx_h.tune.t0,
+                                         ipx_h.tune.t1, c.tlist[0], c.tlist[1], c.tlist[2], c.stat->tn,
+                                         (uint64_t*)c.stat->tedges, 0, ipx_h.st)));
     IPX_LAUNCH(IPX_K_GATHER, ipx_start(early_gather, ipx_k_gather_targets, ge, ipx_h.tb, 0, loop));
 #else
     /* delivery: push along the broadcasters' rows, or, on a symmetric graph

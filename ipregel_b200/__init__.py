@@ -41,7 +41,7 @@ RUNTIME_SYMBOLS = (
     "ipg_graph_from_host", "ipg_graph_from_device", "ipg_graph_generate_rmat", "ipg_graph_generate_er",
     "ipg_graph_view_get", "ipg_graph_set_symmetric", "ipg_graph_check_symmetric", "ipg_graph_build_in",
     "ipg_graph_to_host", "ipg_graph_write", "ipg_graph_free",
-    "ipg_graph_bins", "ipg_degree_classes_noalloc", "ipg_compact", "ipg_bitmap_popc_or", "ipg_sm_count",
+    "ipg_graph_bins", "ipg_degree_classes_noalloc", "ipg_compact", "ipg_compact_unless", "ipg_bitmap_popc_or", "ipg_sm_count",
     "ipg_graph_set_directed", "ipg_memcpy", "ipg_pr_plan_create", "ipg_pr_plan_free", "ipg_pr_plan_info", "ipg_pr_run_f32",
     "ipg_error_f32_f64", "ipg_graph_concat", "ipg_fused_create", "ipg_fused_graph", "ipg_fused_launch",
     "ipg_fused_free", "ipg_server_create", "ipg_server_free", "ipg_server_add_graph", "ipg_server_submit",

@@ -1753,8 +1753,10 @@ __global__ void __launch_bounds__(CT_THREADS) k_compact(uint32_t* __restrict__ b
                                                         const uint64_t* __restrict__ row, uint64_t t0, uint64_t t1,
                                                         uint32_t* __restrict__ l0, uint32_t* __restrict__ l1,
                                                         uint32_t* __restrict__ l2, uint32_t* __restrict__ counts,
-                                                        unsigned long long* __restrict__ edges, int clear)
+                                                        unsigned long long* __restrict__ edges, int clear,
+                                                        const unsigned long long* skip)
 {
+    if (skip && *skip) return;
     __shared__ uint32_t s_cnt[CT_WARPS][3];
     __shared__ uint32_t s_base[3];
     __shared__ unsigned long long s_edges[3];
@@ -1842,6 +1844,14 @@ extern "C" int ipg_compact(uint32_t* d_bitmap, uint64_t V, const uint64_t* d_row
                            uint32_t* d_list0, uint32_t* d_list1, uint32_t* d_list2, uint32_t* d_counts,
                            uint64_t* d_edges, int clear, void* stream)
 {
+    return ipg_compact_unless(nullptr, d_bitmap, V, d_row, t0, t1, d_list0, d_list1, d_list2, d_counts, d_edges, clear,
+                              stream);
+}
+
+extern "C" int ipg_compact_unless(const uint64_t* d_skip, uint32_t* d_bitmap, uint64_t V, const uint64_t* d_row,
+                                  uint64_t t0, uint64_t t1, uint32_t* d_list0, uint32_t* d_list1, uint32_t* d_list2,
+                                  uint32_t* d_counts, uint64_t* d_edges, int clear, void* stream)
+{
     if (V == 0) return IPG_OK;
     if (!d_counts || !d_list0) return fail(IPG_EINVAL, "ipg_compact: null output");
     if (d_row && (!d_list1 || !d_list2)) return fail(IPG_EINVAL, "ipg_compact: three lists needed with degrees");
@@ -1849,7 +1859,8 @@ extern "C" int ipg_compact(uint32_t* d_bitmap, uint64_t V, const uint64_t* d_row
     const uint64_t tiles = (nwords + CT_THREADS - 1) / CT_THREADS;
     uint64_t blocks = std::min<uint64_t>(tiles, (uint64_t)ipg_sm_count() * 8);
     k_compact<<<(uint32_t)blocks, CT_THREADS, 0, (cudaStream_t)stream>>>(
-        d_bitmap, V, d_row, t0, t1, d_list0, d_list1, d_list2, d_counts, (unsigned long long*)d_edges, clear);
+        d_bitmap, V, d_row, t0, t1, d_list0, d_list1, d_list2, d_counts, (unsigned long long*)d_edges, clear,
+        (const unsigned long long*)d_skip);
     IPG_CUDA(cudaGetLastError());
     return IPG_OK;
 }
