@@ -241,6 +241,15 @@ typedef struct ipg_hubs {
 int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64_t chunk,
                    ipg_hubs* hubs);
 
+/* A set of the two calls above (d_set: its d_list[0] or d_hub) stays until the
+ * graph's contents change, its meaning does or it is freed, as long as somebody
+ * holds it; one that nobody holds is valid until the next call of the same kind
+ * and direction with other thresholds.  A hold may be released after the graph
+ * was freed, and on any thread. */
+typedef struct ipg_hold ipg_hold;
+int ipg_graph_hold(ipg_graph* g, const uint32_t* d_set, ipg_hold** hold);
+void ipg_hold_release(ipg_hold* hold);
+
 /* *quads = 1 when the rows' (or in-lists') 32-bit ids, and 4-byte weights if
  * there are any, can be read in aligned groups of four up to the group that
  * holds the last one: always for arrays the runtime allocated. */

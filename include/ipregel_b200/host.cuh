@@ -81,8 +81,9 @@ struct ipx_host_state {
     }* pin = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    ipg_bins gbins;                                    /* static in-degree classes (pulling push versions) */
-    ipg_hubs ghubs;                                    /* hub chunks of the single_broadcast gather */
+    ipg_bins gbins; /* single_broadcast, pulling push versions: static in-degree classes */
+    ipg_hubs ghubs; /* and hub chunks, which other users of the graph leave alone: */
+    ipg_hold* holds[2] = {nullptr, nullptr};
     std::vector<uint64_t> counts;
     double total_seconds = 0.0;
     uint64_t edges = 0;
@@ -216,6 +217,10 @@ static void ipx_release_state(bool keep = false)
         ipx_h.ev0 = ipx_h.ev1 = nullptr;
         ipx_h.st = nullptr;
     }
+    for (auto& h : ipx_h.holds) {
+        ipg_hold_release(h);
+        h = nullptr;
+    }
     if (ipx_h.g && ipx_h.own_graph) ipg_graph_free(ipx_h.g);
     ipx_h.g = nullptr;
     ipx_h.gw = nullptr;
@@ -225,6 +230,13 @@ static void ipx_release_state(bool keep = false)
     ipx_h.host_valid = false;
     ipx_h.host_vertices.clear();
     ipx_h.host_vertices.shrink_to_fit();
+}
+
+/* The attached graph's classes and hubs are this engine's until its next attach. */
+static int ipx_hold_sets()
+{
+    int r = ipg_graph_hold(ipx_h.gw, ipx_h.gbins.d_list[0], &ipx_h.holds[0]);
+    return r == IPG_OK ? ipg_graph_hold(ipx_h.gw, ipx_h.ghubs.d_hub, &ipx_h.holds[1]) : r;
 }
 
 static uint32_t ipx_grid(int per_sm = 8) { return (uint32_t)(ipg_sm_count() * per_sm); }
@@ -464,6 +476,7 @@ static int ipx_setup_state()
         const int in = gv.directed ? 1 : 0;
         IPX_OK(ipg_graph_bins(ipx_h.gw, in, c.push_t[0], c.push_t[1], &ipx_h.gbins));
         IPX_OK(ipg_graph_hubs(ipx_h.gw, in, c.push_t[2], c.push_chunk, &ipx_h.ghubs));
+        IPX_OK(ipx_hold_sets());
         for (int k = 0; k < 3; k++) {
             c.class_list[k] = ipx_h.gbins.d_list[k];
             c.class_n[k] = (uint32_t)ipx_h.gbins.count[k];
@@ -493,6 +506,7 @@ static int ipx_setup_state()
         const uint64_t mid = IPX_GATHER_MID < hub_min ? IPX_GATHER_MID : hub_min;
         IPX_OK(ipg_graph_bins(ipx_h.gw, 1, t0, mid > t0 ? mid : t0, &ipx_h.gbins));
         IPX_OK(ipg_graph_hubs(ipx_h.gw, 1, hub_min, chunk, &ipx_h.ghubs));
+        IPX_OK(ipx_hold_sets());
         c.hub_min = hub_min;
         for (int k = 0; k < 3; k++) {
             c.class_list[k] = ipx_h.gbins.d_list[k];

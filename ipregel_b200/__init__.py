@@ -48,6 +48,7 @@ RUNTIME_SYMBOLS = (
     "ipg_server_poll", "ipg_server_query", "ipg_server_result", "ipg_server_result_device", "ipg_server_release",
     "ipg_server_get_stats", "ipg_server_run_trace", "ipg_server_group_stats",
     "ipg_server_reserve", "ipg_graph_refill_host", "ipg_graph_contents", "ipg_graph_degree_order", "ipg_graph_hubs", "ipg_graph_quads",
+    "ipg_graph_hold", "ipg_hold_release",
 )
 # The reference interface (src/iPregel_preamble.h:66-317) and the ipg_app_*
 # ABI (include/ipregel_b200/host.cuh), exported by every application library.

@@ -80,6 +80,7 @@ struct ipg_pr_plan {
     const uint32_t* new_of_old = nullptr;
     float* xs2 = nullptr;
     ipg_hubs hubs{};                   // rows above hub_min in chunks
+    ipg_hold* holds[2] = {nullptr, nullptr};  // of both
     uint64_t hub_min = 0, chunk = 0;
     bool quads = false;                // the gather lists take 128-bit loads
     float2* partial = nullptr;         // (sum, compensation) of every hub chunk
@@ -553,7 +554,9 @@ extern "C" int ipg_pr_plan_create(ipg_graph* g, ipg_pr_plan** out)
         const uint64_t mid = PR_MID < p->hub_min ? PR_MID : p->hub_min;
         // classes over the gather lists (builds the in-lists of a directed graph)
         if ((r = ipg_graph_bins(gw, 1, ts, mid > ts ? mid : ts, &p->bins)) != IPG_OK) break;
+        if ((r = ipg_graph_hold(gw, p->bins.d_list[0], &p->holds[0])) != IPG_OK) break;
         if ((r = ipg_graph_hubs(gw, 1, p->hub_min, p->chunk, &p->hubs)) != IPG_OK) break;
+        if ((r = ipg_graph_hold(gw, p->hubs.d_hub, &p->holds[1])) != IPG_OK) break;
         if ((r = ipg_graph_view_get(gw, &p->gv)) != IPG_OK) break;
         int quads = 0;
         if ((r = ipg_graph_quads(gw, 1, &quads)) != IPG_OK) break;
@@ -618,6 +621,7 @@ extern "C" void ipg_pr_plan_free(ipg_pr_plan* p)
 {
     if (!p) return;
     for (auto& a : p->allocs) ipg_dev_free(a.first, a.second);
+    for (ipg_hold* h : p->holds) ipg_hold_release(h);
     delete p;
 }
 

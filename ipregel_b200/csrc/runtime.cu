@@ -201,6 +201,17 @@ struct DevBuf {
     template <class T> T* as() { return static_cast<T*>(p); }
 };
 
+// Who uses a set of degree classes or hubs: the graph that keeps it, and each
+// holder.  The last to let go deletes the record; the memory is the graph's.
+struct ipg_hold {
+    std::atomic<int> refs{1};
+};
+
+extern "C" void ipg_hold_release(ipg_hold* hold)
+{
+    if (hold && --hold->refs == 0) delete hold;
+}
+
 // ---------------------------------------------------------------------------
 // Graph object
 // ---------------------------------------------------------------------------
@@ -213,54 +224,53 @@ struct ipg_graph {
     void* in_row = nullptr; uint64_t in_row_bytes = 0;
     void* in_adj = nullptr; uint64_t in_adj_bytes = 0;
     void* in_wgt = nullptr; uint64_t in_wgt_bytes = 0;
-    // Degree classes and hub tables, per direction, least recently asked for
-    // first.  Users of one graph (engines, split plans, servers) ask with
-    // thresholds of their own and hold what they got, so a set stays until
-    // the contents change; past DERIVED_MAX sets, or when memory is short,
-    // the least recently asked for goes.
+    // Degree classes and hub tables, per direction.  Users of one graph
+    // (engines, split plans, servers) ask with thresholds of their own and hold
+    // what they got (ipg_graph_hold): a held set stays until it is let go of or
+    // the contents change; one that nobody holds goes when the next is made.
     template <class S>
     struct Sets {
-        static constexpr size_t DERIVED_MAX = 16;
-        S set[DERIVED_MAX];
-        size_t n = 0;
-        void drop(size_t keep)
-        {
-            for (; n > keep; n--) {
-                ipg_dev_free(set[0].mem, set[0].bytes);
-                std::rotate(set, set + 1, set + n);
-            }
-        }
+        std::vector<S> set;
         template <class F>
-        S* find(F is)
+        const S* find(F is) const
         {
-            S* e = std::find_if(set, set + n, is);
-            if (e == set + n) return nullptr;
-            std::rotate(e, e + 1, set + n);
-            return set + n - 1;
+            auto e = std::find_if(set.begin(), set.end(), is);
+            return e == set.end() ? nullptr : &*e;
         }
-        // memory of a new set, which its maker adds or gives back
-        int alloc(void** p, uint64_t bytes)
+        ipg_hold* holder(const void* mem) const
         {
-            drop(DERIVED_MAX - 1);
-            int r = ipg_dev_alloc(p, bytes);
-            while (r != IPG_OK && n) {
-                drop(n - 1);
-                r = ipg_dev_alloc(p, bytes);
+            const S* e = find([&](const S& s) { return s.mem == mem; });
+            return e ? e->hold : nullptr;
+        }
+        void drop(bool held)
+        {
+            auto gone = std::partition(set.begin(), set.end(), [&](const S& s) { return !held && s.hold->refs > 1; });
+            for (auto e = gone; e != set.end(); ++e) {
+                ipg_dev_free(e->mem, e->bytes);
+                ipg_hold_release(e->hold);
             }
-            return r;
+            set.erase(gone, set.end());
         }
-        void add(const S& s) { set[n++] = s; }
+        int add(S& s)
+        {
+            s.hold = new (std::nothrow) ipg_hold();
+            if (!s.hold) return fail(IPG_ENOMEM, "out of host memory");
+            set.push_back(s);
+            return IPG_OK;
+        }
     };
     struct BinCache {
         uint64_t t0 = 0, t1 = 0;
         void* mem = nullptr;
         uint64_t bytes = 0;
+        ipg_hold* hold = nullptr;
         ipg_bins bins = {};
     };
     struct HubCache {
         uint64_t hub_min = 0, chunk = 0;
         void* mem = nullptr;
         uint64_t bytes = 0;
+        ipg_hold* hold = nullptr;
         ipg_hubs hubs = {};
     };
     Sets<BinCache> bins[2];
@@ -270,8 +280,8 @@ struct ipg_graph {
     {
         for (int k = 0; k < 2; k++) {
             if (which >= 0 && which != k) continue;
-            bins[k].drop(0);
-            hubs[k].drop(0);
+            bins[k].drop(true);
+            hubs[k].drop(true);
         }
     }
     // ipg_graph_refill_host's own stream, device words (check bits, degree
@@ -1916,10 +1926,11 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
         return IPG_OK;
     }
     const uint64_t V = g->v.V;
+    sets.drop(false);
     ipg_graph::BinCache c;
     c.bytes = (V ? V : 1) * 4 + 64;
     SetMem mem(c.bytes);
-    IPG_TRY(sets.alloc(&mem.p, mem.bytes));
+    IPG_TRY(ipg_dev_alloc(&mem.p, mem.bytes));
     c.mem = mem.p;
     DevBuf cnt, l1, l2;
     IPG_TRY(cnt.alloc(64));
@@ -1966,7 +1977,7 @@ extern "C" int ipg_graph_bins(ipg_graph* g, int use_in, uint64_t t0, uint64_t t1
     c.bins.t1 = t1;
     c.t0 = t0;
     c.t1 = t1;
-    sets.add(c);
+    IPG_TRY(sets.add(c));
     mem.p = nullptr;
     *bins = c.bins;
     return IPG_OK;
@@ -2008,10 +2019,11 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     const uint64_t chunks_max = E / chunk + hubs_max + 1;
     if (chunks_max >= (1ULL << 32)) return fail(IPG_EINVAL, "ipg_graph_hubs: too many chunks for 32-bit indices");
     const uint64_t hub_b = align256((hubs_max + 1) * 16), own_b = align256(chunks_max * 4);
+    sets.drop(false);
     ipg_graph::HubCache c;
     c.bytes = hub_b + own_b + 256;
     SetMem mem(c.bytes);
-    IPG_TRY(sets.alloc(&mem.p, mem.bytes));
+    IPG_TRY(ipg_dev_alloc(&mem.p, mem.bytes));
     c.mem = mem.p;
     uint4* hub = (uint4*)c.mem;
     uint32_t* owner = (uint32_t*)((char*)c.mem + hub_b);
@@ -2034,9 +2046,22 @@ extern "C" int ipg_graph_hubs(ipg_graph* g, int use_in, uint64_t hub_min, uint64
     c.hubs.chunks = h.chunks;
     c.hub_min = hub_min;
     c.chunk = chunk;
-    sets.add(c);
+    IPG_TRY(sets.add(c));
     mem.p = nullptr;
     *hubs = c.hubs;
+    return IPG_OK;
+}
+
+extern "C" int ipg_graph_hold(ipg_graph* g, const uint32_t* d_set, ipg_hold** hold)
+{
+    if (!g || !hold) return fail(IPG_EINVAL, "ipg_graph_hold: null argument");
+    *hold = nullptr;
+    for (int k = 0; k < 2 && !*hold; k++) {
+        *hold = g->bins[k].holder(d_set);
+        if (!*hold) *hold = g->hubs[k].holder(d_set);
+    }
+    if (!*hold) return fail(IPG_EINVAL, "ipg_graph_hold: no set of the graph");
+    (*hold)->refs++;
     return IPG_OK;
 }
 

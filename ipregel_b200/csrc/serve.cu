@@ -1292,7 +1292,8 @@ struct Graph {
     Group* pp = nullptr;
     // degree classes over all vertices
     ipg_bins bins{};
-    // the hubs' table (the graph's own may be replaced) and the union-find's words
+    ipg_hold* hold = nullptr;
+    // a copy of the hubs' table, and the union-find's words
     void* cls = nullptr;
     uint64_t cls_bytes = 0;
     Hubs hubs{};
@@ -1438,6 +1439,7 @@ int graph_classes(Graph* Gr, cudaStream_t st)
 {
     if (Gr->classes) return IPG_OK;
     int r = ipg_graph_bins(Gr->g, 0, MP_T0, MP_T1, &Gr->bins);
+    if (r == IPG_OK) r = ipg_graph_hold(Gr->g, Gr->bins.d_list[0], &Gr->hold);
     if (r != IPG_OK) return r;
     ipg_hubs N{};
     if ((r = ipg_graph_hubs(Gr->g, 0, MP_T1, HUB_CHUNK, &N)) != IPG_OK) return r;
@@ -1946,8 +1948,10 @@ extern "C" void ipg_server_free(ipg_server* S)
     cudaStreamSynchronize(S->rel_st);
     cudaStreamDestroy(S->rel_st);
     cudaMemPoolDestroy(S->rpool);
-    for (auto& g : S->graphs)
+    for (auto& g : S->graphs) {
         ipg_dev_free(g->cls, g->cls_bytes);
+        ipg_hold_release(g->hold);
+    }
     delete S;
 }
 
@@ -1967,6 +1971,7 @@ extern "C" int ipg_server_add_graph(ipg_server* S, ipg_graph* g, int* gid)
     // building them synchronises the device
     if ((r = graph_classes(G.get(), nullptr)) != IPG_OK) {
         ipg_dev_free(G->cls, G->cls_bytes);
+        ipg_hold_release(G->hold);
         return r;
     }
     *gid = (int)S->graphs.size();
