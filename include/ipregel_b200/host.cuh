@@ -327,7 +327,8 @@ static int ipx_build_hot_ids(ipx_consts& c)
     if (ipg_dev_alloc(&cnt, tmp_bytes) != IPG_OK) return IPG_OK;
     unsigned long long* hist = (unsigned long long*)((char*)cnt + hist_off);
     uint32_t* out = nullptr;
-    if (ipx_alloc(&out, c.E) != IPG_OK) {
+    /* whole groups of four, as the id arrays themselves: rows are read by them */
+    if (ipx_alloc(&out, (c.E + 3) & ~3ULL) != IPG_OK) {
         ipx_h.err[0] = 0;
         ipg_dev_free(cnt, tmp_bytes);
         return IPG_OK;
