@@ -780,10 +780,13 @@ __device__ __forceinline__ void ipx_block_count(unsigned long long c, unsigned l
     }
 }
 
-/* The loop the kernels run in: a captured one continues by its condition. */
+/* The loop the kernels run in: a captured one continues by its condition.
+ * starts: the superstep is the first that the host enqueued after a wait, and is
+ * timed from its own first kernel, not from the end of the one before. */
 struct ipx_loop {
     cudaGraphConditionalHandle handle;
     int captured;
+    int starts;
     unsigned long long max_supersteps;
 };
 
@@ -808,6 +811,11 @@ __device__ __forceinline__ unsigned long long ipx_now()
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
+}
+
+__device__ __forceinline__ void ipx_start_clock(bool starts)
+{
+    if (starts && blockIdx.x == 0 && threadIdx.x == 0) ipx_c.ctl[IPX_CTL_STAMP] = ipx_now();
 }
 
 /* Direction of the superstep's delivery (push versions). */
@@ -1710,7 +1718,7 @@ __device__ __forceinline__ void ipx_front_flush(const ipx_front_buf& buf, const 
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(IPX_THREADS, IPX_FRONT_CTAS) ipx_k_front(int words)
+__global__ void __launch_bounds__(IPX_THREADS, IPX_FRONT_CTAS) ipx_k_front(int words, bool starts)
 {
     if (ipx_done()) return;
     __shared__ ipx_front_buf s_buf[IPX_THREADS / 32];
@@ -1722,7 +1730,7 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_FRONT_CTAS) ipx_k_front(int w
     [[maybe_unused]] const int pprev = (int)((s + 1) & 1); /* parity of superstep s-1 */
     unsigned long long es[4] = {0, 0, 0, 0};
     uint32_t n[3] = {0, 0, 0};
-    if (s == 0 && blockIdx.x == 0 && threadIdx.x == 0) ipx_c.ctl[IPX_CTL_STAMP] = ipx_now();
+    ipx_start_clock(starts || s == 0);
     for (uint64_t base = (ipx_gtid() >> 5) * (uint64_t)words; base < W; base += step) {
         /* this lane's word */
         const uint64_t wl = base + lane;
@@ -1934,7 +1942,7 @@ __global__ void __launch_bounds__(IPX_THREADS) ipx_k_compute_sb0()
     if (ipx_step() != 0) return;
     if (threadIdx.x == 0) ipx_step_word() = ipd_compute_superstep;
     __syncthreads();
-    if (blockIdx.x == 0 && threadIdx.x == 0) ipx_c.ctl[IPX_CTL_STAMP] = ipx_now();
+    ipx_start_clock(true);
     const uint64_t V = ipx_c.V;
     ipx_sbslot* __restrict__ out = ipx_c.sbslot[0];
     for (uint64_t v = ipx_gtid(); v < V; v += ipx_gstride()) {
@@ -2464,6 +2472,8 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_com
 {
     if (ipx_done()) return;
     const uint64_t s = ipx_step();
+    /* superstep 0 starts with its compute phase, others may with the hubs */
+    ipx_start_clock((IPX_HUB_WARP || !ipx_c.chunks) && loop.starts && s != 0);
     const uint32_t stamp = (uint32_t)s;
     /* HOT: ids of the in-lists carry the flag of the most gathered vertices */
     const ipx_vid* __restrict__ adj = HOT ? reinterpret_cast<const ipx_vid*>(ipx_c.in_adj_hot) : ipx_c.in_adj;
@@ -2492,10 +2502,11 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_com
  * slot loads are issued from shared memory instead of behind a global id
  * load each. */
 template <bool HOT>
-__global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hubs()
+__global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hubs(bool starts)
 {
     if (ipx_done()) return;
     const uint64_t s = ipx_step();
+    ipx_start_clock(starts && s != 0);
     const uint32_t stamp = (uint32_t)s;
     const ipx_vid* __restrict__ adj = HOT ? reinterpret_cast<const ipx_vid*>(ipx_c.in_adj_hot) : ipx_c.in_adj;
     const uint64_t* __restrict__ row = ipx_c.in_row;

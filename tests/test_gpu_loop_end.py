@@ -76,3 +76,27 @@ def test_compact_unless():
                 assert cnt.to_host()[k] == want.size and edges.to_host()[k] == deg[want].sum()
                 np.testing.assert_array_equal(np.sort(lists[k].to_host()[:want.size]), want)
         np.testing.assert_array_equal(bm.to_host(), bits if skip else np.zeros_like(bits))
+
+
+@pytest.mark.parametrize("version", ["combiner", "spread", "single_broadcast", "single_broadcast_spread"])
+@pytest.mark.parametrize("n", [2, 40])
+def test_total_time_is_the_supersteps(version, n, capfd):
+    """The reported total is the sum of the supersteps' durations, without those enqueued beyond the end that do
+    nothing (the durations are printed to a microsecond)."""
+    import ipregel_b200 as ip
+    g = _path(n)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, g.adj)
+    eng = ip.Engine("cc", version)
+    try:
+        eng.set_quiet(False)
+        eng.attach(graph)
+        res = eng.run()
+        ctypes.CDLL(None).fflush(None)
+        out = capfd.readouterr().out
+        times = [float(x.split(":")[1]) for x in out.splitlines() if x.startswith("Superstep") and "Duration" in x]
+        assert len(times) == len(res.counts) and min(times) >= 0
+        assert abs(res.seconds - sum(times)) <= 0.6e-6 * len(times)
+    finally:
+        eng.set_quiet(True)
+        eng.release()
+        graph.free()
