@@ -842,6 +842,7 @@ static int ipx_run_host_loop()
     const ipx_consts& c = ipx_h.c;
     ipx_loop loop = {0, 0, 0, (unsigned long long)ipx_max_supersteps()};
     uint64_t count = ip_active_vertices;
+    if (loop.max_supersteps == 0) return ipx_fail_device(IPX_ERR_SUPERSTEP_LIMIT); /* the device tests it after a superstep */
     IPX_OK(ipx_set_superstep(0));
     for (uint64_t s = 0;;) {
         const int batch = ipx_h.profile ? 1 : IPX_BATCH;

@@ -44,6 +44,27 @@ def test_bounded_run_then_full(version, bound, loop, monkeypatch):
         graph.free()
 
 
+@pytest.mark.parametrize("version", ["combiner", "spread", "single_broadcast", "single_broadcast_spread"])
+def test_bound_of_no_supersteps(version, monkeypatch):
+    """The host-driven loop runs nothing under a bound of 0: no count, and the values as they were initialised."""
+    import ipregel_b200 as ip
+    g = _path(40)
+    graph = ip.Graph.from_csr(g.V, g.E, g.idx, g.adj)
+    eng = ip.Engine("cc", version)
+    eng.set_quiet(True)
+    try:
+        eng.attach(graph)
+        before = eng.values().copy()
+        monkeypatch.setenv("IPG_MAX_SUPERSTEPS", "0")
+        with pytest.raises(ip.IPregelError, match="superstep limit"):
+            eng.run()
+        assert eng.counts() == []
+        np.testing.assert_array_equal(eng.values(), before)
+    finally:
+        eng.release()
+        graph.free()
+
+
 def test_compact_unless():
     """The compaction between the engine's kernels: as ipg_compact while the flag is 0, and nothing appended, summed
     or cleared while it is not."""
