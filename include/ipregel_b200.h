@@ -320,9 +320,10 @@ int ipg_sm_count(void);
  * ------------------------------------------------------------------------ */
 typedef struct ipg_pr_plan ipg_pr_plan;
 
-/* Degree classes and scratch for runs on graph g (32-bit ids); holds
- * 12 bytes per vertex plus 8 bytes per hub chunk of HBM until freed
- * (and builds the graph's in-lists if it is directed). */
+/* Degree classes and scratch for runs on graph g (32-bit ids); holds of HBM
+ * until freed 12 bytes per vertex (16 on the degree-ordered copy), 4 per vertex
+ * of the short rows where there is room, 8 per hub chunk and 4 per hub (and
+ * builds the graph's in-lists if it is directed). */
 int ipg_pr_plan_create(ipg_graph* g, ipg_pr_plan** plan);
 void ipg_pr_plan_free(ipg_pr_plan* plan);
 /* Vertices and edge sums of the rows of a thread each, of several lanes each,

@@ -85,7 +85,7 @@ struct ipg_pr_plan {
     bool quads = false;                // the gather lists take 128-bit loads
     float2* partial = nullptr;         // (sum, compensation) of every hub chunk
     uint32_t* arrived = nullptr;       // per hub the chunks arrived (0 between supersteps)
-    uint32_t* shorts = nullptr;        // the short class: first the vertices with in-edges
+    uint32_t* shorts = nullptr;        // the short class: first the vertices with in-edges (null: unsplit)
     uint64_t empty = 0, empty_dangling = 0;  // the rest of it
     uint64_t class_count[3] = {0, 0, 0}, class_edges[3] = {0, 0, 0};
     int sms = 148;
@@ -470,6 +470,45 @@ int pr_alloc(ipg_pr_plan* p, T** out, uint64_t n)
     return IPG_OK;
 }
 
+// The short class again, vertices without in-edges behind the others.  Where
+// there is no room for it, the class serves as it is, every vertex a row.
+int pr_split_shorts(ipg_pr_plan* p)
+{
+    const uint64_t ns = p->bins.count[0];
+    if (!ns) return IPG_OK;
+    const PrHasEdges has{p->gv.d_in_row};
+    const uint32_t* list = p->bins.d_list[0];
+    size_t tb = 0;
+    void* mem[2] = {nullptr, nullptr};  // the list; scratch and {with in-edges, dangling}
+    cudaError_t e = cub::DevicePartition::If(nullptr, tb, list, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t)ns, has);
+    const uint64_t bytes[2] = {ns * 4, ((uint64_t)tb + 15) / 16 * 16 + 16};
+    int r = IPG_OK;
+    for (int k = 0; k < 2 && e == cudaSuccess && r == IPG_OK; k++) r = ipg_dev_alloc(&mem[k], bytes[k]);
+    unsigned long long h[2] = {0, 0};
+    if (e == cudaSuccess && r == IPG_OK) {
+        uint32_t* shorts = (uint32_t*)mem[0];
+        unsigned long long* cnt = (unsigned long long*)((char*)mem[1] + bytes[1] - 16);
+        e = cudaMemset(cnt, 0, 16);
+        if (e == cudaSuccess) e = cub::DevicePartition::If(mem[1], tb, list, shorts, (uint32_t*)cnt, (int64_t)ns, has);
+        if (e == cudaSuccess) e = cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && h[0] < ns) {
+            k_pr_count_dangling<<<p->grid_flat, PR_THREADS>>>(shorts + h[0], ns - h[0], p->gv.d_row, cnt + 1);
+            e = cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
+        }
+    }
+    ipg_dev_free(mem[1], bytes[1]);
+    if (e != cudaSuccess || r != IPG_OK) {
+        ipg_dev_free(mem[0], bytes[0]);
+        if (e != cudaSuccess) return ipg_internal_fail(IPG_ECUDA, cudaGetErrorString(e));
+        return r == IPG_EBUDGET || r == IPG_ENOMEM ? IPG_OK : r;
+    }
+    p->allocs.push_back({mem[0], bytes[0]});
+    p->shorts = (uint32_t*)mem[0];
+    p->empty = ns - h[0];
+    p->empty_dangling = h[1];
+    return IPG_OK;
+}
+
 // Error of an FP32 vector against an FP64 one: out[0] = max abs, out[1] =
 // max rel (abs where the reference is 0), out[2] = sum of abs, as doubles.
 // Non-negative doubles order as their bit patterns, so the maxima use integer
@@ -573,34 +612,7 @@ extern "C" int ipg_pr_plan_create(ipg_graph* g, ipg_pr_plan** out)
             r = ipg_internal_fail(IPG_ECUDA, cudaGetErrorString(e));
             break;
         }
-        // the short class, vertices without in-edges behind the others
-        const uint64_t ns = p->bins.count[0];
-        if ((r = pr_alloc(p, &p->shorts, ns)) != IPG_OK) break;
-        if (ns) {
-            const PrHasEdges has{p->gv.d_in_row};
-            size_t tb = 0;
-            void* temp = nullptr;
-            e = cub::DevicePartition::If(nullptr, tb, p->bins.d_list[0], p->shorts, (uint32_t*)nullptr, (int64_t)ns, has);
-            const uint64_t bytes = ((uint64_t)tb + 15) / 16 * 16 + 16;
-            if (e == cudaSuccess && (r = ipg_dev_alloc(&temp, bytes)) != IPG_OK) break;
-            unsigned long long* cnt = (unsigned long long*)((char*)temp + bytes - 16);  // {with in-edges, dangling}
-            unsigned long long h[2] = {0, 0};
-            if (e == cudaSuccess) e = cudaMemset(cnt, 0, 16);
-            if (e == cudaSuccess)
-                e = cub::DevicePartition::If(temp, tb, p->bins.d_list[0], p->shorts, (uint32_t*)cnt, (int64_t)ns, has);
-            if (e == cudaSuccess) e = cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
-            if (e == cudaSuccess && h[0] < ns) {
-                k_pr_count_dangling<<<p->grid_flat, PR_THREADS>>>(p->shorts + h[0], ns - h[0], p->gv.d_row, cnt + 1);
-                e = cudaMemcpy(h, cnt, 16, cudaMemcpyDeviceToHost);
-            }
-            ipg_dev_free(temp, bytes);
-            if (e != cudaSuccess) {
-                r = ipg_internal_fail(IPG_ECUDA, cudaGetErrorString(e));
-                break;
-            }
-            p->empty = ns - h[0];
-            p->empty_dangling = h[1];
-        }
+        if ((r = pr_split_shorts(p)) != IPG_OK) break;
         // the classes as the plan's user knows them: thread, lanes, hubs
         p->class_count[0] = p->bins.count[0];
         p->class_edges[0] = p->bins.edges[0];
@@ -643,7 +655,7 @@ extern "C" int ipg_pr_run_f32(ipg_pr_plan* p, uint32_t rounds, double damping, i
         a.list[k] = p->bins.d_list[k];
         a.n[k] = p->bins.count[k];
     }
-    a.list[0] = p->shorts;
+    if (p->shorts) a.list[0] = p->shorts;
     a.n[0] -= p->empty;
     a.empty = p->empty;
     a.empty_dangling = p->empty_dangling;
