@@ -1290,14 +1290,11 @@ struct Graph {
     ipg_graph_view gv{};
     Group* mp = nullptr;
     Group* pp = nullptr;
-    // degree classes over all vertices
+    // degree classes over all vertices, the hubs' table, and the holds of both
     ipg_bins bins{};
-    ipg_hold* hold = nullptr;
-    // a copy of the hubs' table, and the union-find's words
-    void* cls = nullptr;
-    uint64_t cls_bytes = 0;
     Hubs hubs{};
-    uint32_t* cc_err = nullptr;
+    ipg_hold* holds[2] = {nullptr, nullptr};
+    uint32_t* cc_err = nullptr;  // the union-find's words
     uint32_t* cc_giant = nullptr;
     bool classes = false;
 };
@@ -1433,29 +1430,27 @@ bool make_room(ipg_server* S, uint64_t need)
     return true;
 }
 
+void free_classes(Graph* Gr)
+{
+    ipg_dev_free(Gr->cc_err, 8);
+    for (ipg_hold* h : Gr->holds) ipg_hold_release(h);
+}
+
 // Degree classes of all vertices of a graph and its hubs in chunks (built once;
 // the min-plus and PPR groups and the union-find pass use them).
-int graph_classes(Graph* Gr, cudaStream_t st)
+int graph_classes(Graph* Gr)
 {
     if (Gr->classes) return IPG_OK;
     int r = ipg_graph_bins(Gr->g, 0, MP_T0, MP_T1, &Gr->bins);
-    if (r == IPG_OK) r = ipg_graph_hold(Gr->g, Gr->bins.d_list[0], &Gr->hold);
-    if (r != IPG_OK) return r;
+    if (r == IPG_OK) r = ipg_graph_hold(Gr->g, Gr->bins.d_list[0], &Gr->holds[0]);
     ipg_hubs N{};
-    if ((r = ipg_graph_hubs(Gr->g, 0, MP_T1, HUB_CHUNK, &N)) != IPG_OK) return r;
-    const uint64_t bytes = N.hubs * 16 + (N.chunks + 2) * 4;
-    if ((r = ipg_dev_alloc(&Gr->cls, bytes)) != IPG_OK) return r;
-    Gr->cls_bytes = bytes;
-    uint4* hub = (uint4*)Gr->cls;
-    uint32_t* owner = (uint32_t*)(hub + N.hubs);
-    Gr->cc_err = owner + N.chunks;
+    if (r == IPG_OK) r = ipg_graph_hubs(Gr->g, 0, MP_T1, HUB_CHUNK, &N);
+    if (r == IPG_OK) r = ipg_graph_hold(Gr->g, N.d_hub, &Gr->holds[1]);
+    if (r == IPG_OK) r = ipg_dev_alloc((void**)&Gr->cc_err, 8);
+    if (r != IPG_OK) return r;
     Gr->cc_giant = Gr->cc_err + 1;
-    if ((N.hubs && cudaMemcpyAsync(hub, N.d_hub, N.hubs * 16, cudaMemcpyDeviceToDevice, st) != cudaSuccess) ||
-        (N.chunks && cudaMemcpyAsync(owner, N.d_owner, N.chunks * 4, cudaMemcpyDeviceToDevice, st) != cudaSuccess) ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return ipg_internal_fail(IPG_ECUDA, "serve: hub table failed");
-    Gr->hubs.hub = hub;
-    Gr->hubs.owner = owner;
+    Gr->hubs.hub = (const uint4*)N.d_hub;
+    Gr->hubs.owner = N.d_owner;
     Gr->hubs.chunks = N.chunks;
     Gr->hubs.hubs = N.hubs;
     Gr->classes = true;
@@ -1528,7 +1523,7 @@ int create_group(ipg_server* S, Graph* Gr, int kind)
             cudaMemsetAsync(G->stat_d, 0, sizeof(MpStatus), G->st);
         }
     } else {
-        if (r == IPG_OK) r = graph_classes(Gr, G->st);
+        if (r == IPG_OK) r = graph_classes(Gr);
         if (r == IPG_OK) r = galloc(G, &G->b[0], V * PP_K);
         if (r == IPG_OK) r = galloc(G, &G->b[1], V * PP_K);
         if (r == IPG_OK) r = galloc(G, &G->partial, Gr->hubs.chunks * PP_K);
@@ -1641,7 +1636,7 @@ void admit(ipg_server* S, Group* G, double now)
         if (union_find) {
             // CC queries admitted together share one union-find pass
             if (!cc_first) {
-                if (graph_classes(G->G, G->st) != IPG_OK) {
+                if (graph_classes(G->G) != IPG_OK) {
                     release_result(S, q, G->st);
                     q.state = IPG_QUERY_PENDING;
                     ++it;
@@ -1948,10 +1943,7 @@ extern "C" void ipg_server_free(ipg_server* S)
     cudaStreamSynchronize(S->rel_st);
     cudaStreamDestroy(S->rel_st);
     cudaMemPoolDestroy(S->rpool);
-    for (auto& g : S->graphs) {
-        ipg_dev_free(g->cls, g->cls_bytes);
-        ipg_hold_release(g->hold);
-    }
+    for (auto& g : S->graphs) free_classes(g.get());
     delete S;
 }
 
@@ -1969,9 +1961,8 @@ extern "C" int ipg_server_add_graph(ipg_server* S, ipg_graph* g, int* gid)
     // degree classes and hub chunks (the PPR gathers, the union-find pass and
     // the pull supersteps walk them) are built now, before queries arrive:
     // building them synchronises the device
-    if ((r = graph_classes(G.get(), nullptr)) != IPG_OK) {
-        ipg_dev_free(G->cls, G->cls_bytes);
-        ipg_hold_release(G->hold);
+    if ((r = graph_classes(G.get())) != IPG_OK) {
+        free_classes(G.get());
         return r;
     }
     *gid = (int)S->graphs.size();
