@@ -668,6 +668,7 @@ def stored_traffic(name, bytes_per_launch):
                               "algorithmic bytes"}
 
 
+# kernels of the build, and of the launch lists of builds before it
 NCU_KERNEL_NAMES = (("ipx_k_push<0>", "push_thread"), ("ipx_k_push<1>", "push_warp"), ("ipx_k_push<2>", "push_block"),
                     ("ipx_k_compute_spread", "compute"), ("ipx_k_front", "compute"), ("ipx_k_push(", "push"),
                     ("ipx_k_count(", "count_active"))
@@ -681,7 +682,8 @@ def write_traffic(csv_path, line_path, out_path=TRAFFIC_PATH):
     of `bench.py --steps 1 --warmup 1 --no-e2e --no-cpu-baseline --no-extra
     --no-parity` and the JSON line of the same command run without ncu (its
     `kernels` give the algorithmic bytes).  The profiled step runs CC, then
-    SSSP, each superstep opening with one of NCU_SUPERSTEP_OPENERS; k_compact
+    SSSP, each superstep opening with one of NCU_SUPERSTEP_OPENERS; in lists of
+    builds before the compute kernel listed the broadcasters itself, k_compact
     launches alternate broadcasters / next frontier within a superstep."""
     import csv
     line = json.loads(open(line_path).read().strip().splitlines()[-1])

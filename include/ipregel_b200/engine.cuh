@@ -97,8 +97,8 @@ static_assert(sizeof(ipx_msg) <= 8, "iPregel-B200: IP_MESSAGE_TYPE must be at mo
 /* Supersteps the host-driven loop enqueues before it waits for the device. */
 #define IPX_BATCH 8
 
-/* Default degree-class thresholds for the thread / warp / block kernels
- * (runtime tuning parameters). */
+/* Default thresholds of the rows' classes (runtime tuning parameters,
+ * ipg_app_set_tuning). */
 #ifndef IPX_T0
 #define IPX_T0 16
 #endif
@@ -623,7 +623,7 @@ struct ipx_consts {
     unsigned long long pull_threshold;
     /* broadcasters by row length, and the hubs' chunks {vertex, chunk}: rows
      * up to push_t[0] take a thread, up to push_t[1] 8 lanes, up to push_t[2]
-     * 16 lanes, longer ones a warp per push_chunk edges */
+     * 32 lanes, longer ones a warp per push_chunk edges */
     uint32_t* blist[3];
     uint2* bchunk;
     uint64_t push_t[3];
@@ -1342,9 +1342,9 @@ __global__ void __launch_bounds__(IPX_MARK_THREADS, CTAS) ipx_k_mark(uint32_t wo
 /* ------------------------------------------------------------------------ */
 /* Pull gather (ip_fetch_broadcast_messages, combiner_single_broadcast_      */
 /* postamble.h:57-89): fold ip_combine over the in-neighbours that           */
-/* broadcast.  MODE 0 folds in adjacency order, as the reference does; the   */
-/* warp and block modes fold lane-strided runs in order and then combine the */
-/* partial results in a tree.                                                */
+/* broadcast.  A thread alone on a row folds in adjacency order, as the      */
+/* reference does; several lanes fold their runs in order and then combine   */
+/* the partial results in a tree.                                            */
 /* ------------------------------------------------------------------------ */
 __device__ __forceinline__ void ipx_fold(bool& has, ipx_msg& acc, bool oh, ipx_msg om)
 {
@@ -2125,9 +2125,10 @@ __device__ __forceinline__ unsigned long long ipx_hub_chunk_done(const ipx_hub_c
 #ifndef IPX_HUB_UNROLL
 #define IPX_HUB_UNROLL 4
 #endif
-/* The hub class of ipx_k_gather_compute with ids staged in shared memory:
- * two id buffers, each filled by one bulk copy per chunk and completed on
- * its own mbarrier.  Thread 0 locates chunk k+1 and starts its copy before
+#if !IPX_HUB_WARP
+/* The hubs of ipx_k_gather_hubs with ids staged in shared memory: two id
+ * buffers, each filled by one bulk copy per chunk and completed on its own
+ * mbarrier.  Thread 0 locates chunk k+1 and starts its copy before
  * the CTA waits for chunk k's.  Each iteration thread 0 arrives once on the
  * barrier of the chunk it issues (with the copy's byte count, or alone when
  * the chunk has no whole 16-byte group), so buffer j's barrier completes its
@@ -2135,8 +2136,6 @@ __device__ __forceinline__ unsigned long long ipx_hub_chunk_done(const ipx_hub_c
  * global memory.  A wait that gives up (never expected) sets
  * IPX_ERR_COPY_TIMEOUT, and the CTA reads ids from global memory for the
  * rest of the launch; results stay exact. */
-
-#if !IPX_HUB_WARP
 template <bool HOT>
 __device__ __forceinline__ unsigned long long ipx_gather_hubs_staged(
     const uint32_t* __restrict__ adj, const uint64_t* __restrict__ row, const ipx_sbslot* bs,
@@ -2448,9 +2447,9 @@ __device__ __forceinline__ unsigned long long ipx_gather_hubs_warp(
 }
 
 /* Resident CTAs per SM the fused pull kernel is compiled for: it carries
- * ip_compute and the pipeline's registers besides the gather (64 a thread;
- * with 48 or 40 it spills: PageRank at scale 25 78.0 ms with 4 CTAs, 83.4
- * with 5, 95.0 with 6, 80 with 3). */
+ * ip_compute and the pipeline's registers besides the gather (64 a thread, with
+ * 36 bytes of spills for PageRank; many more with 48 or 40: PageRank at scale 25
+ * 78.0 ms with 4 CTAs, 83.4 with 5, 95.0 with 6, 80 with 3). */
 #ifndef IPX_GATHER_CTAS
 #define IPX_GATHER_CTAS 4
 #endif
@@ -2551,8 +2550,8 @@ __global__ void __launch_bounds__(IPX_THREADS, IPX_GATHER_CTAS) ipx_k_gather_hub
 
 #if IPX_VERSION == IPX_SPREAD_SINGLE_BROADCAST
 /* Spread + single broadcast: the targets' fetch (combiner_spread_single_
- * broadcast_postamble.h:249-309), rows by length as in the fused pull kernel,
- * those above t1 a CTA each; then the end of the superstep. */
+ * broadcast_postamble.h:249-309): a thread a target up to t0 in-edges, 16 lanes up to
+ * t1, a CTA beyond; then the end of the superstep. */
 #ifndef IPX_TARGET_CTAS
 #define IPX_TARGET_CTAS 4
 #endif

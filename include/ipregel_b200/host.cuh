@@ -92,8 +92,8 @@ struct ipx_host_state {
     bool ready = false;
     bool dirty = false;
     /* Runtime tuning, applied at the next attach: CTA size of the superstep
-     * kernels, degree-class thresholds (thread up to t0 edges, warp up to
-     * t1, CTAs beyond) and the pull switch of the push versions (pull when
+     * kernels, class thresholds (a thread for rows up to t0 edges, hubs above
+     * t1 or a chunk) and the pull switch of the push versions (pull when
      * the broadcasters' edges exceed E / pull_div; 0 never). */
     struct {
         int block = IPX_THREADS;
@@ -733,12 +733,6 @@ static int ipx_fail_device(uint32_t err)
     return ipx_fail(IPG_EDEVICE, "a kernel reported an error");
 }
 
-/* Enqueues one superstep's kernels on the engine stream.  Nothing here
- * depends on host-side values of the superstep: kernels read it (and the
- * mailbox parity) from device memory, the last one advances it, and a kernel
- * enqueued beyond the program's end returns at once, so the same sequence
- * serves the host loop and the captured loop.  first: superstep 0 may be
- * among those the sequence serves. */
 /* A kernel of a superstep; early: its CTAs come onto the SMs while the kernel
  * before it drains (programmatic dependent launch) and wait there for its end
  * (ipx_done), so the launch is not in the chain of a superstep's three to
@@ -769,6 +763,12 @@ static void ipx_start(bool early, void (*kernel)(P...), uint32_t grid, int block
     cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+/* Enqueues one superstep's kernels on the engine stream.  Nothing here
+ * depends on host-side values of the superstep: kernels read it (and the
+ * mailbox parity) from device memory, the last one advances it, and a kernel
+ * enqueued beyond the program's end returns at once, so the same sequence
+ * serves the host loop and the captured loop.  first: superstep 0 may be
+ * among those the sequence serves. */
 static int ipx_enqueue_superstep(const ipx_loop& loop, bool first)
 {
     const bool early = !loop.captured && !ipx_h.profile;
@@ -1373,8 +1373,8 @@ int ipg_app_set_profile(int on)
     return IPG_OK;
 }
 
-/* Superstep loop mode: 0 drives supersteps from the host (one
- * synchronisation each, the reference's per-superstep log), 1 runs them as a
+/* Superstep loop mode: 0 drives supersteps from the host (a synchronisation
+ * every IPX_BATCH, the reference's per-superstep log), 1 runs them as a
  * captured CUDA graph with a device-evaluated while condition (one launch per
  * ip_run).  Default from IPG_GRAPH_LOOP, else 0. */
 int ipg_app_set_graph_loop(int on)
@@ -1401,17 +1401,20 @@ int ipg_app_set_order(int on)
 int ipg_app_order(void) { return (ipx_h.ready && ipx_h.vid_of) ? 1 : 0; }
 
 /* Tuning of the superstep kernels, applied at the next attach: CTA size
- * (a multiple of 32, at most 256), degree-class thresholds t0 <= t1 (thread
- * per vertex up to t0 edges, warp up to t1, CTAs beyond) and the push
+ * (a multiple of 32, at most 256), class thresholds t0 <= t1 and the push
  * versions' pull switch (pull when the broadcasters' edges exceed
- * E / pull_div; 0 never; needs a symmetric graph or a directed one). */
+ * E / pull_div; 0 never; needs a symmetric graph or a directed one).  Rows up
+ * to t0 edges take a thread, longer ones several lanes, and hubs, whose rows are
+ * cut into chunks that warps share, begin above t1 -- or above a chunk, which
+ * is 256 edges on a small graph and grows with it to 2,048 (push, marking, pull
+ * delivery; from there on t1 alone counts) or 8,192 (single_broadcast), if t1
+ * is larger.  The targets of spread+single_broadcast take a CTA above t1. */
 int ipg_app_set_tuning(int block, uint64_t t0, uint64_t t1, uint64_t pull_div)
 {
     if (block < 32 || block > IPX_THREADS || (block & 31))
         return ipx_fail(IPG_EINVAL, "ipg_app_set_tuning: block must be a multiple of 32 in [32, 256]");
     if (t0 < 1 || t1 < t0) return ipx_fail(IPG_EINVAL, "ipg_app_set_tuning: need 1 <= t0 <= t1");
-    /* a warp of the pull gather sums the degrees of 32 vertices of the
-     * middle class in 32 bits */
+    /* rows that are no hubs are walked with 32-bit positions */
     if (t1 > (1ULL << 26)) return ipx_fail(IPG_EINVAL, "ipg_app_set_tuning: t1 above 2^26");
     ipx_h.tune.block = block;
     ipx_h.tune.t0 = t0;

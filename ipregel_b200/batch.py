@@ -27,9 +27,9 @@ import numpy as np
 
 from . import DeviceArray, Engine, Fused, Graph
 
-#: Candidate settings of the autotuner: CTA size, (t0, t1) degree-class
-#: thresholds (thread per vertex up to t0 edges, warp up to t1, CTAs beyond)
-#: and the pull switch (pull when the broadcasters' edges exceed E / pull_div;
+#: Candidate settings of the autotuner: CTA size, (t0, t1) class thresholds
+#: (rows up to t0 edges take a thread, hubs begin above t1 or, on graphs too
+#: small for it, above a chunk: ipg_app_set_tuning) and the pull switch (pull when the broadcasters' edges exceed E / pull_div;
 #: 0 never pulls).
 BLOCKS = (128, 256)
 THRESHOLDS = ((8, 1024), (16, 4096), (32, 4096))

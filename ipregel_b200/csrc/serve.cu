@@ -14,7 +14,8 @@
 //     are one coalesced line), a bit-packed frontier mask per vertex (u64, a
 //     bit per lane) double-buffered, and the frontier as degree-class lists.
 //     A vertex with few frontier lanes has a thread per edge relax all its
-//     lanes; one with many has a thread per lane relax each edge in turn.
+//     lanes; one with many has a warp walk its row, a thread per quad of lanes
+//     in use and edge.  Rows of more than 256 edges go in chunks.
 //     nd = dist[v][k] + w (w = 0 for a CC lane) goes into dist[u][k] by
 //     atomicMin, and the improved lanes into u's next mask.  A lane whose
 //     frontier empties is finished.
@@ -23,9 +24,9 @@
 //     component); CC queries admitted together share the pass.
 //   PPR group: 32 lanes; the broadcast quotients b[v][lane] = x/deg (FP32,
 //     128 bytes per vertex, one line) double-buffered; a pull gather over
-//     every row: 8 threads per low-degree vertex, each reading one float4
-//     quad of every in-neighbour's row, a warp per vertex of higher degree
-//     (four rows per load instruction), hub rows in chunks.  64 lanes (two
+//     every row: a thread per quad of lanes in use (1, 2, 4 or 8) and low-degree
+//     vertex, each reading one float4 of every in-neighbour's row, four such
+//     groups per vertex of higher degree, hub rows in chunks.  64 lanes (two
 //     lines per row) measured slower in the mixed serving workload: a
 //     superstep cost about twice as much, for half the supersteps.  A lane runs exactly
 //     `rounds` gathers after admission and writes its last values into the
@@ -90,10 +91,11 @@ constexpr int MP_SPARSE = 4;
 // A min-plus superstep pulls (symmetric graphs) when its frontier holds at
 // least E / MP_PULL_DIV edges and at least MP_PULL_LANES lanes are busy.  A
 // pull reads a neighbour's whole 256-byte row, a push the quads of its lanes
-// in use, so a pull pays only where most are: dense supersteps pulled against
-// pushed took, for all queries, 13.0 / 8.1 ms with 32 lanes, 13.6 / 13.5 with
-// 40 and 15.3 / 15.4 with 64 at R-MAT scale 20, 5.5 / 5.8 with 40 and 6.2 /
-// 6.7 with 64 at scale 18, 50 / 47 and 53.6 / 53.6 at scale 22.
+// in use.  Dense supersteps pulled against pushed took, for all queries, 13.0 /
+// 8.1 ms with 32 lanes, 13.6 / 13.5 with 40 and 15.3 / 15.4 with 64 at R-MAT
+// scale 20, 5.5 / 5.8 with 40 and 6.2 / 6.7 with 64 at scale 18, 50 / 47 and
+// 53.6 / 53.6 at scale 22: from 40 lanes on the two are about even, a gain on the
+// smaller graph and a loss on the larger, and below that pushing wins.
 constexpr uint64_t MP_PULL_DIV = 4;
 constexpr int MP_PULL_LANES = 40;
 // Resident CTAs per SM the min-plus kernels are compiled for (64 registers).
