@@ -2341,13 +2341,12 @@ __device__ __forceinline__ unsigned long long ipx_gather_rows(const uint32_t* li
     if (!ipx_c.in_quads) {
         for (; i < n; i += step) {
             const uint64_t v = list[i];
-            const uint64_t e0 = row[v], e1 = row[v + 1];
-            if (SKIP && e1 - e0 > ipx_c.hub_min) continue;
+            if (SKIP && row[v + 1] - row[v] > ipx_c.hub_min) continue;
             ipx_vertex_state x;
             ipx_gather_ahead(v, gl == 0, x);
             bool has = false;
             ipx_msg acc;
-            ipx_gather_fold_edges<HOT>(ids, bs, stamp, e0, e1, gl, G, has, acc);
+            ipx_gather_fold_edges<HOT>(ids, bs, stamp, row[v], row[v + 1], gl, G, has, acc);
             if (G > 1) ipx_group_fold<G>(has, acc, mask);
             if (gl == 0) cnt += ipx_gather_done(v, has, acc, x, out, stamp);
         }
